@@ -135,6 +135,10 @@ int tq_vcode_native_offset(const tq_config* cfg, int32_t token, int32_t canonica
 int tq_decode_workspace_bytes(const tq_config* cfg, int32_t batch, int32_t num_q_heads,
                               int32_t num_kv_heads, int32_t max_splits, size_t* out);
 
+/* Sequence splits per (sequence, kv head) that suit a launch of this shape on a
+ * GPU with `sms` multiprocessors (0: the current device). */
+int32_t tq_decode_splits(int32_t batch, int32_t num_kv_heads, int32_t max_seq_len, int32_t max_ring_len, int32_t sms);
+
 /* Scratch bytes tq_scores needs for n_vectors query vectors. */
 int tq_scores_workspace_bytes(const tq_config* cfg, int64_t n_vectors, size_t* out);
 
@@ -252,13 +256,29 @@ typedef struct tq_decode_args {
     const void* append_k;
     const void* append_v;
     int32_t ring_capacity;
+    int32_t flags;              /* TQ_DECODE_*, 0 = none */
 } tq_decode_args;
+
+/* The lengths are the host's: every sequence holds max_seq_len compressed and max_ring_len exact
+ * tokens (with append_k: the new one is the last of them), seq_lens / ring_lens may be NULL and are
+ * neither read nor written.  For callers that count on the host anyway. */
+#define TQ_DECODE_HOST_LENS 1
+/* Every sequence uses the first row of block_table (several query tokens over one sequence). */
+#define TQ_DECODE_SHARED_TABLE 2
 
 /* One decode-attention step over compressed history plus the exact ring:
  * softmax over [history || ring] jointly, no K/V materialised.  Replaces
  * compute_hybrid_attention (score.py:29-173) and the fused Triton decode
  * (triton_kernels.py:209-356,505-607). */
 int tq_decode(const tq_consts* consts, const tq_pool* pool, const tq_decode_args* args, void* stream);
+
+/* Append `n_tokens` exact tokens to a ring of contiguous (capacity, n_heads, head_dim) key and value
+ * buffers at row `position` (both tensors in one launch).  Replaces the slice assignments of
+ * RingBuffer.write (capture.py:75-112).  Element (t, h, :) of key / value is at base + t*stride_token +
+ * h*stride_head (in elements); rows must be 16-byte aligned. */
+int tq_ring_write(const void* key, const void* value, tq_dtype dtype, int64_t n_tokens, int32_t n_heads, int32_t head_dim,
+                  int64_t stride_token, int64_t stride_head, void* ring_k, void* ring_v, int64_t ring_stride_token,
+                  int64_t position, void* stream);
 
 /* tq_decode for a caller whose step inputs and result live in HOST memory (pinned for the
  * copies to be asynchronous): on `stream`, copies `in_bytes` from `host_in` to the device

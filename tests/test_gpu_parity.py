@@ -1212,3 +1212,24 @@ def test_store_that_reads_the_ring_right_after_a_fused_append(dev):
             assert torch.equal(a.data, b.data)
             assert torch.equal(ring_k[:step + 1].cpu(), k[n:n + step + 1])
     assert E.store_status() == 0 and ws.status() == 0
+
+
+@pytest.mark.parametrize("dtype,n,pos,strided", [(torch.bfloat16, 1, 0, False), (torch.bfloat16, 1, 15, False), (torch.float16, 7, 9, True),
+                                                 (torch.float32, 16, 0, False), (torch.bfloat16, 3, 5, True)])
+def test_ring_write_in_one_launch(dtype, n, pos, strided, dev):
+    """Exact tokens into the ring by the library's kernel (first / last row, a whole ring, rows that are
+    slices of a wider tensor) against slice assignment; nothing else in the ring changes."""
+    from turboquant_b200.capture import RingBuffer
+    h, d, cap = 3, 128, 16
+    g = torch.Generator().manual_seed(n * 31 + pos)
+    ring = RingBuffer(cap, h, d, dev, dtype)
+    before = torch.randn(pos, h, d, generator=g).to(dtype).to(dev)
+    if pos:
+        ring.write(before, before + 1, pos)
+    src = torch.randn(2, n, 2 * h, d, generator=g).to(dtype).to(dev)
+    k, v = (src[0, :, :h], src[1, :, :h]) if strided else (src[0, :, :h].contiguous(), src[1, :, :h].contiguous())
+    assert ring.write(k, v, n) is None and ring.size == pos + n
+    rk, rv = ring.storage
+    assert torch.equal(rk[pos:pos + n], k) and torch.equal(rv[pos:pos + n], v)
+    assert torch.equal(rk[:pos], before) and torch.equal(rv[:pos], before + 1)
+    assert float(rk[pos + n:].abs().max() if pos + n < cap else 0) == 0

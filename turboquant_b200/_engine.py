@@ -14,7 +14,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._lib import TQ_BF16, TQ_BLOCK_TOKENS, TQ_F16, TQ_F32, check, lib
+from ._lib import TQ_BF16, TQ_BLOCK_TOKENS, TQ_F16, TQ_F32, check, host, lib
 from .codebook import get_codebook_tensors
 from .rotation import generate_qjl_matrix, generate_rotation_matrix
 
@@ -111,6 +111,7 @@ class LayerConstants:
             c.m_limbs[i] = self.m_limbs[i].data_ptr() if tensor_core_store else None
             c.s_limbs[i] = self.s_limbs[i].data_ptr() if tensor_core_store else None
         self.c = c
+        self.addr = C.addressof(c)     # what the native host path passes on
 
     @property
     def block_bytes(self) -> int:
@@ -130,6 +131,7 @@ class BlockPool:
         self.num_blocks = 0
         self.data = torch.empty(0, dtype=torch.uint8, device=consts.device)
         self.c = _lib.tq_pool()
+        self.addr = C.addressof(self.c)     # stays valid: the structure is updated in place
         self.resize(max(1, num_blocks))
 
     def resize(self, num_blocks: int) -> None:
@@ -141,7 +143,7 @@ class BlockPool:
         if self.num_blocks:
             new[: self.num_blocks * per_block].copy_(self.data)
         self.data, self.num_blocks = new, num_blocks
-        self.c = _lib.tq_pool(self.data.data_ptr(), num_blocks, self.num_kv_heads)
+        self.c.base, self.c.num_blocks, self.c.num_kv_heads = self.data.data_ptr(), num_blocks, self.num_kv_heads
 
     def nbytes(self) -> int:
         return self.data.numel()
@@ -161,6 +163,7 @@ class BlockPool:
         pool.consts, pool.num_kv_heads, pool.num_blocks = consts, num_kv_heads, n
         pool.data = raw.view(-1)[: n * per_block]
         pool.c = _lib.tq_pool(pool.data.data_ptr(), n, num_kv_heads)
+        pool.addr = C.addressof(pool.c)
         pool.resize = pool._fixed
         return pool
 
@@ -230,17 +233,8 @@ def sm_count(device) -> int:
 
 
 def choose_splits(batch: int, num_kv_heads: int, max_seq_len: int, sms: int, max_ring_len: int = 0) -> int:
-    """Sequence splits per (sequence, kv head).  The decode kernel runs one
-    12-warp CTA per SM when the launch fits one wave: with few (sequence, head)
-    pairs the sequence is cut so that every SM gets one CTA, the ring tokens
-    taking CTAs of their own (64 tokens each when the launch fits one wave -
-    the library applies the same rule); with many pairs a CTA takes at most
-    512 records (8192 tokens) so that long and short sequences balance out."""
-    nblk = (max_seq_len + TQ_BLOCK_TOKENS - 1) // TQ_BLOCK_TOKENS
-    pairs = max(1, batch * num_kv_heads)
-    ring_ctas = (max_ring_len + 63) // 64
-    want = max(sms // pairs - ring_ctas, -(-nblk // 512), 1)
-    return max(1, min(want, max(1, nblk // 12)))
+    """Sequence splits per (sequence, kv head) that suit a launch of this shape on `sms` multiprocessors."""
+    return lib().tq_decode_splits(batch, num_kv_heads, max_seq_len, max_ring_len, sms)
 
 
 def store(consts: LayerConstants, pool: BlockPool, key: torch.Tensor, value: torch.Tensor, *,

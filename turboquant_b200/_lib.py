@@ -9,7 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from .build import LIB_PATH
+from .build import HOST_PATH, LIB_PATH
 
 TQ_BLOCK_TOKENS = 16
 TQ_MAX_CENTROIDS = 16
@@ -59,7 +59,7 @@ class tq_decode_args(C.Structure):
                 ("max_ring_len", C.c_int32), ("ring_stride_seq", C.c_int64), ("ring_stride_token", C.c_int64),
                 ("scale", C.c_float), ("out", C.c_void_p), ("workspace", C.c_void_p),
                 ("workspace_bytes", C.c_size_t), ("num_splits", C.c_int32), ("query_prepared", C.c_int32), ("kernel", C.c_int32), ("append_k", C.c_void_p), ("append_v", C.c_void_p),
-                ("ring_capacity", C.c_int32)]
+                ("ring_capacity", C.c_int32), ("flags", C.c_int32)]
 
 
 # name -> (restype, argtypes); every symbol include/turboquant_b200.h declares
@@ -68,6 +68,9 @@ SIGNATURES = {
     "tq_vcode_native_offset": (C.c_int, [C.POINTER(tq_config), C.c_int32, C.c_int32]),
     "tq_decode_workspace_bytes": (C.c_int, [C.POINTER(tq_config), C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                             C.POINTER(C.c_size_t)]),
+    "tq_decode_splits": (C.c_int32, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32]),
+    "tq_ring_write": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int32, C.c_int64, C.c_int64,
+                                C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]),
     "tq_scores_workspace_bytes": (C.c_int, [C.POINTER(tq_config), C.c_int64, C.POINTER(C.c_size_t)]),
     "tq_strerror": (C.c_char_p, [C.c_int]),
     "tq_version": (C.c_char_p, []),
@@ -124,6 +127,21 @@ def lib() -> C.CDLL:
             fn.argtypes = argtypes
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path of the decode-step calls (csrc/host/tq_host.cpp); raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m turboquant_b200.build`")
+        from . import _host as module
+        _host = module
+    return _host
 
 
 def strerror(status: int) -> str:

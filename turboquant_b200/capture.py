@@ -80,8 +80,12 @@ class RingBuffer:
         evicted_buffers = (total - 1) // cap               # full buffers with a successor
         cut = evicted_buffers * cap - held                 # new tokens that leave with them
         if evicted_buffers == 0:
-            self._keys[held:total] = key[:num_tokens]
-            self._values[held:total] = value[:num_tokens]
+            rc = E.host().ring_write(self._keys, self._values, key, value, held, num_tokens) if self._keys.is_cuda else None
+            if rc is None:
+                self._keys[held:total] = key[:num_tokens]
+                self._values[held:total] = value[:num_tokens]
+            else:
+                E.check(rc, "tq_ring_write")
             self._fill = total
             return None
         out_k = torch.cat((self._keys[:held], key[:cut]), 0)
@@ -99,6 +103,10 @@ class RingBuffer:
         taken = self._keys[: self._fill].clone(), self._values[: self._fill].clone()
         self._fill = 0
         return taken
+
+    def clear(self) -> None:
+        """Forget what is held (the caller has taken it through `peek`)."""
+        self._fill = 0
 
     def peek(self):
         """Views of what is held (None when empty)."""
@@ -164,7 +172,10 @@ class KVCaptureEngine:
         self._prefill_done = True
 
     def ingest_decode(self, key: torch.Tensor, value: torch.Tensor, num_tokens: int) -> None:
-        overflow = self.ring.write(key[:num_tokens], value[:num_tokens], num_tokens)
+        ring = self.ring
+        if ring.is_full and num_tokens == 1:
+            self._compress_ring()              # the same eviction, without copying the ring out first
+        overflow = ring.write(key, value, num_tokens)
         if overflow is not None:
             self.store.append_chunk(*overflow)
 
@@ -181,7 +192,17 @@ class KVCaptureEngine:
         """
         ring, store = self.ring, self.store
         if ring.is_full:                      # the rare step: compress the full ring first
-            self.store.append_chunk(*ring.drain())
+            self._compress_ring()
+        if num_query_heads == query.shape[-2]:
+            res = E.host().step(store.consts.addr, store.pool.addr, store.workspace, store.block_table, store.head_dim,
+                                store._num_tokens, query, key, value, num_query_heads, ring._keys, ring._values,
+                                ring._fill, scale, 16, out)
+            if res is not None:
+                if type(res) is int:
+                    E.check(res, "tq_decode")
+                ring._fill += 1
+                ring._seen += 1
+                return res
         E.require_cuda(query, "query")
         if key.dtype != ring.dtype or value.dtype != ring.dtype:
             raise TypeError(f"key/value must be {ring.dtype} like the ring")
@@ -209,7 +230,7 @@ class KVCaptureEngine:
         """
         ring, store = self.ring, self.store
         if ring.is_full:
-            self.store.append_chunk(*ring.drain())
+            self._compress_ring()
         h, d, qh = store.num_kv_heads, store.head_dim, num_query_heads
         nk, nq = h * d, qh * d
         io = self._host_io
@@ -257,10 +278,16 @@ class KVCaptureEngine:
             E.check(rc, "tq_decode_host_io")
         ring.advance_after_device_append()
 
+    def _compress_ring(self) -> None:
+        """The whole ring into the store, straight out of the ring's buffers: stream order keeps them
+        unchanged until the store has read them, so no copy is needed in between."""
+        held = self.ring.peek()
+        if held is not None:
+            self.store.append_chunk(*held)
+            self.ring.clear()
+
     def flush(self) -> None:
-        data = self.ring.drain()
-        if data is not None:
-            self.store.append_chunk(*data)
+        self._compress_ring()
 
     def reset(self) -> None:
         self.ring.reset()

@@ -1,0 +1,318 @@
+// Host side of the calls a decode step makes, as a CPython extension.
+//
+// A decode step is two or three kernel launches of a few microseconds each; the same step driven through
+// torch slicing, ctypes argument structures and per-step length tensors costs 20-80 us of Python.  The
+// functions here take the tensors as they are, check what the Python wrappers checked, fill the C argument
+// block and launch: about 1 us of their own per call.
+//
+// Every function is a fast path: what it does not take (another device, another layout, a shape the
+// wrappers refuse with a message) it answers with None / NotImplemented-like results BEFORE anything is
+// launched, and the Python wrapper goes its general way.  Status codes of the library come back as ints.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cmath>
+
+#include "turboquant_b200.h"
+
+namespace {
+
+// ------------------------------------------------------------------ argument helpers
+
+inline const at::Tensor* tensor_or_null(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+template <class T>
+inline T* address(PyObject* o) { return reinterpret_cast<T*>(PyLong_AsUnsignedLongLong(o)); }
+inline int dtype_code(at::ScalarType t) {
+    return t == at::kBFloat16 ? TQ_BF16 : t == at::kHalf ? TQ_F16 : t == at::kFloat ? TQ_F32 : -1;
+}
+inline void* stream_of(const at::Tensor& t) {
+    return reinterpret_cast<void*>(c10::cuda::getCurrentCUDAStream(t.get_device()).stream());
+}
+// (n, heads, dim) rows the kernels can read in place: CUDA, `dim` contiguous
+inline bool rows_ok(const at::Tensor& t, int64_t heads, int64_t dim) {
+    return t.is_cuda() && t.dim() == 3 && t.size(1) == heads && t.size(2) == dim && t.stride(2) == 1;
+}
+// The first n rows of t as a contiguous (n, width) block, whatever its shape (rows, heads, dim) or (rows, width)
+inline bool block_ok(const at::Tensor& t, int64_t n, int64_t heads, int64_t dim) {
+    return t.is_cuda() && t.is_contiguous() && (t.dim() == 3 ? t.size(1) == heads && t.size(2) == dim : t.dim() == 2 && t.size(1) == heads * dim) &&
+           t.size(0) >= n;
+}
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Workspace (a Python object with .buf and .ensure(nbytes)): pointer and size once it holds `need` bytes.
+bool workspace(PyObject* ws, size_t need, void** ptr, size_t* bytes) {
+    static PyObject* name = PyUnicode_InternFromString("buf");
+    for (int pass = 0; pass < 2; ++pass) {
+        PyObject* buf = PyObject_GetAttr(ws, name);
+        if (buf == nullptr) return false;
+        const at::Tensor* t = tensor_or_null(buf);
+        const bool fits = t != nullptr && (size_t)t->numel() >= need;
+        if (fits) {
+            *ptr = t->data_ptr();
+            *bytes = (size_t)t->numel();
+        }
+        Py_DECREF(buf);   // the workspace object keeps it
+        if (fits) return true;
+        PyObject* r = PyObject_CallMethod(ws, "ensure", "n", (Py_ssize_t)need);
+        if (r == nullptr) return false;
+        Py_DECREF(r);
+    }
+    PyErr_SetString(PyExc_RuntimeError, "the workspace did not grow");
+    return false;
+}
+
+// Fills what every decode call shares; false with a Python error set when the workspace cannot be had.
+// *rc is the library's answer to the planning calls.
+bool plan(tq_decode_args& a, const tq_consts* c, const tq_pool* pool, PyObject* ws, int batch, int q_heads, int max_seq,
+          int max_ring, int* rc) {
+    size_t need = 0;
+    a.batch = batch;
+    a.num_q_heads = q_heads;
+    a.max_seq_len = max_seq;
+    a.num_splits = tq_decode_splits(batch, pool->num_kv_heads, max_seq, max_ring, 0);
+    *rc = tq_decode_workspace_bytes(&c->cfg, batch, q_heads, pool->num_kv_heads, a.num_splits, &need);
+    if (*rc != TQ_OK) return true;
+    return workspace(ws, need, &a.workspace, &a.workspace_bytes);
+}
+
+#define ARGS(n)                                                                              \
+    if (nargs != (n)) {                                                                      \
+        PyErr_Format(PyExc_TypeError, "%s takes %d arguments, got %zd", __func__, n, nargs); \
+        return nullptr;                                                                      \
+    }
+
+// ------------------------------------------------------------------ ring
+
+// ring_write(ring_k, ring_v, key, value, position, n) -> status, or None: not a case for the kernel
+PyObject* ring_write(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(6);
+    const at::Tensor *rk = tensor_or_null(args[0]), *rv = tensor_or_null(args[1]), *k = tensor_or_null(args[2]),
+                     *v = tensor_or_null(args[3]);
+    const int64_t pos = PyLong_AsLongLong(args[4]), n = PyLong_AsLongLong(args[5]);
+    if (!rk || !rv || !k || !v || !rk->is_cuda() || n < 1 || pos < 0 || rk->dim() != 3 || pos + n > rk->size(0)) Py_RETURN_NONE;
+    const int64_t h = rk->size(1), d = rk->size(2);
+    if (!rows_ok(*k, h, d) || !rows_ok(*v, h, d) || k->size(0) < n || v->size(0) < n || k->scalar_type() != rk->scalar_type() ||
+        v->scalar_type() != rk->scalar_type() || k->get_device() != rk->get_device() || v->get_device() != rk->get_device() ||
+        k->stride(0) != v->stride(0) || k->stride(1) != v->stride(1) || !rk->is_contiguous() || !rv->is_contiguous())
+        Py_RETURN_NONE;
+    const int dt = dtype_code(rk->scalar_type());
+    if (dt < 0) Py_RETURN_NONE;
+    const int rc = tq_ring_write(k->data_ptr(), v->data_ptr(), (tq_dtype)dt, n, (int32_t)h, (int32_t)d, k->stride(0), k->stride(1),
+                                 rk->data_ptr(), rv->data_ptr(), h * d, pos, stream_of(*rk));
+    if (rc == TQ_ERR_ALIGN || rc == TQ_ERR_UNSUPPORTED) Py_RETURN_NONE;
+    return PyLong_FromLong(rc);
+    END_HANDLE_TH_ERRORS
+}
+
+// ------------------------------------------------------------------ store
+
+// store(consts, pool, key, value, head_dim, block_table | None, slots | None, start_pos, n) -> status or None
+PyObject* store(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(9);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const tq_pool* pool = address<const tq_pool>(args[1]);
+    const at::Tensor *k = tensor_or_null(args[2]), *v = tensor_or_null(args[3]);
+    const int64_t d = PyLong_AsLongLong(args[4]), start = PyLong_AsLongLong(args[7]), n = PyLong_AsLongLong(args[8]);
+    const at::Tensor *bt = tensor_or_null(args[5]), *slots = tensor_or_null(args[6]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!k || !v || n < 1 || !rows_ok(*k, pool->num_kv_heads, d) || !rows_ok(*v, pool->num_kv_heads, d) || k->size(0) != n ||
+        v->size(0) != n || k->stride(0) != v->stride(0) || k->stride(1) != v->stride(1) || k->scalar_type() != v->scalar_type() ||
+        k->get_device() != v->get_device())
+        Py_RETURN_NONE;
+    if (slots && (slots->scalar_type() != at::kLong || slots->numel() < n || !slots->is_contiguous() || !slots->is_cuda())) Py_RETURN_NONE;
+    const int dt = dtype_code(k->scalar_type());
+    if (dt < 0 || (!bt && !slots)) Py_RETURN_NONE;
+    return PyLong_FromLong(tq_store(c, k->data_ptr(), v->data_ptr(), (tq_dtype)dt, n, pool->num_kv_heads, k->stride(0), k->stride(1),
+                                    slots ? slots->data_ptr<int64_t>() : nullptr, bt ? bt->data_ptr<int32_t>() : nullptr, start,
+                                    pool, stream_of(*k)));
+    END_HANDLE_TH_ERRORS
+}
+
+// ------------------------------------------------------------------ decode
+
+// hybrid(consts, pool, workspace, block_table, head_dim, n_history, query, n_queries, q_heads, recent_k | None,
+//        recent_v | None, scale | None, min_history, out | None) -> out tensor, status int on failure, or None
+// One sequence: every query attends to the whole history and all recent tokens.  `query` may be
+// (n, q_heads, head_dim) or (n, q_heads * head_dim); with `out` (same dtype, contiguous, at least as long) the
+// result is written there.
+PyObject* hybrid(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(14);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const tq_pool* pool = address<const tq_pool>(args[1]);
+    const at::Tensor* bt = tensor_or_null(args[3]);
+    const int64_t d = PyLong_AsLongLong(args[4]), n = PyLong_AsLongLong(args[5]), t = PyLong_AsLongLong(args[7]),
+                  qh = PyLong_AsLongLong(args[8]), min_history = PyLong_AsLongLong(args[12]);
+    const at::Tensor *q = tensor_or_null(args[6]), *rk = tensor_or_null(args[9]), *rv = tensor_or_null(args[10]),
+                     *out = tensor_or_null(args[13]);
+    const double scale = args[11] == Py_None ? 1.0 / std::sqrt((double)d) : PyFloat_AsDouble(args[11]);
+    if (PyErr_Occurred()) return nullptr;
+    const int64_t h = pool->num_kv_heads;
+    if (!bt || !q || t < 1 || qh < 1 || qh % h != 0 || !block_ok(*q, t, qh, d) || q->get_device() != bt->get_device()) Py_RETURN_NONE;
+    const int dt = dtype_code(q->scalar_type());
+    if (dt < 0 || (out && (!block_ok(*out, t, qh, d) || out->scalar_type() != q->scalar_type() || !aligned16(out->data_ptr()))))
+        Py_RETURN_NONE;
+    tq_decode_args a = {};
+    const int64_t r = rk ? rk->size(0) : 0;
+    if (n < min_history && r == 0) Py_RETURN_NONE;
+    if (r > 0) {
+        if (!rv || !rows_ok(*rk, h, d) || !rows_ok(*rv, h, d) || rk->stride(1) != d || rv->stride(1) != d ||
+            rk->stride(0) != rv->stride(0) || rv->size(0) != r || rk->scalar_type() != rv->scalar_type() || r > 256)
+            Py_RETURN_NONE;
+        const int rdt = dtype_code(rk->scalar_type());
+        if (rdt < 0) Py_RETURN_NONE;
+        a.ring_k = rk->data_ptr();
+        a.ring_v = rv->data_ptr();
+        a.ring_dtype = (tq_dtype)rdt;
+        a.max_ring_len = (int32_t)r;
+        a.ring_stride_token = rk->stride(0);
+    }
+    int rc = TQ_OK;
+    if (!plan(a, c, pool, args[2], (int)t, (int)qh, (int)n, (int)r, &rc)) return nullptr;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    a.query = q->data_ptr();
+    a.q_dtype = (tq_dtype)dt;
+    a.block_table = bt->data_ptr<int32_t>();
+    a.block_table_stride = (int32_t)bt->numel();
+    a.min_history = (int32_t)min_history;
+    a.scale = (float)scale;
+    a.flags = TQ_DECODE_HOST_LENS | TQ_DECODE_SHARED_TABLE;
+    at::Tensor res;
+    if (!out) {
+        res = at::empty({t, qh, d}, q->options());
+        out = &res;
+    }
+    a.out = out->data_ptr();
+    rc = tq_decode(c, pool, &a, stream_of(*q));
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    if (!res.defined()) {
+        Py_INCREF(args[13]);
+        return args[13];
+    }
+    return THPVariable_Wrap(std::move(res));
+    END_HANDLE_TH_ERRORS
+}
+
+// step(consts, pool, workspace, block_table, head_dim, n_history, query, key, value, q_heads, ring_k, ring_v, ring_fill,
+//      scale | None, min_history, out | None) -> out tensor, status int, or None
+// One new token of one sequence: appended to the ring by the launch that prepares the query, then attended.
+PyObject* step(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(16);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const tq_pool* pool = address<const tq_pool>(args[1]);
+    const at::Tensor* bt = tensor_or_null(args[3]);
+    const int64_t d = PyLong_AsLongLong(args[4]), n = PyLong_AsLongLong(args[5]), qh = PyLong_AsLongLong(args[9]),
+                  fill = PyLong_AsLongLong(args[12]), min_history = PyLong_AsLongLong(args[14]);
+    const at::Tensor *q = tensor_or_null(args[6]), *k = tensor_or_null(args[7]), *v = tensor_or_null(args[8]),
+                     *rk = tensor_or_null(args[10]), *rv = tensor_or_null(args[11]), *out = tensor_or_null(args[15]);
+    const double scale = args[13] == Py_None ? 1.0 / std::sqrt((double)d) : PyFloat_AsDouble(args[13]);
+    if (PyErr_Occurred()) return nullptr;
+    const int64_t h = pool->num_kv_heads;
+    if (!bt || !q || !k || !v || !rk || !rv || qh < 1 || qh % h != 0 || q->dim() != 3 || q->size(0) != 1 || q->size(1) != qh ||
+        q->size(2) != d || !q->is_cuda() || !q->is_contiguous() || k->numel() != h * d || v->numel() != h * d || !k->is_contiguous() ||
+        !v->is_contiguous() || k->size(0) != 1 || v->size(0) != 1 || !k->is_cuda() || !v->is_cuda() ||
+        k->scalar_type() != rk->scalar_type() || v->scalar_type() != rk->scalar_type() ||
+        q->get_device() != bt->get_device() || fill < 0 || fill >= rk->size(0) || fill >= 256 || !rk->is_contiguous() || !rv->is_contiguous())
+        Py_RETURN_NONE;
+    const int dt = dtype_code(q->scalar_type()), rdt = dtype_code(rk->scalar_type());
+    if (dt < 0 || rdt < 0 || !aligned16(k->data_ptr()) || !aligned16(v->data_ptr())) Py_RETURN_NONE;
+    if (out && (!block_ok(*out, 1, qh, d) || out->scalar_type() != q->scalar_type() || !aligned16(out->data_ptr()))) Py_RETURN_NONE;
+    tq_decode_args a = {};
+    int rc = TQ_OK;
+    if (!plan(a, c, pool, args[2], 1, (int)qh, (int)n, (int)fill + 1, &rc)) return nullptr;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    a.query = q->data_ptr();
+    a.q_dtype = (tq_dtype)dt;
+    a.block_table = bt->data_ptr<int32_t>();
+    a.block_table_stride = (int32_t)bt->numel();
+    a.min_history = (int32_t)min_history;
+    a.ring_k = rk->data_ptr();
+    a.ring_v = rv->data_ptr();
+    a.ring_dtype = (tq_dtype)rdt;
+    a.max_ring_len = (int32_t)fill + 1;
+    a.ring_stride_token = h * d;
+    a.append_k = k->data_ptr();
+    a.append_v = v->data_ptr();
+    a.ring_capacity = (int32_t)rk->size(0);
+    a.scale = (float)scale;
+    a.flags = TQ_DECODE_HOST_LENS;
+    at::Tensor res;
+    if (!out) {
+        res = at::empty({1, qh, d}, q->options());
+        out = &res;
+    }
+    a.out = out->data_ptr();
+    rc = tq_decode(c, pool, &a, stream_of(*q));
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    if (!res.defined()) {
+        Py_INCREF(args[15]);
+        return args[15];
+    }
+    return THPVariable_Wrap(std::move(res));
+    END_HANDLE_TH_ERRORS
+}
+
+// batch(consts, pool, workspace, head_dim, query, block_tables, seq_lens, max_seq_len, scale | None, min_history, out | None)
+// -> out tensor, status int, or None.  One decode token per sequence of a paged batch, no exact tokens.
+PyObject* batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(11);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const tq_pool* pool = address<const tq_pool>(args[1]);
+    const int64_t d = PyLong_AsLongLong(args[3]), max_seq = PyLong_AsLongLong(args[7]), min_history = PyLong_AsLongLong(args[9]);
+    const at::Tensor *q = tensor_or_null(args[4]), *bt = tensor_or_null(args[5]), *lens = tensor_or_null(args[6]),
+                     *out = tensor_or_null(args[10]);
+    const double scale = args[8] == Py_None ? 1.0 / std::sqrt((double)d) : PyFloat_AsDouble(args[8]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!q || !bt || !lens || q->dim() != 3 || q->size(0) < 1 || q->size(2) != d || !q->is_cuda() || !q->is_contiguous() ||
+        bt->dim() != 2 || bt->scalar_type() != at::kInt || bt->stride(1) != 1 || !bt->is_cuda() || lens->scalar_type() != at::kInt ||
+        !lens->is_contiguous() || !lens->is_cuda() || bt->size(0) < q->size(0) || lens->numel() < q->size(0))
+        Py_RETURN_NONE;
+    const int64_t b = q->size(0), qh = q->size(1);
+    const int dt = dtype_code(q->scalar_type());
+    if (dt < 0 || (out && (!out->is_contiguous() || out->sizes() != q->sizes() || out->scalar_type() != q->scalar_type()))) Py_RETURN_NONE;
+    tq_decode_args a = {};
+    int rc = TQ_OK;
+    if (!plan(a, c, pool, args[2], (int)b, (int)qh, (int)max_seq, 0, &rc)) return nullptr;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    a.query = q->data_ptr();
+    a.q_dtype = (tq_dtype)dt;
+    a.block_table = bt->data_ptr<int32_t>();
+    a.block_table_stride = (int32_t)bt->stride(0);
+    a.seq_lens = lens->data_ptr<int32_t>();
+    a.min_history = (int32_t)min_history;
+    a.scale = (float)scale;
+    at::Tensor res;
+    if (!out) {
+        res = at::empty_like(*q);
+        out = &res;
+    }
+    a.out = out->data_ptr();
+    rc = tq_decode(c, pool, &a, stream_of(*q));
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    if (!res.defined()) {
+        Py_INCREF(args[10]);
+        return args[10];
+    }
+    return THPVariable_Wrap(std::move(res));
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {
+    {"ring_write", (PyCFunction)(void (*)(void))ring_write, METH_FASTCALL, nullptr},
+    {"store", (PyCFunction)(void (*)(void))store, METH_FASTCALL, nullptr},
+    {"hybrid", (PyCFunction)(void (*)(void))hybrid, METH_FASTCALL, nullptr},
+    {"step", (PyCFunction)(void (*)(void))step, METH_FASTCALL, nullptr},
+    {"batch", (PyCFunction)(void (*)(void))batch, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Host side of the decode-step calls", -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host(void) { return PyModule_Create(&module); }

@@ -36,6 +36,7 @@ struct RingAppend {
     int32_t* ring_lens;    // position of the new token; incremented
     int elem_bytes, B, H, capacity;
     int64_t stride_seq, stride_token;   // in elements
+    int host_pos;       // >= 0: position of the new token, known to the host (ring_lens is not touched)
     int early_inputs;   // query and new token come from host memory that no earlier kernel writes:
                         // read them before waiting for the kernel ahead (their latency hides under it)
 };
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
     if (do_append && live) {
         for (int i = threadIdx.x; i < n_app; i += 256) {
             const int c = i % chunks_per_row, h = (i / chunks_per_row) % ap.H, b = i / (chunks_per_row * ap.H);
-            const int pos = ap.ring_lens[b];
+            const int pos = ap.host_pos >= 0 ? ap.host_pos : ap.ring_lens[b];
             if (pos < 0 || pos >= ap.capacity) continue;
             const int64_t dst = ((int64_t)b * ap.stride_seq + (int64_t)pos * ap.stride_token + (int64_t)h * D) * ap.elem_bytes;
             const int64_t src = ((int64_t)(b * ap.H + h) * D) * ap.elem_bytes;
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
                 early ? av : *reinterpret_cast<const uint4*>((const char*)ap.new_v + src + c * 16);
         }
         __syncthreads();
-        for (int b = threadIdx.x; b < ap.B; b += 256)
+        for (int b = threadIdx.x; b < ap.B && ap.host_pos < 0; b += 256)
             if (ap.ring_lens[b] >= 0 && ap.ring_lens[b] < ap.capacity) ap.ring_lens[b] += 1;
     }
 #pragma unroll 1
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(DEC_THREADS) tq_decode_kernel(const DecodePara
 
     if (x < p.num_splits) {
         // ------------------------- compressed history -------------------------
-        int n = p.seq_lens[b];
+        int n = p.seq_lens ? p.seq_lens[b] : p.max_seq_len;
         if (n > p.max_seq_len) {   // the host bound sized the grid and the block-table check
             if (tid == 0) atomicCAS(p.status, 0, (int)TQ_ERR_RANGE);
             n = p.max_seq_len;
@@ -674,6 +675,21 @@ extern "C" int tq_decode_workspace_bytes(const tq_config* cfg, int32_t batch, in
     return TQ_OK;
 }
 
+// The decode kernel runs one 12-warp CTA per SM when the launch fits one wave: with few (sequence, head) pairs the
+// sequence is cut so that every SM gets one CTA, the ring tokens taking CTAs of their own (64 tokens each when the
+// launch fits one wave: ring_tok_for applies the same rule); with many pairs a CTA takes at most 512 records (8192
+// tokens) so that long and short sequences balance out.
+extern "C" int32_t tq_decode_splits(int32_t batch, int32_t num_kv_heads, int32_t max_seq_len, int32_t max_ring_len, int32_t sms) {
+    if (sms <= 0) sms = tq_sm_count();
+    const int nblk = (max_seq_len + TQ_BLOCK_TOKENS - 1) / TQ_BLOCK_TOKENS;
+    const int64_t pairs64 = (int64_t)batch * num_kv_heads;
+    const int pairs = pairs64 < 1 ? 1 : (int)(pairs64 < (1 << 30) ? pairs64 : (1 << 30));
+    int want = sms / pairs - (max_ring_len + 63) / 64;
+    if (want < (nblk + 511) / 512) want = (nblk + 511) / 512;
+    if (want > nblk / 12) want = nblk / 12;
+    return want < 1 ? 1 : want;
+}
+
 extern "C" int tq_scores_workspace_bytes(const tq_config* cfg, int64_t n_vectors, size_t* out) {
     if (!cfg || !out) return TQ_ERR_NULL;
     int rc = tq_check_config(cfg);
@@ -686,7 +702,9 @@ extern "C" int tq_scores_workspace_bytes(const tq_config* cfg, int64_t n_vectors
 static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_decode_args* a, void* stream,
                        int early_inputs, int validate_only = 0) {
     if (!consts || !pool || !a) return TQ_ERR_NULL;
-    if (!pool->base || !a->query || !a->out || !a->workspace || !a->block_table || !a->seq_lens) return TQ_ERR_NULL;
+    if (!pool->base || !a->query || !a->out || !a->workspace || !a->block_table) return TQ_ERR_NULL;
+    const bool host_lens = (a->flags & TQ_DECODE_HOST_LENS) != 0;
+    if (!host_lens && !a->seq_lens) return TQ_ERR_NULL;
     if (!consts->pi_t || !consts->s_t) return TQ_ERR_NULL;
     int rc = tq_check_config(&consts->cfg);
     if (rc != TQ_OK) return rc;
@@ -698,7 +716,7 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     if (G > TQ_MAX_GROUP_HEADS) return TQ_ERR_UNSUPPORTED;
     if ((int64_t)a->block_table_stride * TQ_BLOCK_TOKENS < a->max_seq_len) return TQ_ERR_SHAPE;
     const bool has_ring = a->ring_k != nullptr && a->max_ring_len > 0;
-    if (has_ring && (!a->ring_v || !a->ring_lens)) return TQ_ERR_NULL;
+    if (has_ring && (!a->ring_v || (!host_lens && !a->ring_lens))) return TQ_ERR_NULL;
     if (has_ring && a->max_ring_len > 256) return TQ_ERR_UNSUPPORTED;
     if (((uintptr_t)pool->base & 15) || ((uintptr_t)a->workspace & 255) || ((uintptr_t)a->out & 15)) return TQ_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
@@ -730,6 +748,7 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     uint32_t* qfrag = (uint32_t*)(ws + w.off_qfrag);
     RingAppend ap = {};
     ap.early_inputs = early_inputs;
+    ap.host_pos = host_lens ? a->max_ring_len - 1 : -1;
     if (a->append_k != nullptr) {
         if (!has_ring || !a->append_v || a->query_prepared) return TQ_ERR_NULL;
         if (a->ring_capacity < a->max_ring_len) return TQ_ERR_SHAPE;
@@ -770,8 +789,8 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     p.Qh = a->num_q_heads;
     p.G = G;
     p.block_table = a->block_table;
-    p.bt_stride = a->block_table_stride;
-    p.seq_lens = a->seq_lens;
+    p.bt_stride = (a->flags & TQ_DECODE_SHARED_TABLE) ? 0 : a->block_table_stride;
+    p.seq_lens = host_lens ? nullptr : a->seq_lens;
     p.max_seq_len = a->max_seq_len;
     p.min_history = a->min_history;
     p.qprep = qprep;
@@ -781,7 +800,7 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     p.ring_k = has_ring ? a->ring_k : nullptr;
     p.ring_v = has_ring ? a->ring_v : nullptr;
     p.ring_dtype = a->ring_dtype;
-    p.ring_lens = has_ring ? a->ring_lens : nullptr;
+    p.ring_lens = has_ring && !host_lens ? a->ring_lens : nullptr;
     p.max_ring_len = has_ring ? a->max_ring_len : 0;
     p.ring_stride_seq = a->ring_stride_seq;
     p.ring_stride_token = a->ring_stride_token;
@@ -819,6 +838,56 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
         TQ_DEC(256, 3, 4);
     }
 #undef TQ_DEC
+}
+
+namespace {
+// One or a few exact tokens into the ring, key and value in one launch.  Bound by its launch (a token of 8 heads x 128
+// is 4 KB): two torch slice assignments cost two launches and ~10 us of host time instead of one and ~3 us.
+__global__ void __launch_bounds__(256) tq_ring_write_kernel(const char* __restrict__ k, const char* __restrict__ v, int row16, int n_heads,
+                                                            int64_t total, int64_t src_token, int64_t src_head, char* __restrict__ rk,
+                                                            char* __restrict__ rv, int64_t dst_token) {
+    // the ring may still be read by the launch ahead; only then may the next one begin (it reads pool and tables early)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;   // (token, head, 16-byte chunk)
+    if (i >= total) return;
+    const int c = (int)(i % row16);
+    const int h = (int)((i / row16) % n_heads);
+    const int64_t t = i / ((int64_t)row16 * n_heads);
+    const int64_t src = t * src_token + h * src_head + 16 * c, dst = t * dst_token + ((int64_t)h * row16 + c) * 16;
+    const uint4 a = *reinterpret_cast<const uint4*>(k + src), b = *reinterpret_cast<const uint4*>(v + src);
+    *reinterpret_cast<uint4*>(rk + dst) = a;
+    *reinterpret_cast<uint4*>(rv + dst) = b;
+}
+}  // namespace
+
+extern "C" int tq_ring_write(const void* key, const void* value, tq_dtype dtype, int64_t n_tokens, int32_t n_heads, int32_t head_dim,
+                             int64_t stride_token, int64_t stride_head, void* ring_k, void* ring_v, int64_t ring_stride_token,
+                             int64_t position, void* stream) {
+    if (!key || !value || !ring_k || !ring_v) return TQ_ERR_NULL;
+    if (n_tokens <= 0 || n_heads <= 0 || head_dim <= 0 || position < 0) return TQ_ERR_SHAPE;
+    if (n_tokens > (1 << 20) || n_heads > (1 << 12)) return TQ_ERR_UNSUPPORTED;
+    const int64_t eb = (int64_t)tq_dtype_size(dtype);
+    if (((uintptr_t)key | (uintptr_t)value | (uintptr_t)ring_k | (uintptr_t)ring_v | (uintptr_t)(stride_token * eb) |
+         (uintptr_t)(stride_head * eb) | (uintptr_t)(ring_stride_token * eb) | (uintptr_t)(head_dim * eb)) & 15)
+        return TQ_ERR_ALIGN;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int row16 = (int)(head_dim * eb / 16);
+    const int64_t total = n_tokens * n_heads * row16;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((total + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    tq_note_launch(st, TQ_LAUNCH_DECODE);   // a store behind it may be about to read the ring
+    const int64_t off = position * ring_stride_token * eb;
+    return cudaLaunchKernelEx(&cfg, tq_ring_write_kernel, (const char*)key, (const char*)value, row16, (int)n_heads, total,
+                              stride_token * eb, stride_head * eb, (char*)ring_k + off, (char*)ring_v + off,
+                              ring_stride_token * eb) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
 }
 
 extern "C" int tq_decode(const tq_consts* consts, const tq_pool* pool, const tq_decode_args* a, void* stream) {

@@ -335,7 +335,7 @@ __device__ __forceinline__ void ring_part(const DecodeParams& p, int b, int h, i
     constexpr int MAX_OWN = (GP * D + 127) / 128;   // outputs per thread with at least 128 threads
     const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
     const int rs = slot_idx - p.num_splits;
-    int R = p.ring_lens ? p.ring_lens[b] : 0;
+    int R = p.ring_lens ? p.ring_lens[b] : p.max_ring_len;
     if (R > p.max_ring_len) {   // more than the host promised: the ring CTAs only cover max_ring_len tokens
         if (tid == 0) atomicCAS(p.status, 0, (int)TQ_ERR_RANGE);
         R = p.max_ring_len;

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
 
     // ------------------------------ this CTA's share of the history ------------------------------
     constexpr uint32_t QF_BYTES = qf_words(D, SPLITB ? 8 : 4) * 4u;
-    int n = p.seq_lens[b];
+    int n = p.seq_lens ? p.seq_lens[b] : p.max_seq_len;
     if (n > p.max_seq_len) {   // the host bound sized the grid, the block table and this CTA's table slice
         if (tid == 0) atomicCAS(p.status, 0, (int)TQ_ERR_RANGE);
         n = p.max_seq_len;

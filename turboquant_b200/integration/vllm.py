@@ -201,6 +201,16 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
             return _deliver(_no_alloc_prefill_attention(state, self_impl, query, key, value, attn_metadata),
                             query, output, n)
         if mode == MODE_HYBRID and state.supports_hybrid and state.store.num_tokens >= MIN_HISTORY:
+            if output is not None:                      # straight into the engine's buffer where its layout allows
+                st = state.store
+                rk, rv = state.engine.ring.peek() or (None, None)
+                res = E.host().hybrid(st.consts.addr, st.pool.addr, st.workspace, st.block_table, c.head_dim, st._num_tokens,
+                                      query, n, c.num_query_heads, rk, rv, getattr(self_impl, "scale", None), MIN_HISTORY,
+                                      output)
+                if res is output:
+                    return output
+                if res is not None:
+                    E.check(res, "tq_decode")
             q = _as_heads(query, n, c.num_query_heads, c.head_dim)
             recent = state.engine.ring.peek()
             result = compute_hybrid_attention(q, state.store, recent[0] if recent else None,

@@ -94,6 +94,10 @@ class CompressedPagedKVCache:
         """Compress `key` / `value` (T, H, D) into the slots the engine chose: slot = block * 16 +
         offset, negative = padding token to skip (the contract of vLLM's reshape_and_cache)."""
         t = key.shape[0]
+        rc = E.host().store(self.consts.addr, self.pool.addr, key, value, self.spec.head_dim, None, slot_mapping, 0, t)
+        if rc is not None:
+            E.check(rc, "tq_store")
+            return
         if slot_mapping.dtype != torch.int64 or slot_mapping.numel() < t:
             raise ValueError("slot_mapping must hold one int64 slot per token")
         if key.stride(2) != 1 or value.stride() != key.stride():
@@ -105,6 +109,12 @@ class CompressedPagedKVCache:
                scale: Optional[float] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """One decode token per sequence: query (B, Qh, D), block_tables (B, max_blocks) int32, seq_lens
         (B,) int32 -> (B, Qh, D).  Every sequence of the step in one launch."""
+        res = E.host().batch(self.consts.addr, self.pool.addr, self.workspace, self.spec.head_dim, query, block_tables,
+                             seq_lens, max_seq_len, scale, 1, out)
+        if type(res) is torch.Tensor:
+            return res
+        if res is not None:
+            E.check(res, "tq_decode")
         return E.decode(self.consts, self.pool, self.workspace, query, block_tables, seq_lens, max_seq_len,
                         scale=scale, min_history=1, out=out)
 

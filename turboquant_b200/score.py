@@ -31,6 +31,15 @@ def compute_hybrid_attention(query: torch.Tensor, store: CompressedKVStore, rece
     Every query token attends to all history and all recent tokens (no causal
     mask, as in the reference); history shorter than 16 tokens is ignored.
     """
+    if query.dim() == 3:
+        out = E.host().hybrid(store.consts.addr, store.pool.addr, store.workspace, store.block_table, store.head_dim,
+                              store._num_tokens, query, query.shape[0], num_query_heads, recent_k, recent_v, scale,
+                              MIN_HISTORY_FOR_TQ, None)
+        if type(out) is torch.Tensor:
+            return out
+        if out is not None:
+            E.check(out, "tq_decode")
+    # what the native path does not take: other layouts, nothing to attend to, arguments to refuse
     E.require_cuda(query, "query")
     t, qh, d = query.shape
     if qh != num_query_heads or d != store.head_dim:

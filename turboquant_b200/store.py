@@ -79,6 +79,15 @@ class CompressedKVStore:
         t = key.shape[0]
         if t == 0:
             return
+        n = self._num_tokens
+        if n + t <= self.pool.num_blocks * E.TQ_BLOCK_TOKENS:
+            rc = E.host().store(self.consts.addr, self.pool.addr, key, value, self.head_dim, self.block_table, None, n, t)
+            if rc is not None:
+                E.check(rc, "tq_store")
+                self._num_tokens = n + t
+                self._num_chunks += 1
+                self._flat = None
+                return
         if key.shape != value.shape or key.shape[1] != self.num_kv_heads or key.shape[2] != self.head_dim:
             raise ValueError(f"expected (T, {self.num_kv_heads}, {self.head_dim}) key and value, got "
                              f"{tuple(key.shape)} / {tuple(value.shape)}")

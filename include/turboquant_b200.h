@@ -90,6 +90,12 @@ typedef struct tq_consts {
      * batches at head_dim 128): S split into two bf16 limbs, (D,D) row-major.
      * With either NULL (or pi_limbs missing) the fp32 kernels prepare the queries. */
     const void* s_limbs[2];
+    /* Optional operands of tq_rows_quantize_keys / tq_rows_dequantize_keys at
+     * head_dim 128: 64 Pi, M and S, each as two fp16 limbs, (D,D) row-major.  With
+     * any of them NULL those calls return TQ_ERR_UNSUPPORTED. */
+    const void* rows_pi[2];
+    const void* rows_m[2];
+    const void* rows_s[2];
 } tq_consts;
 
 /* Byte offsets inside one block record. */
@@ -363,6 +369,63 @@ int tq_dequant_keys(const tq_consts* consts, const tq_pool* pool, const int32_t*
  * (kv_cache.py:101-116). */
 int tq_dequant_values(const tq_config* cfg, const tq_pool* pool, const int32_t* block_table,
                       int64_t n_tokens, float* out, void* stream);
+
+/* ---- the single-object cache: both halves of its attention -------------------- */
+
+/* Scratch of tq_cache_scores / tq_cache_attend (one buffer serves both; zero it once,
+ * see tq_workspace_init). */
+int tq_cache_workspace_bytes(const tq_config* cfg, int32_t n_heads, int64_t n_tokens, int64_t n_buf, int32_t n_q, size_t* out);
+
+/* Scaled logits (n_heads, n_q, n_tokens + n_buf) fp32 of query (n_heads, n_q, D) against the compressed
+ * history and n_buf exact keys, element (h, t, :) at buf_keys + h*stride_head + t*stride_token.
+ * Replaces TurboQuantKVCache.attention_scores (kv_cache.py:225-270). */
+int tq_cache_scores(const tq_consts* consts, const tq_pool* pool, const int32_t* block_table, int64_t n_tokens, const void* query,
+                    tq_dtype q_dtype, int32_t n_q, const void* buf_keys, tq_dtype buf_dtype, int64_t n_buf, int64_t stride_head,
+                    int64_t stride_token, float scale, float* logits, void* workspace, size_t workspace_bytes, void* stream);
+
+/* weights (n_heads, n_q, n_tokens + n_buf) times the values, history and exact buffer: out (n_heads, n_q, D)
+ * fp32.  Replaces TurboQuantKVCache.attend (kv_cache.py:272-320). */
+int tq_cache_attend(const tq_consts* consts, const tq_pool* pool, const int32_t* block_table, int64_t n_tokens, const void* weights,
+                    tq_dtype w_dtype, int32_t n_q, const void* buf_values, tq_dtype buf_dtype, int64_t n_buf, int64_t stride_head,
+                    int64_t stride_token, float* out, void* workspace, size_t workspace_bytes, void* stream);
+
+/* ---- the quantiser objects on plain rows and flat planes ------------------- */
+
+/* Group quantisation of n_rows rows of head_dim values (32 per group): codes
+ * (n_rows, head_dim*bits/8) in the reference's packing, scales and zero points
+ * (n_rows, head_dim/32) in the input dtype after their fp16 round trip.
+ * Replaces quantize_values (kv_cache.py:45-98). */
+int tq_rows_quantize_values(const void* v, tq_dtype dtype, int64_t n_rows, int32_t head_dim, int64_t stride_row, int32_t bits,
+                            uint8_t* data, void* scales, void* zeros, void* stream);
+
+/* code * scale + zero, fp32 (kv_cache.py:101-116); scales / zeros of any dtype
+ * pass through fp16. */
+int tq_rows_dequantize_values(const uint8_t* data, const void* scales, const void* zeros, tq_dtype scale_dtype, int64_t n_rows,
+                              int32_t head_dim, int32_t bits, float* out, void* stream);
+
+/* TurboQuantProd.quantize (quantizer.py:231-257) of n_rows vectors: codes
+ * (n_rows, kcode_row), sign bits (n_rows, D/8), norms and residual norms after
+ * their fp16 round trip; codes equal to tq_store's.  head_dim 128, fp32 or fp16
+ * rows (bf16 rows have the tensor-core store), the fp16 operands in `consts`;
+ * anything else returns TQ_ERR_UNSUPPORTED with
+ * nothing launched. */
+int tq_rows_quantize_keys(const tq_consts* consts, const void* x, tq_dtype dtype, int64_t n_rows, int64_t stride_row, uint8_t* codes,
+                          uint8_t* signs, void* norms, tq_dtype norm_dtype, void* residual_norms, tq_dtype residual_dtype,
+                          void* stream);
+
+/* TurboQuantProd.dequantize (quantizer.py:259-272), with_qjl = 0:
+ * TurboQuantMSE.dequantize (quantizer.py:151-165; signs and residual norms may
+ * be NULL).  out (n_rows, D) fp32. */
+int tq_rows_dequantize_keys(const tq_consts* consts, const uint8_t* codes, const uint8_t* signs, const void* norms,
+                            tq_dtype norm_dtype, const void* residual_norms, tq_dtype residual_dtype, int64_t n_rows,
+                            int32_t with_qjl, float* out, void* stream);
+
+/* TurboQuantProd.attention_score (quantizer.py:274-302) on key planes
+ * (n_heads, n_keys, ...): query (n_heads, n_q, D) -> logits (n_heads, n_q,
+ * n_keys).  Workspace as for tq_scores. */
+int tq_rows_scores(const tq_consts* consts, const uint8_t* codes, const uint8_t* signs, const void* norms, tq_dtype norm_dtype,
+                   const void* residual_norms, tq_dtype residual_dtype, int32_t n_heads, int64_t n_keys, const void* query,
+                   tq_dtype q_dtype, int32_t n_q, float* logits, void* workspace, size_t workspace_bytes, void* stream);
 
 /* The integer stages of the store path alone: bucket search + LSB-first code
  * packing of already rotated unit vectors y (n_rows, D) fp32, and sign packing

@@ -1233,3 +1233,108 @@ def test_ring_write_in_one_launch(dtype, n, pos, strided, dev):
     assert torch.equal(rk[pos:pos + n], k) and torch.equal(rv[pos:pos + n], v)
     assert torch.equal(rk[:pos], before) and torch.equal(rv[:pos], before + 1)
     assert float(rk[pos + n:].abs().max() if pos + n < cap else 0) == 0
+
+
+@pytest.mark.parametrize("d,bits,dtype,n", [(128, 3, torch.float32, 1), (128, 3, torch.float32, 129), (128, 4, torch.float32, 1000),
+                                            (128, 3, torch.float16, 16), (128, 4, torch.float16, 127), (256, 3, torch.float32, 33)])
+def test_key_rows_kernels_match_store_and_pool_kernels(d, bits, dtype, n, dev):
+    """Quantise / dequantise / score on plain rows against the same work through a pool of records (edges of the
+    16-row warps and 128-row tiles; a zero row; a key that sits on a decision boundary's neighbour is part of any draw)."""
+    from turboquant_b200 import TurboQuantProd, _engine as E
+    q = TurboQuantProd(d, bits, device=dev)
+    g = torch.Generator().manual_seed(n + bits)
+    x = (torch.randn(n, d, generator=g) * 3).to(dtype).to(dev)
+    x[n // 2] = 0 if n > 1 else x[n // 2]
+    kq = q.quantize(x)
+    ps = q._compress_rows(x)[2]
+    assert _code_frac(kq.mse_indices, ps.mse_indices[0], 4 if bits == 4 else 2) <= TIE_BUDGET
+    assert _bit_frac(kq.qjl_signs, ps.qjl_signs[0]) <= 2 * TIE_BUDGET
+    assert torch.equal(kq.norms.half(), ps.norms[0])
+    assert torch.allclose(kq.residual_norms, ps.residual_norms[0].float(), rtol=2e-3, atol=1e-6)
+    pool, bt, heads, m = q._pool_from(*[t for t in (kq.mse_indices, kq.qjl_signs, kq.norms, kq.residual_norms)])
+    for signs in (True, False):
+        ref = E.dequant_keys(q.consts, pool, bt, m, with_qjl=signs).reshape(n, d)
+        got = q._dequantize(kq.mse_indices, kq.qjl_signs if signs else None, kq.norms, kq.residual_norms if signs else None)
+        assert float((got - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+    query = torch.randn(2, d, generator=g).to(dtype).to(dev)
+    ref = E.scores(q.consts, pool, q._ws, bt, m, query[None])
+    got = q.attention_score(query, kq)
+    assert float((got - ref[0]).abs().max()) <= LOGIT_TOL * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("d,bits,dtype,n,strided", [(128, 2, torch.float32, 1, False), (128, 4, torch.float16, 33, False),
+                                                    (256, 2, torch.bfloat16, 17, True), (256, 4, torch.float32, 300, False)])
+def test_value_rows_kernels_match_oracle(d, bits, dtype, n, strided, dev):
+    from turboquant_b200.kv_cache import dequantize_values, quantize_values
+    g = torch.Generator().manual_seed(d + n)
+    x = torch.randn(n, 2 * d, generator=g).to(dtype).to(dev)
+    x = x[:, :d] if strided else x[:, :d].contiguous()
+    x[n // 2, :32] = 0.5   # a constant group
+    vq = quantize_values(x, bits)
+    lim = 2 ** bits - 1
+    xf = x.float().reshape(n, d // 32, 32)
+    lo, hi = xf.amin(-1), xf.amax(-1)
+    assert torch.equal(vq.zeros.float(), lo.half().to(dtype).float())
+    step = ((hi - lo) / lim).clamp_min(1e-10)
+    assert torch.allclose(vq.scales.float(), step, rtol=1e-2, atol=1e-4)
+    out = dequantize_values(vq)
+    err = (out.reshape(n, d // 32, 32) - xf).abs()
+    assert bool((err <= (0.53 * step + 2e-2 * (hi.abs() + lo.abs()))[..., None]).all())
+
+
+@pytest.mark.parametrize("d,kb,vb,n,n_buf,n_q,dtype", [(128, 3, 2, 1, 1, 1, torch.float32), (128, 3, 2, 63, 17, 1, torch.float16),
+                                                       (128, 4, 4, 200, 5, 3, torch.bfloat16), (256, 3, 2, 1025, 128, 2, torch.float32)])
+def test_cache_object_scores_and_attend_in_one_launch(d, kb, vb, n, n_buf, n_q, dtype, dev):
+    """History and exact buffer in one logits / one output kernel against dequantised rows and plain matrix products,
+    with a split history and twice in a row (the merge tickets return to zero)."""
+    from turboquant_b200 import TurboQuantKVCache, _engine as E
+    g = torch.Generator().manual_seed(n + n_buf)
+    b, h = 2, 3
+    cache = TurboQuantKVCache(head_dim=d, key_bits=kb, value_bits=vb, buffer_size=n_buf, device=dev, dtype=dtype)
+    k, v = (torch.randn(b, h, n + n_buf, d, generator=g).to(dtype).to(dev) for _ in range(2))
+    cache.prefill(k, v)
+    q = torch.randn(b, h, n_q, d, generator=g).to(dtype).to(dev)
+    m = cache._n_quant
+    w = torch.softmax(torch.randn(b, h, n_q, n + n_buf, generator=g), -1).to(dtype).to(dev)
+    for _ in range(2):
+        logits, out = cache.attention_scores(q), cache.attend(w)
+    ref_l, ref_o = [], []
+    if m:
+        kd = E.dequant_keys(cache.consts, cache._pool, cache._bt, m).reshape(b, h, m, d)
+        vd = E.dequant_values(cache.consts, cache._pool, cache._bt, m).reshape(b, h, m, d)
+        ref_l.append(q.float() @ kd.transpose(-1, -2))
+        ref_o.append(w[..., :m].float() @ vd)
+    if n + n_buf > m:
+        ref_l.append(q.float() @ k[..., m:, :].float().transpose(-1, -2))
+        ref_o.append(w[..., m:].float() @ v[..., m:, :].float())
+    ref_l, ref_o = torch.cat(ref_l, -1) / math.sqrt(d), sum(ref_o)
+    tol = 1e-2 if dtype == torch.bfloat16 else 2e-3
+    assert float((logits.float() - ref_l).abs().max()) <= tol * float(ref_l.abs().max())
+    assert _cos(out.float(), ref_o) >= COS_MIN and float((out.float() - ref_o).abs().max()) <= tol * float(ref_o.abs().max())
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (17, 0), (200, 1), (200, 4)])
+def test_conversion_words_and_bytes(n, shift, dev):
+    """Planes at word-aligned and odd addresses survive the way into records and back."""
+    import ctypes as C
+    from turboquant_b200 import _engine as E, _lib
+    consts = E.LayerConstants(128, 3, 2, dev)
+    g = torch.Generator().manual_seed(n)
+    ps, back = E.PlaneSet(consts, 2, n), E.PlaneSet(consts, 2, n)
+    for s in (ps, back):
+        for f in ("mse_indices", "qjl_signs", "v_data"):   # byte planes may start anywhere
+            t = getattr(s, f)
+            raw = torch.randint(0, 256, (t.numel() + 8,), generator=g, dtype=torch.uint8).to(dev)
+            setattr(s, f, raw[shift:shift + t.numel()].view(t.shape))
+        s.c = _lib.tq_planes(s.mse_indices.data_ptr(), s.qjl_signs.data_ptr(), s.norms.data_ptr(), s.residual_norms.data_ptr(),
+                             s.v_data.data_ptr(), s.v_scales.data_ptr(), s.v_zeros.data_ptr(), *[getattr(s.c, x[0]) for x in s.c._fields_[7:]])
+    for f in ("norms", "residual_norms", "v_scales", "v_zeros"):
+        t = getattr(ps, f)
+        t.copy_(torch.rand(t.shape, generator=g))
+    pool = E.BlockPool(consts, 2, E.blocks_for(n))
+    bt = E.identity_block_table(pool.num_blocks, dev)
+    E.planes_to_pool(consts, ps, n, pool, bt)
+    _lib.check(_lib.lib().tq_pool_to_planes(C.byref(consts.cfg), C.byref(pool.c), bt.data_ptr(), n, C.byref(back.c), E.stream_ptr(dev)),
+               "tq_pool_to_planes")
+    for f in ("mse_indices", "qjl_signs", "norms", "residual_norms", "v_data", "v_scales", "v_zeros"):
+        assert torch.equal(getattr(ps, f)[:, :n], getattr(back, f)[:, :n]), f

@@ -44,14 +44,18 @@ def get_layout(head_dim: int, key_bits: int, value_bits: int, group_size: int = 
     return out
 
 
-def _split_bf16(m: torch.Tensor, n_limbs: int) -> list[torch.Tensor]:
-    """m (fp64) as a sum of bf16 limbs, largest first."""
+def _split(m: torch.Tensor, n_limbs: int, dtype: torch.dtype) -> list[torch.Tensor]:
+    """m (fp64) as a sum of limbs of `dtype`, largest first."""
     limbs, rest = [], m.clone()
     for _ in range(n_limbs):
-        limb = rest.to(torch.float32).to(torch.bfloat16)
+        limb = rest.to(torch.float32).to(dtype)
         limbs.append(limb)
         rest = rest - limb.to(torch.float64)
     return limbs
+
+
+def _split_bf16(m: torch.Tensor, n_limbs: int) -> list[torch.Tensor]:
+    return _split(m, n_limbs, torch.bfloat16)
 
 
 class LayerConstants:
@@ -110,8 +114,22 @@ class LayerConstants:
         for i in range(2):
             c.m_limbs[i] = self.m_limbs[i].data_ptr() if tensor_core_store else None
             c.s_limbs[i] = self.s_limbs[i].data_ptr() if tensor_core_store else None
+        self.rows_limbs = None
         self.c = c
         self.addr = C.addressof(c)     # what the native host path passes on
+
+    def ensure_rows(self) -> None:
+        """Operands of the kernels on plain rows (64 Pi, M = S Pi^T and S as two fp16 limbs each): only the quantiser
+        objects use them, which call this when they are made."""
+        if self.rows_limbs is not None or self.head_dim != 128:
+            return
+        pi, s = self.Pi.cpu().double(), self.S.cpu().double()
+        mats, limbs = (pi * 64.0, s @ pi.T, s), []
+        if all(bool(t.abs().max() < 60000.0) for t in mats):   # fp16's range (a caller's own S may be anything)
+            limbs = [[t.contiguous().to(self.device) for t in _split(x, 2, torch.float16)] for x in mats]
+            for i in range(2):
+                self.c.rows_pi[i], self.c.rows_m[i], self.c.rows_s[i] = (x[i].data_ptr() for x in limbs)
+        self.rows_limbs = limbs
 
     @property
     def block_bytes(self) -> int:
@@ -125,7 +143,9 @@ class LayerConstants:
 class BlockPool:
     """A pool of block records for `num_kv_heads` heads (uint8 device tensor)."""
 
-    def __init__(self, consts: LayerConstants, num_kv_heads: int, num_blocks: int):
+    def __init__(self, consts: LayerConstants, num_kv_heads: int, num_blocks: int, zeroed: bool = True):
+        """zeroed=False: for a pool whose blocks are all written before any is read."""
+        self._alloc = torch.zeros if zeroed else torch.empty
         self.consts = consts
         self.num_kv_heads = num_kv_heads
         self.num_blocks = 0
@@ -139,7 +159,7 @@ class BlockPool:
         if num_blocks <= self.num_blocks:
             return
         per_block = self.num_kv_heads * self.consts.block_bytes
-        new = torch.zeros(num_blocks * per_block, dtype=torch.uint8, device=self.consts.device)
+        new = self._alloc(num_blocks * per_block, dtype=torch.uint8, device=self.consts.device)
         if self.num_blocks:
             new[: self.num_blocks * per_block].copy_(self.data)
         self.data, self.num_blocks = new, num_blocks
@@ -351,16 +371,18 @@ def scores(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: 
 class PlaneSet:
     """Flat planes (H, capacity, ...) on the device plus their C descriptor."""
 
-    def __init__(self, consts: LayerConstants, num_kv_heads: int, capacity: int):
+    def __init__(self, consts: LayerConstants, num_kv_heads: int, capacity: int, zeroed: bool = True):
+        """zeroed=False: for planes that a conversion fills completely."""
         lay, dev = consts.layout, consts.device
         h, n = num_kv_heads, max(1, capacity)
-        self.mse_indices = torch.zeros(h, n, lay.kcode_row, dtype=torch.uint8, device=dev)
-        self.qjl_signs = torch.zeros(h, n, lay.ksign_row, dtype=torch.uint8, device=dev)
-        self.norms = torch.zeros(h, n, dtype=torch.float16, device=dev)
-        self.residual_norms = torch.zeros(h, n, dtype=torch.float16, device=dev)
-        self.v_data = torch.zeros(h, n, lay.vcode_row, dtype=torch.uint8, device=dev)
-        self.v_scales = torch.zeros(h, n, lay.n_groups, dtype=torch.float16, device=dev)
-        self.v_zeros = torch.zeros(h, n, lay.n_groups, dtype=torch.float16, device=dev)
+        new = torch.zeros if zeroed else torch.empty
+        self.mse_indices = new(h, n, lay.kcode_row, dtype=torch.uint8, device=dev)
+        self.qjl_signs = new(h, n, lay.ksign_row, dtype=torch.uint8, device=dev)
+        self.norms = new(h, n, dtype=torch.float16, device=dev)
+        self.residual_norms = new(h, n, dtype=torch.float16, device=dev)
+        self.v_data = new(h, n, lay.vcode_row, dtype=torch.uint8, device=dev)
+        self.v_scales = new(h, n, lay.n_groups, dtype=torch.float16, device=dev)
+        self.v_zeros = new(h, n, lay.n_groups, dtype=torch.float16, device=dev)
         self.capacity = n
         self.c = _lib.tq_planes(self.mse_indices.data_ptr(), self.qjl_signs.data_ptr(), self.norms.data_ptr(),
                                 self.residual_norms.data_ptr(), self.v_data.data_ptr(), self.v_scales.data_ptr(),
@@ -382,7 +404,7 @@ class PlaneSet:
 
 
 def pool_to_planes(consts: LayerConstants, pool: BlockPool, block_table: torch.Tensor, n_tokens: int) -> PlaneSet:
-    ps = PlaneSet(consts, pool.num_kv_heads, n_tokens)
+    ps = PlaneSet(consts, pool.num_kv_heads, n_tokens, zeroed=n_tokens < 1)
     check(lib().tq_pool_to_planes(C.byref(consts.cfg), C.byref(pool.c), block_table.data_ptr(), n_tokens,
                                   C.byref(ps.c), stream_ptr(consts.device)), "tq_pool_to_planes")
     return ps
@@ -409,8 +431,161 @@ def dequant_values(consts: LayerConstants, pool: BlockPool, block_table: torch.T
     return out
 
 
+def _float_code(t: torch.Tensor) -> Optional[int]:
+    return _DTYPES.get(t.dtype)
+
+
+def rows_quantize_keys(consts: LayerConstants, x: torch.Tensor):
+    """(n, D) rows -> (codes, sign bits, norms in x's dtype, residual norms fp32), or None where the rows kernel does not
+    take them (head_dim 256, no split operands, unaligned rows)."""
+    if consts.head_dim != 128 or not x.is_cuda or x.dtype not in _DTYPES or x.stride(1) != 1:
+        return None
+    n, lay, dev = x.shape[0], consts.layout, x.device
+    codes = torch.empty(n, lay.kcode_row, dtype=torch.uint8, device=dev)
+    signs = torch.empty(n, lay.ksign_row, dtype=torch.uint8, device=dev)
+    norms = torch.empty(n, dtype=x.dtype, device=dev)
+    rnorms = torch.empty(n, dtype=torch.float32, device=dev)
+    rc = lib().tq_rows_quantize_keys(consts.addr, x.data_ptr(), _DTYPES[x.dtype], n, x.stride(0), codes.data_ptr(), signs.data_ptr(),
+                                     norms.data_ptr(), _DTYPES[x.dtype], rnorms.data_ptr(), TQ_F32, stream_ptr(dev))
+    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN, _lib.TQ_ERR_SHAPE):
+        return None
+    check(rc, "tq_rows_quantize_keys")
+    return codes, signs, norms, rnorms
+
+
+def rows_dequantize_keys(consts: LayerConstants, codes, signs, norms, rnorms) -> Optional[torch.Tensor]:
+    """Contiguous key planes (n, ...) -> (n, D) fp32; signs / rnorms None: the MSE part alone.  None where the rows kernel
+    does not take them."""
+    if not codes.is_cuda or _float_code(norms) is None or (rnorms is not None and _float_code(rnorms) is None):
+        return None
+    n = norms.numel()
+    out = torch.empty(n, consts.head_dim, dtype=torch.float32, device=codes.device)
+    rc = lib().tq_rows_dequantize_keys(consts.addr, codes.data_ptr(), signs.data_ptr() if signs is not None else None, norms.data_ptr(),
+                                       _float_code(norms), rnorms.data_ptr() if rnorms is not None else None,
+                                       _float_code(rnorms) if rnorms is not None else TQ_F32, n, 0 if signs is None else 1,
+                                       out.data_ptr(), stream_ptr(codes.device))
+    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
+        return None
+    check(rc, "tq_rows_dequantize_keys")
+    return out
+
+
+def rows_scores(consts: LayerConstants, ws: "Workspace", codes, signs, norms, rnorms, heads: int, n: int,
+                query: torch.Tensor) -> Optional[torch.Tensor]:
+    """Key planes (heads, n, ...) and query (heads, n_q, D) -> unscaled logits (heads, n_q, n) fp32, or None."""
+    if not codes.is_cuda or not query.is_cuda or None in (_float_code(norms), _float_code(rnorms), _float_code(query)):
+        return None
+    n_q = query.shape[1]
+    ws.ensure(256 + heads * n_q * 2 * consts.head_dim * 4)
+    logits = torch.empty(heads, n_q, n, dtype=torch.float32, device=codes.device)
+    rc = lib().tq_rows_scores(consts.addr, codes.data_ptr(), signs.data_ptr(), norms.data_ptr(), _float_code(norms), rnorms.data_ptr(),
+                              _float_code(rnorms), heads, n, query.data_ptr(), _float_code(query), n_q, logits.data_ptr(), ws.ptr,
+                              ws.nbytes, stream_ptr(codes.device))
+    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
+        return None
+    check(rc, "tq_rows_scores")
+    return logits
+
+
+def rows_quantize_values(v: torch.Tensor, bits: int):
+    """(n, D) rows -> (codes, scales, zero points in v's dtype), or None (unaligned rows)."""
+    n, d = v.shape
+    g = d // 32
+    data = torch.empty(n, d * bits // 8, dtype=torch.uint8, device=v.device)
+    sz = torch.empty(2, n, g, dtype=v.dtype, device=v.device)
+    rc = lib().tq_rows_quantize_values(v.data_ptr(), dtype_code(v.dtype), n, d, v.stride(0), bits, data.data_ptr(), sz[0].data_ptr(),
+                                       sz[1].data_ptr(), stream_ptr(v.device))
+    if rc in (_lib.TQ_ERR_ALIGN, _lib.TQ_ERR_SHAPE):
+        return None
+    check(rc, "tq_rows_quantize_values")
+    return data, sz[0], sz[1]
+
+
+def rows_dequantize_values(data: torch.Tensor, scales: torch.Tensor, zeros: torch.Tensor, bits: int, d: int) -> Optional[torch.Tensor]:
+    """Contiguous value planes -> (n, D) fp32, or None."""
+    if _float_code(scales) is None or zeros.dtype != scales.dtype:
+        return None
+    n = data.numel() // data.shape[-1]
+    out = torch.empty(n, d, dtype=torch.float32, device=data.device)
+    rc = lib().tq_rows_dequantize_values(data.data_ptr(), scales.data_ptr(), zeros.data_ptr(), _float_code(scales), n, d, bits,
+                                         out.data_ptr(), stream_ptr(data.device))
+    if rc == _lib.TQ_ERR_ALIGN:
+        return None
+    check(rc, "tq_rows_dequantize_values")
+    return out
+
+
+def _buffer_rows(buf: Optional[torch.Tensor]):
+    """(b, h, n, d) exact rows as (pointer, dtype, n, stride per (b, h), stride per token), contiguous if need be."""
+    if buf is None or buf.shape[2] == 0:
+        return None, TQ_F32, 0, 0, 0, None
+    es = buf.element_size()
+    if buf.stride(3) != 1 or (buf.shape[0] > 1 and buf.stride(0) != buf.shape[1] * buf.stride(1)) or buf.data_ptr() % 16 or \
+            (buf.stride(1) * es) % 16 or (buf.stride(2) * es) % 16:
+        buf = buf.contiguous()
+    return buf.data_ptr(), dtype_code(buf.dtype), buf.shape[2], buf.stride(1), buf.stride(2), buf
+
+
+def _cache_workspace(consts, ws, heads: int, n: int, n_buf: int, n_q: int) -> None:
+    need = C.c_size_t(0)
+    check(lib().tq_cache_workspace_bytes(C.byref(consts.cfg), heads, n, n_buf, n_q, C.byref(need)), "tq_cache_workspace_bytes")
+    ws.ensure(need.value)
+
+
+def cache_scores(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: torch.Tensor, n: int, query: torch.Tensor,
+                 buf: Optional[torch.Tensor], scale: float) -> Optional[torch.Tensor]:
+    """query (b*h, n_q, D) contiguous -> scaled logits (b*h, n_q, n + buffer) fp32, or None where the kernel does not apply."""
+    if _float_code(query) is None or (buf is not None and buf.dtype not in _DTYPES):
+        return None
+    heads, n_q, _ = query.shape
+    ptr, dt, nb, sh, st, keep = _buffer_rows(buf)
+    _cache_workspace(consts, ws, heads, n, nb, n_q)
+    logits = torch.empty(heads, n_q, n + nb, dtype=torch.float32, device=query.device)
+    rc = lib().tq_cache_scores(consts.addr, pool.addr, block_table.data_ptr(), n, query.data_ptr(), _float_code(query), n_q, ptr, dt, nb,
+                               sh, st, scale, logits.data_ptr(), ws.ptr, ws.nbytes, stream_ptr(query.device))
+    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
+        return None
+    check(rc, "tq_cache_scores")
+    return logits
+
+
+def cache_attend(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: torch.Tensor, n: int, weights: torch.Tensor,
+                 buf: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """weights (b*h, n_q, n + buffer) contiguous -> (b*h, n_q, D) fp32, or None where the kernel does not apply."""
+    if _float_code(weights) is None or (buf is not None and buf.dtype not in _DTYPES):
+        return None
+    heads, n_q, _ = weights.shape
+    ptr, dt, nb, sh, st, keep = _buffer_rows(buf)
+    _cache_workspace(consts, ws, heads, n, nb, n_q)
+    out = torch.empty(heads, n_q, consts.head_dim, dtype=torch.float32, device=weights.device)
+    rc = lib().tq_cache_attend(consts.addr, pool.addr, block_table.data_ptr(), n, weights.data_ptr(), _float_code(weights), n_q, ptr, dt,
+                               nb, sh, st, out.data_ptr(), ws.ptr, ws.nbytes, stream_ptr(weights.device))
+    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
+        return None
+    check(rc, "tq_cache_attend")
+    return out
+
+
 def identity_block_table(n_blocks: int, device) -> torch.Tensor:
     return torch.arange(max(1, n_blocks), dtype=torch.int32, device=device)
+
+
+_IDENTITY: dict[str, torch.Tensor] = {}
+_IDENTITY_ENTRIES = 65536
+
+
+def shared_identity_table(n_blocks: int, device) -> torch.Tensor:
+    """A read-only identity table of at least `n_blocks` entries: one of 64 K entries per device, made once and never
+    replaced, so that any stream may read it; a table of its own beyond that."""
+    key = str(device)
+    t = _IDENTITY.get(key)
+    if n_blocks > _IDENTITY_ENTRIES or (t is None and torch.cuda.is_current_stream_capturing()):
+        return identity_block_table(n_blocks, device)
+    if t is None:
+        t = identity_block_table(_IDENTITY_ENTRIES, device)
+        torch.cuda.current_stream(t.device).synchronize()
+        t = _IDENTITY.setdefault(key, t)
+    return t
 
 
 def blocks_for(n_tokens: int) -> int:

@@ -14,7 +14,7 @@ from .build import HOST_PATH, LIB_PATH
 TQ_BLOCK_TOKENS = 16
 TQ_MAX_CENTROIDS = 16
 TQ_F32, TQ_BF16, TQ_F16 = 0, 1, 2
-TQ_ERR_UNSUPPORTED = -4
+TQ_ERR_SHAPE, TQ_ERR_ALIGN, TQ_ERR_UNSUPPORTED = -2, -3, -4
 
 
 class TQError(RuntimeError):
@@ -32,7 +32,8 @@ class tq_consts(C.Structure):
     _fields_ = [("cfg", tq_config), ("pi", C.c_void_p), ("pi_t", C.c_void_p), ("s", C.c_void_p),
                 ("s_t", C.c_void_p), ("centroids", C.c_float * TQ_MAX_CENTROIDS),
                 ("boundaries", C.c_float * TQ_MAX_CENTROIDS), ("qjl_scale", C.c_float),
-                ("pi_limbs", C.c_void_p * 3), ("m_limbs", C.c_void_p * 2), ("s_limbs", C.c_void_p * 2)]
+                ("pi_limbs", C.c_void_p * 3), ("m_limbs", C.c_void_p * 2), ("s_limbs", C.c_void_p * 2),
+                ("rows_pi", C.c_void_p * 2), ("rows_m", C.c_void_p * 2), ("rows_s", C.c_void_p * 2)]
 
 
 class tq_layout(C.Structure):
@@ -102,6 +103,24 @@ SIGNATURES = {
                                   C.c_void_p, C.c_void_p]),
     "tq_dequant_values": (C.c_int, [C.POINTER(tq_config), C.POINTER(tq_pool), C.c_void_p, C.c_int64, C.c_void_p,
                                     C.c_void_p]),
+    "tq_cache_workspace_bytes": (C.c_int, [C.POINTER(tq_config), C.c_int32, C.c_int64, C.c_int64, C.c_int32, C.POINTER(C.c_size_t)]),
+    "tq_cache_scores": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int,
+                                  C.c_int32, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_int64, C.c_float, C.c_void_p,
+                                  C.c_void_p, C.c_size_t, C.c_void_p]),
+    "tq_cache_attend": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int,
+                                  C.c_int32, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p,
+                                  C.c_size_t, C.c_void_p]),
+    "tq_rows_quantize_values": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int64, C.c_int32, C.c_void_p,
+                                          C.c_void_p, C.c_void_p, C.c_void_p]),
+    "tq_rows_dequantize_values": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int32,
+                                            C.c_void_p, C.c_void_p]),
+    "tq_rows_quantize_keys": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_void_p,
+                                        C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p]),
+    "tq_rows_dequantize_keys": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p,
+                                          C.c_int, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]),
+    "tq_rows_scores": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int,
+                                 C.c_int32, C.c_int64, C.c_void_p, C.c_int, C.c_int32, C.c_void_p, C.c_void_p, C.c_size_t,
+                                 C.c_void_p]),
     "tq_pack_stage": (C.c_int, [C.POINTER(tq_consts), C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p,
                                 C.c_void_p]),
     "tq_workspace_init": (C.c_int, [C.c_void_p, C.c_size_t, C.c_void_p]),

@@ -663,6 +663,10 @@ int ring_tok_for(int max_ring_len, int64_t pairs, int splits) {
 
 }  // namespace
 
+int tq_prepare_queries(const tq_consts* consts, const void* query, int dt, int64_t nvec, float* out, cudaStream_t st) {
+    return launch_qprep(query, dt, nvec, consts->cfg.head_dim, consts->pi_t, consts->s_t, out, nullptr, 1, 1, 2, RingAppend{}, st);
+}
+
 extern "C" int tq_decode_workspace_bytes(const tq_config* cfg, int32_t batch, int32_t num_q_heads,
                                          int32_t num_kv_heads, int32_t max_splits, size_t* out) {
     if (!cfg || !out) return TQ_ERR_NULL;
@@ -911,8 +915,7 @@ extern "C" int tq_scores(const tq_consts* consts, const tq_pool* pool, const int
     cudaStream_t st = (cudaStream_t)stream;
     float* qprep = (float*)((uint8_t*)workspace + TQ_WS_HEADER_BYTES);
     const int64_t nvec = (int64_t)H * n_q;
-    if (launch_qprep(query, q_dtype, nvec, D, consts->pi_t, consts->s_t, qprep, nullptr, 1, 1, 2, RingAppend{}, st) != TQ_OK)
-        return TQ_ERR_CUDA;
+    if (tq_prepare_queries(consts, query, q_dtype, nvec, qprep, st) != TQ_OK) return TQ_ERR_CUDA;
 
     const TqLayout L = tq_make_layout(D, consts->cfg.key_bits, consts->cfg.value_bits);
     ScoreParams p;

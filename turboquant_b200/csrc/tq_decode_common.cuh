@@ -74,17 +74,17 @@ struct ScoreParams {
     int32_t* status;
 };
 
-// Partial logits of one token over dims [dim0, dim0 + D/2) for GP query heads.
+// Partial logits of one key over half of its dims for GP query heads; cw / sw: the key's packed codes and sign bits.
 template <int D, int MSE_BITS, int GP>
-__device__ __forceinline__ void token_half_scores(const uint8_t* rec, const TqLayout& L, int tl, int half,
-                                                  const float* __restrict__ qr, const float* __restrict__ qs,
-                                                  const float* __restrict__ cent, float qjl_scale, float (&out)[GP]) {
+__device__ __forceinline__ void half_row_scores(const uint32_t* cw, const uint32_t* sw, float norm, float rn, int half,
+                                                const float* __restrict__ qr, const float* __restrict__ qs,
+                                                const float* __restrict__ cent, float (&out)[GP]) {
     constexpr int WIDTH = MSE_BITS == 2 ? 2 : 4;
     constexpr int DIMS_PER_CW = 32 / WIDTH;       // dims per 32-bit code word
     constexpr int CW_PER_SW = 32 / DIMS_PER_CW;   // code words per 32-bit sign word
     constexpr uint32_t MASK = (1u << WIDTH) - 1u;
-    const uint32_t* cw = reinterpret_cast<const uint32_t*>(rec + L.off_kcodes + tl * L.kcode_row) + half * (D / 2) / DIMS_PER_CW;
-    const uint32_t* sw = reinterpret_cast<const uint32_t*>(rec + L.off_ksigns + tl * L.ksign_row) + half * (D / 64);
+    cw += half * (D / 2) / DIMS_PER_CW;
+    sw += half * (D / 64);
     float am[GP], aq[GP];
 #pragma unroll
     for (int g = 0; g < GP; ++g) am[g] = aq[g] = 0.f;
@@ -119,10 +119,18 @@ __device__ __forceinline__ void token_half_scores(const uint8_t* rec, const TqLa
             }
         }
     }
-    const float norm = __half2float(reinterpret_cast<const __half*>(rec + L.off_knorm)[tl]);
-    const float rn = __half2float(reinterpret_cast<const __half*>(rec + L.off_krnorm)[tl]) * qjl_scale;
 #pragma unroll
     for (int g = 0; g < GP; ++g) out[g] = norm * am[g] + rn * aq[g];
+}
+// The same for token tl of a block record.
+template <int D, int MSE_BITS, int GP>
+__device__ __forceinline__ void token_half_scores(const uint8_t* rec, const TqLayout& L, int tl, int half,
+                                                  const float* __restrict__ qr, const float* __restrict__ qs,
+                                                  const float* __restrict__ cent, float qjl_scale, float (&out)[GP]) {
+    half_row_scores<D, MSE_BITS, GP>(reinterpret_cast<const uint32_t*>(rec + L.off_kcodes + tl * L.kcode_row),
+                                     reinterpret_cast<const uint32_t*>(rec + L.off_ksigns + tl * L.ksign_row),
+                                     __half2float(reinterpret_cast<const __half*>(rec + L.off_knorm)[tl]),
+                                     __half2float(reinterpret_cast<const __half*>(rec + L.off_krnorm)[tl]) * qjl_scale, half, qr, qs, cent, out);
 }
 
 // Issue the bulk copies of one tile (up to 4 block records) into a stage.
@@ -434,3 +442,5 @@ int tq_decode_mma_launch(const DecodeParams& p, int D, int mse_bits, int val_bit
 // Tensor-core query preparation (tq_qprep_tc.cu): *handled = 0 when the call does not fit it.
 int tq_qprep_tc_launch(const tq_consts* consts, const void* q, int dt, int64_t nvec, float* out, uint32_t* frag, int G,
                        int Qh, int mse_bits, int* status, cudaStream_t st, int* handled);
+// q Pi^T and q S^T of contiguous query vectors as fp32 [n][2][D] (tq_decode.cu).
+int tq_prepare_queries(const tq_consts* consts, const void* query, int dt, int64_t nvec, float* out, cudaStream_t st);

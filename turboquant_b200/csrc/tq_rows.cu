@@ -1,0 +1,874 @@
+// The quantiser objects by themselves (quantizer.py:93-306, kv_cache.py:45-116): plain rows in, the reference's flat
+// planes out, and back.  Nothing goes through a block pool: a call is one kernel that reads its input once and writes
+// its output once.
+//
+//   keys    rows -> codes, sign bits, norms (tensor cores, head_dim 128), planes -> rows
+//   values  rows -> codes, scales, zero points, planes -> rows
+//   scores  query against key planes
+//
+// The products run on mma.sync with fp16 limbs: a number scaled away from fp16's subnormals is the sum of two fp16 numbers
+// to 2^-22, and three products of limbs, accumulated in fp32, give the fp32 product to about the rounding of its own sum
+// (three bf16 limbs would need six).  A warp owns 16 rows from load to packed output with its A operand in registers; the
+// constant operands (two limbs of 128 x 128 each) stay in shared memory, so the kernel is bound by the MMA pipe (8 cycles
+// per m16n8k16 and scheduler) and not by fp32 FMAs, which needed 3 x 16384 per row at a fifth of their peak.
+//
+// Measured (B200, 16000 rows of 128, 3-bit keys): quantise 51 us as half of a store into records plus 10 for the
+// conversion to planes -> 31 (20 without the re-examined coordinates); dequantise 80 -> 12; a whole quantise, score,
+// dequantise pass of keys and values 807 -> 109.
+#include "tq_decode_common.cuh"
+
+using namespace tqdec;
+
+namespace {
+
+// ------------------------------------------------------------------ values
+
+// One thread per group of 32 channels.  Arithmetic of kv_cache.py:64-90 with the rounding of the tensor's dtype after
+// every operation; scale and zero point pass through fp16, the form they are stored in.
+template <int DT, int VAL_BITS>
+__global__ void __launch_bounds__(256) tq_rows_quantize_values_kernel(const void* __restrict__ v, int64_t n_groups, int groups_per_row, int64_t stride_row,
+                                                                      uint8_t* __restrict__ data, void* __restrict__ scales, void* __restrict__ zeros) {
+    using E = TqElem<DT>;
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n_groups) return;
+    const int64_t row = i / groups_per_row;
+    const int grp = (int)(i % groups_per_row);
+    const int64_t at = row * stride_row + grp * 32;
+    float x[32];
+    if (DT == TQ_F32) {
+        const float4* src = reinterpret_cast<const float4*>((const float*)v + at);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 q = src[j];
+            x[4 * j] = q.x;
+            x[4 * j + 1] = q.y;
+            x[4 * j + 2] = q.z;
+            x[4 * j + 3] = q.w;
+        }
+    } else {
+        const uint4* src = reinterpret_cast<const uint4*>((const uint16_t*)v + at);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint4 q = src[j];
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (DT == TQ_BF16) {
+                    x[8 * j + 2 * k] = __uint_as_float(w[k] << 16);
+                    x[8 * j + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+                } else {
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+                    x[8 * j + 2 * k] = f.x;
+                    x[8 * j + 2 * k + 1] = f.y;
+                }
+            }
+        }
+    }
+    float vmin = x[0], vmax = x[0];
+#pragma unroll
+    for (int j = 1; j < 32; ++j) {
+        vmin = fminf(vmin, x[j]);
+        vmax = fmaxf(vmax, x[j]);
+    }
+    constexpr float LEVELS = (float)((1 << VAL_BITS) - 1);
+    float scale = E::round(__fdiv_rn(E::round(vmax - vmin), LEVELS));
+    scale = fmaxf(scale, E::round(1e-10f));
+    constexpr int PER_WORD = 32 / VAL_BITS, WORDS = VAL_BITS;
+    uint32_t out[WORDS];
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        out[w] = 0;
+#pragma unroll
+        for (int j = 0; j < PER_WORD; ++j) {
+            const float r = rintf(E::round(__fdiv_rn(E::round(x[w * PER_WORD + j] - vmin), scale)));
+            out[w] |= (uint32_t)fminf(fmaxf(r, 0.f), LEVELS) << (VAL_BITS * j);
+        }
+    }
+    if (WORDS == 2) *reinterpret_cast<uint2*>(data + i * 8) = make_uint2(out[0], out[1]);
+    else *reinterpret_cast<uint4*>(data + i * 16) = make_uint4(out[0], out[1], out[WORDS - 2], out[WORDS - 1]);
+    E::store(scales, i, __half2float(__float2half_rn(scale)));
+    E::store(zeros, i, __half2float(__float2half_rn(vmin)));
+}
+
+// code * scale + zero in fp32 (kv_cache.py:101-116); one thread per 32-bit word of codes
+template <int VAL_BITS>
+__global__ void __launch_bounds__(256) tq_rows_dequantize_values_kernel(const uint8_t* __restrict__ data, const void* __restrict__ scales,
+                                                                        const void* __restrict__ zeros, int sdt, int64_t n_words, float* __restrict__ out) {
+    constexpr int PER_WORD = 32 / VAL_BITS, WORDS_PER_GROUP = 32 / PER_WORD;
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n_words) return;
+    const uint32_t w = reinterpret_cast<const uint32_t*>(data)[i];
+    const float sc = __half2float(__float2half_rn(tq_load_any(scales, i / WORDS_PER_GROUP, sdt)));
+    const float zr = __half2float(__float2half_rn(tq_load_any(zeros, i / WORDS_PER_GROUP, sdt)));
+    float4* dst = reinterpret_cast<float4*>(out + i * PER_WORD);
+#pragma unroll
+    for (int j = 0; j < PER_WORD / 4; ++j) {
+        float v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = (float)((w >> (VAL_BITS * (4 * j + k))) & ((1u << VAL_BITS) - 1u)) * sc + zr;
+        dst[j] = make_float4(v[0], v[1], v[2], v[3]);
+    }
+}
+
+// ------------------------------------------------------------------ keys, head_dim 128
+
+constexpr int RD = 128, R_WARPS = 8, R_ROWS = 16 * R_WARPS;
+constexpr int R_MAT = RD * RD * 2;                 // one limb of a constant operand in shared memory
+constexpr int KSTEPS = RD / 16;
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <bool TRANS>
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+    if (TRANS)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ uint32_t pack_h(float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// a pair of fp32 numbers as LIMBS packed fp16 pairs
+template <int LIMBS>
+__device__ __forceinline__ void split(float x, float y, uint32_t* l, int step) {
+#pragma unroll
+    for (int i = 0; i < LIMBS; ++i) {
+        const __half2 v = __floats2half2_rn(x, y);
+        l[i * step] = *reinterpret_cast<const uint32_t*>(&v);
+        const float2 f = __half22float2(v);
+        x -= f.x;
+        y -= f.y;
+    }
+}
+
+// (128 x 128) fp16, row-major in global memory -> shared memory, 16-byte chunks of a row swizzled by row % 8
+__device__ __forceinline__ void load_operand(uint8_t* dst, const void* src, int tid, int nt) {
+    for (int i = tid; i < RD * RD / 8; i += nt) {
+        const int row = i >> 4, ch = i & 15;
+        const uint32_t d = tq_smem_u32(dst + row * 256 + ((ch ^ (row & 7)) << 4));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(static_cast<const uint4*>(src) + i) : "memory");
+    }
+}
+// B fragments of columns n0..n0+15, k-step ks: {n8 block 0: b0, b1, block 1: b0, b1}.
+// Rows of the stored matrix are n (TRANS = false) or k (TRANS = true).
+template <bool TRANS>
+__device__ __forceinline__ void b_frag(uint32_t mat, int n0, int ks, int lane, uint32_t (&r)[4]) {
+    // lane l addresses row l % 8 of block l / 8; blocks in the order (n8 0, k8 0), (n8 0, k8 1), (n8 1, k8 0), (n8 1, k8 1)
+    const int blk = lane >> 3, i = lane & 7;
+    const int row = TRANS ? ks * 16 + 8 * (blk & 1) + i : n0 + 8 * (blk >> 1) + i;
+    const int ch = TRANS ? (n0 >> 3) + (blk >> 1) : 2 * ks + (blk & 1);
+    ldsm4<TRANS>(mat + row * 256 + ((ch ^ (row & 7)) << 4), r);
+}
+// acc[2][4] += A (LA limbs in registers) * B (two limbs), without lo * lo
+template <int LA, bool TRANS>
+__device__ __forceinline__ void product(float (&acc)[2][4], const uint32_t (*a)[KSTEPS][4], uint32_t mats, int n0, int lane) {
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks) {
+#pragma unroll
+        for (int lb = 0; lb < 2; ++lb) {
+            uint32_t b[4];
+            b_frag<TRANS>(mats + lb * R_MAT, n0, ks, lane, b);
+#pragma unroll
+            for (int la = 0; la < LA; ++la)
+                if (la + lb < 2) {
+                    mma_f16(acc[0], a[la][ks], b[0], b[1]);
+                    mma_f16(acc[1], a[la][ks], b[2], b[3]);
+                }
+        }
+    }
+}
+
+constexpr float R_SCALE = 64.f;   // of every A operand and of Pi: unit vectors, centroids and residuals are far below 1
+
+struct RowsParams {
+    const void* x;
+    int64_t n, stride_row;
+    const void *pi[2], *other[2];   // limbs of 64 Pi and of M = S Pi^T (quantise) or S (dequantise), (128, 128) row-major
+    const float* pi_t;
+    TqCodebook cb;
+    uint8_t* codes;
+    uint8_t* signs;
+    void* norms;
+    void* rnorms;
+    int norm_dt, rnorm_dt;
+    float qjl_scale;
+    int with_qjl;
+    float* out;
+};
+
+template <int DT>
+__device__ __forceinline__ void load2(const void* p, int64_t i, float& a, float& b) {
+    if (DT == TQ_F32) {
+        const float2 v = *reinterpret_cast<const float2*>((const float*)p + i);
+        a = v.x;
+        b = v.y;
+    } else {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>((const __half*)p + i));
+        a = f.x;
+        b = f.y;
+    }
+}
+template <int DT>
+__device__ __forceinline__ void load4(const void* p, int64_t i, float* x) {
+    load2<DT>(p, i, x[0], x[1]);
+    load2<DT>(p, i + 2, x[2], x[3]);
+}
+
+// The limb products and the fp32 store kernel's chain of fused multiply-adds agree to a few 1e-7 (|u| = 1, rows of Pi have
+// norm 1).  A coordinate that lies closer than this to a decision boundary - some 20 in a million - is computed again as
+// that chain, so that the codes are the fp32 kernel's on both sides of a tie.
+constexpr float NEAR = 1e-6f;
+// Both functions below are off the usual path and run from a cold instruction cache, where a line of eight instructions
+// costs more than the arithmetic in it: loops stay rolled (an unrolled row took 41 us, this form a few).
+// One coordinate by the whole warp: lane l holds the terms l, 32 + l, ...; every lane returns the sum.
+template <int DT>
+__device__ __noinline__ float serial_product(const void* x, int64_t at, float den, const float* pi_t_col, int lane) {
+    using E = TqElem<DT>;
+    float u[RD / 32], w[RD / 32], y = 0.f;
+#pragma unroll
+    for (int i = 0; i < RD / 32; ++i) w[i] = __ldg(pi_t_col + (32 * i + lane) * RD);
+#pragma unroll
+    for (int i = 0; i < RD / 32; ++i) u[i] = E::round(__fdiv_rn(E::load(x, at + 32 * i + lane), den));
+#pragma unroll
+    for (int i = 0; i < RD / 32; ++i)
+#pragma unroll 4
+        for (int l = 0; l < 32; ++l) y = fmaf(__shfl_sync(0xffffffffu, u[i], l), __shfl_sync(0xffffffffu, w[i], l), y);
+    return y;
+}
+// A whole row by that chain, one warp, four coordinates a lane: for the row (one in some 30 000) where it decides
+// differently.  Overwrites the row's codes, sign bits and residual norm.
+template <int DT, int MSE_BITS>
+__device__ __noinline__ void redo_row(const RowsParams& p, int64_t row, float nd, float den, uint32_t sm, int lane) {
+    using E = TqElem<DT>;
+    float u[4], d[4], y[4] = {}, e[4] = {}, r[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float q = __fdiv_rn(E::load(p.x, row * p.stride_row + 4 * lane + c), den);
+        u[c] = E::round(q);
+        d[c] = q - u[c];
+    }
+#pragma unroll 1
+    for (int l = 0; l < 32; l += 2) {
+        float4 w[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w[k] = __ldg(reinterpret_cast<const float4*>(p.pi_t + (4 * l + k) * RD) + lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float uk = __shfl_sync(0xffffffffu, u[k & 3], l + (k >> 2));
+            y[0] = fmaf(uk, w[k].x, y[0]); y[1] = fmaf(uk, w[k].y, y[1]); y[2] = fmaf(uk, w[k].z, y[2]); y[3] = fmaf(uk, w[k].w, y[3]);
+            if (DT != TQ_F32) {
+                const float dk = __shfl_sync(0xffffffffu, d[k & 3], l + (k >> 2));
+                e[0] = fmaf(dk, w[k].x, e[0]); e[1] = fmaf(dk, w[k].y, e[1]); e[2] = fmaf(dk, w[k].z, e[2]); e[3] = fmaf(dk, w[k].w, e[3]);
+            }
+        }
+    }
+    uint32_t packed = 0;
+    float n2 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        uint32_t k = 0;
+        float cv = p.cb.centroids[0];
+#pragma unroll
+        for (int i = 0; i < (1 << MSE_BITS) - 1; ++i)
+            if (p.cb.boundaries[i] < y[c]) {
+                k = i + 1;
+                cv = p.cb.centroids[i + 1];
+            }
+        packed |= k << ((MSE_BITS == 2 ? 2 : 4) * c);
+        r[c] = (y[c] - cv) + e[c];
+        n2 = fmaf(r[c], r[c], n2);
+    }
+    if (MSE_BITS == 2) p.codes[row * (RD / 4) + lane] = (uint8_t)packed;
+    else reinterpret_cast<uint16_t*>(p.codes + row * (RD / 2))[lane] = (uint16_t)packed;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    float pr[4] = {};
+#pragma unroll 1
+    for (int l = 0; l < 32; ++l) {   // columns 4 l .. 4 l + 3 of rows lane + 32 i of M
+        const float rk[4] = {__shfl_sync(0xffffffffu, r[0], l), __shfl_sync(0xffffffffu, r[1], l), __shfl_sync(0xffffffffu, r[2], l),
+                             __shfl_sync(0xffffffffu, r[3], l)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row_m = lane + 32 * i;
+            const uint32_t a = sm + row_m * 256 + (((l >> 1) ^ (row_m & 7)) << 4) + (l & 1) * 8;
+            uint32_t h[2], t[2];
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(h[0]), "=r"(h[1]) : "r"(a));
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(t[0]), "=r"(t[1]) : "r"(a + R_MAT));
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[k])), g = __half22float2(*reinterpret_cast<const __half2*>(&t[k]));
+                pr[i] = fmaf(rk[2 * k], f.x + g.x, pr[i]);
+                pr[i] = fmaf(rk[2 * k + 1], f.y + g.y, pr[i]);
+            }
+        }
+    }
+    uint32_t s[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) s[i] = __ballot_sync(0xffffffffu, pr[i] > 0.f);
+    if (lane == 0) {
+        *reinterpret_cast<uint4*>(p.signs + row * (RD / 8)) = make_uint4(s[0], s[1], s[2], s[3]);
+        tq_store_any(p.rnorms, row, __half2float(__float2half_rn(nd * __fsqrt_rn(n2))), p.rnorm_dt);
+    }
+}
+
+// quantizer.py:129-149,231-257 for 16 rows per warp: norm, x / |x| (rounded to the dtype like torch), Y = u Pi^T, bucket
+// search, residual in rotated space r' = (Y - c) + E, E = (x / |x| - u) Pi^T, sign bits of r' M^T with M = S Pi^T.
+template <int DT, int MSE_BITS>
+__global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(const __grid_constant__ RowsParams p) {
+    using E = TqElem<DT>;
+    constexpr int LU = DT == TQ_F32 ? 2 : 1;   // limbs that hold u
+    constexpr int NB = (1 << MSE_BITS) - 1;
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_WARPS * 32);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) load_operand(smem + (2 + i) * R_MAT, p.other[i], tid, R_WARPS * 32);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const uint32_t sp = tq_smem_u32(smem), sm = sp + 2 * R_MAT;
+    bool first = true;
+#pragma unroll 1
+    for (int64_t tile = blockIdx.x; tile * R_ROWS < p.n; tile += gridDim.x) {
+        const int64_t r0 = tile * R_ROWS + warp * 16 + gid, r1 = r0 + 8;
+        uint32_t a[LU][KSTEPS][4], e[DT == TQ_F32 ? 1 : KSTEPS][4];
+        float nd[2], den[2];
+        {   // norms of the warp's 16 rows, in the fp32 store kernel's order: eight sums of 16 squares, added up in order.
+            // Lane = (row % 4, sum), four rows a lane.
+            const int ch = lane & 7;
+            float own[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int64_t row = tile * R_ROWS + warp * 16 + 4 * i + (lane >> 3);
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; j += 4)
+                    if (row < p.n) load4<DT>(p.x, row * p.stride_row + ch * 16 + j, v + j);
+                    else v[j] = v[j + 1] = v[j + 2] = v[j + 3] = 0.f;
+                float s = 0.f;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) s = fmaf(v[j], v[j], s);
+                float tot = 0.f;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) tot += __shfl_sync(0xffffffffu, s, (lane & 24) + c);
+                own[i] = tot;
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {   // rows gid, gid + 8: slot (row / 4), lanes 8 * (row % 4)
+                const float lo = __shfl_sync(0xffffffffu, own[2 * r], 8 * (gid & 3)), hi = __shfl_sync(0xffffffffu, own[2 * r + 1], 8 * (gid & 3));
+                nd[r] = E::round(__fsqrt_rn(gid < 4 ? lo : hi));
+                den[r] = E::round(nd[r] + 1e-10f);
+            }
+        }
+#pragma unroll
+        for (int ks = 0; ks < KSTEPS; ++ks)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int64_t row = r ? r1 : r0, at = row * p.stride_row + ks * 16 + hf * 8 + 2 * tig;
+                    float v0 = 0.f, v1 = 0.f;
+                    if (row < p.n) load2<DT>(p.x, at, v0, v1);
+                    const float q0 = __fdiv_rn(v0, den[r]), q1 = __fdiv_rn(v1, den[r]);
+                    const float u0 = E::round(q0), u1 = E::round(q1);
+                    split<LU>(u0 * R_SCALE, u1 * R_SCALE, &a[0][ks][hf * 2 + r], KSTEPS * 4);
+                    if (DT != TQ_F32) e[DT == TQ_F32 ? 0 : ks][hf * 2 + r] = pack_h((q0 - u0) * R_SCALE, (q1 - u1) * R_SCALE);
+                }
+        if (first) {
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+        }
+        // ---- codes, r' as limbs in the A layout of the second product ----
+        uint32_t rl[2][KSTEPS][4];
+        uint32_t cw[2][MSE_BITS == 2 ? 2 : 4];    // code words of the two rows, word j in lane j % 4
+        float rn2[2] = {0.f, 0.f};
+        uint32_t near_lo = 0, near_hi = 0;        // coordinates next to a boundary, bit 8 * nb + 4 * n8 + c
+#pragma unroll
+        for (int nb = 0; nb < RD / 16; ++nb) {
+            float acc[2][4] = {};
+            product<LU, false>(acc, a, sp, nb * 16, lane);
+            float er[2][4] = {};
+            if (DT != TQ_F32) {
+#pragma unroll
+                for (int ks = 0; ks < KSTEPS; ++ks) {   // |q - u| <= 2^-12: Pi's first limb is enough
+                    uint32_t b[4];
+                    b_frag<false>(sp, nb * 16, ks, lane, b);
+                    mma_f16(er[0], e[DT == TQ_F32 ? 0 : ks], b[0], b[1]);
+                    mma_f16(er[1], e[DT == TQ_F32 ? 0 : ks], b[2], b[3]);
+                }
+            }
+            uint32_t half[2];   // 2-bit codes: the word's first 16 bits
+#pragma unroll
+            for (int n8 = 0; n8 < 2; ++n8) {
+                uint32_t code[4];
+                float r[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float y = acc[n8][c] * (1.f / (R_SCALE * R_SCALE));
+                    const uint32_t bit = 1u << ((nb & 3) * 8 + n8 * 4 + c);
+                    uint32_t k = 0;
+                    float cv = p.cb.centroids[0], gap = 1.f;
+#pragma unroll
+                    for (int i = 0; i < NB; ++i) {
+                        const float d = y - p.cb.boundaries[i];
+                        gap = fminf(gap, fabsf(d));
+                        if (d > 0.f) {
+                            k = i + 1;
+                            cv = p.cb.centroids[i + 1];
+                        }
+                    }
+                    if (gap < NEAR) (nb < 4 ? near_lo : near_hi) |= bit;
+                    if (y != y) {   // searchsorted orders NaN after every number
+                        k = NB;
+                        cv = p.cb.centroids[NB];
+                    }
+                    code[c] = k;
+                    r[c] = fmaf(er[n8][c], 1.f / (R_SCALE * R_SCALE), y - cv);
+                    rn2[c >> 1] = fmaf(r[c], r[c], rn2[c >> 1]);
+                }
+                split<2>(r[0] * R_SCALE, r[1] * R_SCALE, &rl[0][nb][n8 * 2], KSTEPS * 4);       // row r0
+                split<2>(r[2] * R_SCALE, r[3] * R_SCALE, &rl[0][nb][n8 * 2 + 1], KSTEPS * 4);   // row r1
+#pragma unroll
+                for (int r2 = 0; r2 < 2; ++r2) {
+                    uint32_t w = MSE_BITS == 2 ? (code[2 * r2] | (code[2 * r2 + 1] << 2)) << (4 * tig) : (code[2 * r2] | (code[2 * r2 + 1] << 4)) << (8 * tig);
+                    w |= __shfl_xor_sync(0xffffffffu, w, 1);
+                    w |= __shfl_xor_sync(0xffffffffu, w, 2);
+                    if (MSE_BITS == 2) {
+                        if (n8) w = half[r2] | (w << 16);
+                        else half[r2] = w;
+                    }
+                    const int j = MSE_BITS == 2 ? nb : nb * 2 + n8;
+                    if (tig == (j & 3)) cw[r2][j >> 2] = w;
+                }
+            }
+        }
+        if (first) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            first = false;
+        }
+        // ---- sign bits of r' M^T ----
+        uint32_t sw[2][4] = {};
+#pragma unroll
+        for (int nb = 0; nb < RD / 16; ++nb) {
+            float acc[2][4] = {};
+            product<2, false>(acc, rl, sm, nb * 16, lane);
+#pragma unroll
+            for (int n8 = 0; n8 < 2; ++n8)
+#pragma unroll
+                for (int r2 = 0; r2 < 2; ++r2) {
+                    uint32_t w = ((acc[n8][2 * r2] > 0.f ? 1u : 0u) | (acc[n8][2 * r2 + 1] > 0.f ? 2u : 0u)) << (2 * tig);
+                    sw[r2][nb >> 1] |= w << (8 * (2 * (nb & 1) + n8));
+                }
+        }
+        // ---- out ----
+#pragma unroll
+        for (int r2 = 0; r2 < 2; ++r2) {
+            const int64_t row = r2 ? r1 : r0;
+            float n2 = rn2[r2];
+            n2 += __shfl_xor_sync(0xffffffffu, n2, 1);
+            n2 += __shfl_xor_sync(0xffffffffu, n2, 2);
+            uint32_t s[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t w = sw[r2][i];
+                w |= __shfl_xor_sync(0xffffffffu, w, 1);
+                w |= __shfl_xor_sync(0xffffffffu, w, 2);
+                s[i] = nd[r2] == 0.f ? 0u : w;   // a zero key has a zero residual
+            }
+            if (row >= p.n) continue;
+            constexpr int CB = MSE_BITS == 2 ? RD / 4 : RD / 2;
+            if (tig == 0) *reinterpret_cast<uint4*>(p.signs + row * (RD / 8)) = make_uint4(s[0], s[1], s[2], s[3]);
+#pragma unroll
+            for (int q = 0; q < CB / 16; ++q) *reinterpret_cast<uint32_t*>(p.codes + row * CB + 16 * q + 4 * tig) = cw[r2][q];
+            if (tig == 3) {
+                tq_store_any(p.norms, row, __half2float(__float2half_rn(nd[r2])), p.norm_dt);
+                tq_store_any(p.rnorms, row, nd[r2] == 0.f ? 0.f : __half2float(__float2half_rn(nd[r2] * __fsqrt_rn(n2))), p.rnorm_dt);
+            }
+        }
+        // ---- coordinates next to a boundary, by the fp32 store kernel's chain; a row where it decides differently is redone ----
+        if (r0 >= p.n || nd[0] == 0.f) { near_lo &= 0xccccccccu; near_hi &= 0xccccccccu; }
+        if (r1 >= p.n || nd[1] == 0.f) { near_lo &= 0x33333333u; near_hi &= 0x33333333u; }
+        if (__any_sync(0xffffffffu, (near_lo | near_hi) != 0)) {
+            __syncwarp();   // the warp's codes, read back below
+            uint32_t redo = 0;   // rows of the warp's sixteen
+#pragma unroll 1
+            for (uint32_t who; (who = __ballot_sync(0xffffffffu, (near_lo | near_hi) != 0)) != 0;) {
+                const int from = __ffs(who) - 1;   // this lane's next coordinate, for the whole warp
+                const bool upper = near_lo == 0;
+                const uint32_t m = upper ? near_hi : near_lo, one = m & (0u - m);
+                const int bit = __shfl_sync(0xffffffffu, __ffs(m) - 1 + (upper ? 32 : 0), from);
+                if (lane == from) (upper ? near_hi : near_lo) ^= one;
+                const int col = (bit >> 2) * 8 + 2 * (from & 3) + (bit & 1), rw = (from >> 2) + (bit & 2 ? 8 : 0);
+                const int64_t row = tile * R_ROWS + warp * 16 + rw;
+                const float y = serial_product<DT>(p.x, row * p.stride_row, __shfl_sync(0xffffffffu, bit & 2 ? den[1] : den[0], from), p.pi_t + col, lane);
+                int k = 0;
+#pragma unroll
+                for (int i = 0; i < NB; ++i) k += p.cb.boundaries[i] < y ? 1 : 0;
+                constexpr int PER = MSE_BITS == 2 ? 4 : 2, W = 8 / PER;
+                const int had = (*(volatile const uint8_t*)(p.codes + row * (RD / PER) + col / PER) >> (W * (col % PER))) & ((1 << W) - 1);
+                if (k != had) redo |= 1u << rw;
+            }
+#pragma unroll 1
+            for (; redo != 0; redo &= redo - 1) {
+                const int rw = __ffs(redo) - 1, from = 4 * (rw & 7);
+                redo_row<DT, MSE_BITS>(p, tile * R_ROWS + warp * 16 + rw, __shfl_sync(0xffffffffu, rw & 8 ? nd[1] : nd[0], from),
+                                       __shfl_sync(0xffffffffu, rw & 8 ? den[1] : den[0], from), sm, lane);
+            }
+        }
+    }
+}
+
+// quantizer.py:151-165,259-272 for 16 rows per warp: (c[idx] Pi) * norm + qjl_scale * rnorm * (signs S)
+template <int MSE_BITS>
+__global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_dequantize_keys_kernel(const RowsParams p) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_WARPS * 32);
+    if (p.with_qjl)
+#pragma unroll 1
+        for (int i = 0; i < 2; ++i) load_operand(smem + (2 + i) * R_MAT, p.other[i], tid, R_WARPS * 32);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const uint32_t sp = tq_smem_u32(smem), ssg = sp + 2 * R_MAT;
+    float* cen = reinterpret_cast<float*>(smem + 4 * R_MAT);
+    if (tid < (1 << MSE_BITS)) cen[tid] = p.cb.centroids[tid];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    constexpr int CB = MSE_BITS == 2 ? RD / 4 : RD / 2;
+#pragma unroll 1
+    for (int64_t tile = blockIdx.x; tile * R_ROWS < p.n; tile += gridDim.x) {
+        const int64_t rows[2] = {tile * R_ROWS + warp * 16 + gid, tile * R_ROWS + warp * 16 + gid + 8};
+        uint32_t a[2][KSTEPS][4], sg[1][KSTEPS][4];
+        float norm[2], rn[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const bool live = rows[r] < p.n;
+            norm[r] = live ? 1.f / (R_SCALE * R_SCALE) * __half2float(__float2half_rn(tq_load_any(p.norms, rows[r], p.norm_dt))) : 0.f;
+            rn[r] = live && p.with_qjl ? p.qjl_scale * __half2float(__float2half_rn(tq_load_any(p.rnorms, rows[r], p.rnorm_dt))) : 0.f;
+#pragma unroll
+            for (int ks = 0; ks < KSTEPS; ++ks) {
+                uint32_t cbits = 0, sbits = 0;   // 16 coordinates of the k-step: 2-bit codes in one word, nibbles in two
+                uint32_t cbits2 = 0;
+                if (live) {
+                    if (MSE_BITS == 2) {
+                        cbits = reinterpret_cast<const uint32_t*>(p.codes + rows[r] * CB)[ks];
+                    } else {
+                        const uint2 v = reinterpret_cast<const uint2*>(p.codes + rows[r] * CB)[ks];
+                        cbits = v.x;
+                        cbits2 = v.y;
+                    }
+                    if (p.with_qjl) sbits = reinterpret_cast<const uint16_t*>(p.signs + rows[r] * (RD / 8))[ks];
+                }
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int k = hf * 8 + 2 * tig;
+                    float c0, c1;
+                    if (MSE_BITS == 2) {
+                        c0 = cen[(cbits >> (2 * k)) & 3u];
+                        c1 = cen[(cbits >> (2 * k + 2)) & 3u];
+                    } else {
+                        const uint32_t w = hf ? cbits2 : cbits;
+                        c0 = cen[(w >> (8 * tig)) & 7u];
+                        c1 = cen[(w >> (8 * tig + 4)) & 7u];
+                    }
+                    split<2>(c0 * R_SCALE, c1 * R_SCALE, &a[0][ks][hf * 2 + r], KSTEPS * 4);
+                    const uint32_t b = (sbits >> k) & 3u;   // +1 / -1
+                    sg[0][ks][hf * 2 + r] = ((b & 1u) ? 0x3c00u : 0xbc00u) | ((b & 2u) ? 0x3c000000u : 0xbc000000u);
+                }
+            }
+        }
+#pragma unroll 1
+        for (int nb = 0; nb < RD / 16; ++nb) {
+            float ak[2][4] = {}, as[2][4] = {};
+            product<2, true>(ak, a, sp, nb * 16, lane);
+            if (p.with_qjl) product<1, true>(as, sg, ssg, nb * 16, lane);
+#pragma unroll
+            for (int n8 = 0; n8 < 2; ++n8)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+                    if (rows[r] < p.n)
+                        *reinterpret_cast<float2*>(p.out + rows[r] * RD + nb * 16 + n8 * 8 + 2 * tig) =
+                            make_float2(ak[n8][2 * r] * norm[r] + as[n8][2 * r] * rn[r], ak[n8][2 * r + 1] * norm[r] + as[n8][2 * r + 1] * rn[r]);
+        }
+    }
+}
+
+// The same on CUDA cores for head_dim 256: one CTA of 256 threads (a column each) takes 16 rows.
+__global__ void __launch_bounds__(256) tq_rows_dequantize_keys256_kernel(const RowsParams p, const float* __restrict__ pi, const float* __restrict__ s, int mse_bits) {
+    constexpr int D = 256;
+    __shared__ __align__(16) float yh[D][20], sg[D][20];   // [coordinate][16 rows], padded
+    const int j = threadIdx.x;
+    const int64_t row0 = (int64_t)blockIdx.x * 16;
+    const int width = mse_bits == 2 ? 2 : 4, vpb = 8 / width, cb = D / vpb;
+    for (int t = 0; t < 16; ++t) {
+        float c = 0.f, q = 0.f;
+        if (row0 + t < p.n) {
+            const uint8_t byte = p.codes[(row0 + t) * cb + j / vpb];
+            c = p.cb.centroids[(byte >> ((j % vpb) * width)) & ((1 << width) - 1)];
+            if (p.with_qjl) q = ((p.signs[(row0 + t) * (D / 8) + (j >> 3)] >> (j & 7)) & 1) ? 1.f : -1.f;
+        }
+        yh[j][t] = c;
+        sg[j][t] = q;
+    }
+    __syncthreads();
+    float am[16], aq[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) am[t] = aq[t] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < D; ++k) {
+        const float pv = __ldg(pi + (size_t)k * D + j), sv = p.with_qjl ? __ldg(s + (size_t)k * D + j) : 0.f;
+#pragma unroll
+        for (int t = 0; t < 16; t += 4) {
+            const float4 y = *reinterpret_cast<const float4*>(&yh[k][t]), g = *reinterpret_cast<const float4*>(&sg[k][t]);
+            am[t] = fmaf(y.x, pv, am[t]);
+            am[t + 1] = fmaf(y.y, pv, am[t + 1]);
+            am[t + 2] = fmaf(y.z, pv, am[t + 2]);
+            am[t + 3] = fmaf(y.w, pv, am[t + 3]);
+            aq[t] = fmaf(g.x, sv, aq[t]);
+            aq[t + 1] = fmaf(g.y, sv, aq[t + 1]);
+            aq[t + 2] = fmaf(g.z, sv, aq[t + 2]);
+            aq[t + 3] = fmaf(g.w, sv, aq[t + 3]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        const int64_t r = row0 + t;
+        if (r >= p.n) break;
+        float v = am[t] * __half2float(__float2half_rn(tq_load_any(p.norms, r, p.norm_dt)));
+        if (p.with_qjl) v += aq[t] * (p.qjl_scale * __half2float(__float2half_rn(tq_load_any(p.rnorms, r, p.rnorm_dt))));
+        p.out[r * D + j] = v;
+    }
+}
+
+// ------------------------------------------------------------------ scores of key planes
+
+// Unscaled logits of 64 tokens of one head (two threads per token) for up to eight queries; the queries are prepared (qprep).
+template <int D, int MSE_BITS>
+__global__ void __launch_bounds__(128) tq_rows_scores_kernel(const RowsParams p, const float* __restrict__ qprep, int64_t n_k, int n_q, float* __restrict__ logits) {
+    constexpr int GP = 8;
+    __shared__ __align__(16) float qr[D * GP], qs[D * GP], sp[2 * GP * 64], cent[TQ_MAX_CENTROIDS];
+    const int tid = threadIdx.x, h = blockIdx.y, q0 = blockIdx.z * GP, nq = min(GP, n_q - q0);
+    if (tid < TQ_MAX_CENTROIDS) cent[tid] = p.cb.centroids[tid];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int i = tid; i < D * GP; i += 128) {
+        const int j = i / GP, g = i % GP;
+        const float* src = qprep + ((int64_t)(h * n_q + q0 + g) * 2) * D;
+        qr[i] = g < nq ? src[j] : 0.f;
+        qs[i] = g < nq ? src[D + j] : 0.f;
+    }
+    __syncthreads();
+    const int tk = tid & 63, half = tid >> 6;
+    const int64_t t = (int64_t)blockIdx.x * 64 + tk, row = (int64_t)h * n_k + t;
+    float part[GP];
+#pragma unroll
+    for (int g = 0; g < GP; ++g) part[g] = 0.f;
+    if (t < n_k) {
+        constexpr int CB = MSE_BITS == 2 ? D / 4 : D / 2;
+        const float norm = __half2float(__float2half_rn(tq_load_any(p.norms, row, p.norm_dt)));
+        const float rn = __half2float(__float2half_rn(tq_load_any(p.rnorms, row, p.rnorm_dt))) * p.qjl_scale;
+        half_row_scores<D, MSE_BITS, GP>(reinterpret_cast<const uint32_t*>(p.codes + row * CB), reinterpret_cast<const uint32_t*>(p.signs + row * (D / 8)),
+                                         norm, rn, half, qr, qs, cent, part);
+    }
+#pragma unroll
+    for (int g = 0; g < GP; ++g) sp[(half * GP + g) * 64 + tk] = part[g];
+    __syncthreads();
+    for (int i = tid; i < nq * 64; i += 128) {
+        const int g = i / 64, tt = i % 64;
+        const int64_t at = (int64_t)blockIdx.x * 64 + tt;
+        if (at < n_k) logits[((int64_t)h * n_q + q0 + g) * n_k + at] = sp[g * 64 + tt] + sp[(GP + g) * 64 + tt];
+    }
+}
+
+bool aligned(const void* p, size_t n) { return ((uintptr_t)p & (n - 1)) == 0; }
+
+int fill(RowsParams& p, const tq_consts* c, bool quantise) {
+    for (int i = 0; i < 2; ++i) {
+        p.pi[i] = c->rows_pi[i];
+        p.other[i] = quantise ? c->rows_m[i] : c->rows_s[i];
+        if (c->cfg.head_dim == RD && (!p.pi[i] || !p.other[i] || !aligned(p.pi[i], 16) || !aligned(p.other[i], 16))) return TQ_ERR_UNSUPPORTED;
+    }
+    for (int i = 0; i < TQ_MAX_CENTROIDS; ++i) {
+        p.cb.centroids[i] = c->centroids[i];
+        p.cb.boundaries[i] = c->boundaries[i];
+    }
+    p.qjl_scale = c->qjl_scale;
+    p.pi_t = c->pi_t;
+    return TQ_OK;
+}
+
+unsigned rows_grid(int64_t n) {
+    const int64_t tiles = (n + R_ROWS - 1) / R_ROWS;
+    return (unsigned)(tiles < tq_sm_count() ? tiles : tq_sm_count());
+}
+
+}  // namespace
+
+extern "C" int tq_rows_quantize_values(const void* v, tq_dtype dtype, int64_t n_rows, int32_t head_dim, int64_t stride_row, int32_t bits,
+                                       uint8_t* data, void* scales, void* zeros, void* stream) {
+    if (!v || !data || !scales || !zeros) return TQ_ERR_NULL;
+    if (n_rows < 0 || head_dim <= 0 || head_dim % 32 || stride_row < head_dim) return TQ_ERR_SHAPE;
+    if (bits != 2 && bits != 4) return TQ_ERR_UNSUPPORTED;
+    if (!aligned(v, 16) || (stride_row * (int64_t)tq_dtype_size(dtype)) % 16 || !aligned(data, 16)) return TQ_ERR_ALIGN;
+    if (n_rows == 0) return TQ_OK;
+    const int gpr = head_dim / 32;
+    const int64_t n = n_rows * gpr;
+    const unsigned grid = (unsigned)((n + 255) / 256);
+    cudaStream_t st = (cudaStream_t)stream;
+    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+#define TQ_QV(DT)                                                                                                     \
+    do {                                                                                                              \
+        if (bits == 2) tq_rows_quantize_values_kernel<DT, 2><<<grid, 256, 0, st>>>(v, n, gpr, stride_row, data, scales, zeros); \
+        else tq_rows_quantize_values_kernel<DT, 4><<<grid, 256, 0, st>>>(v, n, gpr, stride_row, data, scales, zeros);  \
+    } while (0)
+    if (dtype == TQ_F32) TQ_QV(TQ_F32);
+    else if (dtype == TQ_BF16) TQ_QV(TQ_BF16);
+    else if (dtype == TQ_F16) TQ_QV(TQ_F16);
+    else return TQ_ERR_UNSUPPORTED;
+#undef TQ_QV
+    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}
+
+extern "C" int tq_rows_dequantize_values(const uint8_t* data, const void* scales, const void* zeros, tq_dtype scale_dtype, int64_t n_rows,
+                                         int32_t head_dim, int32_t bits, float* out, void* stream) {
+    if (!data || !scales || !zeros || !out) return TQ_ERR_NULL;
+    if (n_rows < 0 || head_dim <= 0 || head_dim % 32) return TQ_ERR_SHAPE;
+    if (bits != 2 && bits != 4) return TQ_ERR_UNSUPPORTED;
+    if (!aligned(data, 4) || !aligned(out, 16)) return TQ_ERR_ALIGN;
+    if (n_rows == 0) return TQ_OK;
+    const int64_t words = n_rows * head_dim * bits / 32;
+    const unsigned grid = (unsigned)((words + 255) / 256);
+    cudaStream_t st = (cudaStream_t)stream;
+    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+    if (bits == 2) tq_rows_dequantize_values_kernel<2><<<grid, 256, 0, st>>>(data, scales, zeros, scale_dtype, words, out);
+    else tq_rows_dequantize_values_kernel<4><<<grid, 256, 0, st>>>(data, scales, zeros, scale_dtype, words, out);
+    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}
+
+extern "C" int tq_rows_quantize_keys(const tq_consts* consts, const void* x, tq_dtype dtype, int64_t n_rows, int64_t stride_row, uint8_t* codes,
+                                     uint8_t* signs, void* norms, tq_dtype norm_dtype, void* residual_norms, tq_dtype residual_dtype, void* stream) {
+    if (!consts || !x || !codes || !signs || !norms || !residual_norms) return TQ_ERR_NULL;
+    int rc = tq_check_config(&consts->cfg);
+    if (rc != TQ_OK) return rc;
+    if (consts->cfg.head_dim != RD || dtype == TQ_BF16 || !consts->pi_t) return TQ_ERR_UNSUPPORTED;
+    if (n_rows < 0 || stride_row < RD) return TQ_ERR_SHAPE;
+    if (!aligned(x, 8) || (stride_row * (int64_t)tq_dtype_size(dtype)) % 8 || !aligned(codes, 16) || !aligned(signs, 16)) return TQ_ERR_ALIGN;
+    if (n_rows == 0) return TQ_OK;
+    RowsParams p = {};
+    if ((rc = fill(p, consts, true)) != TQ_OK) return rc;
+    p.x = x;
+    p.n = n_rows;
+    p.stride_row = stride_row;
+    p.codes = codes;
+    p.signs = signs;
+    p.norms = norms;
+    p.rnorms = residual_norms;
+    p.norm_dt = norm_dtype;
+    p.rnorm_dt = residual_dtype;
+    cudaStream_t st = (cudaStream_t)stream;
+    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+    constexpr size_t smem = 4 * R_MAT;
+#define TQ_QK(DT, MB)                                                                            \
+    do {                                                                                         \
+        static TqSmemOptIn opt_in;                                                               \
+        if (tq_opt_in_smem(tq_rows_quantize_keys_kernel<DT, MB>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA; \
+        tq_rows_quantize_keys_kernel<DT, MB><<<rows_grid(n_rows), R_WARPS * 32, smem, st>>>(p);   \
+    } while (0)
+    const int mb = consts->cfg.key_bits - 1;
+    if (dtype == TQ_F32) { if (mb == 2) TQ_QK(TQ_F32, 2); else TQ_QK(TQ_F32, 3); }
+    else if (dtype == TQ_F16) { if (mb == 2) TQ_QK(TQ_F16, 2); else TQ_QK(TQ_F16, 3); }
+    else return TQ_ERR_UNSUPPORTED;
+#undef TQ_QK
+    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}
+
+extern "C" int tq_rows_dequantize_keys(const tq_consts* consts, const uint8_t* codes, const uint8_t* signs, const void* norms, tq_dtype norm_dtype,
+                                       const void* residual_norms, tq_dtype residual_dtype, int64_t n_rows, int32_t with_qjl, float* out, void* stream) {
+    if (!consts || !codes || !norms || !out || (with_qjl && (!signs || !residual_norms))) return TQ_ERR_NULL;
+    int rc = tq_check_config(&consts->cfg);
+    if (rc != TQ_OK) return rc;
+    if (!consts->pi || !consts->s) return TQ_ERR_NULL;
+    if (n_rows < 0) return TQ_ERR_SHAPE;
+    if (!aligned(codes, 8) || (signs && !aligned(signs, 4)) || !aligned(out, 8)) return TQ_ERR_ALIGN;
+    if (n_rows == 0) return TQ_OK;
+    RowsParams p = {};
+    rc = fill(p, consts, false);
+    if (rc != TQ_OK) return rc;
+    p.n = n_rows;
+    p.codes = const_cast<uint8_t*>(codes);
+    p.signs = const_cast<uint8_t*>(signs);
+    p.norms = const_cast<void*>(norms);
+    p.rnorms = const_cast<void*>(residual_norms);
+    p.norm_dt = norm_dtype;
+    p.rnorm_dt = residual_dtype;
+    p.with_qjl = with_qjl;
+    p.out = out;
+    cudaStream_t st = (cudaStream_t)stream;
+    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+    const int mb = consts->cfg.key_bits - 1;
+    if (consts->cfg.head_dim != RD) {
+        tq_rows_dequantize_keys256_kernel<<<(unsigned)((n_rows + 15) / 16), 256, 0, st>>>(p, consts->pi, consts->s, mb);
+        return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+    }
+    constexpr size_t smem = 4 * R_MAT + 16 * sizeof(float);
+    static TqSmemOptIn opt2, opt3;
+    if (mb == 2) {
+        if (tq_opt_in_smem(tq_rows_dequantize_keys_kernel<2>, smem, opt2) != TQ_OK) return TQ_ERR_CUDA;
+        tq_rows_dequantize_keys_kernel<2><<<rows_grid(n_rows), R_WARPS * 32, smem, st>>>(p);
+    } else {
+        if (tq_opt_in_smem(tq_rows_dequantize_keys_kernel<3>, smem, opt3) != TQ_OK) return TQ_ERR_CUDA;
+        tq_rows_dequantize_keys_kernel<3><<<rows_grid(n_rows), R_WARPS * 32, smem, st>>>(p);
+    }
+    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}
+
+extern "C" int tq_rows_scores(const tq_consts* consts, const uint8_t* codes, const uint8_t* signs, const void* norms, tq_dtype norm_dtype,
+                              const void* residual_norms, tq_dtype residual_dtype, int32_t n_heads, int64_t n_keys, const void* query, tq_dtype q_dtype,
+                              int32_t n_q, float* logits, void* workspace, size_t workspace_bytes, void* stream) {
+    if (!consts || !codes || !signs || !norms || !residual_norms || !query || !logits || !workspace) return TQ_ERR_NULL;
+    int rc = tq_check_config(&consts->cfg);
+    if (rc != TQ_OK) return rc;
+    if (!consts->pi_t || !consts->s_t) return TQ_ERR_NULL;
+    if (n_heads <= 0 || n_keys < 0 || n_q <= 0) return TQ_ERR_SHAPE;
+    if (n_heads > 65535 || n_q > 8 * 65535) return TQ_ERR_UNSUPPORTED;
+    if (!aligned(codes, 4) || !aligned(signs, 4) || !aligned(workspace, 256)) return TQ_ERR_ALIGN;
+    size_t need = 0;
+    tq_scores_workspace_bytes(&consts->cfg, (int64_t)n_heads * n_q, &need);
+    if (need > workspace_bytes) return TQ_ERR_WORKSPACE;
+    if (n_keys == 0) return TQ_OK;
+    RowsParams p = {};
+    for (int i = 0; i < TQ_MAX_CENTROIDS; ++i) p.cb.centroids[i] = consts->centroids[i];
+    p.qjl_scale = consts->qjl_scale;
+    p.codes = const_cast<uint8_t*>(codes);
+    p.signs = const_cast<uint8_t*>(signs);
+    p.norms = const_cast<void*>(norms);
+    p.rnorms = const_cast<void*>(residual_norms);
+    p.norm_dt = norm_dtype;
+    p.rnorm_dt = residual_dtype;
+    float* qprep = reinterpret_cast<float*>((uint8_t*)workspace + TQ_WS_HEADER_BYTES);
+    cudaStream_t st = (cudaStream_t)stream;
+    if ((rc = tq_prepare_queries(consts, query, q_dtype, (int64_t)n_heads * n_q, qprep, st)) != TQ_OK) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)((n_keys + 63) / 64), (unsigned)n_heads, (unsigned)((n_q + 7) / 8));
+    cfg.blockDim = dim3(128);
+    cfg.stream = st;
+    const int mb = consts->cfg.key_bits - 1;
+    cudaError_t e;
+    if (consts->cfg.head_dim == 128)
+        e = mb == 2 ? cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<128, 2>, p, (const float*)qprep, n_keys, (int)n_q, logits)
+                    : cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<128, 3>, p, (const float*)qprep, n_keys, (int)n_q, logits);
+    else
+        e = mb == 2 ? cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<256, 2>, p, (const float*)qprep, n_keys, (int)n_q, logits)
+                    : cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<256, 3>, p, (const float*)qprep, n_keys, (int)n_q, logits);
+    return e == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}

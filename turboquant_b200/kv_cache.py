@@ -29,6 +29,16 @@ def _value_consts(d: int, bits: int, device) -> E.LayerConstants:
     return _CONSTS[key]
 
 
+_VALUE_SHAPES: set[tuple] = set()
+
+
+def _check_value_shape(d: int, bits: int) -> None:
+    """The head_dim / bits combinations of the compiled set (raises otherwise)."""
+    if (d, bits) not in _VALUE_SHAPES:
+        E.get_layout(d, 3, bits)
+        _VALUE_SHAPES.add((d, bits))
+
+
 def unpack_values(vq: ValueQuantized) -> torch.Tensor:
     """One uint8 per element from the packed bytes (pure bit slicing)."""
     bits = vq.bits if len(vq) > 3 else 2
@@ -52,12 +62,17 @@ def quantize_values(v: torch.Tensor, bits: int = 2, group_size: int = 32) -> Val
         raise ValueError("only value groups of 32 are compiled")
     E.require_cuda(v, "v")
     d = v.shape[-1]
-    consts = _value_consts(d, bits, v.device)
+    _check_value_shape(d, bits)
     lead = v.shape[:-1]
     v2 = v.reshape(-1, d)
     if v2.stride(-1) != 1:
         v2 = v2.contiguous()
     n = v2.shape[0]
+    got = E.rows_quantize_values(v2, bits) if n else None
+    if got is not None:
+        data, scales, zeros = got
+        return ValueQuantized(data.reshape(*lead, -1), scales.reshape(*lead, -1), zeros.reshape(*lead, -1), bits)
+    consts = _value_consts(d, bits, v.device)
     pool = E.BlockPool(consts, 1, E.blocks_for(n))
     bt = E.identity_block_table(pool.num_blocks, v.device)
     E.store(consts, pool, v2, v2, stride_token=v2.stride(0), stride_head=0, n_tokens=n, n_heads=1,
@@ -73,6 +88,11 @@ def dequantize_values(vq: ValueQuantized, group_size: int = 32) -> torch.Tensor:
     data = vq.data
     E.require_cuda(data, "vq.data")
     d = data.shape[-1] * (4 if bits == 2 else 2)
+    _check_value_shape(d, bits)
+    if data.numel():
+        out = E.rows_dequantize_values(data.contiguous(), vq.scales.contiguous(), vq.zeros.contiguous(), bits, d)
+        if out is not None:
+            return out.reshape(*data.shape[:-1], d)
     consts = _value_consts(d, bits, data.device)
     lay = consts.layout
     n = data.shape[-2]
@@ -116,6 +136,7 @@ class TurboQuantKVCache:
         self._n_quant = 0
         self._lead: Optional[tuple] = None   # (batch, heads)
         self._ws = E.Workspace(self.device)
+        self._ws_attn = E.Workspace(self.device)      # tickets of `attend` live at its start: no other kernel's scratch
 
     # -- compressed segment ---------------------------------------------------
     def _append_compressed(self, keys: torch.Tensor, values: torch.Tensor) -> None:
@@ -187,6 +208,12 @@ class TurboQuantKVCache:
         parts = []
         if self._n_quant > 0:
             b, h = self._lead
+            n_q, buf = query.shape[-2], self.key_buffer
+            if query.is_cuda and (buf is None or buf.dtype == query.dtype):
+                logits = E.cache_scores(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant,
+                                        query.reshape(b * h, n_q, self.head_dim).contiguous(), buf, float(scale))
+                if logits is not None:
+                    return logits.reshape(b, h, n_q, -1)
             q3 = query.reshape(b * h, query.shape[-2], self.head_dim)
             logits = E.scores(self.consts, self._pool, self._ws, self._bt, self._n_quant, q3)
             parts.append(logits.reshape(b, h, query.shape[-2], self._n_quant) * scale)
@@ -199,6 +226,14 @@ class TurboQuantKVCache:
         outs, col = [], 0
         if self._n_quant > 0:
             b, h = self._lead
+            buf = self.value_buffer
+            n_all = self._n_quant + (buf.shape[-2] if buf is not None else 0)
+            if attn_weights.is_cuda and attn_weights.shape[-1] == n_all:
+                n_q = attn_weights.shape[-2]
+                out = E.cache_attend(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant,
+                                     attn_weights.reshape(b * h, n_q, n_all).contiguous(), buf)
+                if out is not None:
+                    return out.reshape(b, h, n_q, self.head_dim)
             v = E.dequant_values(self.consts, self._pool, self._bt, self._n_quant).reshape(b, h, self._n_quant, -1)
             w = attn_weights[..., col: col + self._n_quant]
             outs.append(torch.matmul(w.float(), v))

@@ -50,14 +50,34 @@ class _QuantizerBase(torch.nn.Module):
         # buffers with the reference's attribute names
         self.register_buffer("Pi", self.consts.Pi, persistent=False)
         self.register_buffer("centroids", self.consts.centroids, persistent=False)
+        self.consts.ensure_rows()
         self.register_buffer("boundaries", self.consts.boundaries, persistent=False)
         self.register_buffer("decision_boundaries", self.consts.boundaries[1:-1].contiguous(), persistent=False)
+
+    def _planes_of(self, x2: torch.Tensor):
+        """(codes, sign bits, norms in x's dtype, residual norms fp32) of (rows, d) vectors: one kernel where the rows kernel
+        takes them, the store into a one-head pool and back otherwise."""
+        E.require_cuda(x2, "x")
+        got = E.rows_quantize_keys(self.consts, x2) if x2.shape[0] else None
+        if got is not None:
+            return got
+        _, _, ps = self._compress_rows(x2)
+        return ps.mse_indices[0], ps.qjl_signs[0], ps.norms[0].to(x2.dtype), ps.residual_norms[0].float()
+
+    def _dequantize(self, indices, signs, norms, residual_norms) -> torch.Tensor:
+        if indices.numel():
+            args = [None if t is None else t.contiguous() for t in (indices, signs, norms, residual_norms)]
+            out = E.rows_dequantize_keys(self.consts, *args)
+            if out is not None:
+                return out.reshape(*norms.shape, self.dim)
+        pool, bt, heads, n = self._pool_from(indices, signs, norms, residual_norms)
+        return E.dequant_keys(self.consts, pool, bt, n, with_qjl=signs is not None).reshape(*norms.shape, self.dim)
 
     def _compress_rows(self, x2: torch.Tensor):
         """Store (rows, d) as one head; returns (pool, block table, planes)."""
         n = x2.shape[0]
-        pool = E.BlockPool(self.consts, 1, E.blocks_for(n))
-        bt = E.identity_block_table(pool.num_blocks, self.device)
+        pool = E.BlockPool(self.consts, 1, E.blocks_for(n), zeroed=False)
+        bt = E.shared_identity_table(pool.num_blocks, self.device)
         # the value half of the record is not used here: feed the keys as values
         E.store(self.consts, pool, x2, x2, stride_token=x2.stride(0), stride_head=0, n_tokens=n, n_heads=1,
                 block_table=bt, start_pos=0)
@@ -94,13 +114,11 @@ class TurboQuantMSE(_QuantizerBase):
 
     def quantize(self, x: torch.Tensor) -> MSEQuantized:
         lead, x2 = _rows(x)
-        _, _, ps = self._compress_rows(x2)
-        return MSEQuantized(ps.mse_indices[0].reshape(*lead, -1), ps.norms[0].reshape(lead).to(x.dtype), self.bits)
+        codes, _, norms, _ = self._planes_of(x2)
+        return MSEQuantized(codes.reshape(*lead, -1), norms.reshape(lead), self.bits)
 
     def dequantize(self, q: MSEQuantized) -> torch.Tensor:
-        pool, bt, heads, n = self._pool_from(q.indices, None, q.norms, None)
-        out = E.dequant_keys(self.consts, pool, bt, n, with_qjl=False)
-        return out.reshape(*q.norms.shape, self.dim)
+        return self._dequantize(q.indices, None, q.norms, None)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         return self.dequantize(self.quantize(x))
@@ -128,26 +146,31 @@ class TurboQuantProd(_QuantizerBase):
 
     def quantize(self, x: torch.Tensor) -> ProdQuantized:
         lead, x2 = _rows(x)
-        _, _, ps = self._compress_rows(x2)
-        return ProdQuantized(ps.mse_indices[0].reshape(*lead, -1), ps.qjl_signs[0].reshape(*lead, -1),
-                             ps.residual_norms[0].reshape(lead).float(), ps.norms[0].reshape(lead).to(x.dtype),
+        codes, signs, norms, rnorms = self._planes_of(x2)
+        return ProdQuantized(codes.reshape(*lead, -1), signs.reshape(*lead, -1), rnorms.reshape(lead), norms.reshape(lead),
                              self.bits - 1)
 
     def dequantize(self, q: ProdQuantized) -> torch.Tensor:
-        pool, bt, heads, n = self._pool_from(q.mse_indices, q.qjl_signs, q.norms, q.residual_norms)
-        out = E.dequant_keys(self.consts, pool, bt, n, with_qjl=True)
-        return out.reshape(*q.norms.shape, self.dim)
+        return self._dequantize(q.mse_indices, q.qjl_signs, q.norms, q.residual_norms)
 
     def attention_score(self, query: torch.Tensor, quantized_key: ProdQuantized) -> torch.Tensor:
         """query (..., n_q, d), keys (..., n_k, ...) -> unscaled logits (..., n_q, n_k)."""
-        pool, bt, heads, n = self._pool_from(quantized_key.mse_indices, quantized_key.qjl_signs,
-                                             quantized_key.norms, quantized_key.residual_norms)
+        k = quantized_key
+        n = k.mse_indices.shape[-2]
+        heads = max(1, k.mse_indices.numel() // (n * k.mse_indices.shape[-1])) if n else 1
         n_q = query.shape[-2]
         q3 = query.reshape(-1, n_q, self.dim)
         if q3.shape[0] != heads:
             q3 = q3.expand(heads, n_q, self.dim)
-        logits = E.scores(self.consts, pool, self._ws, bt, n, q3.contiguous())
-        return logits.reshape(*quantized_key.norms.shape[:-1], n_q, n)
+        q3 = q3.contiguous()
+        logits = None
+        if n:
+            logits = E.rows_scores(self.consts, self._ws, k.mse_indices.contiguous(), k.qjl_signs.contiguous(),
+                                   k.norms.contiguous(), k.residual_norms.contiguous(), heads, n, q3)
+        if logits is None:
+            pool, bt, heads, n = self._pool_from(k.mse_indices, k.qjl_signs, k.norms, k.residual_norms)
+            logits = E.scores(self.consts, pool, self._ws, bt, n, q3)
+        return logits.reshape(*k.norms.shape[:-1], n_q, n)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         return self.dequantize(self.quantize(x))

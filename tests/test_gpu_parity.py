@@ -1338,3 +1338,11 @@ def test_conversion_words_and_bytes(n, shift, dev):
                "tq_pool_to_planes")
     for f in ("mse_indices", "qjl_signs", "norms", "residual_norms", "v_data", "v_scales", "v_zeros"):
         assert torch.equal(getattr(ps, f)[:, :n], getattr(back, f)[:, :n]), f
+
+
+@pytest.mark.parametrize("kb,vb,n", [(4, 2, 16), (4, 4, 129), (3, 4, 2047)])
+def test_d256_store_with_wide_records(kb, vb, n, dev):
+    """head_dim 256 with 4-bit keys and / or values (operand ring of 128-row boxes): fp32 store kernel, oracle, and
+    every kind of destination."""
+    test_tensor_core_store_matches_fp32_store_and_oracle(256, kb, vb, 3, n, dev)
+    test_tensor_core_store_destinations(256, kb, vb, dev)

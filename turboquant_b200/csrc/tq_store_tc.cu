@@ -80,10 +80,6 @@ __device__ int g_tq_store_status;   // 0 or a tq_status left by a bounded wait t
 // MMA shapes of this file
 // ---------------------------------------------------------------------------
 constexpr uint32_t IDESC = umma_idesc_bf16(128);        // N = 128
-constexpr uint32_t IDESC_N256 = umma_idesc_bf16(256);   // N = 256
-__device__ __forceinline__ void umma_ss_n256(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t accumulate) {
-    umma_ss(tmem_d, a_desc, b_desc, IDESC_N256, accumulate);
-}
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t accumulate) {
     tqtc::umma_ts(tmem_d, tmem_a, b_desc, IDESC, accumulate);
 }
@@ -783,12 +779,27 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 // over Y, and the constant operands stream through a two-slot ring of 32 KB boxes (256 rows x 64
 // channels), each box used for every product that needs it while it is resident: Pi_hi for Y and E, Pi_lo
 // for Y, M_hi for r'_hi and r'_lo, M_lo for r'_hi - 512 KB from L2 per tile.  One tile in flight.
+// 3-bit keys with 2-bit values have 25 KB of record images and leave room for the two slots of 256 rows;
+// the wider records (33 or 41 KB) take a ring of three 16 KB boxes of 128 rows, every product in two
+// halves of 128 columns: the same number of tensor-core cycles and of bytes, 48 KB of them in flight.
+// Measured (5003 tokens, 4 heads, 4-bit keys, 2-bit values): 300 us in the fp32 kernel -> 77.
 // A compute thread (row, q) owns channels [64q, 64q+64): two value groups, one 128-byte row of a box.
 constexpr int D2 = 256;
 constexpr int D2_TILE_BYTES = 4 * BOX_BYTES;      // 128 rows x 256 bf16: four boxes
-constexpr int D2_CHUNK_BYTES = 2 * BOX_BYTES;     // 256 rows x 64 bf16 of a constant operand
-
+template <int ROWS>
+struct D2Ring {                                   // boxes of ROWS rows x 64 bf16 of a constant operand
+    static constexpr int BYTES = ROWS * 128, SLOTS = ROWS == 256 ? 2 : 3;
+    static constexpr int HALVES = D2 / ROWS, PER_MAT = 4 * HALVES, CHUNKS = 4 * PER_MAT;
+};
 template <int MSE_BITS, int VAL_BITS>
+constexpr int d2_ring_rows() { return MSE_BITS == 2 && VAL_BITS == 2 ? 256 : 128; }
+template <int ROWS>
+constexpr size_t d2_smem(size_t img) {
+    return 2 * (size_t)D2_TILE_BYTES + (size_t)D2Ring<ROWS>::SLOTS * D2Ring<ROWS>::BYTES + img + 4 * TC_TOK * sizeof(float) +
+           13 * sizeof(uint64_t) + 16 + 1024;
+}
+
+template <int MSE_BITS, int VAL_BITS, int ROWS = d2_ring_rows<MSE_BITS, VAL_BITS>()>
 __global__ void __launch_bounds__(TC_LAUNCH, 1)
 tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_kt, const __grid_constant__ CUtensorMap tm_vt,
@@ -797,19 +808,20 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                       const TcParams p) {
     const TqLayout L = tq_make_layout(D2, MSE_BITS + 1, VAL_BITS);
     const int BB = L.block_bytes;
+    using Ring = D2Ring<ROWS>;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (tq_smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* sA0 = smem;                              // key rows -> u -> r'_hi
     uint8_t* sA1 = sA0 + D2_TILE_BYTES;               // value rows -> e' -> r'_lo
-    uint8_t* sBr = sA1 + D2_TILE_BYTES;               // two slots of the constant-operand ring
-    uint8_t* sRec = sBr + 2 * D2_CHUNK_BYTES;         // image of the tile's 8 block records
+    uint8_t* sBr = sA1 + D2_TILE_BYTES;               // the constant-operand ring
+    uint8_t* sRec = sBr + Ring::SLOTS * Ring::BYTES;  // image of the tile's 8 block records
     float* s_ss = reinterpret_cast<float*>(sRec + 8 * BB);   // [4][128] partial sums of squares (x, then r')
     uint64_t* bars = reinterpret_cast<uint64_t*>(s_ss + 4 * TC_TOK);
     uint64_t *bar_k = bars, *bar_v = bars + 1, *bar_m1 = bars + 2, *bar_m2 = bars + 3, *bar_r = bars + 4;
-    uint64_t *bar_full = bars + 5, *bar_empty = bars + 7;     // [2] each: ring slot filled / its products done
-    uint64_t *bar_n = bars + 9, *bar_c = bars + 10;           // 512 arrivals: u, e' written / r' written
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+    uint64_t *bar_full = bars + 5, *bar_empty = bars + 8;     // [2 or 3] each: ring slot filled / its products done
+    uint64_t *bar_n = bars + 11, *bar_c = bars + 12;          // 512 arrivals: u, e' written / r' written
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -826,7 +838,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     }
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 9; ++i) tq_mbar_init(bars + i, 1);
+        for (int i = 0; i < 11; ++i) tq_mbar_init(bars + i, 1);
         tq_mbar_init(bar_n, TC_THREADS);
         tq_mbar_init(bar_c, TC_THREADS);
         *s_fail = 0;
@@ -881,14 +893,14 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         };
         const CUtensorMap* tb[4] = {&tm_b0, &tm_b1, &tm_b2, &tm_b3};
         const uint32_t a0 = tq_smem_u32(sA0), a1 = tq_smem_u32(sA1), ar = tq_smem_u32(sBr);
-        // chunk c of a tile: constant operand c / 4 (Pi_hi, Pi_lo, M_hi, M_lo), channels [64 (c % 4), +64)
+        // chunk c of a tile: constant operand c / PER_MAT (Pi_hi, Pi_lo, M_hi, M_lo), channels [64 kc, +64), rows [ROWS half, +ROWS)
         int g_loaded = 0;       // chunks requested so far, over all tiles of this CTA
         auto load_chunk = [&](int c) -> bool {
-            const int slot = g_loaded & 1;
-            if (g_loaded >= 2 && !wait1(bar_empty + slot, ((g_loaded - 2) >> 1) & 1)) return false;
+            const int slot = g_loaded % Ring::SLOTS, cm = c % Ring::PER_MAT;
+            if (g_loaded >= Ring::SLOTS && !wait1(bar_empty + slot, (g_loaded / Ring::SLOTS - 1) & 1)) return false;
             if (elected()) {
-                tq_mbar_expect_tx(bar_full + slot, D2_CHUNK_BYTES);
-                tma_load_2d(sBr + slot * D2_CHUNK_BYTES, tb[c >> 2], 64 * (c & 3), 0, bar_full + slot);
+                tq_mbar_expect_tx(bar_full + slot, Ring::BYTES);
+                tma_load_2d(sBr + slot * Ring::BYTES, tb[c / Ring::PER_MAT], 64 * (cm / Ring::HALVES), ROWS * (cm % Ring::HALVES), bar_full + slot);
             }
             __syncwarp();
             ++g_loaded;
@@ -896,11 +908,13 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         };
         int g_used = 0;
         auto use_chunk = [&](int c) -> bool {   // issue every product that reads chunk c, then release its slot
-            const int slot = g_used & 1, kc = c & 3, mat = c >> 2;
-            if (!wait1(bar_full + slot, (g_used >> 1) & 1)) return false;
+            const int slot = g_used % Ring::SLOTS, mat = c / Ring::PER_MAT, cm = c % Ring::PER_MAT, kc = cm / Ring::HALVES;
+            const uint32_t col = ROWS * (cm % Ring::HALVES);
+            if (!wait1(bar_full + slot, (g_used / Ring::SLOTS) & 1)) return false;
             tc_fence_after();
             if (elected()) {
-                const uint32_t b_addr = ar + slot * D2_CHUNK_BYTES;
+                constexpr uint32_t ID = umma_idesc_bf16(ROWS);
+                const uint32_t b_addr = ar + slot * Ring::BYTES;
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
                     const uint64_t bd = smem_desc_sw128(b_addr + ks * 32);
@@ -908,20 +922,20 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     const uint64_t d1 = smem_desc_sw128(a1 + kc * BOX_BYTES + ks * 32);
                     const uint32_t first = (kc | ks) == 0 ? 0u : 1u;
                     if (mat == 0) {            // Pi_hi: Y (u) and E (e')
-                        umma_ss_n256(tmem_u + C_Y, d0, bd, first);
-                        umma_ss_n256(tmem_u + C_E, d1, bd, first);
+                        umma_ss(tmem_u + C_Y + col, d0, bd, ID, first);
+                        umma_ss(tmem_u + C_E + col, d1, bd, ID, first);
                     } else if (mat == 1) {     // Pi_lo: Y (u)
-                        umma_ss_n256(tmem_u + C_Y, d0, bd, 1u);
+                        umma_ss(tmem_u + C_Y + col, d0, bd, ID, 1u);
                     } else if (mat == 2) {     // M_hi: P (r'_hi) and P (r'_lo), over Y's columns
-                        umma_ss_n256(tmem_u + C_Y, d0, bd, first);
-                        umma_ss_n256(tmem_u + C_Y, d1, bd, 1u);
+                        umma_ss(tmem_u + C_Y + col, d0, bd, ID, first);
+                        umma_ss(tmem_u + C_Y + col, d1, bd, ID, 1u);
                     } else {                   // M_lo: P (r'_hi)
-                        umma_ss_n256(tmem_u + C_Y, d0, bd, 1u);
+                        umma_ss(tmem_u + C_Y + col, d0, bd, ID, 1u);
                     }
                 }
                 umma_commit(bar_empty + slot);
-                if (c == 7) umma_commit(bar_m1);
-                if (c == 15) umma_commit(bar_m2);
+                if (c == Ring::CHUNKS / 2 - 1) umma_commit(bar_m1);
+                if (c == Ring::CHUNKS - 1) umma_commit(bar_m2);
             }
             __syncwarp();
             ++g_used;
@@ -944,19 +958,19 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             }
             __syncwarp();
         }
-        bool ok = load_chunk(0) && load_chunk(1);
+        bool ok = load_chunk(0) && load_chunk(1) && (Ring::SLOTS < 3 || load_chunk(2));
         int i = 0;
 #pragma unroll 1
         for (int tile = tile0; tile < p.n_tiles && ok; tile += (int)gridDim.x, ++i) {
             const int next = tile + (int)gridDim.x;
             if (!(ok = wait1(bar_n, i & 1))) break;              // u, e' in shared memory
 #pragma unroll 1
-            for (int c = 0; c < 16 && ok; ++c) {
-                if (c == 8 && !(ok = wait1(bar_c, i & 1))) break;   // r' limbs in shared memory
+            for (int c = 0; c < Ring::CHUNKS && ok; ++c) {
+                if (c == Ring::CHUNKS / 2 && !(ok = wait1(bar_c, i & 1))) break;   // r' limbs in shared memory
                 ok = use_chunk(c);
-                // keep the ring full: the chunk two ahead (of this tile, or the first ones of the next tile)
-                const int ahead = c + 2;
-                if (ok && (ahead < 16 || next < p.n_tiles)) ok = load_chunk(ahead & 15);
+                // keep the ring full: the chunk SLOTS ahead (of this tile, or the first ones of the next tile)
+                const int ahead = c + Ring::SLOTS;
+                if (ok && (ahead < Ring::CHUNKS || next < p.n_tiles)) ok = load_chunk(ahead % Ring::CHUNKS);
             }
             if (!ok) break;
             if (next < p.n_tiles) {
@@ -1175,11 +1189,11 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
-// (D x D) bf16 matrix, row-major: boxes of 64 columns x D rows (128 or 256), 128-byte swizzle
-bool make_matrix_map(CUtensorMap* tm, const void* base, int D) {
+// (D x D) bf16 matrix, row-major: boxes of 64 columns x `box_rows` rows, 128-byte swizzle
+bool make_matrix_map(CUtensorMap* tm, const void* base, int D, int box_rows) {
     const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)D};
     const cuuint64_t strides[1] = {(cuuint64_t)D * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)D};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     return encode_tiled_fn()(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1207,10 +1221,10 @@ bool make_rows_map(CUtensorMap* tm, const void* base, int D, int64_t n_tokens, i
 // (a map holds only the address and the geometry, never the matrix).
 struct OperandMapSet {
     const void* ptr[4];
-    int D;
+    int D, box_rows;
     CUtensorMap tm[4];
 };
-bool operand_maps(CUtensorMap (&out)[4], const tq_consts* consts, int D) {
+bool operand_maps(CUtensorMap (&out)[4], const tq_consts* consts, int D, int box_rows) {
     constexpr int SETS = 16;
     static std::mutex mu;
     static OperandMapSet sets[SETS];
@@ -1218,15 +1232,16 @@ bool operand_maps(CUtensorMap (&out)[4], const tq_consts* consts, int D) {
     const void* want[4] = {consts->pi_limbs[0], consts->pi_limbs[1], consts->m_limbs[0], consts->m_limbs[1]};
     std::lock_guard<std::mutex> lock(mu);
     for (int i = 0; i < n_sets; ++i)
-        if (sets[i].D == D && memcmp(sets[i].ptr, want, sizeof(want)) == 0) {
+        if (sets[i].D == D && sets[i].box_rows == box_rows && memcmp(sets[i].ptr, want, sizeof(want)) == 0) {
             memcpy(out, sets[i].tm, sizeof(sets[i].tm));
             return true;
         }
     OperandMapSet fresh;
     memcpy(fresh.ptr, want, sizeof(want));
     fresh.D = D;
+    fresh.box_rows = box_rows;
     for (int i = 0; i < 4; ++i)
-        if (!make_matrix_map(&fresh.tm[i], want[i], D)) return false;
+        if (!make_matrix_map(&fresh.tm[i], want[i], D, box_rows)) return false;
     sets[next] = fresh;
     next = (next + 1) % SETS;
     if (n_sets < SETS) ++n_sets;
@@ -1255,9 +1270,8 @@ bool make_paged_map(CUtensorMap* tm, const void* base, int D, int64_t num_blocks
 
 }  // namespace
 
-// Launches a tensor-core kernel when the call fits one: head_dim 128 (any bit widths) or 256 (3-bit keys
-// with 2-bit values, the combination whose record image fits beside the operands), bf16, 16-byte aligned
-// rows, the split operands present.  Otherwise *handled stays 0 and tq_store runs its fp32 kernel.
+// Launches a tensor-core kernel when the call fits one: head_dim 128 or 256 (any bit widths), bf16, 16-byte
+// aligned rows, the split operands present.  Otherwise *handled stays 0 and tq_store runs its fp32 kernel.
 //
 // `paged` (may be null) makes key / value the two planes of a paged cache: rows are then addressed as
 // (source block from paged->table, token in block) instead of by stride_token from one base.
@@ -1271,9 +1285,8 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     if ((D != TC_D && D != D2) || dtype != TQ_BF16) return TQ_OK;
     const TqLayout L = tq_make_layout(D, cfg.key_bits, cfg.value_bits);
     const size_t img = (size_t)8 * L.block_bytes;
-    const size_t smem256 = 2 * (size_t)D2_TILE_BYTES + 2 * (size_t)D2_CHUNK_BYTES + img + 4 * TC_TOK * sizeof(float) +
-                           11 * sizeof(uint64_t) + 16 + 1024;
-    if (D == D2 && smem256 > SMEM_LIMIT) return TQ_OK;
+    const bool d2_wide = D == D2 && (cfg.key_bits != 3 || cfg.value_bits != 2);   // records of 33 or 41 KB a tile
+    if (paged && d2_wide) return TQ_OK;   // tq_store_paged answers "not supported" for these; its callers gather first
     if (!consts->pi_limbs[0] || !consts->pi_limbs[1] || !consts->m_limbs[0] || !consts->m_limbs[1]) return TQ_OK;
     if (((uintptr_t)key & 15) || ((uintptr_t)value & 15) || (stride_token & 7) || (stride_head & 7)) return TQ_OK;
     if (stride_token < D || (n_heads > 1 && stride_head < D)) return TQ_OK;
@@ -1334,7 +1347,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
         tm_kt = tm_k;
         tm_vt = tm_v;
     }
-    if (!maps_ok || !operand_maps(tm_b, consts, D))
+    if (!maps_ok || !operand_maps(tm_b, consts, D, d2_wide ? 128 : D))
         return TQ_OK;   // a stride pattern the tensor map cannot express: the fp32 kernel takes the call
     *handled = 1;
 
@@ -1352,22 +1365,29 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     lc.stream = st;
     lc.gridDim = dim3(grid);
     lc.blockDim = dim3(TC_LAUNCH);
+    cudaError_t launched = cudaSuccess;
     if (D == D2) {
         p.n_rec_buf = 1;
-        if (mse_bits != 2 || cfg.value_bits != 2) {   // unreachable: no other image passed the size check above
-            *handled = 0;
-            return TQ_OK;
-        }
-        static TqSmemOptIn opt_in;
-        if (tq_opt_in_smem(tq_store_tc256_kernel<2, 2>, smem256, opt_in) != TQ_OK) return TQ_ERR_CUDA;
-        lc.dynamicSmemBytes = smem256;
-        return cudaLaunchKernelEx(&lc, tq_store_tc256_kernel<2, 2>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1], tm_b[2],
-                                  tm_b[3], p) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+#define TQ_TC256(MB, VB)                                                                                         \
+    do {                                                                                                         \
+        static TqSmemOptIn opt_in;                                                                               \
+        const size_t smem = d2_smem<d2_ring_rows<MB, VB>()>(img);                                                \
+        static_assert(d2_ring_rows<2, 2>() == 256 && d2_ring_rows<2, 4>() == 128, "boxes of the operand maps");  \
+        if (tq_opt_in_smem(tq_store_tc256_kernel<MB, VB>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;            \
+        lc.dynamicSmemBytes = smem;                                                                              \
+        launched = cudaLaunchKernelEx(&lc, tq_store_tc256_kernel<MB, VB>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1], \
+                                      tm_b[2], tm_b[3], p);                                                      \
+    } while (0)
+        if (mse_bits == 2 && cfg.value_bits == 2) TQ_TC256(2, 2);
+        else if (mse_bits == 2) TQ_TC256(2, 4);
+        else if (cfg.value_bits == 2) TQ_TC256(3, 2);
+        else TQ_TC256(3, 4);
+#undef TQ_TC256
+        return launched == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
     }
     const size_t fixed = (size_t)6 * MAT_BYTES + 8 * TC_TOK * sizeof(float) + 12 * sizeof(uint64_t) + 16 + 1024;
     p.n_rec_buf = fixed + 2 * img <= SMEM_LIMIT ? 2 : 1;
     const size_t smem = fixed + (size_t)p.n_rec_buf * img;
-    cudaError_t launched = cudaSuccess;
 #define TQ_TC(MB, VB)                                                                                            \
     do {                                                                                                         \
         static TqSmemOptIn opt_in;                                                                               \

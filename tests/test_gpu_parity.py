@@ -1346,3 +1346,28 @@ def test_d256_store_with_wide_records(kb, vb, n, dev):
     every kind of destination."""
     test_tensor_core_store_matches_fp32_store_and_oracle(256, kb, vb, 3, n, dev)
     test_tensor_core_store_destinations(256, kb, vb, dev)
+
+
+@pytest.mark.parametrize("d,kb,vb,qh", [(128, 3, 2, 16), (128, 3, 2, 8), (128, 4, 4, 8), (256, 3, 2, 8)])
+def test_decode_by_pairs_of_records(d, kb, vb, qh, dev):
+    """Several waves of CTAs: 0, 1, 2 or 3 records a warp (a pair without a partner, a partly filled last record), scores
+    that climb along the sequence far past the softmax reference, and stale Inf bytes behind the last token."""
+    from turboquant_b200 import _engine as E
+    h, nseq, nmax = 4, 80, 400                       # 320 CTAs of eight warps, up to 25 records each
+    c = E.LayerConstants(d, kb, vb, dev, seed=5)
+    g = torch.Generator().manual_seed(d + qh)
+    lens = torch.randint(17, nmax + 1, (nseq,), generator=g)
+    lens[:6] = torch.tensor([16, 128, 129, 250, 256, 400])
+    q = (torch.randn(nseq, qh, d, generator=g)).bfloat16().to(dev)
+    k = torch.randn(nmax, h, d, generator=g) + torch.linspace(0, 6, nmax)[:, None, None] * q[0, :h].float().cpu()[None] / 4
+    k, v = k.bfloat16().to(dev), torch.randn(nmax, h, d, generator=g).bfloat16().to(dev)
+    pool = E.BlockPool(c, h, 25)
+    pool.data.fill_(0x7c)                            # stale bytes: fp16 Inf / NaN patterns
+    bt = E.identity_block_table(25, dev)
+    E.store(c, pool, k, v, stride_token=h * d, stride_head=d, n_tokens=nmax, n_heads=h, block_table=bt, start_pos=0)
+    table = bt[None].expand(nseq, -1).contiguous()
+    ws = E.Workspace(dev)
+    a, b = (E.decode(c, pool, ws, q, table, lens.int().to(dev), nmax, num_splits=1, kernel=kern).float() for kern in (0, 1))
+    assert ws.status() == 0 and torch.isfinite(a).all()
+    assert _cos(a, b) >= 0.99995
+    torch.testing.assert_close(a, b, rtol=3e-2, atol=3e-3)

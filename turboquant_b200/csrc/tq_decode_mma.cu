@@ -38,6 +38,9 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 constexpr int NW_WAVE = 12;
 constexpr int NW_MULTI = 8;
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
+// A warp's softmax reference is put this far (in log2) above the largest score of the pair of records that raised it; it
+// moves a few times per sequence then, and not at every new maximum of any of its heads.
+constexpr float MARGIN = 2.f;
 
 
 // 2^x for x <= 0 (softmax terms): the bare approximation instruction, results below 2^-126 flush to 0
@@ -86,6 +89,7 @@ template <int D, int MSE_BITS, int VAL_BITS, bool SPLITB, int NW>
 __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma_kernel(const DecodeParams p) {
     static_assert(MSE_BITS == 2 || SPLITB, "3-bit codes use separate rotated / sketched fragment sets");
     constexpr int NT = NW * 32;
+    constexpr int R = NW == NW_MULTI ? 2 : 1;   // records a warp works on at a time
     constexpr int GP = SPLITB ? 8 : 4;
     constexpr int KS = D / 16;    // score k-steps
     constexpr int NWK = D / 64;   // 32-bit words of 2-bit codes per thread per token; twice the sign words
@@ -180,9 +184,9 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     // (launched with programmatic stream serialisation: everything above overlapped that kernel)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     bool failed = !__all_sync(0xffffffffu, tq_mbar_wait_bounded(bars + NW * NSTW, 0u));   // then no record is processed
-    // Head_dim 256 with separate rotated / sketched sets: two sets of 32 fragment registers do not fit beside
-    // the 64 value accumulators, so the fragments stay in shared memory and are read where they are used.
-    constexpr bool BSM = (D == 256) && SPLITB;
+    // Head_dim 256, and separate rotated / sketched sets in a CTA of 128 registers a thread: the fragments do not fit
+    // beside the value accumulators and two records' score accumulators; they stay in shared memory, read once per pair.
+    constexpr bool BSM = R == 2 ? D == 256 || SPLITB : D == 256 && SPLITB;
     uint32_t bq[BSM ? 1 : 2 * KS];
     uint32_t bsk[(SPLITB && !BSM) ? 2 * KS : 1];
 #define BQ(r) (BSM ? qf_s[QF_HDR + (r) * 32 + lane] : bq[BSM ? 0 : (r)])
@@ -195,7 +199,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         const bool col_live = g_col < p.G;
         if (BSM) {
             if (!col_live)   // columns without a head: nobody wrote their fragments - clear this lane's words
-                for (int r = 0; r < 4 * KS; ++r) qf_s[QF_HDR + r * 32 + lane] = 0u;
+                for (int r = 0; r < (SPLITB ? 4 : 2) * KS; ++r) qf_s[QF_HDR + r * 32 + lane] = 0u;
             __syncwarp();
         } else {
 #pragma unroll
@@ -279,121 +283,158 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         }
     }
 
-    for (int it = 0; it < cnt && !failed; ++it) {
+    // In a launch of several waves a warp takes two records at a time: their six chains of score MMAs, their softmax terms
+    // and their loads are independent, which keeps the pipes of a quarter SM busy with the four warps that the registers
+    // allow (256 sequences of 8192 tokens, 64 heads on 8: 718 -> 625 us).  In one wave a warp has a handful of records,
+    // and taking them in pairs costs more in the odd one than it gives (32768 tokens, head_dim 256: 188 -> 200 us).
+    for (int it = 0; it < cnt && !failed; it += R) {
         const int st = it % NSTW;
-        bool ok = tq_mbar_wait_bounded(my_bar + st, (uint32_t)((it / NSTW) & 1));
+        const uint32_t phase = (uint32_t)((it / NSTW) & 1);
+        const bool both = R == 2 && it + 1 < cnt;
+        bool ok = tq_mbar_wait_bounded(my_bar + st, phase) && (!both || tq_mbar_wait_bounded(my_bar + st + 1, phase));
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
             failed = true;
             break;
         }
-        uint8_t* rec = my_stage + st * BB;
-        const int blk = blk0 + warp + NW * it;
-        const int valid = min(TQ_BLOCK_TOKENS, n - blk * TQ_BLOCK_TOKENS);
-        if (valid < TQ_BLOCK_TOKENS) {
+        uint8_t* rec[R];
+        int valid[R];   // an odd record's partner is itself, with no valid token
+        bool ragged = false;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool there = r == 0 || both;
+            rec[r] = my_stage + (there ? st + r : st) * BB;
+            valid[r] = there ? min(TQ_BLOCK_TOKENS, n - (blk0 + warp + NW * (it + r)) * TQ_BLOCK_TOKENS) : 0;
+            ragged |= valid[r] < TQ_BLOCK_TOKENS;
+        }
+        if (ragged) {
             // the sequence's last, partly filled record: unused slots may hold anything.  Their scores are
             // masked below; their value scales and zero points ([grp][16 tok] fp16, contiguous) are cleared
             // here, so that probability 0 times a stale Inf/NaN cannot reach the value MMAs.
-            __half* sz = reinterpret_cast<__half*>(rec + L.off_vscale);
-            for (int i = lane; i < 2 * NG * TQ_BLOCK_TOKENS; i += 32)
-                if ((i & (TQ_BLOCK_TOKENS - 1)) >= valid) sz[i] = __float2half(0.f);
+            for (int r = 0; r < 1 + (both ? 1 : 0); ++r) {
+                __half* sz = reinterpret_cast<__half*>(my_stage + (st + r) * BB + L.off_vscale);
+                const int live = r == 0 ? valid[0] : valid[R - 1];
+                for (int i = lane; i < 2 * NG * TQ_BLOCK_TOKENS; i += 32)
+                    if ((i & (TQ_BLOCK_TOKENS - 1)) >= live) sz[i] = __float2half(0.f);
+            }
             tq_fence_proxy_async();   // generic writes to a stage that a later bulk copy may refill
             __syncwarp();
         }
 
         // ------------------------------ scores ------------------------------
-        float acc1[4], acc0[4], accs[4];   // written by the first k-step's MMAs
-        if (MSE_BITS == 3) acc1[0] = acc1[1] = acc1[2] = acc1[3] = 0.f;
+        float acc1[R][4], acc0[R][4], accs[R][4];   // written by the first k-step's MMAs
+        if (MSE_BITS == 3)
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc1[r][0] = acc1[r][1] = acc1[r][2] = acc1[r][3] = 0.f;
         if (MSE_BITS == 2) {
-            const uint32_t* cwA = reinterpret_cast<const uint32_t*>(rec + L.off_kcodes + tokA * L.kcode_row) + tig * NWK;
-            const uint32_t* cwB = reinterpret_cast<const uint32_t*>(rec + L.off_kcodes + tokB * L.kcode_row) + tig * NWK;
-            const uint32_t* swA = reinterpret_cast<const uint32_t*>(rec + L.off_ksigns + tokA * L.ksign_row) + tig * (NWK / 2);
-            const uint32_t* swB = reinterpret_cast<const uint32_t*>(rec + L.off_ksigns + tokB * L.ksign_row) + tig * (NWK / 2);
-            uint32_t wA[NWK], wB[NWK], sA[NWK / 2], sB[NWK / 2];
-            if (NWK == 4) {
-                const uint4 a = *reinterpret_cast<const uint4*>(cwA), bb = *reinterpret_cast<const uint4*>(cwB);
-                wA[0] = a.x; wA[1] = a.y; wA[NWK - 2] = a.z; wA[NWK - 1] = a.w;
-                wB[0] = bb.x; wB[1] = bb.y; wB[NWK - 2] = bb.z; wB[NWK - 1] = bb.w;
-                const uint2 c = *reinterpret_cast<const uint2*>(swA), d = *reinterpret_cast<const uint2*>(swB);
-                sA[0] = c.x; sA[NWK / 2 - 1] = c.y;
-                sB[0] = d.x; sB[NWK / 2 - 1] = d.y;
-            } else {
-                const uint2 a = *reinterpret_cast<const uint2*>(cwA), bb = *reinterpret_cast<const uint2*>(cwB);
-                wA[0] = a.x; wA[1] = a.y;
-                wB[0] = bb.x; wB[1] = bb.y;
-                sA[0] = swA[0];
-                sB[0] = swB[0];
+            uint32_t wA[R][NWK], wB[R][NWK], sA[R][NWK / 2], sB[R][NWK / 2];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const uint32_t* cwA = reinterpret_cast<const uint32_t*>(rec[r] + L.off_kcodes + tokA * L.kcode_row) + tig * NWK;
+                const uint32_t* cwB = reinterpret_cast<const uint32_t*>(rec[r] + L.off_kcodes + tokB * L.kcode_row) + tig * NWK;
+                const uint32_t* swA = reinterpret_cast<const uint32_t*>(rec[r] + L.off_ksigns + tokA * L.ksign_row) + tig * (NWK / 2);
+                const uint32_t* swB = reinterpret_cast<const uint32_t*>(rec[r] + L.off_ksigns + tokB * L.ksign_row) + tig * (NWK / 2);
+                if (NWK == 4) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(cwA), bb = *reinterpret_cast<const uint4*>(cwB);
+                    wA[r][0] = a.x; wA[r][1] = a.y; wA[r][NWK - 2] = a.z; wA[r][NWK - 1] = a.w;
+                    wB[r][0] = bb.x; wB[r][1] = bb.y; wB[r][NWK - 2] = bb.z; wB[r][NWK - 1] = bb.w;
+                    const uint2 c = *reinterpret_cast<const uint2*>(swA), d = *reinterpret_cast<const uint2*>(swB);
+                    sA[r][0] = c.x; sA[r][NWK / 2 - 1] = c.y;
+                    sB[r][0] = d.x; sB[r][NWK / 2 - 1] = d.y;
+                } else {
+                    const uint2 a = *reinterpret_cast<const uint2*>(cwA), bb = *reinterpret_cast<const uint2*>(cwB);
+                    wA[r][0] = a.x; wA[r][1] = a.y;
+                    wB[r][0] = bb.x; wB[r][1] = bb.y;
+                    sA[r][0] = swA[0];
+                    sB[r][0] = swB[0];
+                }
             }
 #pragma unroll
             for (int wi = 0; wi < NWK; ++wi) {
-                const uint32_t a_lo = wA[wi], b_lo = wB[wi];
-                const uint32_t a_hi = a_lo >> 6, b_hi = b_lo >> 6;
-                // sign word with bytes 1 and 2 swapped: halves then pair the same dims as the code word
-                const uint32_t sa_lo = __byte_perm(sA[wi >> 1], 0, 0x3120), sb_lo = __byte_perm(sB[wi >> 1], 0, 0x3120);
-                const uint32_t sa_hi = sa_lo >> 6, sb_hi = sb_lo >> 6;
+                uint32_t a_hi[R], b_hi[R], sa_lo[R], sb_lo[R], sa_hi[R], sb_hi[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    a_hi[r] = wA[r][wi] >> 6;
+                    b_hi[r] = wB[r][wi] >> 6;
+                    // sign word with bytes 1 and 2 swapped: halves then pair the same dims as the code word
+                    sa_lo[r] = __byte_perm(sA[r][wi >> 1], 0, 0x3120);
+                    sb_lo[r] = __byte_perm(sB[r][wi >> 1], 0, 0x3120);
+                    sa_hi[r] = sa_lo[r] >> 6;
+                    sb_hi[r] = sb_lo[r] >> 6;
+                }
 #pragma unroll
                 for (int jj = 0; jj < 4; ++jj) {
                     const int s = wi * 4 + jj;
                     const int j0 = 2 * jj, j1 = j0 + 1;
                     const uint32_t m0 = 0x00010001u << (2 * code_pos(j0)), m1 = 0x00010001u << (2 * code_pos(j1));
-                    const uint32_t xa0 = j0 <= 4 ? a_lo : a_hi, xb0 = j0 <= 4 ? b_lo : b_hi;
-                    const uint32_t xa1 = j1 <= 4 ? a_lo : a_hi, xb1 = j1 <= 4 ? b_lo : b_hi;
-                    if (s == 0) {
-                        mma16816_z(acc0, xa0 & m0, xb0 & m0, xa1 & m1, xb1 & m1, BQ(2 * s), BQ(2 * s + 1));
-                        mma16816_z(acc1, xa0 & (m0 << 1), xb0 & (m0 << 1), xa1 & (m1 << 1), xb1 & (m1 << 1), BQ(2 * s),
-                                   BQ(2 * s + 1));
-                    } else {
-                        mma16816(acc0, xa0 & m0, xb0 & m0, xa1 & m1, xb1 & m1, BQ(2 * s), BQ(2 * s + 1));
-                        mma16816(acc1, xa0 & (m0 << 1), xb0 & (m0 << 1), xa1 & (m1 << 1), xb1 & (m1 << 1), BQ(2 * s),
-                                 BQ(2 * s + 1));
-                    }
                     const int sb0 = sign_bit(wi, j0), sb1 = sign_bit(wi, j1);
                     const uint32_t n0 = 0x00010001u << sign_pos(sb0), n1 = 0x00010001u << sign_pos(sb1);
-                    const uint32_t ya0 = sb0 <= 9 ? sa_lo : sa_hi, yb0 = sb0 <= 9 ? sb_lo : sb_hi;
-                    const uint32_t ya1 = sb1 <= 9 ? sa_lo : sa_hi, yb1 = sb1 <= 9 ? sb_lo : sb_hi;
-                    if (s == 0)
-                        mma16816_z(accs, ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, SPLITB ? BSK(0) : BQ(0),
-                                   SPLITB ? BSK(1) : BQ(1));
-                    else if (SPLITB)
-                        mma16816(accs, ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, BSK(2 * s), BSK(2 * s + 1));
-                    else
-                        mma16816(accs, ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, BQ(2 * s), BQ(2 * s + 1));
+                    const uint32_t q0 = BQ(2 * s), q1 = BQ(2 * s + 1);
+                    const uint32_t z0 = SPLITB ? BSK(2 * s) : q0, z1 = SPLITB ? BSK(2 * s + 1) : q1;
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        const uint32_t xa0 = j0 <= 4 ? wA[r][wi] : a_hi[r], xb0 = j0 <= 4 ? wB[r][wi] : b_hi[r];
+                        const uint32_t xa1 = j1 <= 4 ? wA[r][wi] : a_hi[r], xb1 = j1 <= 4 ? wB[r][wi] : b_hi[r];
+                        const uint32_t ya0 = sb0 <= 9 ? sa_lo[r] : sa_hi[r], yb0 = sb0 <= 9 ? sb_lo[r] : sb_hi[r];
+                        const uint32_t ya1 = sb1 <= 9 ? sa_lo[r] : sa_hi[r], yb1 = sb1 <= 9 ? sb_lo[r] : sb_hi[r];
+                        if (s == 0) {
+                            mma16816_z(acc0[r], xa0 & m0, xb0 & m0, xa1 & m1, xb1 & m1, q0, q1);
+                            mma16816_z(acc1[r], xa0 & (m0 << 1), xb0 & (m0 << 1), xa1 & (m1 << 1), xb1 & (m1 << 1), q0, q1);
+                            mma16816_z(accs[r], ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, z0, z1);
+                        } else {
+                            mma16816(acc0[r], xa0 & m0, xb0 & m0, xa1 & m1, xb1 & m1, q0, q1);
+                            mma16816(acc1[r], xa0 & (m0 << 1), xb0 & (m0 << 1), xa1 & (m1 << 1), xb1 & (m1 << 1), q0, q1);
+                            mma16816(accs[r], ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, z0, z1);
+                        }
+                    }
                 }
             }
         }
         if (MSE_BITS == 3) {
             constexpr int NWC = D / 32;    // words of nibble codes per thread per token (8 codes each)
             constexpr int NWS = D / 128;   // sign words per thread per token
-            const uint4* cwA = reinterpret_cast<const uint4*>(rec + L.off_kcodes + tokA * L.kcode_row) + tig * (NWC / 4);
-            const uint4* cwB = reinterpret_cast<const uint4*>(rec + L.off_kcodes + tokB * L.kcode_row) + tig * (NWC / 4);
-            const uint32_t* swA = reinterpret_cast<const uint32_t*>(rec + L.off_ksigns + tokA * L.ksign_row) + tig * NWS;
-            const uint32_t* swB = reinterpret_cast<const uint32_t*>(rec + L.off_ksigns + tokB * L.ksign_row) + tig * NWS;
 #pragma unroll
             for (int q4 = 0; q4 < NWC / 4; ++q4) {
-                const uint4 a4 = cwA[q4], b4 = cwB[q4];
-                const uint32_t wa[4] = {a4.x, a4.y, a4.z, a4.w}, wb[4] = {b4.x, b4.y, b4.z, b4.w};
+                uint32_t wa[R][4], wb[R][4];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint4 a4 = *(reinterpret_cast<const uint4*>(rec[r] + L.off_kcodes + tokA * L.kcode_row) + tig * (NWC / 4) + q4);
+                    const uint4 b4 = *(reinterpret_cast<const uint4*>(rec[r] + L.off_kcodes + tokB * L.kcode_row) + tig * (NWC / 4) + q4);
+                    wa[r][0] = a4.x; wa[r][1] = a4.y; wa[r][2] = a4.z; wa[r][3] = a4.w;
+                    wb[r][0] = b4.x; wb[r][1] = b4.y; wb[r][2] = b4.z; wb[r][3] = b4.w;
+                }
 #pragma unroll
                 for (int wi = 0; wi < 4; ++wi) {
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         // k-step s covers dims 8*(4*q4+wi) + 4*hf + {0,1 | 2,3} of this thread's slice
                         const int s = (q4 * 4 + wi) * 2 + hf;
-                        const uint32_t sa = hf ? wa[wi] >> 16 : wa[wi], sb = hf ? wb[wi] >> 16 : wb[wi];
-                        const uint32_t la = __byte_perm(t_lo0, t_lo1, sa), ha = __byte_perm(t_hi0, t_hi1, sa);
-                        const uint32_t lb = __byte_perm(t_lo0, t_lo1, sb), hb = __byte_perm(t_hi0, t_hi1, sb);
-                        if (s == 0)
-                            mma16816_z(acc0, __byte_perm(la, ha, 0x5140), __byte_perm(lb, hb, 0x5140),
-                                       __byte_perm(la, ha, 0x7362), __byte_perm(lb, hb, 0x7362), BQ(0), BQ(1));
-                        else
-                            mma16816(acc0, __byte_perm(la, ha, 0x5140), __byte_perm(lb, hb, 0x5140),
-                                     __byte_perm(la, ha, 0x7362), __byte_perm(lb, hb, 0x7362), BQ(2 * s), BQ(2 * s + 1));
+                        const uint32_t q0 = BQ(2 * s), q1 = BQ(2 * s + 1);
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            const uint32_t sa = hf ? wa[r][wi] >> 16 : wa[r][wi], sb = hf ? wb[r][wi] >> 16 : wb[r][wi];
+                            const uint32_t la = __byte_perm(t_lo0, t_lo1, sa), ha = __byte_perm(t_hi0, t_hi1, sa);
+                            const uint32_t lb = __byte_perm(t_lo0, t_lo1, sb), hb = __byte_perm(t_hi0, t_hi1, sb);
+                            if (s == 0)
+                                mma16816_z(acc0[r], __byte_perm(la, ha, 0x5140), __byte_perm(lb, hb, 0x5140),
+                                           __byte_perm(la, ha, 0x7362), __byte_perm(lb, hb, 0x7362), q0, q1);
+                            else
+                                mma16816(acc0[r], __byte_perm(la, ha, 0x5140), __byte_perm(lb, hb, 0x5140),
+                                         __byte_perm(la, ha, 0x7362), __byte_perm(lb, hb, 0x7362), q0, q1);
+                        }
                     }
                 }
             }
 #pragma unroll
             for (int sw = 0; sw < NWS; ++sw) {
-                const uint32_t sa_lo = __byte_perm(swA[sw], 0, 0x3120), sb_lo = __byte_perm(swB[sw], 0, 0x3120);
-                const uint32_t sa_hi = sa_lo >> 6, sb_hi = sb_lo >> 6;
+                uint32_t sa_lo[R], sb_lo[R], sa_hi[R], sb_hi[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    sa_lo[r] = __byte_perm((reinterpret_cast<const uint32_t*>(rec[r] + L.off_ksigns + tokA * L.ksign_row) + tig * NWS)[sw], 0, 0x3120);
+                    sb_lo[r] = __byte_perm((reinterpret_cast<const uint32_t*>(rec[r] + L.off_ksigns + tokB * L.ksign_row) + tig * NWS)[sw], 0, 0x3120);
+                    sa_hi[r] = sa_lo[r] >> 6;
+                    sb_hi[r] = sb_lo[r] >> 6;
+                }
 #pragma unroll
                 for (int wi = 2 * sw; wi < 2 * sw + 2; ++wi) {
 #pragma unroll
@@ -401,52 +442,70 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                         const int s = wi * 4 + jj;
                         const int sb0 = sign_bit(wi, 2 * jj), sb1 = sign_bit(wi, 2 * jj + 1);
                         const uint32_t n0 = 0x00010001u << sign_pos(sb0), n1 = 0x00010001u << sign_pos(sb1);
-                        const uint32_t ya0 = sb0 <= 9 ? sa_lo : sa_hi, yb0 = sb0 <= 9 ? sb_lo : sb_hi;
-                        const uint32_t ya1 = sb1 <= 9 ? sa_lo : sa_hi, yb1 = sb1 <= 9 ? sb_lo : sb_hi;
-                        if (s == 0)
-                            mma16816_z(accs, ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, BSK(0), BSK(1));
-                        else
-                            mma16816(accs, ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, BSK(2 * s),
-                                     BSK(2 * s + 1));
+                        const uint32_t z0 = BSK(2 * s), z1 = BSK(2 * s + 1);
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            const uint32_t ya0 = sb0 <= 9 ? sa_lo[r] : sa_hi[r], yb0 = sb0 <= 9 ? sb_lo[r] : sb_hi[r];
+                            const uint32_t ya1 = sb1 <= 9 ? sa_lo[r] : sa_hi[r], yb1 = sb1 <= 9 ? sb_lo[r] : sb_hi[r];
+                            if (s == 0)
+                                mma16816_z(accs[r], ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, z0, z1);
+                            else
+                                mma16816(accs[r], ya0 & n0, yb0 & n0, ya1 & n1, yb1 & n1, z0, z1);
+                        }
                     }
                 }
             }
         }
         if (!SPLITB) {   // sketched-query columns 4..7 live two lanes to the right
 #pragma unroll
-            for (int c = 0; c < 4; ++c) accs[c] = __shfl_xor_sync(0xffffffffu, accs[c], 2);
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) accs[r][c] = __shfl_xor_sync(0xffffffffu, accs[r][c], 2);
         }
 
         // ------------------------------ online softmax ------------------------------
-        const __half* nrm = reinterpret_cast<const __half*>(rec + L.off_knorm);
-        const __half* rnm = reinterpret_cast<const __half*>(rec + L.off_krnorm);
-        const float nA = __half2float(nrm[tokA]) * sm_scale, nB = __half2float(nrm[tokB]) * sm_scale;
-        const float rA = __half2float(rnm[tokA]) * (qjl * sm_scale), rB = __half2float(rnm[tokB]) * (qjl * sm_scale);
-        float sA[2], sB[2], pA[2], pB[2];
-        bool rescale = false;
-        float alpha[2];
+        // The reference m_run is set MARGIN above the largest score seen when it was set and stands until a score passes
+        // it: probabilities stay <= 1, and the reduction over the row groups and the rescaling leave the usual path.
+        float sc_[R][2][2];   // [record][row A, B][column]
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const __half* nrm = reinterpret_cast<const __half*>(rec[r] + L.off_knorm);
+            const __half* rnm = reinterpret_cast<const __half*>(rec[r] + L.off_krnorm);
+            const float nA = __half2float(nrm[tokA]) * sm_scale, nB = __half2float(nrm[tokB]) * sm_scale;
+            const float rA = __half2float(rnm[tokA]) * (qjl * sm_scale), rB = __half2float(rnm[tokB]) * (qjl * sm_scale);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                sc_[r][0][i] = nA * (k0[i] + k1[i] * acc1[r][i] + kb0[i] * acc0[r][i]) + rA * (ksg[i] * accs[r][i] - kq[i]);
+                sc_[r][1][i] = nB * (k0[i] + k1[i] * acc1[r][2 + i] + kb0[i] * acc0[r][2 + i]) + rB * (ksg[i] * accs[r][2 + i] - kq[i]);
+            }
+        }
+        if (ragged) {   // warp-uniform: only the sequence's last record, or a record without a partner
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    if (tokA >= valid[r]) sc_[r][0][i] = -INFINITY;
+                    if (tokB >= valid[r]) sc_[r][1][i] = -INFINITY;
+                }
+        }
+        float mx[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            sA[i] = nA * (k0[i] + k1[i] * acc1[i] + kb0[i] * acc0[i]) + rA * (ksg[i] * accs[i] - kq[i]);
-            sB[i] = nB * (k0[i] + k1[i] * acc1[2 + i] + kb0[i] * acc0[2 + i]) + rB * (ksg[i] * accs[2 + i] - kq[i]);
-            if (valid < TQ_BLOCK_TOKENS) {   // warp-uniform: only the sequence's last record
-                if (tokA >= valid) sA[i] = -INFINITY;
-                if (tokB >= valid) sB[i] = -INFINITY;
-            }
-            float mx = fmaxf(sA[i], sB[i]);
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-            const float m_new = fmaxf(m_run[i], mx);
-            const float m_use = (m_new == -INFINITY) ? 0.f : m_new;
-            alpha[i] = ex2_fast(m_run[i] - m_use);
-            pA[i] = ex2_fast(sA[i] - m_use);
-            pB[i] = ex2_fast(sB[i] - m_use);
-            l_run[i] = l_run[i] * alpha[i] + pA[i] + pB[i];
-            rescale |= (m_new != m_run[i]);
-            m_run[i] = m_new;
+            mx[i] = fmaxf(sc_[0][0][i], sc_[0][1][i]);
+            if (R == 2) mx[i] = fmaxf(mx[i], fmaxf(sc_[R - 1][0][i], sc_[R - 1][1][i]));
         }
-        if (__any_sync(0xffffffffu, rescale && col_ok)) {
+        if (__any_sync(0xffffffffu, col_ok && (mx[0] > m_run[0] || mx[1] > m_run[1]))) {
+            float alpha[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 4));
+                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 8));
+                mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 16));
+                const float m_new = mx[i] > m_run[i] ? mx[i] + MARGIN : m_run[i];
+                alpha[i] = m_new == -INFINITY ? 1.f : ex2_fast(m_run[i] - m_new);
+                l_run[i] *= alpha[i];
+                m_run[i] = m_new;
+            }
 #pragma unroll
             for (int mb = 0; mb < NMB; ++mb) {
                 o[mb][0] *= alpha[0];
@@ -459,22 +518,35 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
             zacc[2] *= alpha[0];
             zacc[3] *= alpha[1];
         }
-        // probabilities (x16, clear of fp16 underflow) -> B fragment of the value MMA
-        const uint32_t t0 = movmatrix_trans(col_ok ? pack_half2(pA[0] * 16.f, pA[1] * 16.f) : 0u);
-        const uint32_t t1 = movmatrix_trans(col_ok ? pack_half2(pB[0] * 16.f, pB[1] * 16.f) : 0u);
+        // probabilities (x16, clear of fp16 underflow) -> B fragments of the value MMAs
+        uint32_t t0[R], t1[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            float pA[2], pB[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const float m_use = m_run[i] == -INFINITY ? 0.f : m_run[i];   // no score yet but -Inf (or NaN)
+                pA[i] = ex2_fast(sc_[r][0][i] - m_use);
+                pB[i] = ex2_fast(sc_[r][1][i] - m_use);
+                l_run[i] += pA[i] + pB[i];
+            }
+            t0[r] = movmatrix_trans(col_ok ? pack_half2(pA[0] * 16.f, pA[1] * 16.f) : 0u);
+            t1[r] = movmatrix_trans(col_ok ? pack_half2(pB[0] * 16.f, pB[1] * 16.f) : 0u);
+        }
 
         // ------------------------------ values ------------------------------
-        {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
             // tokens of this thread's contraction slots: 4*tig .. 4*tig+3
-            const uint2* vsc = reinterpret_cast<const uint2*>(rec + L.off_vscale) + tig;   // [grp][16 tok] fp16: 4 uint2 per group
-            const uint2* vzr = reinterpret_cast<const uint2*>(rec + L.off_vzero) + tig;
+            const uint2* vsc = reinterpret_cast<const uint2*>(rec[r] + L.off_vscale) + tig;   // [grp][16 tok] fp16: 4 uint2 per group
+            const uint2* vzr = reinterpret_cast<const uint2*>(rec[r] + L.off_vzero) + tig;
             // zero-point term: rows = groups
             {
                 uint2 z = make_uint2(0u, 0u);
                 if (gid < NG) z = vzr[gid * 4];
-                mma16816(zacc, z.x, 0u, z.y, 0u, t0, t1);
+                mma16816(zacc, z.x, 0u, z.y, 0u, t0[r], t1[r]);
             }
-            const uint4* vcw = reinterpret_cast<const uint4*>(rec + L.off_vcodes) + lane;   // [chunk][lane] 16 B
+            const uint4* vcw = reinterpret_cast<const uint4*>(rec[r] + L.off_vcodes) + lane;   // [chunk][lane] 16 B
             if (VAL_BITS == 2) {
                 // word (p, gp): [tokA grp 2gp, tokA grp 2gp+1, tokB grp 2gp, tokB grp 2gp+1]
                 constexpr int NGP = NG / 2;
@@ -495,7 +567,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                     for (int odd = 0; odd < 2; ++odd) {
                         const int grp = 2 * gp + odd;
                         const uint2 sc = vsc[grp * 4];
-                        const uint32_t bp0 = hmul2_sat(t0, sc.x), bp1 = hmul2_sat(t1, sc.y);
+                        const uint32_t bp0 = hmul2_sat(t0[r], sc.x), bp1 = hmul2_sat(t1[r], sc.y);
 #pragma unroll
                         for (int hb = 0; hb < 2; ++hb) {   // the two M-blocks of the group
                             const int i_lo = 2 * hb, i_hi = i_lo + 1;
@@ -522,7 +594,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                     const uint32_t w0 = w[grp], w1 = w[NG + grp];
                     const uint32_t w0h = w0 >> 8, w1h = w1 >> 8;
                     const uint2 sc = vsc[grp * 4];
-                    const uint32_t bp0 = hmul2_sat(t0, sc.x), bp1 = hmul2_sat(t1, sc.y);
+                    const uint32_t bp0 = hmul2_sat(t0[r], sc.x), bp1 = hmul2_sat(t1[r], sc.y);
                     mma16816(o[2 * grp], w0 & 0x000f000fu, w0 & 0x00f000f0u, w1 & 0x000f000fu, w1 & 0x00f000f0u, bp0, bp1);
                     mma16816(o[2 * grp + 1], w0h & 0x000f000fu, w0h & 0x00f000f0u, w1h & 0x000f000fu,
                              w1h & 0x00f000f0u, bp0, bp1);
@@ -531,10 +603,10 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         }
 
         __syncwarp();
-        if (lane == 0 && it + NSTW < cnt) {   // refill the stage just consumed
-            tq_mbar_expect_tx(my_bar + st, (uint32_t)BB);
-            tq_bulk_g2s(my_stage + st * BB, p.pool + ((int64_t)bt_s[warp + NW * (it + NSTW)] * p.H + h) * BB,
-                        (uint32_t)BB, my_bar + st);
+        if (lane < R && it + lane + NSTW < cnt) {   // refill the stages just consumed
+            tq_mbar_expect_tx(my_bar + st + lane, (uint32_t)BB);
+            tq_bulk_g2s(my_stage + (st + lane) * BB, p.pool + ((int64_t)bt_s[warp + NW * (it + lane + NSTW)] * p.H + h) * BB,
+                        (uint32_t)BB, my_bar + st + lane);
         }
     }
     if (failed && lane == 0) atomicCAS(p.status, 0, (int)TQ_ERR_TIMEOUT);

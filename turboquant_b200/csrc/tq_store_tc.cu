@@ -84,23 +84,31 @@ __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64
     tqtc::umma_ts(tmem_d, tmem_a, b_desc, IDESC, accumulate);
 }
 
-// Offset inside a block record of byte `cb` of token `tl`'s share (a token owns bytes_per_token bytes:
-// codes, signs, norm, residual norm, value codes, group scales, group zero points - in that order).
-__device__ __forceinline__ int rec_byte_offset(const TqLayout& L, int tl, int cb) {
-    if (cb < L.kcode_row) return L.off_kcodes + tl * L.kcode_row + cb;
+// A token's share of a block record as 16-bit units: codes, signs, norm, residual norm, value codes (whose byte pairs stay
+// together in the native order), group scales, group zero points.  Unit u of token t lies at
+// base + stride * t + (value codes only) tq_vcode_native's token part.
+struct RecUnit {
+    int base, stride;
+    bool vcode;
+};
+__device__ __forceinline__ RecUnit rec_unit(const TqLayout& L, int u) {
+    int cb = 2 * u;
+    if (cb < L.kcode_row) return {L.off_kcodes + cb, L.kcode_row, false};
     cb -= L.kcode_row;
-    if (cb < L.ksign_row) return L.off_ksigns + tl * L.ksign_row + cb;
+    if (cb < L.ksign_row) return {L.off_ksigns + cb, L.ksign_row, false};
     cb -= L.ksign_row;
-    if (cb < 2) return L.off_knorm + tl * 2 + cb;
-    cb -= 2;
-    if (cb < 2) return L.off_krnorm + tl * 2 + cb;
-    cb -= 2;
-    if (cb < L.vcode_row) return L.off_vcodes + tq_vcode_native(L.D, L.val_bits, tl, cb);
+    if (cb < 4) return {cb == 0 ? L.off_knorm : L.off_krnorm, 2, false};
+    cb -= 4;
+    if (cb < L.vcode_row) {   // two-bit codes: one byte each of a pair of groups; four-bit codes: two bytes of a group
+        const int i = cb >> 1, byte = L.val_bits == 2 ? (i >> 3) * 16 + (i & 7) : cb;
+        return {L.off_vcodes + tq_vcode_native(L.D, L.val_bits, 0, byte), 0, true};
+    }
     cb -= L.vcode_row;
-    if (cb < 2 * L.ngroups) return L.off_vscale + ((cb >> 1) * TQ_BLOCK_TOKENS + tl) * 2 + (cb & 1);
-    cb -= 2 * L.ngroups;
-    return L.off_vzero + ((cb >> 1) * TQ_BLOCK_TOKENS + tl) * 2 + (cb & 1);
+    const int grp = cb >> 1;
+    return grp < L.ngroups ? RecUnit{L.off_vscale + grp * 2 * TQ_BLOCK_TOKENS, 2, false}
+                           : RecUnit{L.off_vzero + (grp - L.ngroups) * 2 * TQ_BLOCK_TOKENS, 2, false};
 }
+constexpr int REC_UNITS_MAX = (128 + 32 + 4 + 128 + 32) / 2;   // head_dim 256, four bits each
 
 // ---------------------------------------------------------------------------
 // Values: asymmetric min/max quantisation of ONE 32-channel group of one row in
@@ -210,20 +218,22 @@ struct RecordDest {
     bool asked = false;
 };
 __device__ __forceinline__ void ask_destination(const TcParams& p, int64_t tok0, int warp, int lane, RecordDest& d) {
-    if (warp >= 8) return;
     if (p.slot_mapping == nullptr) {
         const int64_t first = tok0 + warp * TQ_BLOCK_TOKENS;      // token index of the block's first row
-        d.asked = lane == 0 && first < p.n_tokens && first + TQ_BLOCK_TOKENS > 0;
+        d.asked = warp < 8 && lane == 0 && first < p.n_tokens && first + TQ_BLOCK_TOKENS > 0;
         if (d.asked) d.blk = __ldg(p.block_table + ((p.start_pos + first) >> 4));
     } else {
-        const int64_t i = tok0 + warp * TQ_BLOCK_TOKENS + (lane & 15);
+        const int64_t i = tok0 + (warp & 7) * TQ_BLOCK_TOKENS + (lane & 15);
         if (i >= 0 && i < p.n_tokens) d.slot = __ldg(p.slot_mapping + i);
     }
 }
-// Warp j < 8 sends image block j on its way: one bulk (TMA) store when the block is a whole record of
-// the pool, a byte scatter to each token's own slot otherwise.
-__device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout& L, const uint8_t* img, int h, int j,
+// Warps j and j + 8 send image block j on its way: one bulk (TMA) store when the block is a whole record of the pool, a
+// scatter to each token's own slot otherwise, eight tokens a warp.  The scatter works out where a lane's units lie once and
+// moves 16 bits at a time; byte by byte, with the offsets found anew for each, it was two thirds of a decode step's write
+// (5 tokens of 8 heads: 14.8 us a launch, 64 tokens at 4/4 bits 32 us).
+__device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout& L, const uint8_t* img, int h, int warp,
                                               int lane, const RecordDest& d) {
+    const int j = warp & 7;
     const int BB = L.block_bytes;
     if (p.slot_mapping == nullptr) {
         if (d.asked) {
@@ -236,8 +246,7 @@ __device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout&
         }
         return;
     }
-    // slot mapping: sixteen rows that fill one block in order leave as a whole record, anything else is
-    // scattered byte by byte
+    // slot mapping: sixteen rows that fill one block in order leave as a whole record, anything else is scattered
     int64_t slot = d.slot;
     if (slot >= 0 && (slot >> 4) >= p.num_blocks) {
         atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_RANGE);
@@ -246,20 +255,31 @@ __device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout&
     const int64_t slot0 = __shfl_sync(0xffffffffu, slot, 0);
     const bool whole = __all_sync(0xffffffffu, slot0 >= 0 && (slot0 & 15) == 0 && slot == slot0 + (lane & 15));
     if (whole) {
-        if (lane == 0) {
+        if (lane == 0 && warp < 8) {
             tq_bulk_s2g(p.pool + ((slot0 >> 4) * p.H + h) * (int64_t)BB, img + j * BB, (uint32_t)BB);
             tq_bulk_commit();
         }
         return;
     }
-    const int per_tok = BB / TQ_BLOCK_TOKENS;
+    const int units = BB / TQ_BLOCK_TOKENS / 2;
     const uint8_t* src = img + j * BB;
-    for (int t = 0; t < TQ_BLOCK_TOKENS; ++t) {
+    constexpr int NU = (REC_UNITS_MAX + 31) / 32;
+    RecUnit un[NU];
+#pragma unroll
+    for (int i = 0; i < NU; ++i) un[i] = rec_unit(L, min(lane + 32 * i, units - 1));
+    const int half_bytes = L.val_bits == 2 && L.D == 128 ? 8 : L.D * L.val_bits;   // value codes: second token pair of a quad
+    auto vpart = [&](int t) { return (t >> 2) * 16 + ((t >> 1) & 1) * half_bytes + (t & 1) * 2; };
+#pragma unroll 2
+    for (int t = warp & 8; t < (warp & 8) + 8; ++t) {
         const int64_t s = __shfl_sync(0xffffffffu, slot, t);
         if (s < 0) continue;
         uint8_t* dst = p.pool + ((s >> 4) * p.H + h) * (int64_t)BB;
-        for (int cb = lane; cb < per_tok; cb += 32)
-            dst[rec_byte_offset(L, (int)(s & 15), cb)] = src[rec_byte_offset(L, t, cb)];
+        const int td = (int)(s & 15), vs = vpart(t), vd = vpart(td);
+#pragma unroll
+        for (int i = 0; i < NU; ++i)
+            if (lane + 32 * i < units)
+                *reinterpret_cast<uint16_t*>(dst + un[i].base + un[i].stride * td + (un[i].vcode ? vd : 0)) =
+                    *reinterpret_cast<const uint16_t*>(src + un[i].base + un[i].stride * t + (un[i].vcode ? vs : 0));
     }
 }
 
@@ -747,11 +767,9 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             }
 
             // ---------------- the tile's block records leave ----------------
-            if (warp < 8) {
-                if (tile_no == 0) pool_writes_may_begin();
-                leave_records(p, L, img, h, warp, lane, dest);
-                if (lane == 0 && p.n_rec_buf == 1) tq_bulk_wait_all_read();
-            }
+            if (tile_no == 0) pool_writes_may_begin();
+            leave_records(p, L, img, h, warp, lane, dest);
+            if (lane == 0 && warp < 8 && p.n_rec_buf == 1) tq_bulk_wait_all_read();
             if (p.n_rec_buf == 1) {
                 compute_barrier_or(false);                // the single image is rewritten by the values below
                 if (has_next) phase_v(par ^ 1, nimg, tile_tok0(next));
@@ -1152,11 +1170,9 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             }
             tq_fence_proxy_async();
             compute_barrier_or(false);       // record image complete
-            if (warp < 8) {
-                if (tile_no == 0) pool_writes_may_begin();
-                leave_records(p, L, sRec, h, warp, lane, dest);
-                if (lane == 0) tq_bulk_wait_all_read();
-            }
+            if (tile_no == 0) pool_writes_may_begin();
+            leave_records(p, L, sRec, h, warp, lane, dest);
+            if (lane == 0 && warp < 8) tq_bulk_wait_all_read();
             compute_barrier_or(false);       // the image and s_ss are free for the next tile
         }
         if (!ok && tid == 0) atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_TIMEOUT);

@@ -1371,3 +1371,26 @@ def test_decode_by_pairs_of_records(d, kb, vb, qh, dev):
     assert ws.status() == 0 and torch.isfinite(a).all()
     assert _cos(a, b) >= 0.99995
     torch.testing.assert_close(a, b, rtol=3e-2, atol=3e-3)
+
+
+@pytest.mark.parametrize("nseq,n,splits", [(5, 700, 0), (64, 130, 1), (1, 4000, 16)])
+def test_decode_right_behind_a_store(nseq, n, splits, dev):
+    """The query preparation may start under a store; the decode behind it must still see every record of that store.
+    The whole history is rewritten before each decode, compared with a decode after a synchronise."""
+    from turboquant_b200 import _engine as E
+    d, h, qh = 128, 4, 16
+    c = E.LayerConstants(d, 3, 2, dev, seed=3)
+    pool, bt = E.BlockPool(c, h, E.blocks_for(n)), E.identity_block_table(E.blocks_for(n), dev)
+    table = bt[None].expand(nseq, -1).contiguous()
+    lens = torch.full((nseq,), n, dtype=torch.int32, device=dev)
+    ws = E.Workspace(dev)
+    q = O.synth_query(nseq, qh, d, seed=8, dtype=torch.bfloat16).to(dev)
+    kv = [tuple(t.to(dev) for t in O.synth_kv(n, h, d, seed=20 + i, dtype=torch.bfloat16)) for i in range(3)]
+    for i in range(24):
+        k, v = kv[i % 3]
+        E.store(c, pool, k, v, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=bt, start_pos=0)
+        got = [E.decode(c, pool, ws, q, table, lens, n, num_splits=splits).clone() for _ in range(2)]
+        torch.cuda.synchronize()
+        want = E.decode(c, pool, ws, q, table, lens, n, num_splits=splits)
+        assert torch.equal(got[0], want) and torch.equal(got[1], want)
+    assert ws.status() == 0 and E.store_status() == 0

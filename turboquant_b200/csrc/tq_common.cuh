@@ -228,13 +228,21 @@ int tq_sm_count();         // multiprocessors of the current device (148 when th
 //     the new token to the ring - rows a flush then reads - so a store behind a decode launch is launched in
 //     plain stream order;
 //   * the decode family reads sequence lengths, block tables and the first pool records before the wait.
-//     The tensor-core store kernels write the pool and let their dependents begin at once, so the first
-//     kernel of a decode call behind such a store is launched in plain stream order.
+//     The tensor-core store kernels write the pool and let their dependents begin at once.  The query
+//     preparation reads nothing that they write and may start under them; the decode kernel behind it is
+//     then told to wait before its first record (and to let its own dependents begin only after that, so
+//     that no later kernel's early reads reach back to the store).  A decode kernel directly behind a
+//     store is launched in plain stream order.
 // Kernels of other libraries between two of ours never start early and only make the order stricter; a
 // stream the library has not seen counts as unknown.
-enum TqLaunchKind { TQ_LAUNCH_UNKNOWN = 0, TQ_LAUNCH_DECODE = 1, TQ_LAUNCH_STORE_EARLY = 2, TQ_LAUNCH_NEUTRAL = 3 };
+enum TqLaunchKind { TQ_LAUNCH_UNKNOWN = 0, TQ_LAUNCH_DECODE = 1, TQ_LAUNCH_STORE_EARLY = 2, TQ_LAUNCH_NEUTRAL = 3, TQ_LAUNCH_PREP_BEHIND_STORE = 4 };
 void tq_note_launch(cudaStream_t st, int kind);
 int tq_last_launch(cudaStream_t st);
+// notes a launch that prepares a decode call (and neither reads nor writes the pool)
+inline void tq_note_prep_launch(cudaStream_t st) {
+    const int k = tq_last_launch(st);
+    tq_note_launch(st, k == TQ_LAUNCH_STORE_EARLY || k == TQ_LAUNCH_PREP_BEHIND_STORE ? TQ_LAUNCH_PREP_BEHIND_STORE : TQ_LAUNCH_DECODE);
+}
 // programmatic-launch attribute count (0 or 1) for a kernel of the decode family / of the early-starting stores
 inline int tq_pdl_for_decode(cudaStream_t st) { return tq_last_launch(st) == TQ_LAUNCH_STORE_EARLY ? 0 : 1; }
 inline int tq_pdl_for_store(cudaStream_t st) {

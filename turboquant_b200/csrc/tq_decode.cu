@@ -323,8 +323,8 @@ int launch_qprep(const void* q, int dt, int64_t nvec, int D, const float* pi_t, 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // its matrix loads may run under the previous kernel's tail
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = tq_pdl_for_decode(st);   // behind a store that is still writing the pool: plain stream order
-    tq_note_launch(st, TQ_LAUNCH_DECODE);
+    cfg.numAttrs = 1;   // behind a store too: the pool is not touched here
+    tq_note_prep_launch(st);
     cfg.stream = st;
     cfg.blockDim = dim3(256);
     if (nvec >= 4096 && ap.new_k == nullptr && !ap.early_inputs && ((uintptr_t)q & 15) == 0) {   // throughput kernel
@@ -822,6 +822,7 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     p.ring_splits = rsplits;
     p.ring_tok = ring_tok;
     p.land_bytes = 0;
+    p.pool_late = tq_last_launch(st) == TQ_LAUNCH_PREP_BEHIND_STORE ? 1 : 0;
 
     const int mse_bits = consts->cfg.key_bits - 1, vb = consts->cfg.value_bits;
     if (a->kernel != 1) {   // tensor-core kernel where it applies
@@ -1078,8 +1079,8 @@ extern "C" int tq_decode_host_io(const tq_consts* consts, const tq_pool* pool, c
             attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             attr[0].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
-            cfg.numAttrs = tq_pdl_for_decode(st);
-            tq_note_launch(st, TQ_LAUNCH_DECODE);
+            cfg.numAttrs = 1;
+            tq_note_prep_launch(st);
             if (cudaLaunchKernelEx(&cfg, tq_stage_in_kernel, (const uint4*)host_in, (uint4*)dev_in, (int)(in_bytes / 16)) !=
                 cudaSuccess)
                 return TQ_ERR_CUDA;

@@ -116,12 +116,14 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     const int b = blockIdx.z, h = blockIdx.x, x = blockIdx.y;
     // a kernel launched behind this one with programmatic stream serialisation may be scheduled as soon
     // as every CTA of this grid is running; whatever it reads of ours it reads after its own wait
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (pool_late: not before a store ahead of the query preparation is known to have finished)
+    if (!p.pool_late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (x >= p.num_splits) {
         // exact ring tokens: CUDA-core fp32 path shared with the generic kernel.  The ring and its
         // length may have been written by the query-prep grid this launch overlaps with.
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (p.pool_late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         float* scratch = reinterpret_cast<float*>(stages);
         uint8_t* kst = reinterpret_cast<uint8_t*>(scratch + D * GP + 2 * GP * RING_TOK);   // 16-byte aligned
         ring_part<D, GP>(p, b, h, x, scratch, scratch + D * GP, scratch + D * GP + GP * RING_TOK, ml, kst,
@@ -168,6 +170,10 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     // library lets its dependents start early).  Thread 0 waits for them and asks for the fragments
     // before its own warp's records, so that they queue behind as few record copies as possible; the
     // other warps start their copies at once.
+    if (p.pool_late) {   // the records themselves may still be on their way
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
     if (tid == 0) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         tq_mbar_expect_tx(bars + NW * NSTW, QF_BYTES);

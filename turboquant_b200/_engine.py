@@ -120,7 +120,7 @@ class LayerConstants:
 
     def ensure_rows(self) -> None:
         """Operands of the kernels on plain rows (64 Pi, M = S Pi^T and S as two fp16 limbs each): only the quantiser
-        objects use them, which call this when they are made."""
+        objects use them, which call this before their first launch."""
         if self.rows_limbs is not None or self.head_dim != 128:
             return
         pi, s = self.Pi.cpu().double(), self.S.cpu().double()

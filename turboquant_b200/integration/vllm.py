@@ -202,11 +202,10 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
                             query, output, n)
         if mode == MODE_HYBRID and state.supports_hybrid and state.store.num_tokens >= MIN_HISTORY:
             if output is not None:                      # straight into the engine's buffer where its layout allows
-                st = state.store
-                rk, rv = state.engine.ring.peek() or (None, None)
+                st, ring = state.store, state.engine.ring
                 res = E.host().hybrid(st.consts.addr, st.pool.addr, st.workspace, st.block_table, c.head_dim, st._num_tokens,
-                                      query, n, c.num_query_heads, rk, rv, getattr(self_impl, "scale", None), MIN_HISTORY,
-                                      output)
+                                      query, n, c.num_query_heads, *ring.storage, ring.size, getattr(self_impl, "scale", None),
+                                      MIN_HISTORY, output)
                 if res is output:
                     return output
                 if res is not None:
@@ -226,7 +225,7 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
 
 
 def _bind(impl, name: str, fn) -> None:
-    setattr(impl, name, types.MethodType(lambda self, *a, _f=fn, **kw: _f(self, *a, **kw), impl))
+    setattr(impl, name, types.MethodType(fn, impl))
 
 
 def install_hooks(model_runner, key_bits: int = 3, value_bits: int = 2, value_group_size: int = 32,

@@ -50,22 +50,29 @@ class _QuantizerBase(torch.nn.Module):
         # buffers with the reference's attribute names
         self.register_buffer("Pi", self.consts.Pi, persistent=False)
         self.register_buffer("centroids", self.consts.centroids, persistent=False)
-        self.consts.ensure_rows()
         self.register_buffer("boundaries", self.consts.boundaries, persistent=False)
         self.register_buffer("decision_boundaries", self.consts.boundaries[1:-1].contiguous(), persistent=False)
+
+    def _rows_operands(self) -> bool:
+        """The rows kernels' operands, laid out on first use (a store owns a quantiser and never asks for them)."""
+        if self.consts.rows_limbs is None and self.dim == 128:
+            if torch.cuda.is_current_stream_capturing():
+                return False
+            self.consts.ensure_rows()
+        return True
 
     def _planes_of(self, x2: torch.Tensor):
         """(codes, sign bits, norms in x's dtype, residual norms fp32) of (rows, d) vectors: one kernel where the rows kernel
         takes them, the store into a one-head pool and back otherwise."""
         E.require_cuda(x2, "x")
-        got = E.rows_quantize_keys(self.consts, x2) if x2.shape[0] else None
+        got = E.rows_quantize_keys(self.consts, x2) if x2.shape[0] and self._rows_operands() else None
         if got is not None:
             return got
         _, _, ps = self._compress_rows(x2)
         return ps.mse_indices[0], ps.qjl_signs[0], ps.norms[0].to(x2.dtype), ps.residual_norms[0].float()
 
     def _dequantize(self, indices, signs, norms, residual_norms) -> torch.Tensor:
-        if indices.numel():
+        if indices.numel() and self._rows_operands():
             args = [None if t is None else t.contiguous() for t in (indices, signs, norms, residual_norms)]
             out = E.rows_dequantize_keys(self.consts, *args)
             if out is not None:

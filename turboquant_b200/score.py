@@ -33,8 +33,8 @@ def compute_hybrid_attention(query: torch.Tensor, store: CompressedKVStore, rece
     """
     if query.dim() == 3:
         out = E.host().hybrid(store.consts.addr, store.pool.addr, store.workspace, store.block_table, store.head_dim,
-                              store._num_tokens, query, query.shape[0], num_query_heads, recent_k, recent_v, scale,
-                              MIN_HISTORY_FOR_TQ, None)
+                              store._num_tokens, query, query.shape[0], num_query_heads, recent_k, recent_v, None,
+                              scale, MIN_HISTORY_FOR_TQ, None)
         if type(out) is torch.Tensor:
             return out
         if out is not None:

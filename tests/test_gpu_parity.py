@@ -1394,3 +1394,10 @@ def test_decode_right_behind_a_store(nseq, n, splits, dev):
         want = E.decode(c, pool, ws, q, table, lens, n, num_splits=splits)
         assert torch.equal(got[0], want) and torch.equal(got[1], want)
     assert ws.status() == 0 and E.store_status() == 0
+
+
+@pytest.mark.parametrize("qh,h,n,dtype", [(32, 8, 1300, torch.bfloat16), (40, 8, 1025, torch.float16), (12, 4, 3328, torch.bfloat16),
+                                          (300, 100, 130, torch.bfloat16), (304, 8, 1, torch.float16)])
+def test_prefill_attention_pairs_of_query_tiles(qh, h, n, dtype, dev):
+    """Launches of more than two waves of tiles: even and odd numbers of query tiles, a last tile of one row, a single tile."""
+    test_prefill_attention_vs_fp32_reference(128, qh, h, n, dtype, dev)

@@ -391,6 +391,308 @@ tq_prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
+// ---------------------------------------------------------------------------
+// head_dim 128, launches of more than one wave: two query tiles per CTA
+// ---------------------------------------------------------------------------
+// The kernel above spends a tile's time in a chain - scores, row maximum exchanged between four threads, exponentials,
+// probabilities - and its tensor pipe waits for it.  Here a CTA takes two neighbouring query tiles of a head against the
+// same key/value tiles, each with a warpgroup of its own whose threads own whole rows (no exchange, no CTA barrier), and
+// goes through the keys in halves of 64 with two score buffers per query tile: while a warpgroup exponentiates one half,
+// the scores of its next half and the products of the other query tile run.
+//   issue order   S_A(0) S_B(0) S_A(1) S_B(1) | PV_A(h) S_A(h+2) PV_B(h) S_B(h+2) | ...
+// P(h) takes the place of S(h) in tensor memory, S(h+2) that of P(h) (products execute in the order they are issued):
+// S_A 2 x 64 | S_B 2 x 64 | O_A 128 | O_B 128 columns.  One warp issues the products, one the loads.  Per 128 keys and CTA:
+// 32 products of 128 x 128 x 16 or their equivalent (some 2950 cycles at the rate the pipe sustains) against 32768
+// exponentials (2048 cycles of the special-function pipes).  Scaling, sums and the row maximum use the two- and
+// three-operand fp32 forms.  With whole tiles of 128 keys and one score buffer each - softmax, PV and S of a tile in a chain -
+// the pipe stood idle half of the time (5700 cycles per 128 keys, slower than the kernel above).
+constexpr int PP_THREADS = 2 * PA_TOK + 64;
+constexpr int PP_HALF = 64;                        // keys per step
+
+__device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, float* v) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+// ties 32 loaded columns to the wait in front of it: nothing may read them earlier
+__device__ __forceinline__ void tmem_loaded32(float* v) {
+    asm volatile("" : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]),
+                 "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]),
+                 "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]),
+                 "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31]));
+}
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void halves_of(uint64_t p, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(p)); }
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+template <bool BF16>
+__global__ void __launch_bounds__(PP_THREADS, 1)
+tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                       const __grid_constant__ CUtensorMap tm_v, const PrefillParams p) {
+    constexpr int D = 128, TILE_BYTES = 2 * PA_BOX, NST = 2;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (tq_smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* sQ = smem;                           // [2] query tiles
+    uint8_t* sK = sQ + 2 * TILE_BYTES;            // [NST]
+    uint8_t* sV = sK + NST * TILE_BYTES;          // [NST]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NST * TILE_BYTES);
+    uint64_t *bar_q = bars, *bar_k = bars + 1, *bar_v = bars + 3, *free_k = bars + 5, *free_v = bars + 7, *bar_o = bars + 9,
+             *bar_s = bars + 11, *bar_p = bars + 15;   // bar_s, bar_p: [query tile][score buffer]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+    volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tq_smem_u32(tmem_slot)), "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+#pragma unroll
+        for (int i = 0; i < 19; ++i) tq_mbar_init(bars + i, i >= 15 ? PA_TOK : 1);
+        *s_fail = 0;
+        tq_mbar_fence_init();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    constexpr uint32_t C_S = 0, C_O = 256, C_STEP = 128;   // + C_STEP for tile B
+
+    const int pair = (int)gridDim.y - 1 - (int)blockIdx.y;   // longest rows first, over all heads
+    const int qh = blockIdx.x, kvh = qh / p.group;
+    const int n_kv[2] = {2 * pair + 1, 2 * pair + 1 < p.n_tiles ? 2 * pair + 2 : 0};   // key/value tiles of A and of B
+    const int n_all = max(n_kv[0], n_kv[1]);
+
+    // every lane polls: the usual wait is over at the first try, and a vote behind it would cost more than the polls
+    auto wait_fast = [&](uint64_t* bar, uint32_t parity) -> bool {
+        if (tq_mbar_try_wait(bar, parity)) return true;
+        for (int i = 0; i < (1 << 20); ++i) {
+            if (tq_mbar_try_wait(bar, parity)) return true;
+            if ((i & 255) == 255 && *s_fail) break;
+        }
+        *s_fail = 1;
+        return false;
+    };
+    auto wait_warp = [&](uint64_t* bar, uint32_t parity) -> bool {   // the same answer in every lane
+        const bool ok = __all_sync(0xffffffffu, wait_fast(bar, parity));
+        return ok;
+    };
+    auto elected = [&]() -> bool {
+        uint32_t pred;
+        asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+        return pred != 0;
+    };
+
+    if (warp == 9) {
+        // =============================== loads ===============================
+        auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int tok0, int head, bool expect) {
+            if (elected()) {
+                if (expect) tq_mbar_expect_tx(bar, TILE_BYTES);
+                tma_load_3d(dst, tm, 0, head, tok0, bar);
+                tma_load_3d(dst + PA_BOX, tm, 64, head, tok0, bar);
+            }
+            __syncwarp();
+        };
+        const int n_q = n_kv[1] ? 2 : 1;
+        if (elected()) tq_mbar_expect_tx(bar_q, (uint32_t)(n_q * TILE_BYTES));
+        __syncwarp();
+        for (int i = 0; i < n_q; ++i) load_tile(sQ + i * TILE_BYTES, &tm_q, bar_q, (2 * pair + i) * PA_TOK, qh, false);
+        for (int t = 0; t < n_all; ++t) {
+            const int st = t & 1;
+            const uint32_t ph = (uint32_t)((t >> 1) - 1) & 1u;
+            if (t >= NST && !wait_warp(free_k + st, ph)) break;
+            load_tile(sK + st * TILE_BYTES, &tm_k, bar_k + st, t * PA_TOK, kvh, true);
+            if (t >= NST && !wait_warp(free_v + st, ph)) break;
+            load_tile(sV + st * TILE_BYTES, &tm_v, bar_v + st, t * PA_TOK, kvh, true);
+        }
+    } else if (warp == 8) {
+        // =============================== products ===============================
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint32_t aQ = tq_smem_u32(sQ), aK = tq_smem_u32(sK), aV = tq_smem_u32(sV);
+        constexpr uint32_t idesc_s = umma_idesc_bf16(PP_HALF, false, !BF16), idesc_o = umma_idesc_bf16(D, true, !BF16);
+        auto issue_s = [&](int w, int h) {    // S_w(h) = Q_w K(h)^T
+            tc_fence_after();
+            if (elected()) {
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks) {
+                    const uint32_t off = (ks >> 2) * PA_BOX + (ks & 3) * 32;
+                    umma_ss(tmem_u + C_S + w * C_STEP + (h & 1) * PP_HALF, smem_desc_sw128(aQ + w * TILE_BYTES + off),
+                            smem_desc_sw128(aK + ((h >> 1) & 1) * TILE_BYTES + (h & 1) * PP_HALF * 128 + off), idesc_s, ks ? 1u : 0u);
+                }
+                umma_commit(bar_s + 2 * w + (h & 1));
+            }
+            __syncwarp();
+        };
+        auto issue_pv = [&](int w, int h) {   // O_w += P_w(h) V(h)
+            tc_fence_after();
+            if (elected()) {
+#pragma unroll
+                for (int ks = 0; ks < PP_HALF / 16; ++ks)
+                    umma_ts(tmem_u + C_O + w * C_STEP, tmem_u + C_S + w * C_STEP + (h & 1) * PP_HALF + ks * 8,
+                            smem_desc_sw128_mn(aV + ((h >> 1) & 1) * TILE_BYTES + ((h & 1) * (PP_HALF / 16) + ks) * 2048, PA_BOX), idesc_o,
+                            (h | ks) ? 1u : 0u);
+                if (h + 2 >= 2 * n_kv[w]) umma_commit(bar_o + w);   // the last two: phases 0 and 1
+            }
+            __syncwarp();
+        };
+        auto release = [&](uint64_t* bar) {   // completes when everything issued so far has
+            if (elected()) umma_commit(bar);
+            __syncwarp();
+        };
+        bool ok = wait_warp(bar_q, 0) && wait_warp(bar_k, 0);
+        if (ok) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                issue_s(0, h);
+                if (n_kv[1]) issue_s(1, h);
+            }
+            release(free_k);
+        }
+        const int n_h[2] = {2 * n_kv[0], 2 * n_kv[1]}, n_hall = 2 * n_all;
+#pragma unroll 1
+        for (int h = 0; h < n_hall && ok; ++h) {
+            const int t = h >> 1, st = t & 1;
+            const bool odd = h & 1, more = h + 2 < n_hall;
+            if (!odd && !(ok = wait_warp(bar_v + st, (uint32_t)(t >> 1) & 1u))) break;
+            if (!odd && more && !(ok = wait_warp(bar_k + (st ^ 1), (uint32_t)((t + 1) >> 1) & 1u))) break;
+#pragma unroll
+            for (int w = 0; w < 2; ++w) {
+                if (h < n_h[w]) {
+                    if (!(ok = wait_warp(bar_p + 2 * w + (h & 1), (uint32_t)t & 1u))) break;
+                    issue_pv(w, h);
+                }
+                if (w == 1 && odd) release(free_v + st);
+                if (h + 2 < n_h[w]) issue_s(w, h + 2);
+            }
+            if (ok && odd && more) release(free_k + (st ^ 1));
+        }
+    } else {
+        // =============================== softmax: warpgroup w, thread = row ===============================
+        const int w = warp >> 2, row = tid & (PA_TOK - 1), n_h = 2 * n_kv[w], qt = 2 * pair + w;
+        const uint32_t lane_base = tmem + ((uint32_t)(row & ~31) << 16);
+        const uint32_t t_o = lane_base + C_O + w * C_STEP;
+        const uint64_t scale2 = pair_of(p.scale_log2, p.scale_log2);
+        float m_run = -INFINITY, l_run = 0.f;   // the maximum the probabilities are expressed against; the row sum
+        bool ok = true;
+#pragma unroll 1
+        for (int h = 0; h < n_h; ++h) {
+            const uint32_t t_s = lane_base + C_S + w * C_STEP + (h & 1) * PP_HALF;
+            if (!(ok = wait_warp(bar_s + 2 * w + (h & 1), (uint32_t)(h >> 1) & 1u))) break;
+            tc_fence_after();
+            float s[PP_HALF];
+#pragma unroll
+            for (int c = 0; c < PP_HALF / 32; ++c) tmem_ld32_async(t_s + 32 * c, s + 32 * c);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < PP_HALF / 32; ++c) tmem_loaded32(s + 32 * c);
+            if ((h >> 1) == qt) {   // the diagonal tile: a key after the query is masked
+                const int last = row - (h & 1) * PP_HALF;
+#pragma unroll
+                for (int i = 0; i < PP_HALF; ++i)
+                    if (i > last) s[i] = -INFINITY;
+            }
+            float mx4[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                constexpr int Q = PP_HALF / 4;
+                mx4[c] = s[Q * c];
+#pragma unroll
+                for (int i = 1; i + 1 < Q; i += 2) mx4[c] = pa_max3(mx4[c], s[Q * c + i], s[Q * c + i + 1]);
+                mx4[c] = fmaxf(mx4[c], s[Q * c + Q - 1]);
+            }
+            // finite from the first half on: key 0 is never masked
+            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+            const bool move = mx > m_run + PA_RESCALE_STEP;   // also the first half (m_run = -inf)
+            float alpha = 1.f;
+            if (move) {
+                alpha = pa_ex2(m_run - mx);
+                m_run = mx;
+            }
+            if (h > 0 && __any_sync(0xffffffffu, move)) {
+                // PV(h) waits for this warp; PV(h-1) has completed when S(h+1), issued behind it, has
+                if (!(ok = h + 1 < n_h ? wait_warp(bar_s + 2 * w + ((h + 1) & 1), (uint32_t)((h + 1) >> 1) & 1u) : wait_warp(bar_o + w, 0))) break;
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float o[32];
+                    tmem_ld32(t_o + 32 * c, o);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) o[i] *= alpha;
+                    tmem_st32(t_o + 32 * c, o);
+                }
+            }
+            const uint64_t neg_m2 = pair_of(-m_run, -m_run);
+            uint64_t sum2[2] = {0ull, 0ull};
+#pragma unroll
+            for (int c = 0; c < PP_HALF / 32; ++c) {
+                uint32_t pk[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float a, b;
+                    halves_of(fma_pair(pair_of(s[32 * c + 2 * i], s[32 * c + 2 * i + 1]), scale2, neg_m2), a, b);
+                    a = pa_ex2(a);
+                    b = pa_ex2(b);
+                    sum2[i & 1] = add_pair(sum2[i & 1], pair_of(a, b));
+                    pk[i] = pa_pack(a, b, BF16);
+                }
+                tmem_st16(t_s + 16 * c, pk);
+            }
+            float a, b;
+            halves_of(add_pair(sum2[0], sum2[1]), a, b);
+            l_run = fmaf(l_run, alpha, a + b);
+            tmem_st_wait();
+            tc_fence_before();
+            pa_arrive(bar_p + 2 * w + (h & 1));
+        }
+        if (ok && n_h > 0) ok = wait_warp(bar_o + w, 0) && wait_warp(bar_o + w, 1);
+        if (ok && n_h > 0) {
+            tc_fence_after();
+            const float inv = 1.f / l_run;
+            const int64_t tok = (int64_t)qt * PA_TOK + row;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float o[32];
+                tmem_ld32(t_o + 32 * c, o);
+                if (tok < p.n_tokens) {
+                    uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + tok * p.out_stride_token +
+                                                          (int64_t)qh * p.out_stride_head + 32 * c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        dst[i] = make_uint4(pa_pack(o[8 * i] * inv, o[8 * i + 1] * inv, BF16), pa_pack(o[8 * i + 2] * inv, o[8 * i + 3] * inv, BF16),
+                                            pa_pack(o[8 * i + 4] * inv, o[8 * i + 5] * inv, BF16), pa_pack(o[8 * i + 6] * inv, o[8 * i + 7] * inv, BF16));
+                }
+            }
+        }
+        if (!ok && row == 0) atomicCAS(&g_tq_prefill_status, 0, (int)TQ_ERR_TIMEOUT);
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -466,7 +768,20 @@ extern "C" int tq_prefill_attention(const void* query, const void* key, const vo
         return (size_t)(1 + 2 * nst) * (D / 64) * PA_BOX + (size_t)2 * tpr * PA_TOK * sizeof(float) + 11 * sizeof(uint64_t) +
                16 + 1024;
     };
-    if (D == 128) {
+    // Pairs of query tiles where the launch is more than two waves of single tiles; below that the single tiles' four
+    // threads per row and twice the number of CTAs finish sooner.
+    if (D == 128 && (int64_t)p.n_tiles * num_q_heads > 2 * tq_sm_count()) {
+        const size_t smem = (size_t)6 * 2 * PA_BOX + 19 * sizeof(uint64_t) + 16 + 1024;
+        const dim3 pairs((unsigned)num_q_heads, (unsigned)((p.n_tiles + 1) / 2));
+        static TqSmemOptIn opt_b, opt_h;
+        if (bf16) {
+            if (tq_opt_in_smem(tq_prefill_pair_kernel<true>, smem, opt_b) != TQ_OK) return TQ_ERR_CUDA;
+            tq_prefill_pair_kernel<true><<<pairs, PP_THREADS, smem, st>>>(tm_q, tm_k, tm_v, p);
+        } else {
+            if (tq_opt_in_smem(tq_prefill_pair_kernel<false>, smem, opt_h) != TQ_OK) return TQ_ERR_CUDA;
+            tq_prefill_pair_kernel<false><<<pairs, PP_THREADS, smem, st>>>(tm_q, tm_k, tm_v, p);
+        }
+    } else if (D == 128) {
         const size_t smem = smem_of(2, PA_TPR);
         static TqSmemOptIn opt_in;
         if (tq_opt_in_smem(tq_prefill_attn_kernel<128, PA_AHEAD>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;

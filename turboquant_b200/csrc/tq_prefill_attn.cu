@@ -461,7 +461,7 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: known to be uniform
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tq_smem_u32(tmem_slot)), "r"(512)
@@ -532,28 +532,28 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
         const uint32_t aQ = tq_smem_u32(sQ), aK = tq_smem_u32(sK), aV = tq_smem_u32(sV);
         constexpr uint32_t idesc_s = umma_idesc_bf16(PP_HALF, false, !BF16), idesc_o = umma_idesc_bf16(D, true, !BF16);
-        auto issue_s = [&](int w, int h) {    // S_w(h) = Q_w K(h)^T
+        auto issue_s = [&](int w, int t, int odd) {    // S_w(h) = Q_w K(h)^T, h = 2 t + odd
             tc_fence_after();
             if (elected()) {
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks) {
                     const uint32_t off = (ks >> 2) * PA_BOX + (ks & 3) * 32;
-                    umma_ss(tmem_u + C_S + w * C_STEP + (h & 1) * PP_HALF, smem_desc_sw128(aQ + w * TILE_BYTES + off),
-                            smem_desc_sw128(aK + ((h >> 1) & 1) * TILE_BYTES + (h & 1) * PP_HALF * 128 + off), idesc_s, ks ? 1u : 0u);
+                    umma_ss(tmem_u + C_S + w * C_STEP + odd * PP_HALF, smem_desc_sw128(aQ + w * TILE_BYTES + off),
+                            smem_desc_sw128(aK + (t & 1) * TILE_BYTES + odd * PP_HALF * 128 + off), idesc_s, ks ? 1u : 0u);
                 }
-                umma_commit(bar_s + 2 * w + (h & 1));
+                umma_commit(bar_s + 2 * w + odd);
             }
             __syncwarp();
         };
-        auto issue_pv = [&](int w, int h) {   // O_w += P_w(h) V(h)
+        auto issue_pv = [&](int w, int t, int odd) {   // O_w += P_w(h) V(h)
             tc_fence_after();
             if (elected()) {
 #pragma unroll
                 for (int ks = 0; ks < PP_HALF / 16; ++ks)
-                    umma_ts(tmem_u + C_O + w * C_STEP, tmem_u + C_S + w * C_STEP + (h & 1) * PP_HALF + ks * 8,
-                            smem_desc_sw128_mn(aV + ((h >> 1) & 1) * TILE_BYTES + ((h & 1) * (PP_HALF / 16) + ks) * 2048, PA_BOX), idesc_o,
-                            (h | ks) ? 1u : 0u);
-                if (h + 2 >= 2 * n_kv[w]) umma_commit(bar_o + w);   // the last two: phases 0 and 1
+                    umma_ts(tmem_u + C_O + w * C_STEP, tmem_u + C_S + w * C_STEP + odd * PP_HALF + ks * 8,
+                            smem_desc_sw128_mn(aV + (t & 1) * TILE_BYTES + (odd * (PP_HALF / 16) + ks) * 2048, PA_BOX), idesc_o,
+                            (t | odd | ks) ? 1u : 0u);
+                if (t + 1 >= n_kv[w]) umma_commit(bar_o + w);   // the last two: phases 0 and 1
             }
             __syncwarp();
         };
@@ -565,28 +565,28 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         if (ok) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                issue_s(0, h);
-                if (n_kv[1]) issue_s(1, h);
+                issue_s(0, 0, h);
+                if (n_kv[1]) issue_s(1, 0, h);
             }
             release(free_k);
         }
-        const int n_h[2] = {2 * n_kv[0], 2 * n_kv[1]}, n_hall = 2 * n_all;
 #pragma unroll 1
-        for (int h = 0; h < n_hall && ok; ++h) {
-            const int t = h >> 1, st = t & 1;
-            const bool odd = h & 1, more = h + 2 < n_hall;
-            if (!odd && !(ok = wait_warp(bar_v + st, (uint32_t)(t >> 1) & 1u))) break;
-            if (!odd && more && !(ok = wait_warp(bar_k + (st ^ 1), (uint32_t)((t + 1) >> 1) & 1u))) break;
+        for (int t = 0; t < n_all && ok; ++t) {
+            const int st = t & 1;
+            const bool more = t + 1 < n_all;
+            if (!(ok = wait_warp(bar_v + st, (uint32_t)(t >> 1) & 1u))) break;
+            if (more && !(ok = wait_warp(bar_k + (st ^ 1), (uint32_t)((t + 1) >> 1) & 1u))) break;
 #pragma unroll
-            for (int w = 0; w < 2; ++w) {
-                if (h < n_h[w]) {
-                    if (!(ok = wait_warp(bar_p + 2 * w + (h & 1), (uint32_t)t & 1u))) break;
-                    issue_pv(w, h);
+            for (int hw = 0; hw < 4 && ok; ++hw) {   // halves, and in each both query tiles
+                const int odd = hw >> 1, w = hw & 1;
+                if (t < n_kv[w]) {
+                    if (!(ok = wait_warp(bar_p + 2 * w + odd, (uint32_t)t & 1u))) break;
+                    issue_pv(w, t, odd);
                 }
                 if (w == 1 && odd) release(free_v + st);
-                if (h + 2 < n_h[w]) issue_s(w, h + 2);
+                if (t + 1 < n_kv[w]) issue_s(w, t + 1, odd);
             }
-            if (ok && odd && more) release(free_k + (st ^ 1));
+            if (ok && more) release(free_k + (st ^ 1));
         }
     } else {
         // =============================== softmax: warpgroup w, thread = row ===============================

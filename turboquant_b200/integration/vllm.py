@@ -137,12 +137,13 @@ def _deliver(result: torch.Tensor, query: torch.Tensor, output, n: int):
     return result.to(query.dtype) if query.dim() == 3 else flat
 
 
-def _no_alloc_prefill_attention(state: LayerState, impl, query, key, value, attn_metadata) -> torch.Tensor:
+def _no_alloc_prefill_attention(state: LayerState, impl, query, key, value, attn_metadata, output=None) -> torch.Tensor:
     """Causal prefill attention from the layer's own K/V when no paged cache exists (reference
     vllm.py:150-180).  16-bit CUDA tensors with head_dim 128 / 256 go through the library's tensor-core
     kernel, which reads each kv head in place for its group of query heads (no repeat_interleave) and
     lets the store of the same K/V, launched next on the stream, begin under its tail; anything else
-    takes torch's attention like the reference."""
+    takes torch's attention like the reference.  Where the engine's `output` has the layout the kernel writes, the result
+    goes straight there (and is a view of it)."""
     c = state.config
     n = attn_metadata.num_actual_tokens
     q = _as_heads(query, n, c.num_query_heads, c.head_dim)
@@ -150,7 +151,12 @@ def _no_alloc_prefill_attention(state: LayerState, impl, query, key, value, attn
     v = _as_heads(value, n, c.num_kv_heads, c.head_dim)
     scale = getattr(impl, "scale", 1.0 / math.sqrt(c.head_dim))
     if E.prefill_attention_supported(q, k, v):
-        return E.prefill_attention(q, k, v, scale=scale)
+        out = None
+        if output is not None and output.dtype == q.dtype and output.device == q.device and output.is_contiguous() and \
+                output.shape[0] >= n and output[:n].numel() == q.numel() and output.data_ptr() % 16 == 0 and \
+                output.untyped_storage().data_ptr() not in [t.untyped_storage().data_ptr() for t in (q, k, v)]:
+            out = output[:n].view(q.shape)
+        return E.prefill_attention(q, k, v, scale=scale, out=out)
     rep = c.num_query_heads // c.num_kv_heads
     if rep > 1:
         k, v = k.repeat_interleave(rep, dim=1), v.repeat_interleave(rep, dim=1)
@@ -198,8 +204,10 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
         if attn_metadata.max_query_len > 1:            # prefill
             if not no_alloc:
                 return original(*args)
-            return _deliver(_no_alloc_prefill_attention(state, self_impl, query, key, value, attn_metadata),
-                            query, output, n)
+            result = _no_alloc_prefill_attention(state, self_impl, query, key, value, attn_metadata, output)
+            if output is not None and result.data_ptr() == output.data_ptr() and result.device == output.device:
+                return output
+            return _deliver(result, query, output, n)
         if mode == MODE_HYBRID and state.supports_hybrid and state.store.num_tokens >= MIN_HISTORY:
             if output is not None:                      # straight into the engine's buffer where its layout allows
                 st, ring = state.store, state.engine.ring

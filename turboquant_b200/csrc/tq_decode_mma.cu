@@ -35,7 +35,11 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 // Warps per CTA.  A launch that fits one wave runs 12-warp CTAs, one per SM (all of an SM's warps
 // share one set of query fragments and one merge).  A launch of several waves runs 8-warp CTAs, two
 // per SM, so that the set-up and the merge of one CTA overlap the main loop of the other.
+// One sequence at head_dim 128 runs 16 warps an SM instead (128 registers are enough there, and a fourth warp per scheduler
+// shortens the main loop: 4096 tokens 13.9 -> 12.9 us, eight layers of 16000 tokens 134 -> 124 us); at head_dim 256 it costs
+// registers (32768 tokens: 188 -> 195 us), and a few short sequences behind a paged write prefer the lighter CTA (25.8, not 26.5).
 constexpr int NW_WAVE = 12;
+constexpr int NW_SINGLE = 16;
 constexpr int NW_MULTI = 8;
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
 // A warp's softmax reference is put this far (in log2) above the largest score of the pair of records that raised it; it
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     bool failed = !__all_sync(0xffffffffu, tq_mbar_wait_bounded(bars + NW * NSTW, 0u));   // then no record is processed
     // Head_dim 256, and separate rotated / sketched sets in a CTA of 128 registers a thread: the fragments do not fit
     // beside the value accumulators and two records' score accumulators; they stay in shared memory, read once per pair.
-    constexpr bool BSM = R == 2 ? D == 256 || SPLITB : D == 256 && SPLITB;
+    constexpr bool BSM = R == 2 ? D == 256 || SPLITB : SPLITB && (D == 256 || NW == NW_SINGLE);
     uint32_t bq[BSM ? 1 : 2 * KS];
     uint32_t bsk[(SPLITB && !BSM) ? 2 * KS : 1];
 #define BQ(r) (BSM ? qf_s[QF_HDR + (r) * 32 + lane] : bq[BSM ? 0 : (r)])
@@ -719,7 +723,7 @@ size_t mma_land_bytes(int block_bytes, int nslot) {
     constexpr int GP = SPLITB ? 8 : 4;
     size_t s = (size_t)NW * NSTW * block_bytes + sizeof(float) * (2 * NW * GP) + sizeof(int) * BT_MAX;
     const size_t want = (size_t)nslot * GP * (D + 2) * sizeof(float);
-    if (NW == NW_WAVE && want > s && want <= 200 * 1024) s = want;
+    if (NW != NW_MULTI && want > s && want <= 200 * 1024) s = want;
     return (s + 127) / 128 * 128;
 }
 template <int D, bool SPLITB, int NW>
@@ -771,6 +775,9 @@ int launch_mma(const DecodeParams& p, int batch, cudaStream_t st, int* handled) 
     // two 8-warp CTAs per SM need two merge scratch areas in shared memory: only with few slots
     if (fits_multi && ((ctas > tq_sm_count() && nslot <= 128) || !fits_wave))
         return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_MULTI>(p, batch, st);
+    if constexpr (D == 128)
+        if (batch == 1 && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
+            return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_SINGLE>(p, batch, st);
     if (fits_wave) return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_WAVE>(p, batch, st);
     *handled = 0;
     return TQ_OK;

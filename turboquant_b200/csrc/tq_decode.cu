@@ -91,6 +91,13 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
             av = *reinterpret_cast<const uint4*>((const char*)ap.new_v + src + c * 16);
         }
     }
+    // The query's own bytes belong to the kernel ahead, but moving their lines into L2 reads nothing: whoever writes them
+    // does so there.  Saves the trip to memory behind the wait when the query was not written just now.
+    if (!ap.early_inputs) {
+        const int es = dt == TQ_F32 ? 4 : 2;
+        const int i = threadIdx.x * 128;
+        if (i < nv * D * es) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(q) + v0 * D * es + i));
+    }
     // Two passes over the same instructions.  The first is a rehearsal that runs while this grid would
     // otherwise sit waiting for the kernel ahead of it: it computes on whatever the query buffer holds
     // and stores nothing outside shared memory, but it pulls the code of the second pass - which is on

@@ -1401,3 +1401,22 @@ def test_decode_right_behind_a_store(nseq, n, splits, dev):
 def test_prefill_attention_pairs_of_query_tiles(qh, h, n, dtype, dev):
     """Launches of more than two waves of tiles: even and odd numbers of query tiles, a last tile of one row, a single tile."""
     test_prefill_attention_vs_fp32_reference(128, qh, h, n, dtype, dev)
+
+
+@pytest.mark.parametrize("d,kb,vb", [(128, 3, 2), (128, 4, 4), (256, 4, 2)])
+@pytest.mark.parametrize("n", [2048, 2049])
+def test_scattered_slots_on_both_sides_of_the_step_limit(d, kb, vb, n, dev):
+    """Shuffled slot mappings through both forms of the scatter: the same records as one aligned call."""
+    from turboquant_b200 import _engine as E
+    h = 2
+    c = E.LayerConstants(d, kb, vb, dev, seed=49)
+    k, v = (t.to(dev) for t in O.synth_kv(n, h, d, seed=n, dtype=torch.bfloat16))
+    nb = E.blocks_for(n)
+    a, b = E.BlockPool(c, h, nb), E.BlockPool(c, h, nb)
+    E.store(c, a, k, v, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=E.identity_block_table(nb, dev), start_pos=0)
+    order = torch.randperm(n, generator=torch.Generator().manual_seed(n)).to(dev)
+    E.store(c, b, k[order], v[order], stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, slot_mapping=order)
+    bt = E.identity_block_table(nb, dev)
+    for f in ("mse_indices", "qjl_signs", "norms", "residual_norms", "v_data", "v_scales", "v_zeros"):
+        assert torch.equal(getattr(E.pool_to_planes(c, a, bt, n), f), getattr(E.pool_to_planes(c, b, bt, n), f)), f
+    assert E.store_status() == 0

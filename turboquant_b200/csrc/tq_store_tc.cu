@@ -42,6 +42,7 @@ using namespace tqtc;
 
 namespace {
 
+constexpr int64_t SCATTER_MAX = 2048;           // slot mappings up to here are taken for a decode step's (see leave_records)
 constexpr int TC_D = 128;
 constexpr int TC_TOK = 128;
 constexpr int TC_THREADS = 512;                 // compute threads
@@ -82,6 +83,24 @@ __device__ int g_tq_store_status;   // 0 or a tq_status left by a bounded wait t
 constexpr uint32_t IDESC = umma_idesc_bf16(128);        // N = 128
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t accumulate) {
     tqtc::umma_ts(tmem_d, tmem_a, b_desc, IDESC, accumulate);
+}
+
+// Offset inside a block record of byte `cb` of token `tl`'s share (a token owns bytes_per_token bytes:
+// codes, signs, norm, residual norm, value codes, group scales, group zero points - in that order).
+__device__ __forceinline__ int rec_byte_offset(const TqLayout& L, int tl, int cb) {
+    if (cb < L.kcode_row) return L.off_kcodes + tl * L.kcode_row + cb;
+    cb -= L.kcode_row;
+    if (cb < L.ksign_row) return L.off_ksigns + tl * L.ksign_row + cb;
+    cb -= L.ksign_row;
+    if (cb < 2) return L.off_knorm + tl * 2 + cb;
+    cb -= 2;
+    if (cb < 2) return L.off_krnorm + tl * 2 + cb;
+    cb -= 2;
+    if (cb < L.vcode_row) return L.off_vcodes + tq_vcode_native(L.D, L.val_bits, tl, cb);
+    cb -= L.vcode_row;
+    if (cb < 2 * L.ngroups) return L.off_vscale + ((cb >> 1) * TQ_BLOCK_TOKENS + tl) * 2 + (cb & 1);
+    cb -= 2 * L.ngroups;
+    return L.off_vzero + ((cb >> 1) * TQ_BLOCK_TOKENS + tl) * 2 + (cb & 1);
 }
 
 // A token's share of a block record as 16-bit units: codes, signs, norm, residual norm, value codes (whose byte pairs stay
@@ -217,25 +236,29 @@ struct RecordDest {
     int64_t slot = -1;    // slot mode: slot of row `lane & 15`
     bool asked = false;
 };
+template <bool SCATTER>
 __device__ __forceinline__ void ask_destination(const TcParams& p, int64_t tok0, int warp, int lane, RecordDest& d) {
-    if (p.slot_mapping == nullptr) {
+    if (!SCATTER && warp >= 8) return;
+    if (!SCATTER && p.slot_mapping == nullptr) {
         const int64_t first = tok0 + warp * TQ_BLOCK_TOKENS;      // token index of the block's first row
-        d.asked = warp < 8 && lane == 0 && first < p.n_tokens && first + TQ_BLOCK_TOKENS > 0;
+        d.asked = lane == 0 && first < p.n_tokens && first + TQ_BLOCK_TOKENS > 0;
         if (d.asked) d.blk = __ldg(p.block_table + ((p.start_pos + first) >> 4));
     } else {
-        const int64_t i = tok0 + (warp & 7) * TQ_BLOCK_TOKENS + (lane & 15);
+        const int64_t i = tok0 + (SCATTER ? warp & 7 : warp) * TQ_BLOCK_TOKENS + (lane & 15);
         if (i >= 0 && i < p.n_tokens) d.slot = __ldg(p.slot_mapping + i);
     }
 }
-// Warps j and j + 8 send image block j on its way: one bulk (TMA) store when the block is a whole record of the pool, a
-// scatter to each token's own slot otherwise, eight tokens a warp.  The scatter works out where a lane's units lie once and
-// moves 16 bits at a time; byte by byte, with the offsets found anew for each, it was two thirds of a decode step's write
-// (5 tokens of 8 heads: 14.8 us a launch, 64 tokens at 4/4 bits 32 us).
+// Warp j < 8 (SCATTER: warps j and j + 8) sends image block j on its way: one bulk (TMA) store when the block is a whole record of
+// the pool, a byte scatter to each token's own slot otherwise.
+// SCATTER is for the writes of a decode step, where next to every row goes to a block of its own: the offsets of a lane's
+// units are worked out once, sixteen warps share the rows.  Byte by byte, with the offsets found anew for each, the scatter was
+// two thirds of such a write (5 tokens of 8 heads 14.8 us, 64 tokens at 4/4 bits 32 us; now 8.7 and 14).  Whole records leave
+// the same way in both; the kernel without it stays 3 % faster on long chunks (16 x 8192 tokens: 331 against 340 us).
+template <bool SCATTER>
 __device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout& L, const uint8_t* img, int h, int warp,
                                               int lane, const RecordDest& d) {
-    const int j = warp & 7;
-    const int BB = L.block_bytes;
-    if (p.slot_mapping == nullptr) {
+    const int BB = L.block_bytes, j = SCATTER ? warp & 7 : warp;
+    if (!SCATTER && p.slot_mapping == nullptr) {
         if (d.asked) {
             if (d.blk >= 0 && d.blk < p.num_blocks) {
                 tq_bulk_s2g(p.pool + ((int64_t)d.blk * p.H + h) * (int64_t)BB, img + j * BB, (uint32_t)BB);
@@ -246,7 +269,8 @@ __device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout&
         }
         return;
     }
-    // slot mapping: sixteen rows that fill one block in order leave as a whole record, anything else is scattered
+    // slot mapping: sixteen rows that fill one block in order leave as a whole record, anything else is
+    // scattered byte by byte
     int64_t slot = d.slot;
     if (slot >= 0 && (slot >> 4) >= p.num_blocks) {
         atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_RANGE);
@@ -255,31 +279,43 @@ __device__ __forceinline__ void leave_records(const TcParams& p, const TqLayout&
     const int64_t slot0 = __shfl_sync(0xffffffffu, slot, 0);
     const bool whole = __all_sync(0xffffffffu, slot0 >= 0 && (slot0 & 15) == 0 && slot == slot0 + (lane & 15));
     if (whole) {
-        if (lane == 0 && warp < 8) {
+        if (lane == 0 && (!SCATTER || warp < 8)) {
             tq_bulk_s2g(p.pool + ((slot0 >> 4) * p.H + h) * (int64_t)BB, img + j * BB, (uint32_t)BB);
             tq_bulk_commit();
         }
         return;
     }
-    const int units = BB / TQ_BLOCK_TOKENS / 2;
-    const uint8_t* src = img + j * BB;
-    constexpr int NU = (REC_UNITS_MAX + 31) / 32;
-    RecUnit un[NU];
+    if (SCATTER) {
+        const int units = BB / TQ_BLOCK_TOKENS / 2;
+        const uint8_t* src = img + j * BB;
+        constexpr int NU = (REC_UNITS_MAX + 31) / 32;
+        RecUnit un[NU];
 #pragma unroll
-    for (int i = 0; i < NU; ++i) un[i] = rec_unit(L, min(lane + 32 * i, units - 1));
-    const int half_bytes = L.val_bits == 2 && L.D == 128 ? 8 : L.D * L.val_bits;   // value codes: second token pair of a quad
-    auto vpart = [&](int t) { return (t >> 2) * 16 + ((t >> 1) & 1) * half_bytes + (t & 1) * 2; };
+        for (int i = 0; i < NU; ++i) un[i] = rec_unit(L, min(lane + 32 * i, units - 1));
+        const int half_bytes = L.val_bits == 2 && L.D == 128 ? 8 : L.D * L.val_bits;   // value codes: second token pair of a quad
+        auto vpart = [&](int t) { return (t >> 2) * 16 + ((t >> 1) & 1) * half_bytes + (t & 1) * 2; };
 #pragma unroll 2
-    for (int t = warp & 8; t < (warp & 8) + 8; ++t) {
+        for (int t = warp & 8; t < (warp & 8) + 8; ++t) {
+            const int64_t s = __shfl_sync(0xffffffffu, slot, t);
+            if (s < 0) continue;
+            uint8_t* dst = p.pool + ((s >> 4) * p.H + h) * (int64_t)BB;
+            const int td = (int)(s & 15), vs = vpart(t), vd = vpart(td);
+#pragma unroll
+            for (int i = 0; i < NU; ++i)
+                if (lane + 32 * i < units)
+                    *reinterpret_cast<uint16_t*>(dst + un[i].base + un[i].stride * td + (un[i].vcode ? vd : 0)) =
+                        *reinterpret_cast<const uint16_t*>(src + un[i].base + un[i].stride * t + (un[i].vcode ? vs : 0));
+        }
+        return;
+    }
+    const int per_tok = BB / TQ_BLOCK_TOKENS;
+    const uint8_t* src = img + j * BB;
+    for (int t = 0; t < TQ_BLOCK_TOKENS; ++t) {
         const int64_t s = __shfl_sync(0xffffffffu, slot, t);
         if (s < 0) continue;
         uint8_t* dst = p.pool + ((s >> 4) * p.H + h) * (int64_t)BB;
-        const int td = (int)(s & 15), vs = vpart(t), vd = vpart(td);
-#pragma unroll
-        for (int i = 0; i < NU; ++i)
-            if (lane + 32 * i < units)
-                *reinterpret_cast<uint16_t*>(dst + un[i].base + un[i].stride * td + (un[i].vcode ? vd : 0)) =
-                    *reinterpret_cast<const uint16_t*>(src + un[i].base + un[i].stride * t + (un[i].vcode ? vs : 0));
+        for (int cb = lane; cb < per_tok; cb += 32)
+            dst[rec_byte_offset(L, (int)(s & 15), cb)] = src[rec_byte_offset(L, t, cb)];
     }
 }
 
@@ -341,7 +377,7 @@ __device__ __forceinline__ bool compute_barrier_or(bool flag) {
 // Compute thread (row = tid % 128, q = tid / 128), tid < 512, owns channels [32q, 32q+32) of token row
 // `row` - one value group, 16 packed columns of an A operand, 32 accumulator columns.  Warp w reads
 // and writes TMEM lanes of quarter w % 4 = row / 32, as the hardware requires.  Warp 16 only issues.
-template <int MSE_BITS, int VAL_BITS>
+template <int MSE_BITS, int VAL_BITS, bool SCATTER>
 __global__ void __launch_bounds__(TC_LAUNCH, 1)
 tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                    const __grid_constant__ CUtensorMap tm_kt, const __grid_constant__ CUtensorMap tm_vt,
@@ -375,7 +411,7 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool slot_mode = p.slot_mapping != nullptr;
+    const bool slot_mode = SCATTER || p.slot_mapping != nullptr;
     // The launch that follows in the stream may take over each SM as soon as this CTA leaves it; whatever
     // it reads or writes in the pool comes after its own wait for this grid (see pool_writes_may_begin).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -668,7 +704,7 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             uint8_t* rec = img + blk_l * BB;
 
             RecordDest dest;
-            ask_destination(p, tok0, warp, lane, dest);
+            ask_destination<SCATTER>(p, tok0, warp, lane, dest);
 
             // ---------------- C: codes and rotated-space residual of channels [32q, 32q+32) ----------------
             bad |= !wait_warp(bar_y, par);
@@ -767,9 +803,11 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             }
 
             // ---------------- the tile's block records leave ----------------
-            if (tile_no == 0) pool_writes_may_begin();
-            leave_records(p, L, img, h, warp, lane, dest);
-            if (lane == 0 && warp < 8 && p.n_rec_buf == 1) tq_bulk_wait_all_read();
+            if (SCATTER || warp < 8) {   // the other warps need not wait for the launch ahead
+                if (tile_no == 0) pool_writes_may_begin();
+                leave_records<SCATTER>(p, L, img, h, warp, lane, dest);
+                if (lane == 0 && warp < 8 && p.n_rec_buf == 1) tq_bulk_wait_all_read();
+            }
             if (p.n_rec_buf == 1) {
                 compute_barrier_or(false);                // the single image is rewritten by the values below
                 if (has_next) phase_v(par ^ 1, nimg, tile_tok0(next));
@@ -817,7 +855,7 @@ constexpr size_t d2_smem(size_t img) {
            13 * sizeof(uint64_t) + 16 + 1024;
 }
 
-template <int MSE_BITS, int VAL_BITS, int ROWS = d2_ring_rows<MSE_BITS, VAL_BITS>()>
+template <int MSE_BITS, int VAL_BITS, bool SCATTER, int ROWS = d2_ring_rows<MSE_BITS, VAL_BITS>()>
 __global__ void __launch_bounds__(TC_LAUNCH, 1)
 tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_kt, const __grid_constant__ CUtensorMap tm_vt,
@@ -843,7 +881,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool slot_mode = p.slot_mapping != nullptr;
+    const bool slot_mode = SCATTER || p.slot_mapping != nullptr;
     // The launch that follows in the stream may take over each SM as soon as this CTA leaves it; whatever
     // it reads or writes in the pool comes after its own wait for this grid (see pool_writes_may_begin).
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1039,7 +1077,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             const bool wr = tok0 + row >= 0;
             uint8_t* rec = sRec + blk_l * BB;
             RecordDest dest;
-            ask_destination(p, tok0, warp, lane, dest);
+            ask_destination<SCATTER>(p, tok0, warp, lane, dest);
 
             // ---------------- V: the two value groups of channels [64q, 64q+64) ----------------
             if (tile_no == 0 && rmw) bad |= !wait_warp(bar_r, 0);
@@ -1170,9 +1208,11 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             }
             tq_fence_proxy_async();
             compute_barrier_or(false);       // record image complete
-            if (tile_no == 0) pool_writes_may_begin();
-            leave_records(p, L, sRec, h, warp, lane, dest);
-            if (lane == 0 && warp < 8) tq_bulk_wait_all_read();
+            if (SCATTER || warp < 8) {
+                if (tile_no == 0) pool_writes_may_begin();
+                leave_records<SCATTER>(p, L, sRec, h, warp, lane, dest);
+                if (lane == 0 && warp < 8) tq_bulk_wait_all_read();
+            }
             compute_barrier_or(false);       // the image and s_ss are free for the next tile
         }
         if (!ok && tid == 0) atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_TIMEOUT);
@@ -1368,6 +1408,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     *handled = 1;
 
     const int mse_bits = cfg.key_bits - 1;
+    const bool scatter = slot_mapping != nullptr && n_tokens <= SCATTER_MAX;
     const int sms = tq_sm_count();
     const unsigned grid = (unsigned)(p.n_tiles < sms ? p.n_tiles : sms);
     // programmatic dependent launch: this grid may begin under the tail of the launch ahead of it
@@ -1384,39 +1425,43 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     cudaError_t launched = cudaSuccess;
     if (D == D2) {
         p.n_rec_buf = 1;
-#define TQ_TC256(MB, VB)                                                                                         \
+#define TQ_TC256_(MB, VB, SL)                                                                                         \
     do {                                                                                                         \
         static TqSmemOptIn opt_in;                                                                               \
         const size_t smem = d2_smem<d2_ring_rows<MB, VB>()>(img);                                                \
         static_assert(d2_ring_rows<2, 2>() == 256 && d2_ring_rows<2, 4>() == 128, "boxes of the operand maps");  \
-        if (tq_opt_in_smem(tq_store_tc256_kernel<MB, VB>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;            \
+        if (tq_opt_in_smem(tq_store_tc256_kernel<MB, VB, SL>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;            \
         lc.dynamicSmemBytes = smem;                                                                              \
-        launched = cudaLaunchKernelEx(&lc, tq_store_tc256_kernel<MB, VB>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1], \
+        launched = cudaLaunchKernelEx(&lc, tq_store_tc256_kernel<MB, VB, SL>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1], \
                                       tm_b[2], tm_b[3], p);                                                      \
     } while (0)
+#define TQ_TC256(MB, VB) do { if (scatter) TQ_TC256_(MB, VB, true); else TQ_TC256_(MB, VB, false); } while (0)
         if (mse_bits == 2 && cfg.value_bits == 2) TQ_TC256(2, 2);
         else if (mse_bits == 2) TQ_TC256(2, 4);
         else if (cfg.value_bits == 2) TQ_TC256(3, 2);
         else TQ_TC256(3, 4);
 #undef TQ_TC256
+#undef TQ_TC256_
         return launched == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
     }
     const size_t fixed = (size_t)6 * MAT_BYTES + 8 * TC_TOK * sizeof(float) + 12 * sizeof(uint64_t) + 16 + 1024;
     p.n_rec_buf = fixed + 2 * img <= SMEM_LIMIT ? 2 : 1;
     const size_t smem = fixed + (size_t)p.n_rec_buf * img;
-#define TQ_TC(MB, VB)                                                                                            \
+#define TQ_TC_(MB, VB, SL)                                                                                            \
     do {                                                                                                         \
         static TqSmemOptIn opt_in;                                                                               \
-        if (tq_opt_in_smem(tq_store_tc_kernel<MB, VB>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;               \
+        if (tq_opt_in_smem(tq_store_tc_kernel<MB, VB, SL>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;               \
         lc.dynamicSmemBytes = smem;                                                                              \
-        launched = cudaLaunchKernelEx(&lc, tq_store_tc_kernel<MB, VB>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1],   \
+        launched = cudaLaunchKernelEx(&lc, tq_store_tc_kernel<MB, VB, SL>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1],   \
                                       tm_b[2], tm_b[3], p);                                                      \
     } while (0)
+#define TQ_TC(MB, VB) do { if (scatter) TQ_TC_(MB, VB, true); else TQ_TC_(MB, VB, false); } while (0)
     if (mse_bits == 2 && cfg.value_bits == 2) TQ_TC(2, 2);
     else if (mse_bits == 2) TQ_TC(2, 4);
     else if (cfg.value_bits == 2) TQ_TC(3, 2);
     else TQ_TC(3, 4);
 #undef TQ_TC
+#undef TQ_TC_
     return launched == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
 }
 

@@ -1420,3 +1420,21 @@ def test_scattered_slots_on_both_sides_of_the_step_limit(d, kb, vb, n, dev):
     for f in ("mse_indices", "qjl_signs", "norms", "residual_norms", "v_data", "v_scales", "v_zeros"):
         assert torch.equal(getattr(E.pool_to_planes(c, a, bt, n), f), getattr(E.pool_to_planes(c, b, bt, n), f)), f
     assert E.store_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_rows_of_a_wider_tensor_equal_contiguous_rows(dtype, dev):
+    """What the native calls leave to the general way (strided rows, a query shared by the heads) gives the same tensors."""
+    from turboquant_b200 import TurboQuantProd
+    from turboquant_b200.kv_cache import quantize_values
+    g = torch.Generator().manual_seed(5)
+    wide = torch.randn(2, 40, 256, generator=g).to(dtype).to(dev)
+    x, q = wide[..., :128], torch.randn(2, 3, 128, generator=g).to(dtype).to(dev)
+    z = TurboQuantProd(128, 3, device=dev)
+    a, b = z.quantize(x), z.quantize(x.contiguous())
+    for s, t in zip(a[:4], b[:4]):
+        assert s.shape == t.shape and s.dtype == t.dtype and torch.equal(s, t)
+    for s, t in zip(quantize_values(x, 2)[:3], quantize_values(x.contiguous(), 2)[:3]):
+        assert s.shape == t.shape and s.dtype == t.dtype and torch.equal(s, t)
+    one = z.quantize(x[0].contiguous())
+    assert torch.equal(z.attention_score(q[:1].expand(2, 3, 128), a)[0], z.attention_score(q[0], one))

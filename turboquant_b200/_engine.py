@@ -431,6 +431,14 @@ def dequant_values(consts: LayerConstants, pool: BlockPool, block_table: torch.T
     return out
 
 
+def taken(result, what: str):
+    """What a call of the native host path returned: its tensors, None where it left the call to the general way; raises on a
+    status."""
+    if type(result) is int:
+        check(result, what)
+    return result
+
+
 def _float_code(t: torch.Tensor) -> Optional[int]:
     return _DTYPES.get(t.dtype)
 

@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cmath>
+#include <vector>
 
 #include "turboquant_b200.h"
 
@@ -306,7 +307,150 @@ PyObject* batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
+// ------------------------------------------------------------------ the quantiser objects on plain rows
+
+// sizes of `t` without its last dimension, then `tail`
+inline std::vector<int64_t> lead_shape(const at::Tensor& t, std::initializer_list<int64_t> tail) {
+    std::vector<int64_t> s(t.sizes().begin(), t.sizes().end() - 1);
+    s.insert(s.end(), tail);
+    return s;
+}
+inline bool rows_tensor(const at::Tensor* t) { return t && t->is_cuda() && t->is_contiguous() && t->dim() >= 1 && t->numel() > 0; }
+inline bool declined(int rc) { return rc == TQ_ERR_UNSUPPORTED || rc == TQ_ERR_ALIGN || rc == TQ_ERR_SHAPE; }
+PyObject* tuple_of(std::initializer_list<at::Tensor> ts) {
+    PyObject* r = PyTuple_New((Py_ssize_t)ts.size());
+    Py_ssize_t i = 0;
+    for (const at::Tensor& t : ts) PyTuple_SET_ITEM(r, i++, THPVariable_Wrap(t));
+    return r;
+}
+
+// quantize_keys(consts, x (..., D)) -> (codes, sign bits, norms, residual norms), status, or None
+PyObject* quantize_keys(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(2);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const at::Tensor* x = tensor_or_null(args[1]);
+    if (PyErr_Occurred()) return nullptr;
+    const int64_t d = c->cfg.head_dim;
+    if (!rows_tensor(x) || x->size(-1) != d) Py_RETURN_NONE;
+    const int dt = dtype_code(x->scalar_type());
+    if (dt != TQ_F32 && dt != TQ_F16) Py_RETURN_NONE;
+    const auto bytes = x->options().dtype(at::kByte);
+    at::Tensor codes = at::empty(lead_shape(*x, {c->cfg.key_bits == 3 ? d / 4 : d / 2}), bytes), signs = at::empty(lead_shape(*x, {d / 8}), bytes),
+               norms = at::empty(lead_shape(*x, {}), x->options()), rnorms = at::empty(lead_shape(*x, {}), x->options().dtype(at::kFloat));
+    const int rc = tq_rows_quantize_keys(c, x->data_ptr(), (tq_dtype)dt, x->numel() / d, d, codes.data_ptr<uint8_t>(), signs.data_ptr<uint8_t>(),
+                                         norms.data_ptr(), (tq_dtype)dt, rnorms.data_ptr(), TQ_F32, stream_of(*x));
+    if (declined(rc)) Py_RETURN_NONE;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    return tuple_of({codes, signs, norms, rnorms});
+    END_HANDLE_TH_ERRORS
+}
+
+// dequantize_keys(consts, codes, sign bits | None, norms, residual norms | None) -> rows fp32, status, or None
+PyObject* dequantize_keys(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(5);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const at::Tensor *codes = tensor_or_null(args[1]), *signs = tensor_or_null(args[2]), *norms = tensor_or_null(args[3]), *rn = tensor_or_null(args[4]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!rows_tensor(codes) || !rows_tensor(norms) || (signs && !rows_tensor(signs)) || (rn && !rows_tensor(rn)) || (signs != nullptr) != (rn != nullptr))
+        Py_RETURN_NONE;
+    const int64_t d = c->cfg.head_dim, n = norms->numel(), row = c->cfg.key_bits == 3 ? d / 4 : d / 2;
+    const int dn = dtype_code(norms->scalar_type()), dr = rn ? dtype_code(rn->scalar_type()) : TQ_F32;
+    if (dn < 0 || dr < 0 || codes->scalar_type() != at::kByte || codes->numel() != n * row || (signs && (signs->scalar_type() != at::kByte ||
+        signs->numel() != n * (d / 8) || rn->numel() != n)))
+        Py_RETURN_NONE;
+    std::vector<int64_t> shape(norms->sizes().begin(), norms->sizes().end());
+    shape.push_back(d);
+    at::Tensor out = at::empty(shape, norms->options().dtype(at::kFloat));
+    const int rc = tq_rows_dequantize_keys(c, codes->data_ptr<uint8_t>(), signs ? signs->data_ptr<uint8_t>() : nullptr, norms->data_ptr(), (tq_dtype)dn,
+                                           rn ? rn->data_ptr() : nullptr, (tq_dtype)dr, n, signs ? 1 : 0, out.data_ptr<float>(), stream_of(*codes));
+    if (declined(rc)) Py_RETURN_NONE;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
+// key_scores(consts, workspace, query (..., n_q, D), codes, sign bits, norms (..., n), residual norms) -> logits, status, or None
+PyObject* key_scores(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(7);
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const at::Tensor *q = tensor_or_null(args[2]), *codes = tensor_or_null(args[3]), *signs = tensor_or_null(args[4]), *norms = tensor_or_null(args[5]),
+                     *rn = tensor_or_null(args[6]);
+    if (PyErr_Occurred()) return nullptr;
+    const int64_t d = c->cfg.head_dim;
+    if (!rows_tensor(q) || !rows_tensor(codes) || !rows_tensor(signs) || !rows_tensor(norms) || !rows_tensor(rn) || q->dim() < 2 || q->size(-1) != d)
+        Py_RETURN_NONE;
+    const int64_t n = norms->size(-1), heads = norms->numel() / n, n_q = q->size(-2);
+    const int dq = dtype_code(q->scalar_type()), dn = dtype_code(norms->scalar_type()), dr = dtype_code(rn->scalar_type());
+    if (dq < 0 || dn < 0 || dr < 0 || q->numel() != heads * n_q * d || rn->numel() != norms->numel() || codes->scalar_type() != at::kByte ||
+        signs->scalar_type() != at::kByte || codes->numel() != heads * n * (c->cfg.key_bits == 3 ? d / 4 : d / 2) || signs->numel() != heads * n * (d / 8))
+        Py_RETURN_NONE;
+    size_t need = 0, bytes = 0;
+    void* ws = nullptr;
+    int rc = tq_scores_workspace_bytes(&c->cfg, heads * n_q, &need);
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    if (!workspace(args[1], need, &ws, &bytes)) return nullptr;
+    std::vector<int64_t> shape(norms->sizes().begin(), norms->sizes().end() - 1);
+    shape.push_back(n_q);
+    shape.push_back(n);
+    at::Tensor logits = at::empty(shape, norms->options().dtype(at::kFloat));
+    rc = tq_rows_scores(c, codes->data_ptr<uint8_t>(), signs->data_ptr<uint8_t>(), norms->data_ptr(), (tq_dtype)dn, rn->data_ptr(), (tq_dtype)dr,
+                        (int32_t)heads, n, q->data_ptr(), (tq_dtype)dq, (int32_t)n_q, logits.data_ptr<float>(), ws, bytes, stream_of(*q));
+    if (declined(rc)) Py_RETURN_NONE;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(logits));
+    END_HANDLE_TH_ERRORS
+}
+
+// quantize_values(v (..., D), bits) -> (codes, scales, zero points), status, or None
+PyObject* quantize_values(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(2);
+    const at::Tensor* v = tensor_or_null(args[0]);
+    const int64_t bits = PyLong_AsLongLong(args[1]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!rows_tensor(v)) Py_RETURN_NONE;
+    const int64_t d = v->size(-1);
+    const int dt = dtype_code(v->scalar_type());
+    if (dt < 0 || (d != 128 && d != 256) || (bits != 2 && bits != 4)) Py_RETURN_NONE;
+    at::Tensor data = at::empty(lead_shape(*v, {d * bits / 8}), v->options().dtype(at::kByte)), scales = at::empty(lead_shape(*v, {d / 32}), v->options()),
+               zeros = at::empty(lead_shape(*v, {d / 32}), v->options());
+    const int rc = tq_rows_quantize_values(v->data_ptr(), (tq_dtype)dt, v->numel() / d, (int32_t)d, d, (int32_t)bits, data.data_ptr<uint8_t>(),
+                                           scales.data_ptr(), zeros.data_ptr(), stream_of(*v));
+    if (declined(rc)) Py_RETURN_NONE;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    return tuple_of({data, scales, zeros});
+    END_HANDLE_TH_ERRORS
+}
+
+// dequantize_values(codes, scales, zero points, bits) -> rows fp32, status, or None
+PyObject* dequantize_values(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(4);
+    const at::Tensor *data = tensor_or_null(args[0]), *sc = tensor_or_null(args[1]), *zr = tensor_or_null(args[2]);
+    const int64_t bits = PyLong_AsLongLong(args[3]);
+    if (PyErr_Occurred()) return nullptr;
+    if (!rows_tensor(data) || !rows_tensor(sc) || !rows_tensor(zr) || (bits != 2 && bits != 4) || data->scalar_type() != at::kByte) Py_RETURN_NONE;
+    const int64_t d = data->size(-1) * 8 / bits, n = data->numel() / data->size(-1);
+    const int dt = dtype_code(sc->scalar_type());
+    if (dt < 0 || (d != 128 && d != 256) || zr->scalar_type() != sc->scalar_type() || sc->numel() != n * (d / 32) || zr->numel() != sc->numel()) Py_RETURN_NONE;
+    at::Tensor out = at::empty(lead_shape(*data, {d}), data->options().dtype(at::kFloat));
+    const int rc = tq_rows_dequantize_values(data->data_ptr<uint8_t>(), sc->data_ptr(), zr->data_ptr(), (tq_dtype)dt, n, (int32_t)d, (int32_t)bits,
+                                             out.data_ptr<float>(), stream_of(*data));
+    if (declined(rc)) Py_RETURN_NONE;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"quantize_keys", (PyCFunction)(void (*)(void))quantize_keys, METH_FASTCALL, nullptr},
+    {"dequantize_keys", (PyCFunction)(void (*)(void))dequantize_keys, METH_FASTCALL, nullptr},
+    {"key_scores", (PyCFunction)(void (*)(void))key_scores, METH_FASTCALL, nullptr},
+    {"quantize_values", (PyCFunction)(void (*)(void))quantize_values, METH_FASTCALL, nullptr},
+    {"dequantize_values", (PyCFunction)(void (*)(void))dequantize_values, METH_FASTCALL, nullptr},
     {"ring_write", (PyCFunction)(void (*)(void))ring_write, METH_FASTCALL, nullptr},
     {"store", (PyCFunction)(void (*)(void))store, METH_FASTCALL, nullptr},
     {"hybrid", (PyCFunction)(void (*)(void))hybrid, METH_FASTCALL, nullptr},

@@ -63,6 +63,9 @@ def quantize_values(v: torch.Tensor, bits: int = 2, group_size: int = 32) -> Val
     E.require_cuda(v, "v")
     d = v.shape[-1]
     _check_value_shape(d, bits)
+    got = E.taken(E.host().quantize_values(v, bits), "tq_rows_quantize_values")
+    if got is not None:
+        return ValueQuantized(*got, bits)
     lead = v.shape[:-1]
     v2 = v.reshape(-1, d)
     if v2.stride(-1) != 1:
@@ -89,6 +92,9 @@ def dequantize_values(vq: ValueQuantized, group_size: int = 32) -> torch.Tensor:
     E.require_cuda(data, "vq.data")
     d = data.shape[-1] * (4 if bits == 2 else 2)
     _check_value_shape(d, bits)
+    out = E.taken(E.host().dequantize_values(data, vq.scales, vq.zeros, bits), "tq_rows_dequantize_values")
+    if out is not None:
+        return out
     if data.numel():
         out = E.rows_dequantize_values(data.contiguous(), vq.scales.contiguous(), vq.zeros.contiguous(), bits, d)
         if out is not None:

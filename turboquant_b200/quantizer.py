@@ -73,6 +73,9 @@ class _QuantizerBase(torch.nn.Module):
 
     def _dequantize(self, indices, signs, norms, residual_norms) -> torch.Tensor:
         if indices.numel() and self._rows_operands():
+            out = E.taken(E.host().dequantize_keys(self.consts.addr, indices, signs, norms, residual_norms), "tq_rows_dequantize_keys")
+            if out is not None:
+                return out
             args = [None if t is None else t.contiguous() for t in (indices, signs, norms, residual_norms)]
             out = E.rows_dequantize_keys(self.consts, *args)
             if out is not None:
@@ -152,6 +155,10 @@ class TurboQuantProd(_QuantizerBase):
         return self._mse
 
     def quantize(self, x: torch.Tensor) -> ProdQuantized:
+        if x.is_cuda and self._rows_operands():
+            got = E.taken(E.host().quantize_keys(self.consts.addr, x), "tq_rows_quantize_keys")
+            if got is not None:
+                return ProdQuantized(got[0], got[1], got[3], got[2], self.bits - 1)
         lead, x2 = _rows(x)
         codes, signs, norms, rnorms = self._planes_of(x2)
         return ProdQuantized(codes.reshape(*lead, -1), signs.reshape(*lead, -1), rnorms.reshape(lead), norms.reshape(lead),
@@ -163,6 +170,10 @@ class TurboQuantProd(_QuantizerBase):
     def attention_score(self, query: torch.Tensor, quantized_key: ProdQuantized) -> torch.Tensor:
         """query (..., n_q, d), keys (..., n_k, ...) -> unscaled logits (..., n_q, n_k)."""
         k = quantized_key
+        logits = E.taken(E.host().key_scores(self.consts.addr, self._ws, query, k.mse_indices, k.qjl_signs, k.norms, k.residual_norms),
+                         "tq_rows_scores") if query.is_cuda else None
+        if logits is not None:
+            return logits
         n = k.mse_indices.shape[-2]
         heads = max(1, k.mse_indices.numel() // (n * k.mse_indices.shape[-1])) if n else 1
         n_q = query.shape[-2]

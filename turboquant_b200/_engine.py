@@ -523,54 +523,23 @@ def rows_dequantize_values(data: torch.Tensor, scales: torch.Tensor, zeros: torc
     return out
 
 
-def _buffer_rows(buf: Optional[torch.Tensor]):
-    """(b, h, n, d) exact rows as (pointer, dtype, n, stride per (b, h), stride per token), contiguous if need be."""
-    if buf is None or buf.shape[2] == 0:
-        return None, TQ_F32, 0, 0, 0, None
-    es = buf.element_size()
-    if buf.stride(3) != 1 or (buf.shape[0] > 1 and buf.stride(0) != buf.shape[1] * buf.stride(1)) or buf.data_ptr() % 16 or \
-            (buf.stride(1) * es) % 16 or (buf.stride(2) * es) % 16:
-        buf = buf.contiguous()
-    return buf.data_ptr(), dtype_code(buf.dtype), buf.shape[2], buf.stride(1), buf.stride(2), buf
-
-
-def _cache_workspace(consts, ws, heads: int, n: int, n_buf: int, n_q: int) -> None:
-    need = C.c_size_t(0)
-    check(lib().tq_cache_workspace_bytes(C.byref(consts.cfg), heads, n, n_buf, n_q, C.byref(need)), "tq_cache_workspace_bytes")
-    ws.ensure(need.value)
-
-
 def cache_scores(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: torch.Tensor, n: int, query: torch.Tensor,
                  buf: Optional[torch.Tensor], scale: float) -> Optional[torch.Tensor]:
-    """query (b*h, n_q, D) contiguous -> scaled logits (b*h, n_q, n + buffer) fp32, or None where the kernel does not apply."""
-    if _float_code(query) is None or (buf is not None and buf.dtype not in _DTYPES):
-        return None
-    heads, n_q, _ = query.shape
-    ptr, dt, nb, sh, st, keep = _buffer_rows(buf)
-    _cache_workspace(consts, ws, heads, n, nb, n_q)
-    logits = torch.empty(heads, n_q, n + nb, dtype=torch.float32, device=query.device)
-    rc = lib().tq_cache_scores(consts.addr, pool.addr, block_table.data_ptr(), n, query.data_ptr(), _float_code(query), n_q, ptr, dt, nb,
-                               sh, st, scale, logits.data_ptr(), ws.ptr, ws.nbytes, stream_ptr(query.device))
-    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
-        return None
-    check(rc, "tq_cache_scores")
-    return logits
+    """query (b, h, n_q, D) -> scaled logits (b, h, n_q, n + buffer) fp32, or None where the kernel does not apply."""
+    call = lambda q, x: taken(host().cache_scores(consts.addr, pool.addr, ws, block_table, n, q, x, scale), "tq_cache_scores")  # noqa: E731
+    out = call(query, buf)
+    if out is None:   # strides the kernel does not read in place
+        out = call(query.contiguous(), buf.contiguous() if buf is not None else None)
+    return out
 
 
 def cache_attend(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: torch.Tensor, n: int, weights: torch.Tensor,
                  buf: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """weights (b*h, n_q, n + buffer) contiguous -> (b*h, n_q, D) fp32, or None where the kernel does not apply."""
-    if _float_code(weights) is None or (buf is not None and buf.dtype not in _DTYPES):
-        return None
-    heads, n_q, _ = weights.shape
-    ptr, dt, nb, sh, st, keep = _buffer_rows(buf)
-    _cache_workspace(consts, ws, heads, n, nb, n_q)
-    out = torch.empty(heads, n_q, consts.head_dim, dtype=torch.float32, device=weights.device)
-    rc = lib().tq_cache_attend(consts.addr, pool.addr, block_table.data_ptr(), n, weights.data_ptr(), _float_code(weights), n_q, ptr, dt,
-                               nb, sh, st, out.data_ptr(), ws.ptr, ws.nbytes, stream_ptr(weights.device))
-    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
-        return None
-    check(rc, "tq_cache_attend")
+    """weights (b, h, n_q, n + buffer) -> (b, h, n_q, D) fp32, or None where the kernel does not apply."""
+    call = lambda w, x: taken(host().cache_attend(consts.addr, pool.addr, ws, block_table, n, w, x), "tq_cache_attend")  # noqa: E731
+    out = call(weights, buf)
+    if out is None:
+        out = call(weights.contiguous(), buf.contiguous() if buf is not None else None)
     return out
 
 

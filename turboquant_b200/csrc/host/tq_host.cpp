@@ -445,7 +445,64 @@ PyObject* dequantize_values(PyObject*, PyObject* const* args, Py_ssize_t nargs) 
     END_HANDLE_TH_ERRORS
 }
 
+// ------------------------------------------------------------------ the single-object cache
+
+// cache_scores(consts, pool, workspace, block_table, n, query (b, h, n_q, D), exact keys (b, h, m, D) | None, scale)
+//   -> scaled logits (b, h, n_q, n + m)
+// cache_attend(consts, pool, workspace, block_table, n, weights (b, h, n_q, n + m), exact values | None) -> (b, h, n_q, D)
+// Both: the tensor, a status, or None.
+PyObject* cache_call(PyObject* const* args, bool scores) {
+    const tq_consts* c = address<const tq_consts>(args[0]);
+    const tq_pool* pool = address<const tq_pool>(args[1]);
+    const at::Tensor *bt = tensor_or_null(args[3]), *x = tensor_or_null(args[5]), *buf = tensor_or_null(args[6]);
+    const int64_t n = PyLong_AsLongLong(args[4]), d = c->cfg.head_dim;
+    const double scale = scores ? PyFloat_AsDouble(args[7]) : 0.0;
+    if (PyErr_Occurred()) return nullptr;
+    if (!bt || !rows_tensor(x) || x->dim() != 4 || x->get_device() != bt->get_device() || n < 1) Py_RETURN_NONE;
+    const int64_t b = x->size(0), h = x->size(1), n_q = x->size(2), m = buf ? buf->size(2) : 0;
+    const int dt = dtype_code(x->scalar_type()), db = m ? dtype_code(buf->scalar_type()) : TQ_F32;
+    if (dt < 0 || db < 0 || b * h != pool->num_kv_heads || x->size(3) != (scores ? d : n + m)) Py_RETURN_NONE;
+    if (m) {
+        const int64_t es = (int64_t)buf->element_size();
+        if (buf->dim() != 4 || buf->size(0) != b || buf->size(1) != h || buf->size(3) != d || !buf->is_cuda() || buf->get_device() != x->get_device() ||
+            buf->stride(3) != 1 || (b > 1 && buf->stride(0) != h * buf->stride(1)) || !aligned16(buf->data_ptr()) || (buf->stride(1) * es) % 16 ||
+            (buf->stride(2) * es) % 16)
+            Py_RETURN_NONE;
+    }
+    size_t need = 0, bytes = 0;
+    void* ws = nullptr;
+    int rc = tq_cache_workspace_bytes(&c->cfg, (int32_t)(b * h), n, m, (int32_t)n_q, &need);
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    if (!workspace(args[2], need, &ws, &bytes)) return nullptr;
+    at::Tensor out = at::empty({b, h, n_q, scores ? n + m : d}, x->options().dtype(at::kFloat));
+    const void* rows = m ? buf->data_ptr() : nullptr;
+    const int64_t sh = m ? buf->stride(1) : 0, st = m ? buf->stride(2) : 0;
+    if (scores)
+        rc = tq_cache_scores(c, pool, bt->data_ptr<int32_t>(), n, x->data_ptr(), (tq_dtype)dt, (int32_t)n_q, rows, (tq_dtype)db, m, sh, st,
+                             (float)scale, out.data_ptr<float>(), ws, bytes, stream_of(*x));
+    else
+        rc = tq_cache_attend(c, pool, bt->data_ptr<int32_t>(), n, x->data_ptr(), (tq_dtype)dt, (int32_t)n_q, rows, (tq_dtype)db, m, sh, st,
+                             out.data_ptr<float>(), ws, bytes, stream_of(*x));
+    if (rc == TQ_ERR_UNSUPPORTED || rc == TQ_ERR_ALIGN) Py_RETURN_NONE;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(out));
+}
+PyObject* cache_scores(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(8);
+    return cache_call(args, true);
+    END_HANDLE_TH_ERRORS
+}
+PyObject* cache_attend(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    ARGS(7);
+    return cache_call(args, false);
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {
+    {"cache_scores", (PyCFunction)(void (*)(void))cache_scores, METH_FASTCALL, nullptr},
+    {"cache_attend", (PyCFunction)(void (*)(void))cache_attend, METH_FASTCALL, nullptr},
     {"quantize_keys", (PyCFunction)(void (*)(void))quantize_keys, METH_FASTCALL, nullptr},
     {"dequantize_keys", (PyCFunction)(void (*)(void))dequantize_keys, METH_FASTCALL, nullptr},
     {"key_scores", (PyCFunction)(void (*)(void))key_scores, METH_FASTCALL, nullptr},

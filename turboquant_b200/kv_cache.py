@@ -216,10 +216,10 @@ class TurboQuantKVCache:
             b, h = self._lead
             n_q, buf = query.shape[-2], self.key_buffer
             if query.is_cuda and (buf is None or buf.dtype == query.dtype):
-                logits = E.cache_scores(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant,
-                                        query.reshape(b * h, n_q, self.head_dim).contiguous(), buf, float(scale))
+                q4 = query if query.shape[:2] == (b, h) else query.reshape(b, h, n_q, self.head_dim)
+                logits = E.cache_scores(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant, q4, buf, float(scale))
                 if logits is not None:
-                    return logits.reshape(b, h, n_q, -1)
+                    return logits
             q3 = query.reshape(b * h, query.shape[-2], self.head_dim)
             logits = E.scores(self.consts, self._pool, self._ws, self._bt, self._n_quant, q3)
             parts.append(logits.reshape(b, h, query.shape[-2], self._n_quant) * scale)
@@ -236,10 +236,10 @@ class TurboQuantKVCache:
             n_all = self._n_quant + (buf.shape[-2] if buf is not None else 0)
             if attn_weights.is_cuda and attn_weights.shape[-1] == n_all:
                 n_q = attn_weights.shape[-2]
-                out = E.cache_attend(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant,
-                                     attn_weights.reshape(b * h, n_q, n_all).contiguous(), buf)
+                w4 = attn_weights if attn_weights.shape[:2] == (b, h) else attn_weights.reshape(b, h, n_q, n_all)
+                out = E.cache_attend(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant, w4, buf)
                 if out is not None:
-                    return out.reshape(b, h, n_q, self.head_dim)
+                    return out
             v = E.dequant_values(self.consts, self._pool, self._bt, self._n_quant).reshape(b, h, self._n_quant, -1)
             w = attn_weights[..., col: col + self._n_quant]
             outs.append(torch.matmul(w.float(), v))

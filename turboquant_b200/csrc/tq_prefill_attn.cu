@@ -408,6 +408,7 @@ tq_prefill_attn_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 // the pipe stood idle half of the time (5700 cycles per 128 keys, slower than the kernel above).
 constexpr int PP_THREADS = 2 * PA_TOK + 64;
 constexpr int PP_HALF = 64;                        // keys per step
+constexpr int PP_BARS = 21;
 
 __device__ __forceinline__ void tmem_ld32_async(uint32_t taddr, float* v) {
     uint32_t* r = reinterpret_cast<uint32_t*>(v);
@@ -457,8 +458,8 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     uint8_t* sV = sK + NST * TILE_BYTES;          // [NST]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sV + NST * TILE_BYTES);
     uint64_t *bar_q = bars, *bar_k = bars + 1, *bar_v = bars + 3, *free_k = bars + 5, *free_v = bars + 7, *bar_o = bars + 9,
-             *bar_s = bars + 11, *bar_p = bars + 15;   // bar_s, bar_p: [query tile][score buffer]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+             *bar_s = bars + 13, *bar_p = bars + 17;   // bar_o, bar_s, bar_p: [query tile][half]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + PP_BARS);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // warp: known to be uniform
@@ -470,7 +471,7 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 19; ++i) tq_mbar_init(bars + i, i >= 15 ? PA_TOK : 1);
+        for (int i = 0; i < PP_BARS; ++i) tq_mbar_init(bars + i, i >= 17 ? PA_TOK : 1);
         *s_fail = 0;
         tq_mbar_fence_init();
     }
@@ -553,7 +554,9 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                     umma_ts(tmem_u + C_O + w * C_STEP, tmem_u + C_S + w * C_STEP + odd * PP_HALF + ks * 8,
                             smem_desc_sw128_mn(aV + (t & 1) * TILE_BYTES + (odd * (PP_HALF / 16) + ks) * 2048, PA_BOX), idesc_o,
                             (t | odd | ks) ? 1u : 0u);
-                if (t + 1 >= n_kv[w]) umma_commit(bar_o + w);   // the last two: phases 0 and 1
+                // The last two halves, a barrier each: nobody need have seen the first complete when the second does, and a
+                // wait on a parity cannot tell the phase before last from the one to come.
+                if (t + 1 >= n_kv[w]) umma_commit(bar_o + 2 * w + odd);
             }
             __syncwarp();
         };
@@ -632,7 +635,7 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             }
             if (h > 0 && __any_sync(0xffffffffu, move)) {
                 // PV(h) waits for this warp; PV(h-1) has completed when S(h+1), issued behind it, has
-                if (!(ok = h + 1 < n_h ? wait_warp(bar_s + 2 * w + ((h + 1) & 1), (uint32_t)((h + 1) >> 1) & 1u) : wait_warp(bar_o + w, 0))) break;
+                if (!(ok = h + 1 < n_h ? wait_warp(bar_s + 2 * w + ((h + 1) & 1), (uint32_t)((h + 1) >> 1) & 1u) : wait_warp(bar_o + 2 * w, 0))) break;
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -666,7 +669,7 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             tc_fence_before();
             pa_arrive(bar_p + 2 * w + (h & 1));
         }
-        if (ok && n_h > 0) ok = wait_warp(bar_o + w, 0) && wait_warp(bar_o + w, 1);
+        if (ok && n_h > 0) ok = wait_warp(bar_o + 2 * w + 1, 0);   // its commit covers every product issued before it
         if (ok && n_h > 0) {
             tc_fence_after();
             const float inv = 1.f / l_run;
@@ -771,7 +774,7 @@ extern "C" int tq_prefill_attention(const void* query, const void* key, const vo
     // Pairs of query tiles where single tiles would take more than one wave; below that their four threads per row and
     // twice the number of CTAs finish sooner (128 tiles of 2048 tokens: 27 against 33 us; 176 tiles of 1400: 29 against 24).
     if (D == 128 && (int64_t)p.n_tiles * num_q_heads > tq_sm_count()) {
-        const size_t smem = (size_t)6 * 2 * PA_BOX + 19 * sizeof(uint64_t) + 16 + 1024;
+        const size_t smem = (size_t)6 * 2 * PA_BOX + PP_BARS * sizeof(uint64_t) + 16 + 1024;
         const dim3 pairs((unsigned)num_q_heads, (unsigned)((p.n_tiles + 1) / 2));
         static TqSmemOptIn opt_b, opt_h;
         if (bf16) {

@@ -696,6 +696,19 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
 }
 
+// Pairs of query tiles where single tiles would take more than one wave - by the more tiles, the longer the last row of them
+// is: a CTA of the pair kernel takes 1.38 times as long for it as one of the other, which has four threads a row, and with few
+// heads the launch is that long, while the tiles of the second wave are short ones.  Time of pairs / of single tiles, query
+// heads x query tiles: 32 x 5 0.69, 16 x 10 0.94, 15 x 10 1.21, 14 x 12 0.97, 13 x 12 1.18, 12 x 14 1.02, 12 x 15 0.97, 8 x 20
+// 1.28, 8 x 24 1.04, 8 x 27 0.94, 6 x 36 1.03, 6 x 39 0.98, 4 x 50 1.23, 4 x 63 1.00, 4 x 74 0.90, 2 x 100 1.39, 2 x 185 1.00.
+bool pairs_are_faster(int64_t n_tiles, int64_t heads) {
+    int64_t more = 5 * (n_tiles - 9);
+    if (more < 0) more = 0;
+    if (more > 2 * n_tiles) more = 2 * n_tiles;
+    if (more > 60 + n_tiles * 7 / 8) more = 60 + n_tiles * 7 / 8;
+    return n_tiles * heads > tq_sm_count() + more;
+}
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -771,9 +784,7 @@ extern "C" int tq_prefill_attention(const void* query, const void* key, const vo
         return (size_t)(1 + 2 * nst) * (D / 64) * PA_BOX + (size_t)2 * tpr * PA_TOK * sizeof(float) + 11 * sizeof(uint64_t) +
                16 + 1024;
     };
-    // Pairs of query tiles where single tiles would take more than one wave; below that their four threads per row and
-    // twice the number of CTAs finish sooner (128 tiles of 2048 tokens: 27 against 33 us; 176 tiles of 1400: 29 against 24).
-    if (D == 128 && (int64_t)p.n_tiles * num_q_heads > tq_sm_count()) {
+    if (D == 128 && pairs_are_faster(p.n_tiles, num_q_heads)) {
         const size_t smem = (size_t)6 * 2 * PA_BOX + PP_BARS * sizeof(uint64_t) + 16 + 1024;
         const dim3 pairs((unsigned)num_q_heads, (unsigned)((p.n_tiles + 1) / 2));
         static TqSmemOptIn opt_b, opt_h;

@@ -626,7 +626,23 @@ tq_prefill_pair_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
                 mx4[c] = fmaxf(mx4[c], s[Q * c + Q - 1]);
             }
             // finite from the first half on: key 0 is never masked
-            const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2;
+            float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+            // The first reference is the maximum of the whole first tile, as in the kernel above: the largest probability of a
+            // short row is then 1 and exact in 16 bits.  With that of the first half alone the error against 64 bits was 0.8 %
+            // larger; 64 heads of 400 tokens take 13.6 us in the place of 13.4, 32 of 4096 the same.
+            if (h == 0) {
+                if (!(ok = wait_warp(bar_s + 2 * w + 1, 0))) break;
+                tc_fence_after();
+#pragma unroll
+                for (int c = 0; c < PP_HALF / 32; ++c) {
+                    float v[32];
+                    tmem_ld32(t_s + PP_HALF + 32 * c, v);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (qt > 0 || PP_HALF + 32 * c + i <= row) mx = fmaxf(mx, v[i]);
+                }
+            }
+            mx *= p.scale_log2;
             const bool move = mx > m_run + PA_RESCALE_STEP;   // also the first half (m_run = -inf)
             float alpha = 1.f;
             if (move) {

@@ -67,3 +67,40 @@ def test_prefill_pairs_are_as_exact_as_single_tiles(dtype, dev):
     ref = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v.double().repeat_interleave(rep, 1))
     err = [float((x.double() - ref).norm() / ref.norm()) for x in (pairs, single)]
     assert err[0] <= 1.002 * err[1]
+
+
+@pytest.mark.parametrize("d,kb,vb,qh", [(128, 3, 2, 32), (128, 4, 4, 16), (256, 3, 2, 16)])
+def test_decode_weighs_the_largest_score_exactly(d, kb, vb, qh, dev):
+    """Two tokens that score alike, in records that one warp takes one after the other, and nothing else of weight: the
+    softmax reference is the larger score, whose probability is 1 and exact in fp16, and the smaller one was 1 when it came.
+    What is left is the ratio of the two: 1.7 units of log2 by queries rounded to fp16 (2^-12 / sqrt(3 d) rms, four sigmas:
+    6e-5), and scores of 86 in fp32 (ulp 7.6e-6, a few roundings each: 3e-5), together some 1e-4, where half an ulp of an
+    fp16 probability (2.4e-4) comes to 8e-4 of the difference of two values."""
+    from turboquant_b200 import _engine as E
+    h, nseq, n = 4, 96, 2000
+    c = E.LayerConstants(d, kb, vb, dev, seed=5)
+    g = torch.Generator().manual_seed(d + kb)
+    u = torch.randn(h, d, generator=g)
+    u = u / u.norm(dim=-1, keepdim=True)
+    k = 0.01 * torch.randn(n, h, d, generator=g)
+    a, b = 5, 5 + 16 * 16
+    k[a] = k[b] = 8.0 * u
+    v = torch.randn(n, h, d, generator=g)
+    q = (u.repeat_interleave(qh // h, 0) * 10.0 * math.sqrt(d)).expand(nseq, qh, d).contiguous()
+    q = q * (1 + 0.1 * torch.rand(nseq, qh, 1, generator=g))
+    k, v, q = k.bfloat16().to(dev), v.bfloat16().to(dev), q.to(dev)
+    pool, bt = E.BlockPool(c, h, E.blocks_for(n)), E.identity_block_table(E.blocks_for(n), dev)
+    E.store(c, pool, k, v, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=bt, start_pos=0)
+    ps = E.pool_to_planes(c, pool, bt, n)
+    up = 1 + torch.rand(h, generator=g).to(dev) / 70                # the same vector, up to 1.7 more in log2
+    ps.norms[:, b], ps.residual_norms[:, b] = ps.norms[:, a] * up, ps.residual_norms[:, a] * up
+    E.planes_to_pool(c, ps, n, pool, bt)
+    k64 = _keys64(c, ps.mse_indices, ps.qjl_signs, ps.norms, ps.residual_norms)
+    v64 = _unpack(ps.v_data, vb).double().reshape(h, n, -1, 32) * ps.v_scales.double()[..., None] + ps.v_zeros.double()[..., None]
+    s = torch.einsum("bhgd,hnd->bhgn", q.double().reshape(nseq, h, -1, d), k64) / math.sqrt(d)
+    ref = torch.einsum("bhgn,hnd->bhgd", torch.softmax(s, -1), v64.flatten(-2)).reshape(nseq, qh, d)
+    ws = E.Workspace(dev)
+    lens = torch.full((nseq,), n, dtype=torch.int32, device=dev)
+    out = E.decode(c, pool, ws, q, bt[None].expand(nseq, -1).contiguous(), lens, n, num_splits=1)
+    assert ws.status() == 0
+    assert float(((out.double() - ref).norm(dim=-1) / ref.norm(dim=-1)).max()) <= 1.5e-4

@@ -42,9 +42,6 @@ constexpr int NW_WAVE = 12;
 constexpr int NW_SINGLE = 16;
 constexpr int NW_MULTI = 8;
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
-// A warp's softmax reference is put this far (in log2) above the largest score of the pair of records that raised it; it
-// moves a few times per sequence then, and not at every new maximum of any of its heads.
-constexpr float MARGIN = 2.f;
 
 
 // 2^x for x <= 0 (softmax terms): the bare approximation instruction, results below 2^-126 flush to 0
@@ -474,8 +471,10 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         }
 
         // ------------------------------ online softmax ------------------------------
-        // The reference m_run is set MARGIN above the largest score seen when it was set and stands until a score passes
-        // it: probabilities stay <= 1, and the reduction over the row groups and the rescaling leave the usual path.
+        // The reference m_run is the largest score of the column so far: the probability that counts most is 1 and exact in
+        // fp16.  (With a reference put 2 in log2 above it, which moves a few times per sequence only, 256 sequences of 8192
+        // tokens took 612 us in the place of 621, but the error against 64 bits rose by 3 to 12 %, by as much again for
+        // heads that look at one token, and a wider fp16 scale returned only the second part.)
         float sc_[R][2][2];   // [record][row A, B][column]
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -511,7 +510,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                 mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 4));
                 mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 8));
                 mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 16));
-                const float m_new = mx[i] > m_run[i] ? mx[i] + MARGIN : m_run[i];
+                const float m_new = fmaxf(m_run[i], mx[i]);
                 alpha[i] = m_new == -INFINITY ? 1.f : ex2_fast(m_run[i] - m_new);
                 l_run[i] *= alpha[i];
                 m_run[i] = m_new;

@@ -104,3 +104,49 @@ def test_decode_weighs_the_largest_score_exactly(d, kb, vb, qh, dev):
     out = E.decode(c, pool, ws, q, bt[None].expand(nseq, -1).contiguous(), lens, n, num_splits=1)
     assert ws.status() == 0
     assert float(((out.double() - ref).norm(dim=-1) / ref.norm(dim=-1)).max()) <= 1.5e-4
+
+
+@pytest.mark.parametrize("d,kb,vb,qh", [(128, 3, 2, 16), (128, 3, 2, 32), (128, 4, 4, 16), (256, 3, 2, 16), (256, 4, 4, 8)])
+@pytest.mark.parametrize("records", [1, 56, 57, 73, 124, 125])
+def test_decode_on_both_sides_of_the_lines_for_pairs(d, kb, vb, qh, records, dev):
+    """Launches of several waves: records one by one and in pairs (also an odd number a warp), a ragged last record, scores
+    that climb along the sequence, stale bytes behind the last token."""
+    from turboquant_b200 import _engine as E
+    h, nseq, n = 4, 50, 16 * records - 3
+    c = E.LayerConstants(d, kb, vb, dev, seed=5)
+    g = torch.Generator().manual_seed(d + qh + records)
+    lens = torch.randint(min(n, 17), n + 1, (nseq,), generator=g)
+    lens[0] = n
+    q = torch.randn(nseq, qh, d, generator=g).bfloat16().to(dev)
+    k = torch.randn(n, h, d, generator=g) + torch.linspace(0, 6, n)[:, None, None] * q[0, :h].float().cpu()[None] / 4
+    k, v = k.bfloat16().to(dev), torch.randn(n, h, d, generator=g).bfloat16().to(dev)
+    pool = E.BlockPool(c, h, records)
+    pool.data.fill_(0x7c)                            # fp16 Inf / NaN patterns
+    bt = E.identity_block_table(records, dev)
+    E.store(c, pool, k, v, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=bt, start_pos=0)
+    table, ws = bt[None].expand(nseq, -1).contiguous(), E.Workspace(dev)
+    a, b = (E.decode(c, pool, ws, q, table, lens.int().to(dev), n, num_splits=1, min_history=1, kernel=kern).float() for kern in (0, 1))
+    assert ws.status() == 0 and torch.isfinite(a).all()
+    assert _cos(a, b) >= 0.99995
+    torch.testing.assert_close(a, b, rtol=3e-2, atol=3e-3)
+
+
+@pytest.mark.parametrize("kb,vb,h,qh", [(3, 2, 8, 32), (4, 2, 2, 8), (3, 4, 8, 64)])
+@pytest.mark.parametrize("ring", [0, 47, 48, 128])
+@pytest.mark.parametrize("n", [300, 13000])
+def test_decode_of_one_sequence_on_both_sides_of_the_lines_for_warps(kb, vb, h, qh, ring, n, dev):
+    """Twelve or sixteen warps an SM at head_dim 128 by the ring's length and the records a CTA takes."""
+    from turboquant_b200 import _engine as E
+    d = 128
+    c = E.LayerConstants(d, kb, vb, dev, seed=5)
+    k, v = (t.to(dev) for t in O.synth_kv(n + ring, h, d, seed=ring + n, dtype=torch.bfloat16))
+    pool, bt = E.BlockPool(c, h, E.blocks_for(n)), E.identity_block_table(E.blocks_for(n), dev)
+    E.store(c, pool, k, v, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=bt, start_pos=0)
+    q = O.synth_query(1, qh, d, seed=3, dtype=torch.bfloat16).to(dev)
+    count = lambda x: torch.tensor([x], dtype=torch.int32, device=dev)  # noqa: E731
+    kw = dict(ring_k=k[n:], ring_v=v[n:], ring_lens=count(ring), max_ring_len=ring, ring_stride_token=h * d) if ring else {}
+    ws = E.Workspace(dev)
+    a, b = (E.decode(c, pool, ws, q, bt[None], count(n), n, kernel=kern, **kw).float() for kern in (0, 1))
+    assert ws.status() == 0
+    assert _cos(a, b) >= 0.99995
+    torch.testing.assert_close(a, b, rtol=3e-2, atol=3e-3)

@@ -35,12 +35,16 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 // Warps per CTA.  A launch that fits one wave runs 12-warp CTAs, one per SM (all of an SM's warps
 // share one set of query fragments and one merge).  A launch of several waves runs 8-warp CTAs, two
 // per SM, so that the set-up and the merge of one CTA overlap the main loop of the other.
-// One sequence at head_dim 128 runs 16 warps an SM instead (128 registers are enough there, and a fourth warp per scheduler
-// shortens the main loop: 4096 tokens 13.9 -> 12.9 us, eight layers of 16000 tokens 134 -> 124 us); at head_dim 256 it costs
-// registers (32768 tokens: 188 -> 195 us), and a few short sequences behind a paged write prefer the lighter CTA (25.8, not 26.5).
+// At head_dim 128 a single sequence with a ring may run 16 warps an SM: 128 registers are enough there, the CTAs of the ring
+// (CUDA-core work, up to 64 tokens each) finish sooner with more threads, and they are what such a launch waits for.  Of the
+// launch's time at 8 kv heads, sixteen warps / twelve: 0.93 (one set of fragments) and 0.97 (two sets) from 64 ring tokens on
+// and up to 8000 of history, which is 32 records a CTA; 0.98 at 48 records; 0.98 to 1.03 at 63; 0.95 to 1.02 with 40 ring
+// tokens; 1.00 to 1.06 with 1 or 16, 1.00 to 1.13 without a ring (two sets do not fit the registers and are read from shared
+// memory).  At head_dim 256 it costs registers.
 constexpr int NW_WAVE = 12;
 constexpr int NW_SINGLE = 16;
 constexpr int NW_MULTI = 8;
+constexpr int SINGLE_RING = 48, SINGLE_RECORDS = 48;   // at least so many ring tokens, at most so many records a CTA
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
 
 
@@ -86,11 +90,10 @@ __device__ __forceinline__ uint32_t hmul2_sat(uint32_t a, uint32_t b) {
 // nibbles are byte-table selectors - two PRMTs look up the low and high bytes of four fp16 centroids, two more
 // interleave them into two A registers - so the A operand holds true centroid values, one plane, and the
 // rotated query needs no per-position scaling; it always uses separate rotated / sketched fragment sets.
-template <int D, int MSE_BITS, int VAL_BITS, bool SPLITB, int NW>
+template <int D, int MSE_BITS, int VAL_BITS, bool SPLITB, int NW, int R>
 __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma_kernel(const DecodeParams p) {
     static_assert(MSE_BITS == 2 || SPLITB, "3-bit codes use separate rotated / sketched fragment sets");
     constexpr int NT = NW * 32;
-    constexpr int R = NW == NW_MULTI ? 2 : 1;   // records a warp works on at a time
     constexpr int GP = SPLITB ? 8 : 4;
     constexpr int KS = D / 16;    // score k-steps
     constexpr int NWK = D / 64;   // 32-bit words of 2-bit codes per thread per token; twice the sign words
@@ -290,10 +293,8 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         }
     }
 
-    // In a launch of several waves a warp takes two records at a time: their six chains of score MMAs, their softmax terms
-    // and their loads are independent, which keeps the pipes of a quarter SM busy with the four warps that the registers
-    // allow (256 sequences of 8192 tokens, 64 heads on 8: 718 -> 625 us).  In one wave a warp has a handful of records,
-    // and taking them in pairs costs more in the odd one than it gives (32768 tokens, head_dim 256: 188 -> 200 us).
+    // R = 2: a warp takes two records at a time.  Their six chains of score MMAs, their softmax terms and their loads are
+    // independent, which keeps the pipes of a quarter SM busy with the four warps that the registers allow.
     for (int it = 0; it < cnt && !failed; it += R) {
         const int st = it % NSTW;
         const uint32_t phase = (uint32_t)((it / NSTW) & 1);
@@ -735,7 +736,7 @@ size_t mma_smem_bytes(int block_bytes, int nslot) {
     return s;
 }
 
-template <int D, int MSE_BITS, int VAL_BITS, bool SPLITB, int NW>
+template <int D, int MSE_BITS, int VAL_BITS, bool SPLITB, int NW, int R = 1>
 int launch_mma_nw(const DecodeParams& p_in, int batch, cudaStream_t st) {
     DecodeParams p = p_in;
     constexpr int NT = NW * 32;
@@ -743,7 +744,7 @@ int launch_mma_nw(const DecodeParams& p_in, int batch, cudaStream_t st) {
     const int nslot = p.num_splits + p.ring_splits;
     const size_t smem = mma_smem_bytes<D, SPLITB, NW>(L.block_bytes, nslot);
     p.land_bytes = (uint32_t)mma_land_bytes<D, SPLITB, NW>(L.block_bytes, nslot);
-    auto kern = tq_decode_mma_kernel<D, MSE_BITS, VAL_BITS, SPLITB, NW>;
+    auto kern = tq_decode_mma_kernel<D, MSE_BITS, VAL_BITS, SPLITB, NW, R>;
     static TqSmemOptIn opt_in;
     if (tq_opt_in_smem(kern, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;
     cudaLaunchConfig_t cfg = {};
@@ -770,12 +771,23 @@ int launch_mma(const DecodeParams& p, int batch, cudaStream_t st, int* handled) 
     const int64_t ctas = (int64_t)nslot * p.H * batch;
     const bool fits_wave = mma_smem_bytes<D, SPLITB, NW_WAVE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX;
     const bool fits_multi = mma_smem_bytes<D, SPLITB, NW_MULTI>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX;
+    // records a CTA takes at most
+    const int records = ((p.max_seq_len + TQ_BLOCK_TOKENS - 1) / TQ_BLOCK_TOKENS + p.num_splits - 1) / p.num_splits;
     *handled = 1;
     // two 8-warp CTAs per SM need two merge scratch areas in shared memory: only with few slots
-    if (fits_multi && ((ctas > tq_sm_count() && nslot <= 128) || !fits_wave))
+    if (fits_multi && ((ctas > tq_sm_count() && nslot <= 128) || !fits_wave)) {
+        // Pairs of records where a launch of several waves gives a warp enough of them: a record without a partner costs as
+        // much as a pair.  Time with pairs / without, 64 sequences: head_dim 256, or two sets of fragments: 1.00 to 1.10 at 40
+        // to 400 tokens, 1.02 to 1.05 at 600 (5 records a warp), 0.97 to 1.00 at 800, 0.94 to 0.99 from 900 (57 records a CTA)
+        // on but for odd counts (1.01 at 9 a warp), 0.89 at 8192; head_dim 128 with one set: 0.98 to 1.05 up to 1600 tokens,
+        // 0.97 to 1.00 from 2000 (125) on.  In one wave: 1.02 to 1.07 (head_dim 256 with 4-bit keys and values).
+        constexpr int PAIR_RECORDS = D == 128 && !SPLITB ? 125 : 57;
+        if (ctas > tq_sm_count() && records >= PAIR_RECORDS)
+            return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_MULTI, 2>(p, batch, st);
         return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_MULTI>(p, batch, st);
+    }
     if constexpr (D == 128)
-        if (batch == 1 && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
+        if (batch == 1 && p.max_ring_len >= SINGLE_RING && records <= SINGLE_RECORDS && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
             return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_SINGLE>(p, batch, st);
     if (fits_wave) return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_WAVE>(p, batch, st);
     *handled = 0;

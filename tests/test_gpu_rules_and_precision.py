@@ -150,3 +150,28 @@ def test_decode_of_one_sequence_on_both_sides_of_the_lines_for_warps(kb, vb, h, 
     assert ws.status() == 0
     assert _cos(a, b) >= 0.99995
     torch.testing.assert_close(a, b, rtol=3e-2, atol=3e-3)
+
+
+def test_planes_of_another_size_type_or_place_are_not_read(dev):
+    """What the kernels on plain rows would read out of range goes the general way, which raises or moves it."""
+    from turboquant_b200 import TurboQuantProd
+    from turboquant_b200.kv_cache import dequantize_values, quantize_values
+    z3, z4 = TurboQuantProd(128, 3, device=dev), TurboQuantProd(128, 4, device=dev)
+    x = torch.randn(2, 50, 128, device=dev)
+    kq, q = z3.quantize(x), torch.randn(2, 3, 128, device=dev)
+    for bad in (kq._replace(qjl_signs=kq.qjl_signs[:, :20].contiguous()), kq._replace(norms=kq.norms[:1]),
+                kq._replace(residual_norms=kq.residual_norms[:, ::2].contiguous())):
+        for call in (lambda: z3.dequantize(bad), lambda: z3.attention_score(q, bad)):
+            with pytest.raises(RuntimeError):
+                call()
+    with pytest.raises(RuntimeError):                  # 3-bit codes in a 4-bit quantiser
+        z4.dequantize(kq)
+    there = kq._replace(norms=kq.norms.cpu(), residual_norms=kq.residual_norms.cpu())
+    assert torch.equal(z3.dequantize(there), z3.dequantize(kq)) or \
+        torch.allclose(z3.dequantize(there), z3.dequantize(kq), rtol=1e-4, atol=1e-4)
+    wide = kq._replace(mse_indices=kq.mse_indices.int())
+    assert torch.allclose(z3.dequantize(wide), z3.dequantize(kq), rtol=1e-4, atol=1e-4)
+    vq = quantize_values(x, 2)
+    with pytest.raises(RuntimeError):
+        dequantize_values(vq._replace(scales=vq.scales[:, :20].contiguous()))
+    assert torch.equal(dequantize_values(vq._replace(zeros=vq.zeros.half())), dequantize_values(vq))

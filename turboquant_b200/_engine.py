@@ -461,12 +461,30 @@ def rows_quantize_keys(consts: LayerConstants, x: torch.Tensor):
     return codes, signs, norms, rnorms
 
 
+def key_planes_fit(consts: LayerConstants, n: int, codes, signs, norms, rnorms) -> bool:
+    """Whether contiguous planes hold n keys of this configuration, byte planes as bytes, all on one device: what the kernels
+    on plain rows take on trust.  signs / rnorms may both be None."""
+    lay = consts.layout
+    planes = [(codes, n * lay.kcode_row, True), (norms, n, False)]
+    if signs is not None or rnorms is not None:
+        planes += [(signs, n * lay.ksign_row, True), (rnorms, n, False)]
+    return all(t is not None and t.device == codes.device and t.numel() == count and t.is_contiguous()
+               and (t.dtype == torch.uint8 if is_bytes else t.dtype in _DTYPES) for t, count, is_bytes in planes)
+
+
+def value_planes_fit(n: int, d: int, bits: int, data, scales, zeros) -> bool:
+    """The same for value codes, scales and zero points of n rows of d values."""
+    return (data.dtype == torch.uint8 and data.numel() == n * d * bits // 8 and scales.dtype in _DTYPES and zeros.dtype == scales.dtype
+            and all(t.device == data.device and t.numel() == n * (d // 32) for t in (scales, zeros))
+            and all(t.is_contiguous() for t in (data, scales, zeros)))
+
+
 def rows_dequantize_keys(consts: LayerConstants, codes, signs, norms, rnorms) -> Optional[torch.Tensor]:
     """Contiguous key planes (n, ...) -> (n, D) fp32; signs / rnorms None: the MSE part alone.  None where the rows kernel
     does not take them."""
-    if not codes.is_cuda or _float_code(norms) is None or (rnorms is not None and _float_code(rnorms) is None):
-        return None
     n = norms.numel()
+    if not codes.is_cuda or not key_planes_fit(consts, n, codes, signs, norms, rnorms):
+        return None
     out = torch.empty(n, consts.head_dim, dtype=torch.float32, device=codes.device)
     rc = lib().tq_rows_dequantize_keys(consts.addr, codes.data_ptr(), signs.data_ptr() if signs is not None else None, norms.data_ptr(),
                                        _float_code(norms), rnorms.data_ptr() if rnorms is not None else None,
@@ -481,10 +499,13 @@ def rows_dequantize_keys(consts: LayerConstants, codes, signs, norms, rnorms) ->
 def rows_scores(consts: LayerConstants, ws: "Workspace", codes, signs, norms, rnorms, heads: int, n: int,
                 query: torch.Tensor) -> Optional[torch.Tensor]:
     """Key planes (heads, n, ...) and query (heads, n_q, D) -> unscaled logits (heads, n_q, n) fp32, or None."""
-    if not codes.is_cuda or not query.is_cuda or None in (_float_code(norms), _float_code(rnorms), _float_code(query)):
+    if not codes.is_cuda or query.device != codes.device or _float_code(query) is None or \
+            not key_planes_fit(consts, heads * n, codes, signs, norms, rnorms) or query.shape[::2] != (heads, consts.head_dim):
         return None
     n_q = query.shape[1]
-    ws.ensure(256 + heads * n_q * 2 * consts.head_dim * 4)
+    need = C.c_size_t(0)
+    check(lib().tq_scores_workspace_bytes(C.byref(consts.cfg), heads * n_q, C.byref(need)), "tq_scores_workspace_bytes")
+    ws.ensure(need.value)
     logits = torch.empty(heads, n_q, n, dtype=torch.float32, device=codes.device)
     rc = lib().tq_rows_scores(consts.addr, codes.data_ptr(), signs.data_ptr(), norms.data_ptr(), _float_code(norms), rnorms.data_ptr(),
                               _float_code(rnorms), heads, n, query.data_ptr(), _float_code(query), n_q, logits.data_ptr(), ws.ptr,
@@ -511,9 +532,9 @@ def rows_quantize_values(v: torch.Tensor, bits: int):
 
 def rows_dequantize_values(data: torch.Tensor, scales: torch.Tensor, zeros: torch.Tensor, bits: int, d: int) -> Optional[torch.Tensor]:
     """Contiguous value planes -> (n, D) fp32, or None."""
-    if _float_code(scales) is None or zeros.dtype != scales.dtype:
-        return None
     n = data.numel() // data.shape[-1]
+    if not data.is_cuda or not value_planes_fit(n, d, bits, data, scales, zeros):
+        return None
     out = torch.empty(n, d, dtype=torch.float32, device=data.device)
     rc = lib().tq_rows_dequantize_values(data.data_ptr(), scales.data_ptr(), zeros.data_ptr(), _float_code(scales), n, d, bits,
                                          out.data_ptr(), stream_ptr(data.device))

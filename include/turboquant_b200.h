@@ -372,8 +372,11 @@ int tq_dequant_values(const tq_config* cfg, const tq_pool* pool, const int32_t* 
 
 /* ---- the single-object cache: both halves of its attention -------------------- */
 
-/* Scratch of tq_cache_scores / tq_cache_attend (one buffer serves both; zero it once,
- * see tq_workspace_init). */
+/* Scratch of tq_cache_scores and of tq_cache_attend; TQ_ERR_UNSUPPORTED where the call itself would answer
+ * that (more than 128 queries, or more heads and queries than there are merge tickets, in tq_cache_attend).
+ * One zeroed buffer (see tq_workspace_init) may serve both calls; tq_cache_workspace_bytes is its size. */
+int tq_cache_scores_workspace_bytes(const tq_config* cfg, int32_t n_heads, int32_t n_q, size_t* out);
+int tq_cache_attend_workspace_bytes(const tq_config* cfg, int32_t n_heads, int64_t n_tokens, int64_t n_buf, int32_t n_q, size_t* out);
 int tq_cache_workspace_bytes(const tq_config* cfg, int32_t n_heads, int64_t n_tokens, int64_t n_buf, int32_t n_q, size_t* out);
 
 /* Scaled logits (n_heads, n_q, n_tokens + n_buf) fp32 of query (n_heads, n_q, D) against the compressed

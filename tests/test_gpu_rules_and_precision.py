@@ -175,3 +175,26 @@ def test_planes_of_another_size_type_or_place_are_not_read(dev):
     with pytest.raises(RuntimeError):
         dequantize_values(vq._replace(scales=vq.scales[:, :20].contiguous()))
     assert torch.equal(dequantize_values(vq._replace(zeros=vq.zeros.half())), dequantize_values(vq))
+
+
+@pytest.mark.parametrize("n_q", [128, 129])
+def test_cache_object_with_many_queries(n_q, dev):
+    """Both sides of the line between the attend kernel and the matrix product on dequantised values; no scratch for a call
+    that is declined, the logits' scratch is the prepared queries."""
+    from turboquant_b200 import TurboQuantKVCache, _engine as E
+    d, h, n = 128, 3, 700
+    cache = TurboQuantKVCache(d, 3, 2, buffer_size=32, device=dev, dtype=torch.float32)
+    g = torch.Generator().manual_seed(n_q)
+    k, v = (torch.randn(1, h, n, d, generator=g).to(dev) for _ in range(2))
+    cache.prefill(k, v)
+    q, w = torch.randn(1, h, n_q, d, generator=g).to(dev), torch.softmax(torch.randn(1, h, n_q, n, generator=g), -1).to(dev)
+    m = cache._n_quant
+    logits = cache.attention_scores(q)
+    scratch = cache._ws_attn.buf.numel()
+    assert scratch <= 32768 + h * n_q * 2 * d * 4
+    out = cache.attend(w)
+    assert (cache._ws_attn.buf.numel() == scratch) == (n_q > 128)
+    keys = torch.cat((E.dequant_keys(cache.consts, cache._pool, cache._bt, m).reshape(1, h, m, d), k[..., m:, :]), -2).double()
+    vals = torch.cat((E.dequant_values(cache.consts, cache._pool, cache._bt, m).reshape(1, h, m, d), v[..., m:, :]), -2).double()
+    for got, ref in ((logits, q.double() @ keys.transpose(-1, -2) / math.sqrt(d)), (out, w.double() @ vals)):
+        assert float((got.double() - ref).norm() / ref.norm()) <= 2e-6      # fp32 sums of some hundred terms

@@ -27,3 +27,26 @@ def test_planes_are_measured_before_a_kernel_reads_them(d, kb, vb):
     for bad in ((data[:4], scales, zeros), (data.int(), scales, zeros), (data, scales[:, 1:], zeros), (data, scales, zeros[:4]),
                 (data, scales, zeros.half()), (data, scales.double(), zeros.double()), (data, scales.to("meta"), zeros)):
         assert not E.value_planes_fit(n, d, vb, *bad)
+
+
+def test_scratch_of_the_cache_object_is_sized_by_call():
+    cfg, out = _lib.tq_config(128, 3, 2, 32), C.c_size_t(0)
+    lib = _lib.lib()
+
+    def size(name, *args):
+        rc = getattr(lib, name)(C.byref(cfg), *args, C.byref(out))
+        return out.value if rc == 0 else rc
+
+    base = size("tq_cache_scores_workspace_bytes", 1, 1) - 2 * 128 * 4
+    assert size("tq_cache_scores_workspace_bytes", 32, 4096) == base + 32 * 4096 * 2 * 128 * 4
+    # partial sums: no more than the history dequantised to fp32, whatever the number of queries taken
+    for heads, n in ((8, 32768), (1, 128)):
+        assert size("tq_cache_attend_workspace_bytes", heads, n, 0, 128) == base + heads * n * 128 * 4
+        assert size("tq_cache_attend_workspace_bytes", heads, n, 0, 129) == _lib.TQ_ERR_UNSUPPORTED
+    assert size("tq_cache_attend_workspace_bytes", 4097, 128, 0, 1) == _lib.TQ_ERR_UNSUPPORTED     # merge tickets
+    assert size("tq_cache_attend_workspace_bytes", 4096, 128, 0, 4) > 0
+    both = size("tq_cache_workspace_bytes", 8, 4096, 128, 2)
+    assert both == max(size("tq_cache_scores_workspace_bytes", 8, 2), size("tq_cache_attend_workspace_bytes", 8, 4096, 128, 2))
+    assert size("tq_cache_workspace_bytes", 8, 4096, 0, 4096) == size("tq_cache_scores_workspace_bytes", 8, 4096)
+    for bad in ((0, 16, 0, 1), (1, -1, 0, 1), (1, 16, -1, 1), (1, 16, 0, 0)):
+        assert size("tq_cache_workspace_bytes", *bad) == _lib.TQ_ERR_SHAPE

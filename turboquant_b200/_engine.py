@@ -544,24 +544,26 @@ def rows_dequantize_values(data: torch.Tensor, scales: torch.Tensor, zeros: torc
     return out
 
 
+def _cache_call(fn, consts, pool, ws, block_table, n, x, buf, *scale) -> Optional[torch.Tensor]:
+    """One of the cache object's native calls; a second time on contiguous copies where the strides were the reason."""
+    out = fn(consts.addr, pool.addr, ws, block_table, n, x, buf, *scale)
+    if out is None:
+        args = x.contiguous(), buf.contiguous() if buf is not None else None
+        if args[0] is not x or args[1] is not buf:
+            out = fn(consts.addr, pool.addr, ws, block_table, n, *args, *scale)
+    return None if out is NotImplemented else taken(out, fn.__name__)
+
+
 def cache_scores(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: torch.Tensor, n: int, query: torch.Tensor,
                  buf: Optional[torch.Tensor], scale: float) -> Optional[torch.Tensor]:
     """query (b, h, n_q, D) -> scaled logits (b, h, n_q, n + buffer) fp32, or None where the kernel does not apply."""
-    call = lambda q, x: taken(host().cache_scores(consts.addr, pool.addr, ws, block_table, n, q, x, scale), "tq_cache_scores")  # noqa: E731
-    out = call(query, buf)
-    if out is None:   # strides the kernel does not read in place
-        out = call(query.contiguous(), buf.contiguous() if buf is not None else None)
-    return out
+    return _cache_call(host().cache_scores, consts, pool, ws, block_table, n, query, buf, scale)
 
 
 def cache_attend(consts: LayerConstants, pool: BlockPool, ws: Workspace, block_table: torch.Tensor, n: int, weights: torch.Tensor,
                  buf: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
     """weights (b, h, n_q, n + buffer) -> (b, h, n_q, D) fp32, or None where the kernel does not apply."""
-    call = lambda w, x: taken(host().cache_attend(consts.addr, pool.addr, ws, block_table, n, w, x), "tq_cache_attend")  # noqa: E731
-    out = call(weights, buf)
-    if out is None:
-        out = call(weights.contiguous(), buf.contiguous() if buf is not None else None)
-    return out
+    return _cache_call(host().cache_attend, consts, pool, ws, block_table, n, weights, buf)
 
 
 def identity_block_table(n_blocks: int, device) -> torch.Tensor:

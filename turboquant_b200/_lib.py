@@ -103,6 +103,8 @@ SIGNATURES = {
                                   C.c_void_p, C.c_void_p]),
     "tq_dequant_values": (C.c_int, [C.POINTER(tq_config), C.POINTER(tq_pool), C.c_void_p, C.c_int64, C.c_void_p,
                                     C.c_void_p]),
+    "tq_cache_scores_workspace_bytes": (C.c_int, [C.POINTER(tq_config), C.c_int32, C.c_int32, C.POINTER(C.c_size_t)]),
+    "tq_cache_attend_workspace_bytes": (C.c_int, [C.POINTER(tq_config), C.c_int32, C.c_int64, C.c_int64, C.c_int32, C.POINTER(C.c_size_t)]),
     "tq_cache_workspace_bytes": (C.c_int, [C.POINTER(tq_config), C.c_int32, C.c_int64, C.c_int64, C.c_int32, C.POINTER(C.c_size_t)]),
     "tq_cache_scores": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_int,
                                   C.c_int32, C.c_void_p, C.c_int, C.c_int64, C.c_int64, C.c_int64, C.c_float, C.c_void_p,

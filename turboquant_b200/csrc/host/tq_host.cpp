@@ -450,7 +450,8 @@ PyObject* dequantize_values(PyObject*, PyObject* const* args, Py_ssize_t nargs) 
 // cache_scores(consts, pool, workspace, block_table, n, query (b, h, n_q, D), exact keys (b, h, m, D) | None, scale)
 //   -> scaled logits (b, h, n_q, n + m)
 // cache_attend(consts, pool, workspace, block_table, n, weights (b, h, n_q, n + m), exact values | None) -> (b, h, n_q, D)
-// Both: the tensor, a status, or None.
+// Both: the tensor, a status, None where strides or types are not the kernel's, NotImplemented where the call is too large for it
+// (nothing has been allocated then).
 PyObject* cache_call(PyObject* const* args, bool scores) {
     const tq_consts* c = address<const tq_consts>(args[0]);
     const tq_pool* pool = address<const tq_pool>(args[1]);
@@ -458,10 +459,17 @@ PyObject* cache_call(PyObject* const* args, bool scores) {
     const int64_t n = PyLong_AsLongLong(args[4]), d = c->cfg.head_dim;
     const double scale = scores ? PyFloat_AsDouble(args[7]) : 0.0;
     if (PyErr_Occurred()) return nullptr;
-    if (!bt || !rows_tensor(x) || x->dim() != 4 || x->get_device() != bt->get_device() || n < 1) Py_RETURN_NONE;
+    if (!bt || !x || !x->is_cuda() || x->dim() != 4 || x->numel() == 0 || x->get_device() != bt->get_device() || n < 1) Py_RETURN_NONE;
     const int64_t b = x->size(0), h = x->size(1), n_q = x->size(2), m = buf ? buf->size(2) : 0;
     const int dt = dtype_code(x->scalar_type()), db = m ? dtype_code(buf->scalar_type()) : TQ_F32;
     if (dt < 0 || db < 0 || b * h != pool->num_kv_heads || x->size(3) != (scores ? d : n + m)) Py_RETURN_NONE;
+    size_t need = 0, bytes = 0;
+    void* ws = nullptr;
+    int rc = scores ? tq_cache_scores_workspace_bytes(&c->cfg, (int32_t)(b * h), (int32_t)n_q, &need)
+                    : tq_cache_attend_workspace_bytes(&c->cfg, (int32_t)(b * h), n, m, (int32_t)n_q, &need);
+    if (rc == TQ_ERR_UNSUPPORTED) Py_RETURN_NOTIMPLEMENTED;
+    if (rc != TQ_OK) return PyLong_FromLong(rc);
+    if (!x->is_contiguous()) Py_RETURN_NONE;
     if (m) {
         const int64_t es = (int64_t)buf->element_size();
         if (buf->dim() != 4 || buf->size(0) != b || buf->size(1) != h || buf->size(3) != d || !buf->is_cuda() || buf->get_device() != x->get_device() ||
@@ -469,10 +477,6 @@ PyObject* cache_call(PyObject* const* args, bool scores) {
             (buf->stride(2) * es) % 16)
             Py_RETURN_NONE;
     }
-    size_t need = 0, bytes = 0;
-    void* ws = nullptr;
-    int rc = tq_cache_workspace_bytes(&c->cfg, (int32_t)(b * h), n, m, (int32_t)n_q, &need);
-    if (rc != TQ_OK) return PyLong_FromLong(rc);
     if (!workspace(args[2], need, &ws, &bytes)) return nullptr;
     at::Tensor out = at::empty({b, h, n_q, scores ? n + m : d}, x->options().dtype(at::kFloat));
     const void* rows = m ? buf->data_ptr() : nullptr;

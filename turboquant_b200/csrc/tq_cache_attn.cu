@@ -16,6 +16,11 @@ namespace {
 constexpr int CA_TOK = 64;        // tokens per CTA (logits)
 constexpr int AT_REC = 8;         // records per CTA (values): 128 tokens
 constexpr int AT_NQ = 4;          // queries a CTA accumulates at a time
+// Queries of one call: the partial sums of so many take as much memory as the dequantised history of the way that this kernel
+// replaces (a split is 128 tokens), and its matrix product overtakes the kernel's passes over the records between 128 and 256
+// (8 heads of 128, 4096 / 32768 tokens: 108 against 162 us and 750 against 904 at 128 queries, 195 against 164 and 1459 against
+// 907 at 256; 4 heads of 256, 8192 tokens: 205 against 261, 387 against 265).
+constexpr int AT_NQ_MAX = 128;
 constexpr int AT_TICKETS = 4096;  // heads x groups of AT_NQ queries; at a fixed place, so that no call's scratch lands on them
 
 struct CacheParams {
@@ -131,7 +136,7 @@ __global__ void __launch_bounds__(128) tq_cache_scores_kernel(const CacheParams 
 template <int D, int VAL_BITS>
 __global__ void __launch_bounds__(D) tq_cache_attend_kernel(const CacheParams p, int key_bits) {
     const TqLayout L = tq_make_layout(D, key_bits, VAL_BITS);
-    constexpr int TOK = AT_REC * TQ_BLOCK_TOKENS, NG = D / 32;
+    constexpr int TOK = AT_REC * TQ_BLOCK_TOKENS;
     __shared__ __align__(16) float w[AT_NQ][TOK];
     __shared__ int last;
     const int d = threadIdx.x, h = blockIdx.y, q0 = blockIdx.z * AT_NQ, nq = min(AT_NQ, p.n_q - q0);
@@ -186,7 +191,6 @@ __global__ void __launch_bounds__(D) tq_cache_attend_kernel(const CacheParams p,
                 for (int q = 0; q < AT_NQ; ++q) acc[q] = fmaf(w[q][16 * r + t], v, acc[q]);
             }
         }
-        (void)NG;
     } else {
 #pragma unroll 8
         for (int t = 0; t < n_here; ++t) {
@@ -251,15 +255,35 @@ constexpr size_t SCRATCH_AT = TQ_WS_HEADER_BYTES + AT_TICKETS * sizeof(int32_t);
 
 }  // namespace
 
-extern "C" int tq_cache_workspace_bytes(const tq_config* cfg, int32_t n_heads, int64_t n_tokens, int64_t n_buf, int32_t n_q, size_t* out) {
+extern "C" int tq_cache_scores_workspace_bytes(const tq_config* cfg, int32_t n_heads, int32_t n_q, size_t* out) {
+    if (!cfg || !out) return TQ_ERR_NULL;
+    const int rc = tq_check_config(cfg);
+    if (rc != TQ_OK) return rc;
+    if (n_heads <= 0 || n_q <= 0) return TQ_ERR_SHAPE;
+    if (n_q > 8 * 65535 || n_heads > 65535) return TQ_ERR_UNSUPPORTED;
+    *out = SCRATCH_AT + (size_t)n_heads * n_q * 2 * cfg->head_dim * sizeof(float);
+    return TQ_OK;
+}
+
+extern "C" int tq_cache_attend_workspace_bytes(const tq_config* cfg, int32_t n_heads, int64_t n_tokens, int64_t n_buf, int32_t n_q, size_t* out) {
     if (!cfg || !out) return TQ_ERR_NULL;
     const int rc = tq_check_config(cfg);
     if (rc != TQ_OK) return rc;
     if (n_heads <= 0 || n_tokens < 0 || n_buf < 0 || n_q <= 0) return TQ_ERR_SHAPE;
     const int64_t zs = tiles(n_q, AT_NQ), splits = tiles(n_tokens, AT_REC * TQ_BLOCK_TOKENS) + tiles(n_buf, AT_REC * TQ_BLOCK_TOKENS);
-    const size_t queries = (size_t)n_heads * n_q * 2 * cfg->head_dim * sizeof(float);
-    const size_t partials = (size_t)(zs * n_heads * splits * AT_NQ * cfg->head_dim) * sizeof(float);
-    *out = SCRATCH_AT + (queries > partials ? queries : partials);
+    if (n_q > AT_NQ_MAX || n_heads > 65535 || zs * n_heads > AT_TICKETS) return TQ_ERR_UNSUPPORTED;
+    *out = SCRATCH_AT + (size_t)(zs * n_heads * splits * AT_NQ * cfg->head_dim) * sizeof(float);
+    return TQ_OK;
+}
+
+extern "C" int tq_cache_workspace_bytes(const tq_config* cfg, int32_t n_heads, int64_t n_tokens, int64_t n_buf, int32_t n_q, size_t* out) {
+    size_t scores = 0, attend = 0;
+    int rc = tq_cache_scores_workspace_bytes(cfg, n_heads, n_q, &scores);
+    if (rc == TQ_OK) rc = tq_cache_attend_workspace_bytes(cfg, n_heads, n_tokens, n_buf, n_q, &attend);
+    if (rc != TQ_OK && rc != TQ_ERR_UNSUPPORTED) return rc;
+    if (scores == 0 && attend == 0) return rc;
+    if (!out) return TQ_ERR_NULL;
+    *out = scores > attend ? scores : attend;
     return TQ_OK;
 }
 
@@ -272,7 +296,7 @@ extern "C" int tq_cache_scores(const tq_consts* consts, const tq_pool* pool, con
     if (!query || !logits || !consts->pi_t || !consts->s_t) return TQ_ERR_NULL;
     const int D = consts->cfg.head_dim;
     size_t need = 0;
-    tq_cache_workspace_bytes(&consts->cfg, p.H, n_tokens, n_buf, n_q, &need);
+    if ((rc = tq_cache_scores_workspace_bytes(&consts->cfg, p.H, n_q, &need)) != TQ_OK) return rc;
     if (need > workspace_bytes) return TQ_ERR_WORKSPACE;
     float* qprep = reinterpret_cast<float*>((uint8_t*)workspace + SCRATCH_AT);
     cudaStream_t st = (cudaStream_t)stream;
@@ -302,12 +326,12 @@ extern "C" int tq_cache_attend(const tq_consts* consts, const tq_pool* pool, con
                                tq_dtype w_dtype, int32_t n_q, const void* buf_values, tq_dtype buf_dtype, int64_t n_buf, int64_t stride_head,
                                int64_t stride_token, float* out, void* workspace, size_t workspace_bytes, void* stream) {
     CacheParams p = {};
-    const int rc = common(p, consts, pool, block_table, n_tokens, n_q, buf_values, buf_dtype, n_buf, stride_head, stride_token, workspace);
+    int rc = common(p, consts, pool, block_table, n_tokens, n_q, buf_values, buf_dtype, n_buf, stride_head, stride_token, workspace);
     if (rc != TQ_OK) return rc;
     if (!weights || !out) return TQ_ERR_NULL;
     const int D = consts->cfg.head_dim;
     size_t need = 0;
-    tq_cache_workspace_bytes(&consts->cfg, p.H, n_tokens, n_buf, n_q, &need);
+    if ((rc = tq_cache_attend_workspace_bytes(&consts->cfg, p.H, n_tokens, n_buf, n_q, &need)) != TQ_OK) return rc;
     if (need > workspace_bytes) return TQ_ERR_WORKSPACE;
     const int64_t zs = tiles(n_q, AT_NQ);
     p.weights = weights;
@@ -316,7 +340,6 @@ extern "C" int tq_cache_attend(const tq_consts* consts, const tq_pool* pool, con
     p.splits = (int)(tiles(n_tokens, AT_REC * TQ_BLOCK_TOKENS) + tiles(n_buf, AT_REC * TQ_BLOCK_TOKENS));
     p.tickets = reinterpret_cast<int32_t*>((uint8_t*)workspace + TQ_WS_HEADER_BYTES);
     p.partials = reinterpret_cast<float*>((uint8_t*)workspace + SCRATCH_AT);
-    if (zs * p.H > AT_TICKETS) return TQ_ERR_UNSUPPORTED;
     const dim3 grid((unsigned)p.splits, (unsigned)p.H, (unsigned)zs);
     cudaStream_t st = (cudaStream_t)stream;
     tq_note_launch(st, TQ_LAUNCH_UNKNOWN);

@@ -50,3 +50,23 @@ def test_scratch_of_the_cache_object_is_sized_by_call():
     assert size("tq_cache_workspace_bytes", 8, 4096, 0, 4096) == size("tq_cache_scores_workspace_bytes", 8, 4096)
     for bad in ((0, 16, 0, 1), (1, -1, 0, 1), (1, 16, -1, 1), (1, 16, 0, 0)):
         assert size("tq_cache_workspace_bytes", *bad) == _lib.TQ_ERR_SHAPE
+
+
+def test_the_shared_identity_table_belongs_to_the_device_that_is_current(monkeypatch):
+    """A device without an index means the current one at the call, not at the first call."""
+    made, now = [], [0]
+
+    def table(n, device):
+        made.append(torch.device(device))
+        return torch.arange(n, dtype=torch.int32)
+
+    monkeypatch.setattr(E, "_IDENTITY", {})
+    monkeypatch.setattr(E, "identity_block_table", table)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: now[0])
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: type("S", (), {"synchronize": lambda self: None})())
+    first = E.shared_identity_table(10, "cuda")
+    now[0] = 1
+    second = E.shared_identity_table(10, torch.device("cuda"))
+    assert second is not first and made == [torch.device("cuda", 0), torch.device("cuda", 1)]
+    assert E.shared_identity_table(10, torch.device("cuda", 0)) is first and E.shared_identity_table(5, "cuda:1") is second

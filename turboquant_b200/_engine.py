@@ -576,7 +576,11 @@ _IDENTITY_ENTRIES = 65536
 
 def shared_identity_table(n_blocks: int, device) -> torch.Tensor:
     """A read-only identity table of at least `n_blocks` entries: one of 64 K entries per device, made once and never
-    replaced, so that any stream may read it; a table of its own beyond that."""
+    replaced, so that any stream may read it; a table of its own beyond that.  A device without an index means the
+    current one, at this call."""
+    device = torch.device(device)
+    if device.index is None:
+        device = torch.device(device.type, torch.cuda.current_device())
     key = str(device)
     t = _IDENTITY.get(key)
     if n_blocks > _IDENTITY_ENTRIES or (t is None and torch.cuda.is_current_stream_capturing()):

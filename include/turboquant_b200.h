@@ -90,9 +90,11 @@ typedef struct tq_consts {
      * batches at head_dim 128): S split into two bf16 limbs, (D,D) row-major.
      * With either NULL (or pi_limbs missing) the fp32 kernels prepare the queries. */
     const void* s_limbs[2];
-    /* Optional operands of tq_rows_quantize_keys / tq_rows_dequantize_keys at
-     * head_dim 128: 64 Pi, M and S, each as two fp16 limbs, (D,D) row-major.  With
-     * any of them NULL those calls return TQ_ERR_UNSUPPORTED. */
+    /* Optional: 64 Pi, M and S, each as two fp16 limbs, (D,D) row-major.  Operands of
+     * tq_rows_quantize_keys / tq_rows_dequantize_keys at head_dim 128, which return
+     * TQ_ERR_UNSUPPORTED with any of them NULL, and (64 Pi and M) of the tensor-core
+     * store at head_dim 256 with 4-bit keys or values, which the fp32 kernel replaces
+     * then.  For the store, rows of Pi of norm < 8 and centroids < 8. */
     const void* rows_pi[2];
     const void* rows_m[2];
     const void* rows_s[2];

@@ -198,3 +198,41 @@ def test_cache_object_with_many_queries(n_q, dev):
     vals = torch.cat((E.dequant_values(cache.consts, cache._pool, cache._bt, m).reshape(1, h, m, d), v[..., m:, :]), -2).double()
     for got, ref in ((logits, q.double() @ keys.transpose(-1, -2) / math.sqrt(d)), (out, w.double() @ vals)):
         assert float((got.double() - ref).norm() / ref.norm()) <= 2e-6      # fp32 sums of some hundred terms
+
+
+@pytest.mark.parametrize("kb,vb", [(4, 2), (3, 4)])
+def test_d256_wide_records_are_as_exact_as_the_fp32_store(kb, vb, dev):
+    """Codes next to a boundary and sign bits next to zero that come out otherwise than in 64 bits: not more than from the
+    fp32 kernel, up to three standard deviations of the two counts (bf16 limbs gave six to twelve times as many)."""
+    from turboquant_b200 import _engine as E
+    n, h, d = 16384, 8, 256
+    g = torch.Generator(device=dev)
+    g.manual_seed(11)
+    x = (torch.randn(n, h, d, generator=g, device=dev) * torch.exp(0.5 * torch.randn(d, generator=g, device=dev))).bfloat16()
+    wrong = []
+    for tensor_cores in (True, False):
+        c = E.LayerConstants(d, kb, vb, dev, tensor_core_store=tensor_cores)
+        pool, bt = E.BlockPool(c, h, E.blocks_for(n)), E.identity_block_table(E.blocks_for(n), dev)
+        E.store(c, pool, x, x, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=bt)
+        ps = E.pool_to_planes(c, pool, bt, n)
+        wrong.append([sum(w) for w in zip(*(_wrong(c, x[:, i], ps.mse_indices[i], ps.qjl_signs[i]) for i in range(h)))])
+    for fast, exact in zip(*wrong):
+        assert fast <= exact + 3 * math.sqrt(fast + exact), wrong
+    assert E.store_status() == 0
+
+
+def test_d256_wide_store_without_fp16_operands(dev):
+    """A rotation whose residuals would leave fp16's range has no operands for the tensor-core kernel: the fp32 one runs."""
+    from turboquant_b200 import _engine as E
+    n, h, d = 100, 2, 256
+    x = torch.randn(n, h, d, generator=torch.Generator().manual_seed(1)).bfloat16().to(dev)
+    pi = 20.0 * E.LayerConstants(d, 4, 2, dev).Pi
+    planes = []
+    for tensor_cores in (True, False):
+        c = E.LayerConstants(d, 4, 2, dev, Pi=pi, tensor_core_store=tensor_cores)
+        assert c.rows_limbs is None
+        pool, bt = E.BlockPool(c, h, E.blocks_for(n)), E.identity_block_table(E.blocks_for(n), dev)
+        E.store(c, pool, x, x, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h, block_table=bt)
+        planes.append(E.pool_to_planes(c, pool, bt, n))
+    for f in ("mse_indices", "qjl_signs", "norms", "residual_norms"):
+        assert torch.equal(getattr(planes[0], f), getattr(planes[1], f))

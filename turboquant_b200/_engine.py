@@ -115,8 +115,21 @@ class LayerConstants:
             c.m_limbs[i] = self.m_limbs[i].data_ptr() if tensor_core_store else None
             c.s_limbs[i] = self.s_limbs[i].data_ptr() if tensor_core_store else None
         self.rows_limbs = None
+        if tensor_core_store and head_dim == 256 and (key_bits, value_bits) != (3, 2):
+            # the wide records' store keeps 22 bits of Pi and M; its residuals must stay in fp16's range
+            if float(pi.norm(dim=1).max()) < 8 and float(self.centroids_cpu.abs().max()) < 8:
+                self.rows_limbs = self._fp16_limbs(pi.double() * 64.0, m)
+                for i in range(2 if self.rows_limbs else 0):
+                    c.rows_pi[i], c.rows_m[i] = (x[i].data_ptr() for x in self.rows_limbs)
         self.c = c
         self.addr = C.addressof(c)     # what the native host path passes on
+
+    def _fp16_limbs(self, *mats: torch.Tensor) -> list:
+        """Each matrix as two fp16 limbs on the device; nothing where one leaves fp16's range (a caller's own S may be
+        anything)."""
+        if not all(bool(t.abs().max() < 60000.0) for t in mats):
+            return []
+        return [[t.contiguous().to(self.device) for t in _split(x, 2, torch.float16)] for x in mats]
 
     def ensure_rows(self) -> None:
         """Operands of the kernels on plain rows (64 Pi, M = S Pi^T and S as two fp16 limbs each): only the quantiser

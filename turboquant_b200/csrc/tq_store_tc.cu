@@ -214,13 +214,14 @@ struct BookRegs {
 
 // Bucket search of one rotated coordinate y (torch.searchsorted on the interior boundaries, left: the
 // code is the number of boundaries below y) and y minus its centroid.  `code` comes back as a float.
-template <int MSE_BITS>
+// SCALE: y, c0 and the steps are this power of two times theirs, the boundaries in nb are not.
+template <int MSE_BITS, int SCALE = 1>
 __device__ __forceinline__ void bucket(const BookRegs<MSE_BITS>& bk, float y, float& code, float& y_minus_c) {
     constexpr int NB = (1 << MSE_BITS) - 1, MID = NB / 2;   // the middle boundary is (next to) zero
     float k = 0.f, r = y - bk.c0;
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
-        float t = fma_sat(y, BIG, bk.nb[i]);
+        float t = fma_sat(y, BIG / SCALE, bk.nb[i]);
         if (i == MID) t = mul_sat(t, BIG);
         k += t;
         r = fmaf(-t, bk.step[i], r);
@@ -838,7 +839,16 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 // 3-bit keys with 2-bit values have 25 KB of record images and leave room for the two slots of 256 rows;
 // the wider records (33 or 41 KB) take a ring of three 16 KB boxes of 128 rows, every product in two
 // halves of 128 columns: the same number of tensor-core cycles and of bytes, 48 KB of them in flight.
-// Measured (5003 tokens, 4 heads, 4-bit keys, 2-bit values): 300 us in the fp32 kernel -> 77.
+// They also keep the precision of the fp32 kernel, on which these widths ran before (with the products of the narrow records
+// codes next to a boundary came out wrong eleven times as often, sign bits next to zero eight times):
+//   * fp16 limbs in the place of bf16 ones, scaled clear of the subnormals by powers of two: 22 bits of Pi, r' and M;
+//   * the accumulators drop what does not fit with every step of 16 channels, so the long chains are cut: Y is two
+//     accumulators of 128 channels each, P one of the high limbs and one of the rest, small products first, sums in fp32.
+//     Two accumulators of Y leave room for half of its columns beside E: the first half's r' limbs wait in registers
+//     until the products of the second have read u and e'.  A box holds 32 columns of each compute thread's 64.
+// Measured (5003 tokens, 4 heads, 4-bit keys, 2-bit values, with the gather in front): 376 us with the fp32 kernel, 120.5 with
+// the narrow records' products, 122.8 so; codes and sign bits that 64-bit arithmetic decides otherwise, of 46 million each with
+// 4-bit keys: 127 and 394, 1390 and 3070, 106 and 331.
 // A compute thread (row, q) owns channels [64q, 64q+64): two value groups, one 128-byte row of a box.
 constexpr int D2 = 256;
 constexpr int D2_TILE_BYTES = 4 * BOX_BYTES;      // 128 rows x 256 bf16: four boxes
@@ -846,13 +856,21 @@ template <int ROWS>
 struct D2Ring {                                   // boxes of ROWS rows x 64 bf16 of a constant operand
     static constexpr int BYTES = ROWS * 128, SLOTS = ROWS == 256 ? 2 : 3;
     static constexpr int HALVES = D2 / ROWS, PER_MAT = 4 * HALVES, CHUNKS = 4 * PER_MAT;
+    static constexpr int BOX_ROWS = ROWS == 256 ? 256 : 32;   // a slot of 128 rows: 32 of each 64
 };
 template <int MSE_BITS, int VAL_BITS>
 constexpr int d2_ring_rows() { return MSE_BITS == 2 && VAL_BITS == 2 ? 256 : 128; }
+// What the operands of the wide records carry: u, e' and Pi are 64 times theirs, so Y, E and r' are 4096 times.
+constexpr float D2_OP = 64.f, D2_ACC = D2_OP * D2_OP;
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+constexpr int D2_BARS = 15;
 template <int ROWS>
 constexpr size_t d2_smem(size_t img) {
     return 2 * (size_t)D2_TILE_BYTES + (size_t)D2Ring<ROWS>::SLOTS * D2Ring<ROWS>::BYTES + img + 4 * TC_TOK * sizeof(float) +
-           13 * sizeof(uint64_t) + 16 + 1024;
+           D2_BARS * sizeof(uint64_t) + 16 + 1024;
 }
 
 template <int MSE_BITS, int VAL_BITS, bool SCATTER, int ROWS = d2_ring_rows<MSE_BITS, VAL_BITS>()>
@@ -865,6 +883,8 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     const TqLayout L = tq_make_layout(D2, MSE_BITS + 1, VAL_BITS);
     const int BB = L.block_bytes;
     using Ring = D2Ring<ROWS>;
+    constexpr bool F16 = MSE_BITS != 2 || VAL_BITS != 2;
+    constexpr float OP = F16 ? D2_OP : 1.f, ACC = F16 ? D2_ACC : 1.f;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (tq_smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -876,8 +896,10 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     uint64_t* bars = reinterpret_cast<uint64_t*>(s_ss + 4 * TC_TOK);
     uint64_t *bar_k = bars, *bar_v = bars + 1, *bar_m1 = bars + 2, *bar_m2 = bars + 3, *bar_r = bars + 4;
     uint64_t *bar_full = bars + 5, *bar_empty = bars + 8;     // [2 or 3] each: ring slot filled / its products done
-    uint64_t *bar_n = bars + 11, *bar_c = bars + 12;          // 512 arrivals: u, e' written / r' written
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+    uint64_t* bar_m1b = bars + 11;                            // F16: the second half of Y and E (bar_m1: the first)
+    uint64_t *bar_n = bars + 12, *bar_c = bars + 13;          // 512 arrivals: u, e' written / r' written
+    uint64_t* bar_y = bars + 14;                              // F16, 512 arrivals: the first half of Y has been read
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + D2_BARS);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -894,9 +916,10 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     }
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 11; ++i) tq_mbar_init(bars + i, 1);
+        for (int i = 0; i < 12; ++i) tq_mbar_init(bars + i, 1);
         tq_mbar_init(bar_n, TC_THREADS);
         tq_mbar_init(bar_c, TC_THREADS);
+        tq_mbar_init(bar_y, TC_THREADS);
         *s_fail = 0;
         tq_mbar_fence_init();
     }
@@ -949,14 +972,32 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         };
         const CUtensorMap* tb[4] = {&tm_b0, &tm_b1, &tm_b2, &tm_b3};
         const uint32_t a0 = tq_smem_u32(sA0), a1 = tq_smem_u32(sA1), ar = tq_smem_u32(sBr);
-        // chunk c of a tile: constant operand c / PER_MAT (Pi_hi, Pi_lo, M_hi, M_lo), channels [64 kc, +64), rows [ROWS half, +ROWS)
+        // Chunk c of a tile: constant operand mat (Pi_hi, Pi_lo, M_hi, M_lo), channels [64 kc, +64), rows [ROWS half, +ROWS) -
+        // F16: rows [64 g + 32 half, +32) for g = 0..3.  In order of operand, channels, half, but with F16 all of Y's and E's
+        // first half before the second, and Pi_lo before Pi_hi.
+        struct Chunk {
+            int mat, kc, half;
+        };
+        auto chunk = [](int c) -> Chunk {
+            if (F16 && c < Ring::CHUNKS / 2) return {1 - ((c >> 2) & 1), c & 3, c >> 3};
+            const int cm = c % Ring::PER_MAT;
+            return {c / Ring::PER_MAT, cm / Ring::HALVES, cm % Ring::HALVES};
+        };
         int g_loaded = 0;       // chunks requested so far, over all tiles of this CTA
         auto load_chunk = [&](int c) -> bool {
-            const int slot = g_loaded % Ring::SLOTS, cm = c % Ring::PER_MAT;
+            const int slot = g_loaded % Ring::SLOTS;
+            const Chunk ch = chunk(c);
             if (g_loaded >= Ring::SLOTS && !wait1(bar_empty + slot, (g_loaded / Ring::SLOTS - 1) & 1)) return false;
             if (elected()) {
                 tq_mbar_expect_tx(bar_full + slot, Ring::BYTES);
-                tma_load_2d(sBr + slot * Ring::BYTES, tb[c / Ring::PER_MAT], 64 * (cm / Ring::HALVES), ROWS * (cm % Ring::HALVES), bar_full + slot);
+                uint8_t* dst = sBr + slot * Ring::BYTES;
+                if (F16) {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g)
+                        tma_load_2d(dst + g * Ring::BOX_ROWS * 128, tb[ch.mat], 64 * ch.kc, 64 * g + 32 * ch.half, bar_full + slot);
+                } else {
+                    tma_load_2d(dst, tb[ch.mat], 64 * ch.kc, ROWS * ch.half, bar_full + slot);
+                }
             }
             __syncwarp();
             ++g_loaded;
@@ -964,12 +1005,14 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         };
         int g_used = 0;
         auto use_chunk = [&](int c) -> bool {   // issue every product that reads chunk c, then release its slot
-            const int slot = g_used % Ring::SLOTS, mat = c / Ring::PER_MAT, cm = c % Ring::PER_MAT, kc = cm / Ring::HALVES;
-            const uint32_t col = ROWS * (cm % Ring::HALVES);
+            const int slot = g_used % Ring::SLOTS;
+            const Chunk ch = chunk(c);
+            const int mat = ch.mat, kc = ch.kc;
+            const uint32_t col = ROWS * ch.half;
             if (!wait1(bar_full + slot, (g_used / Ring::SLOTS) & 1)) return false;
             tc_fence_after();
             if (elected()) {
-                constexpr uint32_t ID = umma_idesc_bf16(ROWS);
+                constexpr uint32_t ID = umma_idesc_bf16(ROWS, false, F16);
                 const uint32_t b_addr = ar + slot * Ring::BYTES;
 #pragma unroll
                 for (int ks = 0; ks < 4; ++ks) {
@@ -977,7 +1020,13 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     const uint64_t d0 = smem_desc_sw128(a0 + kc * BOX_BYTES + ks * 32);
                     const uint64_t d1 = smem_desc_sw128(a1 + kc * BOX_BYTES + ks * 32);
                     const uint32_t first = (kc | ks) == 0 ? 0u : 1u;
-                    if (mat == 0) {            // Pi_hi: Y (u) and E (e')
+                    if (F16 && mat < 2) {      // Y (u): channels 0-127 and 128-255 apart, Pi_lo first; E (e') with Pi_hi
+                        umma_ss(tmem_u + C_Y + 128 * (kc >> 1), d0, bd, ID, mat == 0 || (kc & 1) || ks ? 1u : 0u);
+                        if (mat == 0) umma_ss(tmem_u + C_E + col, d1, bd, ID, first);
+                    } else if (F16) {          // P: r'_hi M_hi over Y's columns, r'_lo M_hi + r'_hi M_lo over E's
+                        umma_ss(tmem_u + (mat == 2 ? C_Y : C_E) + col, d0, bd, ID, mat == 2 ? first : 1u);
+                        if (mat == 2) umma_ss(tmem_u + C_E + col, d1, bd, ID, first);
+                    } else if (mat == 0) {     // Pi_hi: Y (u) and E (e')
                         umma_ss(tmem_u + C_Y + col, d0, bd, ID, first);
                         umma_ss(tmem_u + C_E + col, d1, bd, ID, first);
                     } else if (mat == 1) {     // Pi_lo: Y (u)
@@ -990,7 +1039,8 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     }
                 }
                 umma_commit(bar_empty + slot);
-                if (c == Ring::CHUNKS / 2 - 1) umma_commit(bar_m1);
+                if (c == Ring::CHUNKS / 2 - 1) umma_commit(F16 ? bar_m1b : bar_m1);
+                if (F16 && c == Ring::CHUNKS / 4 - 1) umma_commit(bar_m1);
                 if (c == Ring::CHUNKS - 1) umma_commit(bar_m2);
             }
             __syncwarp();
@@ -1022,6 +1072,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             if (!(ok = wait1(bar_n, i & 1))) break;              // u, e' in shared memory
 #pragma unroll 1
             for (int c = 0; c < Ring::CHUNKS && ok; ++c) {
+                if (F16 && c == Ring::CHUNKS / 4 && !(ok = wait1(bar_y, i & 1))) break;   // Y's columns are free for its second half
                 if (c == Ring::CHUNKS / 2 && !(ok = wait1(bar_c, i & 1))) break;   // r' limbs in shared memory
                 ok = use_chunk(c);
                 // keep the ring full: the chunk SLOTS ahead (of this tile, or the first ones of the next tile)
@@ -1041,11 +1092,11 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         const int blk_l = row >> 4, tl = row & 15;
         const uint32_t lane_base = (uint32_t)(row & ~31) << 16;
         BookRegs<MSE_BITS> bk;
-        bk.c0 = p.cb.centroids[0];
+        bk.c0 = p.cb.centroids[0] * ACC;
 #pragma unroll
         for (int i = 0; i < (1 << MSE_BITS) - 1; ++i) {
             bk.nb[i] = -p.cb.boundaries[i] * BIG;
-            bk.step[i] = p.cb.centroids[i + 1] - p.cb.centroids[i];
+            bk.step[i] = (p.cb.centroids[i + 1] - p.cb.centroids[i]) * ACC;
         }
         auto wait_warp = [&](uint64_t* bar, uint32_t parity) -> bool {
             uint32_t ok = 1;
@@ -1113,7 +1164,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 }
                 ss = (s_ss[row] + s_ss[TC_TOK + row]) + (s_ss[2 * TC_TOK + row] + s_ss[3 * TC_TOK + row]);
                 nd = bf16r(__fsqrt_rn(ss));
-                const float rden = __frcp_rn(bf16r(nd + 1e-10f));
+                const float rden = __frcp_rn(bf16r(nd + 1e-10f)) * OP;
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
                     uint32_t up[4], ep[4];
@@ -1121,7 +1172,9 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     for (int i = 0; i < 4; ++i) {
                         const float q0 = bf_lo(xw[4 * c + i]) * rden, q1 = bf_hi(xw[4 * c + i]) * rden;
                         up[i] = pack_bf16(q0, q1);
-                        ep[i] = pack_bf16(q0 - bf_lo(up[i]), q1 - bf_hi(up[i]));
+                        const float u0 = bf_lo(up[i]), u1 = bf_hi(up[i]);
+                        if (F16) up[i] = pack_f16(u0, u1);   // eight bits: exact down to 2^-22 of the row's norm
+                        ep[i] = F16 ? pack_f16(q0 - u0, q1 - u1) : pack_bf16(q0 - u0, q1 - u1);
                     }
                     *row_chunk(sA0, c) = make_uint4(up[0], up[1], up[2], up[3]);
                     *row_chunk(sA1, c) = make_uint4(ep[0], ep[1], ep[2], ep[3]);
@@ -1134,10 +1187,27 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             bad |= !wait_warp(bar_m1, par);
             tc_fence_after();
             float rn2 = 0.f;
+            uint4 held[F16 ? 8 : 1];   // F16: the first half's limbs while u and e' are still read
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 float y[32];
-                tmem_ld32(tmem + lane_base + C_Y + q * 64 + hf * 32, y);
+                if (F16) {
+                    if (hf == 1) {
+                        bad |= !wait_warp(bar_m1b, par);
+                        tc_fence_after();
+                    }
+                    float y2[32];
+                    tmem_ld32(tmem + lane_base + C_Y + q * 32, y);
+                    tmem_ld32(tmem + lane_base + C_Y + 128 + q * 32, y2);
+                    if (hf == 0) {
+                        tc_fence_before();
+                        mbar_arrive(bar_y);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) y[i] += y2[i];
+                } else {
+                    tmem_ld32(tmem + lane_base + C_Y + q * 64 + hf * 32, y);
+                }
                 constexpr int WIDTH = MSE_BITS == 2 ? 2 : 4, PER_HALF = 16 / WIDTH;
                 uint32_t halves[32 / PER_HALF];
 #pragma unroll
@@ -1146,7 +1216,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
                     for (int jj = 0; jj < PER_HALF; ++jj) {
                         float code;
-                        bucket<MSE_BITS>(bk, y[w * PER_HALF + jj], code, y[w * PER_HALF + jj]);
+                        bucket<MSE_BITS, (int)ACC>(bk, y[w * PER_HALF + jj], code, y[w * PER_HALF + jj]);
                         wf = fmaf(code, (float)(1u << (WIDTH * jj)), wf);
                     }
                     halves[w] = __float_as_uint(wf + 8388608.f) & 0xffffu;
@@ -1158,7 +1228,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     for (int w = 0; w < 16 / PER_HALF; ++w) kc[w] = halves[2 * w] | (halves[2 * w + 1] << 16);
                 }
                 float er[32];
-                tmem_ld32(tmem + lane_base + C_E + q * 64 + hf * 32, er);
+                tmem_ld32(tmem + lane_base + C_E + (F16 ? hf * 128 + q * 32 : q * 64 + hf * 32), er);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     uint32_t hi[4], lo[4];
@@ -1167,11 +1237,29 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                         const float a = y[8 * c + 2 * i] + er[8 * c + 2 * i], b = y[8 * c + 2 * i + 1] + er[8 * c + 2 * i + 1];
                         rn2 = fmaf(a, a, rn2);
                         rn2 = fmaf(b, b, rn2);
-                        hi[i] = pack_bf16(a, b);
-                        lo[i] = pack_bf16(a - bf_lo(hi[i]), b - bf_hi(hi[i]));
+                        if (F16) {
+                            hi[i] = pack_f16(a, b);
+                            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi[i]));
+                            lo[i] = pack_f16(a - f.x, b - f.y);
+                        } else {
+                            hi[i] = pack_bf16(a, b);
+                            lo[i] = pack_bf16(a - bf_lo(hi[i]), b - bf_hi(hi[i]));
+                        }
                     }
-                    *row_chunk(sA0, 4 * hf + c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                    *row_chunk(sA1, 4 * hf + c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    if (F16 && hf == 0) {
+                        held[F16 ? c : 0] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        held[F16 ? 4 + c : 0] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    } else {
+                        *row_chunk(sA0, 4 * hf + c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *row_chunk(sA1, 4 * hf + c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    }
+                }
+            }
+            if (F16) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    *row_chunk(sA0, c) = held[F16 ? c : 0];
+                    *row_chunk(sA1, c) = held[F16 ? 4 + c : 0];
                 }
             }
             s_ss[q * TC_TOK + row] = rn2;
@@ -1185,7 +1273,13 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 float pr[32];
-                tmem_ld32(tmem + lane_base + C_Y + q * 64 + hf * 32, pr);
+                tmem_ld32(tmem + lane_base + C_Y + (F16 ? hf * 128 + q * 32 : q * 64 + hf * 32), pr);
+                if (F16) {
+                    float p2[32];
+                    tmem_ld32(tmem + lane_base + C_E + hf * 128 + q * 32, p2);
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) pr[i] += p2[i];
+                }
                 float w_lo = 0.f, w_hi = 0.f;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
@@ -1204,7 +1298,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             if (q == 0 && wr) {
                 const float r2 = (s_ss[row] + s_ss[TC_TOK + row]) + (s_ss[2 * TC_TOK + row] + s_ss[3 * TC_TOK + row]);
                 reinterpret_cast<__half*>(rec + L.off_knorm)[tl] = __float2half_rn(nd);
-                reinterpret_cast<__half*>(rec + L.off_krnorm)[tl] = __float2half_rn(nd * __fsqrt_rn(r2));
+                reinterpret_cast<__half*>(rec + L.off_krnorm)[tl] = __float2half_rn(nd * (__fsqrt_rn(r2) * (1.f / ACC)));
             }
             tq_fence_proxy_async();
             compute_barrier_or(false);       // record image complete
@@ -1280,12 +1374,11 @@ struct OperandMapSet {
     int D, box_rows;
     CUtensorMap tm[4];
 };
-bool operand_maps(CUtensorMap (&out)[4], const tq_consts* consts, int D, int box_rows) {
+bool operand_maps(CUtensorMap (&out)[4], const void* const (&want)[4], int D, int box_rows) {
     constexpr int SETS = 16;
     static std::mutex mu;
     static OperandMapSet sets[SETS];
     static int n_sets = 0, next = 0;
-    const void* want[4] = {consts->pi_limbs[0], consts->pi_limbs[1], consts->m_limbs[0], consts->m_limbs[1]};
     std::lock_guard<std::mutex> lock(mu);
     for (int i = 0; i < n_sets; ++i)
         if (sets[i].D == D && sets[i].box_rows == box_rows && memcmp(sets[i].ptr, want, sizeof(want)) == 0) {
@@ -1343,7 +1436,11 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     const size_t img = (size_t)8 * L.block_bytes;
     const bool d2_wide = D == D2 && (cfg.key_bits != 3 || cfg.value_bits != 2);   // records of 33 or 41 KB a tile
     if (paged && d2_wide) return TQ_OK;   // tq_store_paged answers "not supported" for these; its callers gather first
-    if (!consts->pi_limbs[0] || !consts->pi_limbs[1] || !consts->m_limbs[0] || !consts->m_limbs[1]) return TQ_OK;
+    // wide records: fp16 limbs of 64 Pi and M; elsewhere bf16 limbs
+    const void* const* pi = d2_wide ? consts->rows_pi : consts->pi_limbs;
+    const void* const* m = d2_wide ? consts->rows_m : consts->m_limbs;
+    const void* const limbs[4] = {pi[0], pi[1], m[0], m[1]};
+    if (!limbs[0] || !limbs[1] || !limbs[2] || !limbs[3]) return TQ_OK;
     if (((uintptr_t)key & 15) || ((uintptr_t)value & 15) || (stride_token & 7) || (stride_head & 7)) return TQ_OK;
     if (stride_token < D || (n_heads > 1 && stride_head < D)) return TQ_OK;
     if (n_heads == 1) stride_head = stride_token > D ? D : stride_token;
@@ -1355,7 +1452,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
             return TQ_OK;
     }   // never dereferenced; keep the map well formed
     for (int i = 0; i < 2; ++i)
-        if (((uintptr_t)consts->pi_limbs[i] & 15) || ((uintptr_t)consts->m_limbs[i] & 15)) return TQ_OK;
+        if (((uintptr_t)pi[i] & 15) || ((uintptr_t)m[i] & 15)) return TQ_OK;
     if (n_tokens >= ((int64_t)1 << 31) - 256) return TQ_OK;   // 32-bit box coordinates
     if (encode_tiled_fn() == nullptr) return TQ_OK;
     {   // the kernel's comparison arithmetic treats only the middle boundary as possibly (next to) zero
@@ -1403,7 +1500,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
         tm_kt = tm_k;
         tm_vt = tm_v;
     }
-    if (!maps_ok || !operand_maps(tm_b, consts, D, d2_wide ? 128 : D))
+    if (!maps_ok || !operand_maps(tm_b, limbs, D, d2_wide ? D2Ring<128>::BOX_ROWS : D))
         return TQ_OK;   // a stride pattern the tensor map cannot express: the fp32 kernel takes the call
     *handled = 1;
 

@@ -70,3 +70,27 @@ def test_the_shared_identity_table_belongs_to_the_device_that_is_current(monkeyp
     second = E.shared_identity_table(10, torch.device("cuda"))
     assert second is not first and made == [torch.device("cuda", 0), torch.device("cuda", 1)]
     assert E.shared_identity_table(10, torch.device("cuda", 0)) is first and E.shared_identity_table(5, "cuda:1") is second
+
+
+def test_threads_share_one_set_of_operands(monkeypatch):
+    """Two threads that need the operands first at the same time: the structure keeps the addresses of the tensors that the
+    object keeps."""
+    consts = E.LayerConstants(128, 3, 2, "cpu")
+    split, meet = E._split, threading.Barrier(2, timeout=0.5)
+
+    def slow(m, limbs, dtype):
+        try:
+            meet.wait()        # both threads inside, if both can be
+        except threading.BrokenBarrierError:
+            pass
+        return split(m, limbs, dtype)
+
+    monkeypatch.setattr(E, "_split", slow)
+    made, keep = [], E.LayerConstants.__setattr__
+    monkeypatch.setattr(E.LayerConstants, "__setattr__", lambda self, k, v: (made.append(v) if k == "rows_limbs" else None, keep(self, k, v))[1])
+    threads = [threading.Thread(target=consts.ensure_rows) for _ in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert len(made) == 1
+    for i in range(2):
+        assert [consts.c.rows_pi[i], consts.c.rows_m[i], consts.c.rows_s[i]] == [x[i].data_ptr() for x in consts.rows_limbs]

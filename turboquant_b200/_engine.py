@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from typing import Optional
 
 import torch
@@ -56,6 +57,9 @@ def _split(m: torch.Tensor, n_limbs: int, dtype: torch.dtype) -> list[torch.Tens
 
 def _split_bf16(m: torch.Tensor, n_limbs: int) -> list[torch.Tensor]:
     return _split(m, n_limbs, torch.bfloat16)
+
+
+_ROWS_LOCK = threading.Lock()
 
 
 class LayerConstants:
@@ -136,13 +140,14 @@ class LayerConstants:
         objects use them, which call this before their first launch."""
         if self.rows_limbs is not None or self.head_dim != 128:
             return
-        pi, s = self.Pi.cpu().double(), self.S.cpu().double()
-        mats, limbs = (pi * 64.0, s @ pi.T, s), []
-        if all(bool(t.abs().max() < 60000.0) for t in mats):   # fp16's range (a caller's own S may be anything)
-            limbs = [[t.contiguous().to(self.device) for t in _split(x, 2, torch.float16)] for x in mats]
-            for i in range(2):
+        with _ROWS_LOCK:   # one set per object: the structure holds the addresses of the tensors that rows_limbs keeps
+            if self.rows_limbs is not None:
+                return
+            pi, s = self.Pi.cpu().double(), self.S.cpu().double()
+            limbs = self._fp16_limbs(pi * 64.0, s @ pi.T, s)
+            for i in range(2 if limbs else 0):
                 self.c.rows_pi[i], self.c.rows_m[i], self.c.rows_s[i] = (x[i].data_ptr() for x in limbs)
-        self.rows_limbs = limbs
+            self.rows_limbs = limbs
 
     @property
     def block_bytes(self) -> int:

@@ -236,3 +236,46 @@ def test_d256_wide_store_without_fp16_operands(dev):
         planes.append(E.pool_to_planes(c, pool, bt, n))
     for f in ("mse_indices", "qjl_signs", "norms", "residual_norms"):
         assert torch.equal(getattr(planes[0], f), getattr(planes[1], f))
+
+
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_key_rows_kernels_are_as_exact_as_fp32(bits, dtype, dev):
+    """Quantising and dequantising plain rows by limb products against 64 bits and against the fp32 kernels on records:
+    the same codes, not more wrong sign bits (three standard deviations), no larger error of the rows that come back."""
+    from turboquant_b200 import TurboQuantProd, _engine as E
+    n = 200000
+    z = TurboQuantProd(128, bits, device=dev)
+    g = torch.Generator(device=dev)
+    g.manual_seed(13)
+    x = (torch.randn(n, 128, generator=g, device=dev) * torch.exp(0.5 * torch.randn(128, generator=g, device=dev))).to(dtype)
+    kq, ps = z.quantize(x), z._compress_rows(x)[2]
+    assert torch.equal(kq.mse_indices, ps.mse_indices[0])
+    fast, exact = (_wrong(z.consts, x, s.mse_indices.view(n, -1), s.qjl_signs.view(n, -1))[1] for s in (kq, ps))
+    assert fast <= exact + 3 * math.sqrt(fast + exact)
+    ref = _keys64(z.consts, kq.mse_indices, kq.qjl_signs, kq.norms, kq.residual_norms)
+    pool, bt, _, m = z._pool_from(kq.mse_indices, kq.qjl_signs, kq.norms, kq.residual_norms)
+    err = [float((t.reshape(n, 128).double() - ref).norm() / ref.norm()) for t in (z.dequantize(kq), E.dequant_keys(z.consts, pool, bt, m))]
+    assert err[0] <= err[1]
+
+
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_key_rows_on_the_decision_boundaries(bits, dtype, dev):
+    """Rows with half of their rotated coordinates on a boundary, where the limb product decides otherwise than the fp32
+    chain in many a row, which is then redone as a whole: codes, residual norms and sign bits are the fp32 store's."""
+    from turboquant_b200 import TurboQuantProd
+    n = 3000
+    z = TurboQuantProd(128, bits, device=dev)
+    g = torch.Generator().manual_seed(bits)
+    inner = z.consts.boundaries_cpu[1:-1].double()
+    y = inner[torch.randint(0, len(inner), (n, 128), generator=g)]
+    rest = torch.randn(n, 64, generator=g).double()
+    room = (1 - y[:, :64].pow(2).sum(1, keepdim=True)).clamp_min(1e-3).sqrt()
+    y[:, 64:] = rest / rest.norm(dim=1, keepdim=True) * room
+    x = (y @ z.consts.Pi.cpu().double()).to(dtype).to(dev)
+    kq, ps = z.quantize(x), z._compress_rows(x)[2]
+    assert torch.equal(kq.mse_indices, ps.mse_indices[0])
+    assert torch.equal(kq.norms.half(), ps.norms[0])
+    torch.testing.assert_close(kq.residual_norms, ps.residual_norms[0].float(), rtol=1.1e-3, atol=0)   # an ulp of fp16
+    assert _bit_frac(kq.qjl_signs, ps.qjl_signs[0]) <= 2e-5     # sums of 128 terms within 1e-6 of zero

@@ -164,23 +164,45 @@ __device__ __forceinline__ void b_frag(uint32_t mat, int n0, int ks, int lane, u
     const int ch = TRANS ? (n0 >> 3) + (blk >> 1) : 2 * ks + (blk & 1);
     ldsm4<TRANS>(mat + row * 256 + ((ch ^ (row & 7)) << 4), r);
 }
-// acc[2][4] += A (LA limbs in registers) * B (two limbs), without lo * lo
-template <int LA, bool TRANS>
+// The same onto zero
+__device__ __forceinline__ void mma_f16_z(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// acc[2][4] += A (LA limbs in registers) * B (two limbs), without lo * lo.
+// The pipe drops what does not fit its accumulator instead of rounding, so the large products (hi * hi) must not pass through
+// it together with the small ones, which have accumulators of their own.  STEPS: not with each other either - every k-step's
+// sum is added up in fp32.  Error of a product against 64 bits, unit vectors: one chain for all 4.6e-7 of the result (5.6e-7
+// with 3-bit codes), two chains 1.9e-7 (2.5e-7), STEPS 0.9e-7 (1.1e-7); the fp32 fused multiply-adds of the kernels on records
+// 2.0e-7.  16000 rows: two chains cost nothing, STEPS 2.4 us where both products of a dequantisation take it.
+template <int LA, bool TRANS, bool STEPS>
 __device__ __forceinline__ void product(float (&acc)[2][4], const uint32_t (*a)[KSTEPS][4], uint32_t mats, int n0, int lane) {
+    float low[2][4] = {};
 #pragma unroll
     for (int ks = 0; ks < KSTEPS; ++ks) {
+        uint32_t b[4], bl[4];
+        b_frag<TRANS>(mats, n0, ks, lane, b);
+        b_frag<TRANS>(mats + R_MAT, n0, ks, lane, bl);
 #pragma unroll
-        for (int lb = 0; lb < 2; ++lb) {
-            uint32_t b[4];
-            b_frag<TRANS>(mats + lb * R_MAT, n0, ks, lane, b);
+        for (int n8 = 0; n8 < 2; ++n8) {
+            if (STEPS) {
+                float t[4];
+                mma_f16_z(t, a[0][ks], b[2 * n8], b[2 * n8 + 1]);
 #pragma unroll
-            for (int la = 0; la < LA; ++la)
-                if (la + lb < 2) {
-                    mma_f16(acc[0], a[la][ks], b[0], b[1]);
-                    mma_f16(acc[1], a[la][ks], b[2], b[3]);
-                }
+                for (int c = 0; c < 4; ++c) acc[n8][c] += t[c];
+            } else {
+                mma_f16(acc[n8], a[0][ks], b[2 * n8], b[2 * n8 + 1]);
+            }
+            if (LA == 2) mma_f16(low[n8], a[LA - 1][ks], b[2 * n8], b[2 * n8 + 1]);
+            mma_f16(low[n8], a[0][ks], bl[2 * n8], bl[2 * n8 + 1]);
         }
     }
+#pragma unroll
+    for (int n8 = 0; n8 < 2; ++n8)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[n8][c] += low[n8][c];
 }
 
 constexpr float R_SCALE = 64.f;   // of every A operand and of Pi: unit vectors, centroids and residuals are far below 1
@@ -391,7 +413,7 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
 #pragma unroll
         for (int nb = 0; nb < RD / 16; ++nb) {
             float acc[2][4] = {};
-            product<LU, false>(acc, a, sp, nb * 16, lane);
+            product<LU, false, false>(acc, a, sp, nb * 16, lane);
             float er[2][4] = {};
             if (DT != TQ_F32) {
 #pragma unroll
@@ -457,7 +479,7 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
 #pragma unroll
         for (int nb = 0; nb < RD / 16; ++nb) {
             float acc[2][4] = {};
-            product<2, false>(acc, rl, sm, nb * 16, lane);
+            product<2, false, false>(acc, rl, sm, nb * 16, lane);
 #pragma unroll
             for (int n8 = 0; n8 < 2; ++n8)
 #pragma unroll
@@ -586,8 +608,8 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_dequantize_keys_kerne
 #pragma unroll 1
         for (int nb = 0; nb < RD / 16; ++nb) {
             float ak[2][4] = {}, as[2][4] = {};
-            product<2, true>(ak, a, sp, nb * 16, lane);
-            if (p.with_qjl) product<1, true>(as, sg, ssg, nb * 16, lane);
+            product<2, true, true>(ak, a, sp, nb * 16, lane);
+            if (p.with_qjl) product<1, true, true>(as, sg, ssg, nb * 16, lane);
 #pragma unroll
             for (int n8 = 0; n8 < 2; ++n8)
 #pragma unroll

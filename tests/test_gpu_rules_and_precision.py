@@ -279,3 +279,39 @@ def test_key_rows_on_the_decision_boundaries(bits, dtype, dev):
     assert torch.equal(kq.norms.half(), ps.norms[0])
     torch.testing.assert_close(kq.residual_norms, ps.residual_norms[0].float(), rtol=1.1e-3, atol=0)   # an ulp of fp16
     assert _bit_frac(kq.qjl_signs, ps.qjl_signs[0]) <= 2e-5     # sums of 128 terms within 1e-6 of zero
+
+
+def test_captured_decode_reads_its_lengths_at_replay(dev):
+    """A step captured at the longest history and replayed after a shorter one took its place attends to the shorter one;
+    a captured fused step appends behind the tokens that the ring then holds."""
+    from turboquant_b200 import CompressedKVStore, KVCaptureEngine, compute_hybrid_attention
+    d, h, qh, n = 128, 4, 16, 600
+    k, v = (t.to(dev) for t in O.synth_kv(n + 40, h, d, seed=1, dtype=torch.bfloat16))
+    q = O.synth_query(1, qh, d, seed=2, dtype=torch.bfloat16).to(dev)
+    store = CompressedKVStore(d, h, 3, 2, device=dev, capacity_tokens=n)
+    engine = KVCaptureEngine(store, ring_capacity=64, device=dev)
+    store.append_chunk(k[:n], v[:n])
+    engine.ingest_decode(k[n:n + 20], v[n:n + 20], 20)
+    rk, rv = engine.ring.peek()
+    store.seq_len_device, engine.ring.device_len()
+    compute_hybrid_attention(q, store, rk, rv, qh)      # scratch at its size
+    one, step = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(one):
+        out = compute_hybrid_attention(q, store, rk, rv, qh)
+    store.reset()
+    store.append_chunk(k[:200], v[:200])
+    store.seq_len_device
+    one.replay()
+    torch.cuda.synchronize()
+    want = compute_hybrid_attention(q, store, rk, rv, qh)
+    torch.testing.assert_close(out.float(), want.float(), rtol=2e-2, atol=2e-3)
+
+    engine.decode_step(q, k[n + 20:n + 21], v[n + 20:n + 21], qh)
+    engine.ring.device_len()
+    with torch.cuda.graph(step):
+        engine.decode_step(q, k[n + 21:n + 22], v[n + 21:n + 22], qh)
+    step.replay()
+    step.replay()                                       # the second behind the first
+    torch.cuda.synchronize()
+    keys = engine.ring.storage[0]
+    assert torch.equal(keys[21], k[n + 21]) and torch.equal(keys[22], k[n + 21])

@@ -315,3 +315,24 @@ def test_captured_decode_reads_its_lengths_at_replay(dev):
     torch.cuda.synchronize()
     keys = engine.ring.storage[0]
     assert torch.equal(keys[21], k[n + 21]) and torch.equal(keys[22], k[n + 21])
+
+
+def test_cache_object_takes_weights_that_broadcast(dev):
+    """Weights shared by the heads or the batch, or without a batch: what the matrix products broadcast or refuse."""
+    from turboquant_b200 import TurboQuantKVCache
+    g = torch.Generator().manual_seed(4)
+    for b, shapes, bad in ((2, ((2, 3, 2), (2, 1, 2), (1, 3, 2), (1, 1, 2)), ((3, 2, 2), (6, 2))), (1, ((1, 3, 2), (3, 2), (3, 1, 2)), ((1, 2, 2), (2, 2)))):
+        cache = TurboQuantKVCache(128, 3, 2, buffer_size=16, device=dev, dtype=torch.float32)
+        k, v = (torch.randn(b, 3, 200, 128, generator=g).to(dev) for _ in range(2))
+        cache.prefill(k, v)
+        eye = torch.eye(200, device=dev).expand(b, 3, 200, 200).contiguous()
+        values = torch.cat([cache.attend(eye[..., i:i + 100, :].contiguous()) for i in (0, 100)], -2)
+        for lead in shapes:
+            w = torch.softmax(torch.randn(*lead, 200, generator=g), -1).to(dev)
+            got = cache.attend(w)
+            want = torch.matmul(w, values)
+            assert got.shape == want.shape
+            torch.testing.assert_close(got, want, rtol=1e-4, atol=1e-5)
+        for lead in bad:
+            with pytest.raises(RuntimeError):
+                cache.attend(torch.ones(*lead, 200, device=dev))

@@ -207,6 +207,13 @@ class TurboQuantKVCache:
             self.key_buffer = self.key_buffer[..., n_flush:, :]
             self.value_buffer = self.value_buffer[..., n_flush:, :]
 
+    def _by_heads(self, t: torch.Tensor) -> Optional[torch.Tensor]:
+        """`t` as (batch, heads, ...) where every head of the history has rows of its own in it; None for what the matrix
+        products of the general way broadcast or refuse."""
+        if t.dim() == 3 and self._lead[0] == 1:
+            t = t.unsqueeze(0)
+        return t if t.dim() == 4 and tuple(t.shape[:2]) == self._lead else None
+
     def attention_scores(self, query: torch.Tensor, scale: float = None) -> torch.Tensor:
         """query (batch, heads, n_q, d) -> logits (batch, heads, n_q, seq_len)."""
         if scale is None:
@@ -214,9 +221,8 @@ class TurboQuantKVCache:
         parts = []
         if self._n_quant > 0:
             b, h = self._lead
-            n_q, buf = query.shape[-2], self.key_buffer
-            if query.is_cuda and (buf is None or buf.dtype == query.dtype):
-                q4 = query if query.shape[:2] == (b, h) else query.reshape(b, h, n_q, self.head_dim)
+            q4, buf = self._by_heads(query), self.key_buffer
+            if query.is_cuda and q4 is not None and (buf is None or buf.dtype == query.dtype):
                 logits = E.cache_scores(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant, q4, buf, float(scale))
                 if logits is not None:
                     return logits
@@ -234,9 +240,8 @@ class TurboQuantKVCache:
             b, h = self._lead
             buf = self.value_buffer
             n_all = self._n_quant + (buf.shape[-2] if buf is not None else 0)
-            if attn_weights.is_cuda and attn_weights.shape[-1] == n_all:
-                n_q = attn_weights.shape[-2]
-                w4 = attn_weights if attn_weights.shape[:2] == (b, h) else attn_weights.reshape(b, h, n_q, n_all)
+            w4 = self._by_heads(attn_weights)
+            if attn_weights.is_cuda and w4 is not None and attn_weights.shape[-1] == n_all:
                 out = E.cache_attend(self.consts, self._pool, self._ws_attn, self._bt, self._n_quant, w4, buf)
                 if out is not None:
                     return out

@@ -336,3 +336,16 @@ def test_cache_object_takes_weights_that_broadcast(dev):
         for lead in bad:
             with pytest.raises(RuntimeError):
                 cache.attend(torch.ones(*lead, 200, device=dev))
+
+
+def test_hybrid_attention_on_strided_tensors_equals_contiguous_ones(dev):
+    from turboquant_b200 import CompressedKVStore, compute_hybrid_attention
+    g = torch.Generator(device=dev)
+    g.manual_seed(8)
+    wide = lambda *s: torch.randn(*s, 256, generator=g, device=dev).bfloat16()[..., :128]  # noqa: E731
+    store = CompressedKVStore(128, 4, 3, 2, device=dev, capacity_tokens=500)
+    store.append_chunk(wide(500, 4).contiguous(), wide(500, 4).contiguous())
+    q, rk, rv = wide(3, 16), wide(30, 4), wide(30, 4)
+    want = compute_hybrid_attention(q.contiguous(), store, rk.contiguous(), rv.contiguous(), 16)
+    assert torch.equal(compute_hybrid_attention(q, store, rk, rv, 16), want)
+    assert torch.equal(compute_hybrid_attention(q, store, rk.contiguous(), rv, 16), want)

@@ -32,9 +32,15 @@ def compute_hybrid_attention(query: torch.Tensor, store: CompressedKVStore, rece
     mask, as in the reference); history shorter than 16 tokens is ignored.
     """
     if query.dim() == 3:
-        out = E.host().hybrid(store.consts.addr, store.pool.addr, store.workspace, store.block_table, store.head_dim,
-                              store._num_tokens, query, query.shape[0], num_query_heads, recent_k, recent_v, None,
-                              scale, MIN_HISTORY_FOR_TQ, None)
+        native, args = E.host().hybrid, (store.consts.addr, store.pool.addr, store.workspace, store.block_table, store.head_dim,
+                                         store._num_tokens)
+        rest = (None, scale, MIN_HISTORY_FOR_TQ, None)
+        out = native(*args, query, query.shape[0], num_query_heads, recent_k, recent_v, *rest)
+        if out is None and query.is_cuda:      # once more where strides were the reason
+            q = query.contiguous()
+            rk, rv = (t.contiguous() if isinstance(t, torch.Tensor) else t for t in (recent_k, recent_v))
+            if q is not query or rk is not recent_k or rv is not recent_v:
+                out = native(*args, q, q.shape[0], num_query_heads, rk, rv, *rest)
         if type(out) is torch.Tensor:
             return out
         if out is not None:

@@ -349,3 +349,16 @@ def test_hybrid_attention_on_strided_tensors_equals_contiguous_ones(dev):
     want = compute_hybrid_attention(q.contiguous(), store, rk.contiguous(), rv.contiguous(), 16)
     assert torch.equal(compute_hybrid_attention(q, store, rk, rv, 16), want)
     assert torch.equal(compute_hybrid_attention(q, store, rk.contiguous(), rv, 16), want)
+
+
+def test_a_host_tensor_is_no_place_for_a_result(dev):
+    from turboquant_b200 import CompressedCacheSpec, CompressedPagedKVCache
+    cache = CompressedPagedKVCache.allocate(CompressedCacheSpec(128, 2, 3, 2), 4, dev)
+    k = torch.randn(40, 2, 128, device=dev).bfloat16()
+    cache.write(k, k, torch.arange(40, device=dev))
+    q, table, lens = torch.randn(1, 8, 128, device=dev).bfloat16(), torch.arange(4, dtype=torch.int32, device=dev)[None], \
+        torch.tensor([40], dtype=torch.int32, device=dev)
+    with pytest.raises((TypeError, ValueError, RuntimeError)):
+        cache.decode(q, table, lens, 40, out=torch.empty(1, 8, 128, dtype=torch.bfloat16))
+    out = torch.empty_like(q)
+    assert cache.decode(q, table, lens, 40, out=out) is out

@@ -338,6 +338,7 @@ def decode(consts: LayerConstants, pool: BlockPool, ws: Workspace, query: torch.
     query = query.contiguous()
     if out is None:
         out = torch.empty_like(query)
+    require_cuda(out, "out")
     if scale is None:
         scale = 1.0 / math.sqrt(d)
     h = pool.num_kv_heads

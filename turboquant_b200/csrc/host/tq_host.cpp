@@ -285,7 +285,7 @@ PyObject* batch(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         Py_RETURN_NONE;
     const int64_t b = q->size(0), qh = q->size(1);
     const int dt = dtype_code(q->scalar_type());
-    if (dt < 0 || (out && (!out->is_contiguous() || out->sizes() != q->sizes() || out->scalar_type() != q->scalar_type()))) Py_RETURN_NONE;
+    if (dt < 0 || (out && (!out->is_cuda() || !out->is_contiguous() || out->sizes() != q->sizes() || out->scalar_type() != q->scalar_type()))) Py_RETURN_NONE;
     tq_decode_args a = {};
     int rc = TQ_OK;
     if (!plan(a, c, pool, args[2], (int)b, (int)qh, (int)max_seq, 0, &rc)) return nullptr;

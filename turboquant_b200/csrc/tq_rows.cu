@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(128) tq_rows_scores_kernel(const RowsParams p,
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int i = tid; i < D * GP; i += 128) {
         const int j = i / GP, g = i % GP;
-        const float* src = qprep + ((int64_t)(h * n_q + q0 + g) * 2) * D;
+        const float* src = qprep + (((int64_t)h * n_q + q0 + g) * 2) * D;
         qr[i] = g < nq ? src[j] : 0.f;
         qs[i] = g < nq ? src[D + j] : 0.f;
     }

@@ -829,6 +829,7 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     p.ring_splits = rsplits;
     p.ring_tok = ring_tok;
     p.land_bytes = 0;
+    p.host_io = early_inputs;
     p.pool_late = tq_last_launch(st) == TQ_LAUNCH_PREP_BEHIND_STORE ? 1 : 0;
 
     const int mse_bits = consts->cfg.key_bits - 1, vb = consts->cfg.value_bits;

@@ -41,6 +41,7 @@ struct DecodeParams {
     int num_splits, ring_splits;
     int ring_tok;          // ring tokens per ring CTA, a multiple of RING_TOK
     uint32_t land_bytes;   // tensor-core kernel: shared memory in front of its barriers, reusable by the merge
+    int host_io;           // the query is read from host memory
     int pool_late;         // a store ahead of the query preparation may still be writing records: wait before the first one
 };
 

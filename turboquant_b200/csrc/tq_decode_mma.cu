@@ -40,11 +40,13 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 // launch's time at 8 kv heads, sixteen warps / twelve: 0.93 (one set of fragments) and 0.97 (two sets) from 64 ring tokens on
 // and up to 8000 of history, which is 32 records a CTA; 0.98 at 48 records; 0.98 to 1.03 at 63; 0.95 to 1.02 with 40 ring
 // tokens; 1.00 to 1.06 with 1 or 16, 1.00 to 1.13 without a ring (two sets do not fit the registers and are read from shared
-// memory).  At head_dim 256 it costs registers.
+// memory); the ring's CTAs take 32 tokens at a time.  With the query in host memory they also fetch it from there, the more at
+// a time the more threads: a step of decode_step_host 18.2 us for 20.4 at 4000 tokens, whatever the ring holds, and 23.4 for
+// 24.1 at 30000.  At head_dim 256 sixteen warps cost registers.
 constexpr int NW_WAVE = 12;
 constexpr int NW_SINGLE = 16;
 constexpr int NW_MULTI = 8;
-constexpr int SINGLE_RING = 48, SINGLE_RECORDS = 48;   // at least so many ring tokens, at most so many records a CTA
+constexpr int SINGLE_RING = 33, SINGLE_RECORDS = 48;   // at least so many ring tokens, at most so many records a CTA
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
 
 
@@ -787,7 +789,7 @@ int launch_mma(const DecodeParams& p, int batch, cudaStream_t st, int* handled) 
         return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_MULTI>(p, batch, st);
     }
     if constexpr (D == 128)
-        if (batch == 1 && p.max_ring_len >= SINGLE_RING && records <= SINGLE_RECORDS && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
+        if (batch == 1 && (p.host_io || (p.max_ring_len >= SINGLE_RING && records <= SINGLE_RECORDS)) && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
             return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_SINGLE>(p, batch, st);
     if (fits_wave) return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_WAVE>(p, batch, st);
     *handled = 0;

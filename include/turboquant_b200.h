@@ -94,7 +94,7 @@ typedef struct tq_consts {
      * tq_rows_quantize_keys / tq_rows_dequantize_keys at head_dim 128, which return
      * TQ_ERR_UNSUPPORTED with any of them NULL, and (64 Pi and M) of the tensor-core
      * store at head_dim 256 with 4-bit keys or values, which the fp32 kernel replaces
-     * then.  For the store, rows of Pi of norm < 8 and centroids < 8. */
+     * then.  For the store, rows of Pi of norm < 8 and centroids < 7. */
     const void* rows_pi[2];
     const void* rows_m[2];
     const void* rows_s[2];

@@ -94,3 +94,16 @@ def test_threads_share_one_set_of_operands(monkeypatch):
     assert len(made) == 1
     for i in range(2):
         assert [consts.c.rows_pi[i], consts.c.rows_m[i], consts.c.rows_s[i]] == [x[i].data_ptr() for x in consts.rows_limbs]
+
+
+@pytest.mark.parametrize("row,top,taken", [(1.0, 0.2, True), (7.9, 0.2, True), (8.1, 0.2, False), (1.0, 6.9, True), (1.0, 7.1, False)])
+def test_operands_of_the_wide_store_keep_residuals_inside_fp16(row, top, taken):
+    """Residuals are carried 4096 times: |u| |row of Pi| + |centroid| + what E adds must stay below 65504 / 4096."""
+    unit = E.LayerConstants(256, 4, 2, "cpu")
+    pi = unit.Pi / unit.Pi.norm(dim=1, keepdim=True) * row
+    cents = torch.linspace(-top, top, 8)
+    bounds = torch.cat((torch.tensor([-10.0 * top]), (cents[1:] + cents[:-1]) / 2, torch.tensor([10.0 * top])))
+    consts = E.LayerConstants(256, 4, 2, "cpu", Pi=pi, centroids=cents, boundaries=bounds)
+    assert (consts.rows_limbs is not None) == taken and (consts.c.rows_pi[0] is not None) == taken
+    if taken:
+        assert (row * (1 + 2 ** -8 + 2 ** -9) * (1 + 2 ** -8) + top) * 4096 < 65504

@@ -121,7 +121,7 @@ class LayerConstants:
         self.rows_limbs = None
         if tensor_core_store and head_dim == 256 and (key_bits, value_bits) != (3, 2):
             # the wide records' store keeps 22 bits of Pi and M; its residuals must stay in fp16's range
-            if float(pi.norm(dim=1).max()) < 8 and float(self.centroids_cpu.abs().max()) < 8:
+            if float(pi.norm(dim=1).max()) < 8 and float(self.centroids_cpu.abs().max()) < 7:
                 self.rows_limbs = self._fp16_limbs(pi.double() * 64.0, m)
                 for i in range(2 if self.rows_limbs else 0):
                     c.rows_pi[i], c.rows_m[i] = (x[i].data_ptr() for x in self.rows_limbs)

@@ -197,6 +197,8 @@ int tq_prefill_attention_read_status(int32_t* out);
  * is launched in plain stream order; likewise the first kernel of a tq_decode*
  * call that follows one of these stores (the decode kernels fetch lengths,
  * block tables and their first records before they wait for the launch ahead).
+ * With a block table the kernels may fill the slots of the last block behind the last token (a later
+ * append overwrites them): tokens are appended, not rewritten in the middle of a sequence.
  * Device-side status: tq_store_read_status. */
 int tq_store(const tq_consts* consts, const void* key, const void* value, tq_dtype dtype,
              int64_t n_tokens, int32_t n_heads, int64_t stride_token, int64_t stride_head,

@@ -1239,7 +1239,7 @@ def test_ring_write_in_one_launch(dtype, n, pos, strided, dev):
                                             (128, 3, torch.float16, 16), (128, 4, torch.float16, 127), (256, 3, torch.float32, 33)])
 def test_key_rows_kernels_match_store_and_pool_kernels(d, bits, dtype, n, dev):
     """Quantise / dequantise / score on plain rows against the same work through a pool of records (edges of the
-    16-row warps and 128-row tiles; a zero row; a key that sits on a decision boundary's neighbour is part of any draw)."""
+    16-row warps and 128-row tiles; a zero row)."""
     from turboquant_b200 import TurboQuantProd, _engine as E
     q = TurboQuantProd(d, bits, device=dev)
     g = torch.Generator().manual_seed(n + bits)
@@ -1350,8 +1350,8 @@ def test_d256_store_with_wide_records(kb, vb, n, dev):
 
 @pytest.mark.parametrize("d,kb,vb,qh", [(128, 3, 2, 16), (128, 3, 2, 8), (128, 4, 4, 8), (256, 3, 2, 8)])
 def test_decode_by_pairs_of_records(d, kb, vb, qh, dev):
-    """Several waves of CTAs: 0, 1, 2 or 3 records a warp (a pair without a partner, a partly filled last record), scores
-    that climb along the sequence far past the softmax reference, and stale Inf bytes behind the last token."""
+    """Several waves of CTAs with 0 to 4 records a warp (taken one by one; a partly filled last record), scores that climb
+    along the sequence far past the softmax reference, and stale Inf bytes behind the last token."""
     from turboquant_b200 import _engine as E
     h, nseq, nmax = 4, 80, 400                       # 320 CTAs of eight warps, up to 25 records each
     c = E.LayerConstants(d, kb, vb, dev, seed=5)
@@ -1399,7 +1399,7 @@ def test_decode_right_behind_a_store(nseq, n, splits, dev):
 @pytest.mark.parametrize("qh,h,n,dtype", [(32, 8, 1300, torch.bfloat16), (40, 8, 1025, torch.float16), (12, 4, 3328, torch.bfloat16),
                                           (300, 100, 130, torch.bfloat16), (304, 8, 1, torch.float16)])
 def test_prefill_attention_pairs_of_query_tiles(qh, h, n, dtype, dev):
-    """Launches of more than two waves of tiles: even and odd numbers of query tiles, a last tile of one row, a single tile."""
+    """Launches of several waves of tiles: even and odd numbers of query tiles, a last tile of one row, a single tile."""
     test_prefill_attention_vs_fp32_reference(128, qh, h, n, dtype, dev)
 
 

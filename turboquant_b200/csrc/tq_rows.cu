@@ -13,8 +13,8 @@
 // per m16n8k16 and scheduler) and not by fp32 FMAs, which needed 3 x 16384 per row at a fifth of their peak.
 //
 // Measured (B200, 16000 rows of 128, 3-bit keys): quantise 51 us as half of a store into records plus 10 for the
-// conversion to planes -> 31 (20 without the re-examined coordinates); dequantise 80 -> 12; a whole quantise, score,
-// dequantise pass of keys and values 807 -> 109, 70 with the native host path.
+// conversion to planes -> 22 back to back; dequantise 80 -> 12.6; a whole quantise, score, dequantise pass of keys and
+// values 807 -> 67 to 73.
 #include "tq_decode_common.cuh"
 
 using namespace tqdec;
@@ -176,7 +176,9 @@ __device__ __forceinline__ void mma_f16_z(float (&c)[4], const uint32_t (&a)[4],
 // it together with the small ones, which have accumulators of their own.  STEPS: not with each other either - every k-step's
 // sum is added up in fp32.  Error of a product against 64 bits, unit vectors: one chain for all 4.6e-7 of the result (5.6e-7
 // with 3-bit codes), two chains 1.9e-7 (2.5e-7), STEPS 0.9e-7 (1.1e-7); the fp32 fused multiply-adds of the kernels on records
-// 2.0e-7.  16000 rows: two chains cost nothing, STEPS 2.4 us where both products of a dequantisation take it.
+// 2.0e-7.  Of 384 million fp32 coordinates 319, 129 and 58 sign bits came out wrong, 259 in the fp32 store.  A pass over 16000
+// rows (quantise, score, dequantise) takes 73 us with one chain, 67 with two for quantising and STEPS for dequantising, 75 with
+// STEPS everywhere.
 template <int LA, bool TRANS, bool STEPS>
 __device__ __forceinline__ void product(float (&acc)[2][4], const uint32_t (*a)[KSTEPS][4], uint32_t mats, int n0, int lane) {
     float low[2][4] = {};

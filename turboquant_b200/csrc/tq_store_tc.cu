@@ -847,7 +847,7 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 //     Two accumulators of Y leave room for half of its columns beside E: the first half's r' limbs wait in registers
 //     until the products of the second have read u and e'.  A box holds 32 columns of each compute thread's 64.
 // Measured (5003 tokens, 4 heads, 4-bit keys, 2-bit values, with the gather in front): 376 us with the fp32 kernel, 120.5 with
-// the narrow records' products, 122.8 so; codes and sign bits that 64-bit arithmetic decides otherwise, of 46 million each with
+// the narrow records' products, 122.8 so; codes and sign bits that 64-bit arithmetic decides otherwise, of 384 million each with
 // 4-bit keys: 127 and 394, 1390 and 3070, 106 and 331.
 // A compute thread (row, q) owns channels [64q, 64q+64): two value groups, one 128-byte row of a box.
 constexpr int D2 = 256;

@@ -1,0 +1,79 @@
+"""Edges of the kernels' splits - ring tokens over warps, partial results over threads, queries over CTAs, rows over tiles -
+against 64-bit arithmetic on what the records hold."""
+
+import math
+
+import pytest
+import torch
+
+from tests.test_gpu_rules_and_precision import _keys64, _unpack
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    return torch.device("cuda:0")
+
+
+def _history64(consts, planes, n, vb):
+    """Dequantised keys and values (H, n, D) in 64 bits."""
+    k = _keys64(consts, planes.mse_indices[:, :n], planes.qjl_signs[:, :n], planes.norms[:, :n], planes.residual_norms[:, :n])
+    code = _unpack(planes.v_data[:, :n], vb).double()
+    scale, zero = (t[:, :n].double().repeat_interleave(32, -1) for t in (planes.v_scales, planes.v_zeros))
+    return k, code * scale + zero
+
+
+def _attend64(q, k, v, group):
+    """q (T, Qh, D), k / v (H, N, D) -> (T, Qh, D)"""
+    k, v = (t.repeat_interleave(group, 0) for t in (k, v))
+    p = torch.softmax(torch.einsum("thd,hnd->thn", q.double(), k) / math.sqrt(q.shape[-1]), -1)
+    return torch.einsum("thn,hnd->thd", p, v)
+
+
+def _rel(got, want):
+    return float((got.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("d,h,qh", [(128, 8, 32), (128, 2, 16), (128, 3, 3), (256, 4, 16), (256, 2, 16)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_ring_lengths_on_both_sides_of_every_split(d, h, qh, dtype, dev):
+    """Ring tokens alone (a history below 16 tokens does not count): fp32 all the way.  A score is a sum of D products,
+    wrong by at most (log2(D) + 8) 2^-24 sum |q k| / sqrt(D) <= 16 * 6e-8 * 13 = 1.2e-5, which is the relative error of a
+    probability; the 2^-22 of the exponential's approximation and the output's own rounding come on top."""
+    from turboquant_b200 import CompressedKVStore, compute_hybrid_attention
+    store = CompressedKVStore(d, h, 3, 2, device=dev)
+    g = torch.Generator(device=dev).manual_seed(d + qh)
+    r_max = 256
+    k, v = (torch.randn(r_max, h, d, generator=g, device=dev, dtype=dtype) for _ in range(2))
+    q = torch.randn(1, qh, d, generator=g, device=dev, dtype=dtype)
+    tol = 3e-5 + {torch.float32: 0.0, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dtype]
+    for r in (1, 2, 3, 23, 24, 25, 31, 32, 33, 47, 48, 49, 63, 64, 65, 95, 97, 127, 128, 129, 191, 193, 256):
+        out = compute_hybrid_attention(q, store, k[:r], v[:r], qh)
+        want = _attend64(q, k[:r].double().transpose(0, 1), v[:r].double().transpose(0, 1), qh // h)
+        assert _rel(out, want) <= tol, r
+    assert store.workspace.status() == 0
+
+
+@pytest.mark.parametrize("d,h,qh,kb,vb", [(128, 2, 8, 3, 2), (128, 1, 8, 4, 4), (256, 1, 4, 3, 2), (256, 2, 16, 4, 2)])
+def test_merge_of_any_number_of_partial_results(d, h, qh, kb, vb, dev):
+    """One CTA up to more slots than a warp looks at twice, with and without ring slots between.  Probabilities are fp16
+    (2^-12 each, 5e-4 measured for whole outputs), so twice what they give bounds a slot left out or taken twice, which
+    would cost at least 1 / 140."""
+    from turboquant_b200 import CompressedKVStore, _engine as E
+    n = 2240
+    store = CompressedKVStore(d, h, kb, vb, device=dev, capacity_tokens=n)
+    g = torch.Generator(device=dev).manual_seed(7 * d + qh)
+    k, v = (torch.randn(n, h, d, generator=g, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    store.append_chunk(k, v)
+    rk, rv = (torch.randn(70, h, d, generator=g, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    q = torch.randn(1, qh, d, generator=g, device=dev)
+    k64, v64 = _history64(store.consts, E.pool_to_planes(store.consts, store.pool, store.block_table, n), n, vb)
+    lens, ring_lens = (torch.tensor([x], dtype=torch.int32, device=dev) for x in (n, 70))
+    for splits in (1, 2, 3, 4, 13, 14, 37, 40, 63, 64, 65, 100, 128, 140):
+        for ring in (False, True):
+            kw = dict(ring_k=rk, ring_v=rv, ring_lens=ring_lens, max_ring_len=70, ring_stride_token=h * d) if ring else {}
+            out = E.decode(store.consts, store.pool, store.workspace, q, store.block_table[None], lens, n, num_splits=splits, **kw)
+            ks, vs = ((torch.cat((a, b.double().transpose(0, 1)), 1) if ring else a) for a, b in ((k64, rk), (v64, rv)))
+            assert _rel(out, _attend64(q, ks, vs, qh // h)) <= 1e-3, (splits, ring)
+    assert store.workspace.status() == 0

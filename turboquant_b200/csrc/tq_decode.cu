@@ -98,6 +98,32 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
         const int i = threadIdx.x * 128;
         if (i < nv * D * es) asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const char*>(q) + v0 * D * es + i));
     }
+    // Where this thread's column goes among the fragments: the same for every vector but for the vector's own offset, whose
+    // divisions are done here, in front of the wait, for the first group.
+    const bool split = G > 4 || mse_bits == 3;   // separate rotated / sketched fragment sets
+    const int tig = col / (D / 4), rem = col % (D / 4);
+    int r = (rem >> 4) * 8 + (rem & 7), half = (rem >> 3) & 1;
+    int sh = which ? sign_pos(sign_bit(rem >> 4, rem & 7)) : 2 * code_pos(rem & 7);
+    if (mse_bits == 3 && which == 0) {
+        // nibble codes: registers pair adjacent dims, k-step = 4 dims, true centroid values (no scaling)
+        r = rem >> 1;
+        half = rem & 1;
+        sh = 0;
+    }
+    struct Place {
+        float* header;
+        __half* entry;
+    };
+    auto place = [&](int64_t vec64) -> Place {   // fragments of 2^31 vectors do not fit any memory
+        const uint32_t vec = (uint32_t)vec64, seq = vec / (uint32_t)Qh, qh = vec - seq * (uint32_t)Qh;
+        const uint32_t kvh = qh / (uint32_t)G, g = qh - kvh * (uint32_t)G;
+        uint32_t* base = frag + (int64_t)(seq * (uint32_t)(Qh / G) + kvh) * qf_words(D, split ? 8 : 4);   // (sequence, kv head)
+        const int gid = split ? g : g + 4 * which, set = split ? which : 0;
+        return {reinterpret_cast<float*>(base) + which * 8 + g,
+                reinterpret_cast<__half*>(base + QF_HDR + ((set * (D / 8) + r) * 32 + gid * 4 + tig)) + half};
+    };
+    Place at = {nullptr, nullptr};
+    if (frag != nullptr && threadIdx.x < VPC * 32) at = place(v0 + (threadIdx.x >> 5));
     // Two passes over the same instructions.  The first is a rehearsal that runs while this grid would
     // otherwise sit waiting for the kernel ahead of it: it computes on whatever the query buffer holds
     // and stores nothing outside shared memory, but it pulls the code of the second pass - which is on
@@ -164,29 +190,12 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
         if (v < nv) {
             if (live) out[((v0 + v) * 2 + which) * D + col] = t;
             if (frag != nullptr) {
-                const int64_t vec = v0 + v;
-                const int qh = (int)(vec % Qh), g = qh % G;
-                const int64_t pair = (vec / Qh) * (Qh / G) + qh / G;   // (sequence, kv head)
-                const bool split = G > 4 || mse_bits == 3;   // separate rotated / sketched fragment sets
-                uint32_t* base = frag + pair * qf_words(D, split ? 8 : 4);
+                if (gi > 0) at = place(v0 + v);
                 const float bound = sqrtf(qn2[v]) * (which ? 2.f * sqrtf((float)D) : 1.f);
                 int e = 0;
                 if (bound > 0.f && bound < 3.0e38f) e = max(-100, min(100, 14 - ilogbf(bound)));
-                if (live && chunk == 0 && lane == 0) reinterpret_cast<float*>(base)[which * 8 + g] = (float)e;
-                const int tig = col / (D / 4), rem = col % (D / 4);
-                int wi = rem >> 4, half = (rem >> 3) & 1, jf = rem & 7;
-                int r = wi * 8 + jf;
-                int sh = which ? sign_pos(sign_bit(wi, jf)) : 2 * code_pos(jf);
-                if (mse_bits == 3 && which == 0) {
-                    // nibble codes: registers pair adjacent dims, k-step = 4 dims, true centroid values (no scaling)
-                    r = rem >> 1;
-                    half = rem & 1;
-                    sh = 0;
-                }
-                const int gid = split ? g : g + 4 * which;
-                const int set = split ? which : 0;
-                __half* dst = reinterpret_cast<__half*>(base + QF_HDR + ((set * (D / 8) + r) * 32 + gid * 4 + tig));
-                if (live) dst[half] = __float2half_rn(t * __int_as_float((127 + e - sh) << 23));
+                if (live && chunk == 0 && lane == 0) *at.header = (float)e;
+                if (live) *at.entry = __float2half_rn(t * __int_as_float((127 + e - sh) << 23));
             }
         }
     }
@@ -535,7 +544,7 @@ __global__ void __launch_bounds__(DEC_THREADS) tq_decode_kernel(const DecodePara
         }
         __syncthreads();
         write_partial_regs<D, GP>(p, b, h, x, acc, m_run, l_run);
-        ticket_and_merge<D, GP>(p, b, h, wsm);
+        ticket_and_merge<D, GP, DEC_THREADS>(p, b, h, wsm, nullptr);
         return;
     }
 
@@ -543,7 +552,7 @@ __global__ void __launch_bounds__(DEC_THREADS) tq_decode_kernel(const DecodePara
     __syncthreads();
     // m_run, l_run are adjacent: [2*GP]; the stage region (sized for it by the launcher) holds the ring rows
     ring_part<D, GP>(p, b, h, x, qr, sp, pp, m_run, stages, stages + RING_TOK * D * 4);
-    ticket_and_merge<D, GP>(p, b, h, wsm);
+    ticket_and_merge<D, GP, DEC_THREADS>(p, b, h, wsm, nullptr);
 }
 
 // Unscaled logits of up to 8 query vectors per CTA against one 64-token tile.
@@ -828,7 +837,6 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     p.num_splits = splits;
     p.ring_splits = rsplits;
     p.ring_tok = ring_tok;
-    p.land_bytes = 0;
     p.host_io = early_inputs;
     p.pool_late = tq_last_launch(st) == TQ_LAUNCH_PREP_BEHIND_STORE ? 1 : 0;
 

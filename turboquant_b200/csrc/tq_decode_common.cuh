@@ -40,7 +40,6 @@ struct DecodeParams {
     int32_t* status;
     int num_splits, ring_splits;
     int ring_tok;          // ring tokens per ring CTA, a multiple of RING_TOK
-    uint32_t land_bytes;   // tensor-core kernel: shared memory in front of its barriers, reusable by the merge
     int host_io;           // the query is read from host memory
     int pool_late;         // a store ahead of the query preparation may still be writing records: wait before the first one
 };
@@ -176,24 +175,35 @@ __device__ __forceinline__ void write_partial_regs(const DecodeParams& p, int b,
         for (int i = 0; i < DPT; ++i) mine[2 * GP + g * D + tid * DPT + i] = acc[g][i];
 }
 
+// How the threads of the last CTA share the merge: a unit is four channels of one head over one of CHUNKS ranges of slots,
+// a thread takes UNITS of them with BATCH loads of each in flight.  A CTA pulls about 64 bytes a cycle out of L2, and every
+// thread's loads together ask for all of it at once.
+template <int D, int GP, int NT>
+struct MergeShape {
+    static constexpr int ITEMS = GP * (D / 4);
+    static constexpr int CHUNKS = NT == 384 ? 3 : (NT > ITEMS ? NT / ITEMS : 1);
+    static constexpr int UNITS = ITEMS * CHUNKS / NT;
+    static constexpr int BATCH = NT <= 256 ? 8 / (UNITS < 2 ? UNITS : 2) : UNITS >= 4 ? 7 : 13;
+    static constexpr size_t SCRATCH = CHUNKS > 1 ? (size_t)ITEMS * CHUNKS * sizeof(float4) : 0;
+    static_assert(ITEMS * CHUNKS % NT == 0, "every thread takes as many units");
+};
+
 // After a CTA has written its partial: take a ticket; the last CTA of this
 // (sequence, kv head) merges all partials and writes the output.  Nobody waits.
 // Every partial is always fully written with finite numbers, so the merge is
-// branch free: a float4 of one head per thread, slots unrolled.
+// branch free.
 //
-// `land` / `land_bytes`: shared memory the CTA no longer needs.  When all the
-// partials of the pair fit there, the last CTA fetches them with bulk copies
-// (one trip to L2 instead of a chain of dependent loads) and merges out of
-// shared memory; otherwise it reads them from global memory.
-template <int D, int GP>
+// The partials go from L2 straight into registers, their loads asked for before the slots' weights are worked out (whose own
+// loads go first): bound by the 64 bytes a cycle at which one SM reads L2.
+template <int D, int GP, int NT>
 __device__ __forceinline__ void ticket_and_merge(const DecodeParams& p, int b, int h,
-                                                 float* wsm /* [max(nslot,128)*GP + 2*GP] */,
-                                                 uint8_t* land = nullptr, uint32_t land_bytes = 0) {
+                                                 float* wsm /* [nslot * GP + GP] */,
+                                                 float4* scratch /* MergeShape::SCRATCH bytes */) {
+    using M = MergeShape<D, GP, NT>;
     constexpr int PS = GP * (D + 2);
-    const int tid = threadIdx.x, nt = blockDim.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nslot = p.num_splits + p.ring_splits;
     __shared__ int s_last;
-    __shared__ __align__(8) uint64_t s_bar;
     __syncthreads();          // every thread's part of the partial is written ...
     if (tid == 0) {
         // ... and, release being cumulative, visible device-wide before the ticket; the acquire half orders
@@ -206,128 +216,102 @@ __device__ __forceinline__ void ticket_and_merge(const DecodeParams& p, int b, i
     if (!s_last) return;
 
     const float* base = p.partials + (int64_t)(b * p.H + h) * nslot * PS;
-    const uint32_t total = (uint32_t)nslot * PS * 4u;
-    const bool staged = land != nullptr && total <= land_bytes && total < (1u << 20);
-    if (staged) {
-        if (tid == 0) {
-            tq_mbar_init(&s_bar, 1);
-            tq_mbar_fence_init();
-            asm volatile("fence.proxy.async;" ::: "memory");   // other CTAs' generic writes -> this bulk read
-            tq_mbar_expect_tx(&s_bar, total);
-            for (uint32_t off = 0; off < total; off += 32768u)
-                tq_bulk_g2s(land + off, reinterpret_cast<const uint8_t*>(base) + off, min(32768u, total - off), &s_bar);
-        }
-        __syncthreads();
-        bool ok = tq_mbar_wait_bounded(&s_bar, 0u);
-        if (!__syncthreads_and(ok)) {   // never arrived: report; the kernel must not touch `land` again
-            if (tid == 0) {
-                atomicCAS(p.status, 0, (int)TQ_ERR_TIMEOUT);
-                p.tickets[b * p.H + h] = 0;   // the output of this launch is lost, the workspace stays usable
-            }
-            return;
-        }
-        // Out of shared memory: a thread owns four channels of one head; the head is the same for a whole
-        // warp, so the warp works out the slots' weights once into its own row of `wsm` (padded with
-        // zeros to a multiple of eight) and then takes the slots eight at a time, all loads first.
-        const float* sb = reinterpret_cast<const float*>(land);
-        const int lane = tid & 31;
-        const int items = p.G * (D / 4);
-        const int wstride = (nslot + 7) & ~7;
-        float* ww = wsm + (tid >> 5) * wstride;   // tensor-core kernel: wsm holds one row of max(nslot,128) + 8 floats per warp
-        for (int i0 = (tid >> 5) * 32; i0 < items; i0 += nt) {   // D/4 is a multiple of 32: one head per warp pass
-            const int i = i0 + lane;
-            const int g = i0 / (D / 4), d = (i % (D / 4)) * 4;
-            float mx = -INFINITY;
-            for (int s = lane; s < nslot; s += 32) mx = fmaxf(mx, sb[s * PS + g]);
-            mx = tq_warp_max(mx);
-            float l = 0.f;
-            for (int s = lane; s < wstride; s += 32) {
-                float wm = 0.f;
-                if (s < nslot) {
-                    const float ms = sb[s * PS + g];
-                    wm = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
-                    l = fmaf(wm, sb[s * PS + GP + g], l);
-                }
-                ww[s] = wm;
-            }
-            l = tq_warp_sum(l);
-            __syncwarp();
-            const float4* src = reinterpret_cast<const float4*>(sb + 2 * GP + g * D + d);
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int s = 0; s < nslot; s += 8) {
-                float4 v[8];
-                float w8[8];
+    // maxima and sums of head `warp`: the first 64 slots from registers
+    float ms[2] = {-INFINITY, -INFINITY}, ls[2] = {0.f, 0.f};
+    if (warp < GP) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    v[u] = src[min(s + u, nslot - 1) * (PS / 4)];   // past the end: a valid slot, weight 0
-                    w8[u] = ww[s + u];
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    o.x = fmaf(w8[u], v[u].x, o.x);
-                    o.y = fmaf(w8[u], v[u].y, o.y);
-                    o.z = fmaf(w8[u], v[u].z, o.z);
-                    o.w = fmaf(w8[u], v[u].w, o.w);
-                }
+        for (int u = 0; u < 2; ++u)
+            if (lane + 32 * u < nslot) {
+                ms[u] = __ldcg(base + (int64_t)(lane + 32 * u) * PS + warp);
+                ls[u] = __ldcg(base + (int64_t)(lane + 32 * u) * PS + GP + warp);
             }
-            __syncwarp();   // the row of weights is rewritten by the warp's next pass
-            const float inv = l > 0.f ? 1.f / l : 0.f;
-            const int64_t dst = ((int64_t)b * p.Qh + h * p.G + g) * D + d;
-            tq_store4_any(p.out, dst, o.x * inv, o.y * inv, o.z * inv, o.w * inv, p.q_dtype);
-        }
-        if (tid == 0) p.tickets[b * p.H + h] = 0;  // ready for the next launch
-        return;
     }
-
-    float* wL = wsm;             // [GP] global sum
-    float* w = wsm + 2 * GP;     // [nslot][GP] weight of each partial
-    const int warp = tid >> 5, lane = tid & 31;
-    for (int g = warp; g < GP; g += nt / 32) {
-        float mx = -INFINITY;
-        for (int s = lane; s < nslot; s += 32) mx = fmaxf(mx, __ldcg(base + (int64_t)s * PS + g));
+    float4 v[M::UNITS][M::BATCH], o[M::UNITS];
+    int s0[M::UNITS], s1[M::UNITS];
+    auto fetch = [&](int at) {   // slots [at, at + BATCH) of every unit's range
+#pragma unroll
+        for (int k = 0; k < M::UNITS; ++k) {
+            const float4* src = reinterpret_cast<const float4*>(base + 2 * GP) + (tid + k * NT) % M::ITEMS;   // PS*4 and 8*GP are multiples of 16
+#pragma unroll
+            for (int u = 0; u < M::BATCH; ++u)
+                v[k][u] = s0[k] + at + u < s1[k] ? __ldcg(src + (int64_t)(s0[k] + at + u) * (PS / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+#pragma unroll
+    for (int k = 0; k < M::UNITS; ++k) {
+        const int unit = tid + k * NT, item = unit % M::ITEMS, chunk = unit / M::ITEMS;
+        o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        s0[k] = chunk * nslot / M::CHUNKS;
+        s1[k] = item / (D / 4) < p.G ? (chunk + 1) * nslot / M::CHUNKS : s0[k];
+    }
+    fetch(0);
+    float* wL = wsm + nslot * GP;   // [GP] sum over all slots; in front of it [GP][nslot] weights
+    for (int g = warp; g < GP; g += NT / 32) {
+        if (g != warp)   // fewer warps than heads
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool in = lane + 32 * u < nslot;
+                ms[u] = in ? __ldcg(base + (int64_t)(lane + 32 * u) * PS + g) : -INFINITY;
+                ls[u] = in ? __ldcg(base + (int64_t)(lane + 32 * u) * PS + GP + g) : 0.f;
+            }
+        float mx = fmaxf(ms[0], ms[1]);
+        for (int s = lane + 64; s < nslot; s += 32) mx = fmaxf(mx, __ldcg(base + (int64_t)s * PS + g));
         mx = tq_warp_max(mx);
         float sum = 0.f;
         for (int s = lane; s < nslot; s += 32) {
-            const float ms = __ldcg(base + (int64_t)s * PS + g);
-            const float ls = __ldcg(base + (int64_t)s * PS + GP + g);
-            const float ws = (ms == -INFINITY) ? 0.f : __expf(ms - mx);
-            w[s * GP + g] = ws;
-            sum += ws * ls;
+            const float m = s < 32 ? ms[0] : s < 64 ? ms[1] : __ldcg(base + (int64_t)s * PS + g);
+            const float l = s < 32 ? ls[0] : s < 64 ? ls[1] : __ldcg(base + (int64_t)s * PS + GP + g);
+            const float w = m == -INFINITY ? 0.f : __expf(m - mx);
+            wsm[g * nslot + s] = w;
+            sum = fmaf(w, l, sum);
         }
         sum = tq_warp_sum(sum);
         if (lane == 0) wL[g] = sum;
     }
     __syncthreads();
-    for (int i = tid; i < p.G * (D / 4); i += nt) {
-        const int g = i / (D / 4), d = (i % (D / 4)) * 4;
-        const float4* src = reinterpret_cast<const float4*>(base + 2 * GP + g * D + d);   // PS*4 and (2GP+gD+d)*4 are multiples of 16
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-        int s = 0;
-        for (; s + 8 <= nslot; s += 8) {
-            float4 v[8];
+    const int longest = (nslot + M::CHUNKS - 1) / M::CHUNKS;
+    for (int at = 0; at < longest; at += M::BATCH) {
+        if (at > 0) fetch(at);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = __ldcg(src + (int64_t)(s + u) * (PS / 4));
+        for (int k = 0; k < M::UNITS; ++k) {
+            const float* w = wsm + (tid + k * NT) % M::ITEMS / (D / 4) * nslot + s0[k] + at;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const float ws = w[(s + u) * GP + g];
-                o.x = fmaf(ws, v[u].x, o.x);
-                o.y = fmaf(ws, v[u].y, o.y);
-                o.z = fmaf(ws, v[u].z, o.z);
-                o.w = fmaf(ws, v[u].w, o.w);
+            for (int u = 0; u < M::BATCH; ++u) {
+                const float ws = s0[k] + at + u < s1[k] ? w[u] : 0.f;
+                o[k].x = fmaf(ws, v[k][u].x, o[k].x);
+                o[k].y = fmaf(ws, v[k][u].y, o[k].y);
+                o[k].z = fmaf(ws, v[k][u].z, o[k].z);
+                o[k].w = fmaf(ws, v[k][u].w, o[k].w);
             }
         }
-        for (; s < nslot; ++s) {
-            const float4 v = __ldcg(src + (int64_t)s * (PS / 4));
-            const float ws = w[s * GP + g];
-            o.x = fmaf(ws, v.x, o.x);
-            o.y = fmaf(ws, v.y, o.y);
-            o.z = fmaf(ws, v.z, o.z);
-            o.w = fmaf(ws, v.w, o.w);
+    }
+    if (M::CHUNKS > 1)
+#pragma unroll
+        for (int k = 0; k < M::UNITS; ++k) scratch[tid + k * NT] = o[k];
+    if (M::CHUNKS > 1) __syncthreads();
+    for (int i = tid; i < p.G * (D / 4); i += NT) {
+        const int g = i / (D / 4), d = (i % (D / 4)) * 4;
+        float4 r;
+        if (M::CHUNKS > 1) {
+            r = scratch[i];
+#pragma unroll
+            for (int c = 1; c < M::CHUNKS; ++c) {
+                const float4 t = scratch[c * M::ITEMS + i];
+                r.x += t.x;
+                r.y += t.y;
+                r.z += t.z;
+                r.w += t.w;
+            }
+        } else {
+            r = o[0];
+#pragma unroll
+            for (int k = 1; k < M::UNITS; ++k)
+                if (i == tid + k * NT) r = o[k];
         }
         const float l = wL[g];
         const float inv = l > 0.f ? 1.f / l : 0.f;
         const int64_t dst = ((int64_t)b * p.Qh + h * p.G + g) * D + d;
-        tq_store4_any(p.out, dst, o.x * inv, o.y * inv, o.z * inv, o.w * inv, p.q_dtype);
+        tq_store4_any(p.out, dst, r.x * inv, r.y * inv, r.z * inv, r.w * inv, p.q_dtype);
     }
     if (tid == 0) p.tickets[b * p.H + h] = 0;  // ready for the next launch
 }

@@ -35,18 +35,14 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 // Warps per CTA.  A launch that fits one wave runs 12-warp CTAs, one per SM (all of an SM's warps
 // share one set of query fragments and one merge).  A launch of several waves runs 8-warp CTAs, two
 // per SM, so that the set-up and the merge of one CTA overlap the main loop of the other.
-// At head_dim 128 a single sequence with a ring may run 16 warps an SM: 128 registers are enough there, the CTAs of the ring
-// (CUDA-core work, up to 64 tokens each) finish sooner with more threads, and they are what such a launch waits for.  Of the
-// launch's time at 8 kv heads, sixteen warps / twelve: 0.93 (one set of fragments) and 0.97 (two sets) from 64 ring tokens on
-// and up to 8000 of history, which is 32 records a CTA; 0.98 at 48 records; 0.98 to 1.03 at 63; 0.95 to 1.02 with 40 ring
-// tokens; 1.00 to 1.06 with 1 or 16, 1.00 to 1.13 without a ring (two sets do not fit the registers and are read from shared
-// memory); the ring's CTAs take 32 tokens at a time.  With the query in host memory they also fetch it from there, the more at
-// a time the more threads: a step of decode_step_host 18.2 us for 20.4 at 4000 tokens, whatever the ring holds, and 23.4 for
-// 24.1 at 30000.  At head_dim 256 sixteen warps cost registers.
+// At head_dim 128 a single sequence whose query lies in host memory runs 16 warps an SM: 128 registers are enough there, and
+// the ring's CTAs fetch the query from the host, the more at a time the more threads.  Steps of decode_step_host, sixteen warps /
+// twelve: 0.94 to 0.99 (13.0 us for 13.7 at 4000 tokens of 8 heads, 17.3 for 17.6 at 16000; two sets of fragments 16.6 for 17.3).
+// With everything on the device they are no faster: 1.00 to 1.01 with the ring's tokens a warp each, 1.06 with 3-bit codes.  At
+// head_dim 256 sixteen warps cost registers.
 constexpr int NW_WAVE = 12;
 constexpr int NW_SINGLE = 16;
 constexpr int NW_MULTI = 8;
-constexpr int SINGLE_RING = 33, SINGLE_RECORDS = 48;   // at least so many ring tokens, at most so many records a CTA
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
 
 
@@ -88,6 +84,132 @@ __device__ __forceinline__ uint32_t hmul2_sat(uint32_t a, uint32_t b) {
     return *reinterpret_cast<const uint32_t*>(&r);
 }
 
+// Exact attention over this CTA's slice of the ring, up to 64 tokens, fp32 like the reference's matmul path (score.py:154-170).
+// A lane owns eight channels (16 bytes of a 16-bit row), so a token takes a whole warp at head_dim 256 and half a warp at 128;
+// every warp asks for all its key rows, and its value rows where registers allow, in one go and keeps a softmax of its own: one
+// trip to memory, one barrier (for the query) and no shared memory in between.  Leaves the warp's maxima, sums and weighted
+// values where the warps of a history CTA leave theirs.  (With the rows staged in shared memory 32 at a time, a barrier between
+// scores, softmax and values, these CTAs took 5.9 us at head_dim 128 and 12.4 us at 256 for 64 tokens, and were what a launch
+// for one sequence waited for.)
+template <int D, int GP, int NW, int DT>
+__device__ __forceinline__ void ring_warps(const DecodeParams& p, int b, int h, int first, int nr, const float* qf /* [GP][D] */,
+                                           float* osm, float* ml) {
+    static_assert(GP % 4 == 0, "heads are taken in fours");
+    constexpr int TPW = 256 / D;                              // tokens a warp holds side by side
+    constexpr int LANES = 32 / TPW;
+    constexpr int TB = (64 + NW * TPW - 1) / (NW * TPW);      // such rows of tokens
+    constexpr int CH = DT == TQ_F32 ? 2 : 1;                  // 16-byte chunks a lane reads of a row
+    constexpr bool PRE = TB * CH <= 6;                        // value rows on their way under the scores; else they take the keys' registers
+    constexpr int DP = D + 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane % LANES, part = lane / LANES;
+    const int64_t eb = DT == TQ_F32 ? 4 : 2;
+    const int64_t at0 = ((int64_t)b * p.ring_stride_seq + (int64_t)first * p.ring_stride_token + (int64_t)h * D) * eb + l * 16 * CH;
+    uint4 kr[TB][CH], later[PRE ? TB : 1][CH];
+    auto fetch = [&](uint4 (*r)[CH], const void* base) {
+#pragma unroll
+        for (int t = 0; t < TB; ++t) {
+            const int tok = (warp + NW * t) * TPW + part;
+#pragma unroll
+            for (int c = 0; c < CH; ++c)
+                r[t][c] = tok < nr ? *reinterpret_cast<const uint4*>((const char*)base + at0 + tok * p.ring_stride_token * eb + 16 * c)
+                                   : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    auto widen = [&](const uint4 (&r)[CH], float (&x)[8]) {
+        const uint32_t w[8] = {r[0].x, r[0].y, r[0].z, r[0].w, r[CH - 1].x, r[CH - 1].y, r[CH - 1].z, r[CH - 1].w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (DT == TQ_F32) x[i] = __uint_as_float(w[i]);
+            else if (DT == TQ_BF16) x[i] = __uint_as_float((i & 1) ? w[i >> 1] & 0xffff0000u : w[i >> 1] << 16);
+            else x[i] = __half2float(__ushort_as_half((unsigned short)((i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu)));
+        }
+    };
+    fetch(kr, p.ring_k);
+    if (PRE) fetch(later, p.ring_v);
+    __syncthreads();   // the query is in shared memory
+    const float sm_scale = p.scale * 1.4426950408889634f;   // softmax in base 2
+#pragma unroll 1
+    for (int g0 = 0; g0 < GP; g0 += 4) {   // four heads at a time
+        float q[4][8], sc[TB];
+        if (!PRE && g0 > 0) fetch(kr, p.ring_k);
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const float4 x = *reinterpret_cast<const float4*>(qf + (g0 + g) * D + 8 * l + 4 * c);
+                q[g][4 * c] = x.x; q[g][4 * c + 1] = x.y; q[g][4 * c + 2] = x.z; q[g][4 * c + 3] = x.w;
+            }
+        float m = -INFINITY;
+#pragma unroll
+        for (int t = 0; t < TB; ++t) {
+            float x[8], a[4] = {0.f, 0.f, 0.f, 0.f};
+            widen(kr[t], x);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int g = 0; g < 4; ++g) a[g] = fmaf(q[g][i], x[i], a[g]);
+            // sums over the token's lanes: lane l ends up with head l % 4
+            const bool hi = lane & 2, odd = lane & 1;
+            const float b0 = (hi ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[2], 2);
+            const float b1 = (hi ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, hi ? a[1] : a[3], 2);
+            float s = (odd ? b1 : b0) + __shfl_xor_sync(0xffffffffu, odd ? b0 : b1, 1);
+#pragma unroll
+            for (int o = 4; o < LANES; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            sc[t] = (warp + NW * t) * TPW + part < nr ? s * sm_scale : -INFINITY;
+            m = fmaxf(m, sc[t]);
+        }
+        if (TPW == 2) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        float sum = 0.f;
+#pragma unroll
+        for (int t = 0; t < TB; ++t) {
+            sc[t] = sc[t] == -INFINITY ? 0.f : ex2_fast(sc[t] - m);
+            sum += sc[t];
+        }
+        if (TPW == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        if (lane < 4) {
+            ml[(warp * 2 + 0) * GP + g0 + lane] = m;
+            ml[(warp * 2 + 1) * GP + g0 + lane] = sum;
+        }
+        if (!PRE) fetch(kr, p.ring_v);
+        float acc[4][8];
+#pragma unroll
+        for (int g = 0; g < 4; ++g)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
+#pragma unroll
+        for (int t = 0; t < TB; ++t) {
+            float x[8];
+            widen(PRE ? later[PRE ? t : 0] : kr[t], x);
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const float pg = __shfl_sync(0xffffffffu, sc[t], g, LANES);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[g][i] = fmaf(pg, x[i], acc[g][i]);
+            }
+        }
+        float* dst = osm + (warp * GP + g0) * DP + 8 * l;
+        if (TPW == 2) {   // the two halves add up: each keeps two heads
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                float r[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    r[i] = (part ? acc[2 + g][i] : acc[g][i]) + __shfl_xor_sync(0xffffffffu, part ? acc[g][i] : acc[2 + g][i], 16);
+                float4* d4 = reinterpret_cast<float4*>(dst + (2 * part + g) * DP);
+                d4[0] = make_float4(r[0], r[1], r[2], r[3]);
+                d4[1] = make_float4(r[4], r[5], r[6], r[7]);
+            }
+        } else {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                float4* d4 = reinterpret_cast<float4*>(dst + g * DP);
+                d4[0] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+                d4[1] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
+            }
+        }
+    }
+}
+
 // MSE_BITS == 2: bit-plane scores as described above.  MSE_BITS == 3 (codes in nibbles, 8 centroids): the
 // nibbles are byte-table selectors - two PRMTs look up the low and high bytes of four fp16 centroids, two more
 // interleave them into two A registers - so the A operand holds true centroid values, one plane, and the
@@ -97,6 +219,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     static_assert(MSE_BITS == 2 || SPLITB, "3-bit codes use separate rotated / sketched fragment sets");
     constexpr int NT = NW * 32;
     constexpr int GP = SPLITB ? 8 : 4;
+    static_assert(MergeShape<D, GP, NT>::SCRATCH <= (size_t)NW * NSTW * 1600, "the merge's sums fit the stages");
     constexpr int KS = D / 16;    // score k-steps
     constexpr int NWK = D / 64;   // 32-bit words of 2-bit codes per thread per token; twice the sign words
     constexpr int NMB = D / 16;   // value M-blocks
@@ -105,14 +228,16 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     const int BB = L.block_bytes;
 
     extern __shared__ __align__(128) uint8_t smem[];
-    // [0, land_bytes): stages, ml, bt_s (+ padding) - all dead once the CTA's partial is written, so the
-    // merge may land every partial of the pair there
-    uint8_t* stages = smem;                                              // [NW warps][NSTW][BB]; reused after the loop
+    uint8_t* stages = smem;                                              // [NW warps][NSTW][BB]; reused after the loop, by the merge too
     float* ml = reinterpret_cast<float*>(smem + NW * NSTW * BB);         // [NW warps][2][GP]
     int* bt_s = reinterpret_cast<int*>(ml + 2 * NW * GP);                // [BT_MAX] physical blocks of this CTA
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + p.land_bytes);   // [NW][NSTW] + 1 for the query fragments
+    uint64_t* bars = reinterpret_cast<uint64_t*>(bt_s + BT_MAX);         // [NW][NSTW] + 1 for the query fragments
     uint32_t* qf_s = reinterpret_cast<uint32_t*>(bars + NW * NSTW + 2);  // query fragments of this (sequence, kv head)
     float* wsm = reinterpret_cast<float*>(qf_s + qf_words(D, SPLITB ? 8 : 4));   // merge scratch
+    // [NW warps][GP][D + 4] weighted values of each warp: the padding spreads the four lanes that share a channel quad (one
+    // per pair of heads) over different banks; a thread stores the quad of a head with one 16-byte store
+    constexpr int DP = D + 4;
+    float* osm = reinterpret_cast<float*>(stages);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int gid = lane >> 2, tig = lane & 3;
@@ -126,17 +251,23 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     if (!p.pool_late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (x >= p.num_splits) {
-        // exact ring tokens: CUDA-core fp32 path shared with the generic kernel.  The ring and its
-        // length may have been written by the query-prep grid this launch overlaps with.
+        // ------------------------------ exact ring tokens ------------------------------
+        // The ring and its length may have been written by the query-prep grid this launch overlaps with.
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (p.pool_late) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        float* scratch = reinterpret_cast<float*>(stages);
-        uint8_t* kst = reinterpret_cast<uint8_t*>(scratch + D * GP + 2 * GP * RING_TOK);   // 16-byte aligned
-        ring_part<D, GP>(p, b, h, x, scratch, scratch + D * GP, scratch + D * GP + GP * RING_TOK, ml, kst,
-                         kst + RING_TOK * D * 4);
-        ticket_and_merge<D, GP>(p, b, h, wsm, smem, p.land_bytes);
-        return;
-    }
+        int len = p.ring_lens ? p.ring_lens[b] : p.max_ring_len;
+        if (len > p.max_ring_len) {   // more than the host promised: the ring CTAs only cover max_ring_len tokens
+            if (tid == 0) atomicCAS(p.status, 0, (int)TQ_ERR_RANGE);
+            len = p.max_ring_len;
+        }
+        const int first = (x - p.num_splits) * p.ring_tok, nr = max(0, min(p.ring_tok, len - first));
+        float* qf = reinterpret_cast<float*>(qf_s);   // the query as it is, in the place of its fragments
+        for (int i = tid; i < GP * D; i += NT)
+            qf[i] = i / D < p.G ? tq_load_any(p.query, ((int64_t)b * p.Qh + h * p.G) * D + i, p.q_dtype) : 0.f;
+        if (p.ring_dtype == TQ_BF16) ring_warps<D, GP, NW, TQ_BF16>(p, b, h, first, nr, qf, osm, ml);
+        else if (p.ring_dtype == TQ_F16) ring_warps<D, GP, NW, TQ_F16>(p, b, h, first, nr, qf, osm, ml);
+        else ring_warps<D, GP, NW, TQ_F32>(p, b, h, first, nr, qf, osm, ml);
+    } else {
 
     // ------------------------------ this CTA's share of the history ------------------------------
     constexpr uint32_t QF_BYTES = qf_words(D, SPLITB ? 8 : 4) * 4u;
@@ -638,10 +769,6 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         zrow[grp][1] = __shfl_sync(0xffffffffu, zacc[1], grp * 4 + tig);
     }
     __syncthreads();   // every warp is done with its stages: reuse them
-    // [NW warps][GP][D + 4]: the padding spreads the four lanes that share a channel quad (one per
-    // pair of heads) over different banks; a thread stores the quad of a head with one 16-byte store
-    constexpr int DP = D + 4;
-    float* osm = reinterpret_cast<float*>(stages);
     if (col_ok) {
 #pragma unroll
         for (int grp = 0; grp < NG; ++grp) {
@@ -672,6 +799,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
             }
         }
     }
+    }   // history
     __syncthreads();
     // Every thread owns four channels of one head: it weighs the warps' partials itself (NW exp2f)
     // instead of waiting for a serial pass over the heads.
@@ -715,27 +843,15 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         }
     }
     __syncthreads();   // wsm is reused by the merge
-    ticket_and_merge<D, GP>(p, b, h, wsm, smem, p.land_bytes);
+    ticket_and_merge<D, GP, NT>(p, b, h, wsm, reinterpret_cast<float4*>(stages));
 }
 
-// Bytes in front of the barriers: stages, ml, bt_s, grown (one CTA per SM only) until the merge
-// can land all `nslot` partials of a (sequence, kv head) there.
-template <int D, bool SPLITB, int NW>
-size_t mma_land_bytes(int block_bytes, int nslot) {
-    constexpr int GP = SPLITB ? 8 : 4;
-    size_t s = (size_t)NW * NSTW * block_bytes + sizeof(float) * (2 * NW * GP) + sizeof(int) * BT_MAX;
-    const size_t want = (size_t)nslot * GP * (D + 2) * sizeof(float);
-    if (NW != NW_MULTI && want > s && want <= 200 * 1024) s = want;
-    return (s + 127) / 128 * 128;
-}
 template <int D, bool SPLITB, int NW>
 size_t mma_smem_bytes(int block_bytes, int nslot) {
     constexpr int GP = SPLITB ? 8 : 4;
-    size_t s = mma_land_bytes<D, SPLITB, NW>(block_bytes, nslot);
+    size_t s = (size_t)NW * NSTW * block_bytes + sizeof(float) * (2 * NW * GP) + sizeof(int) * BT_MAX;
     s += sizeof(uint64_t) * (NW * NSTW + 2) + sizeof(uint32_t) * qf_words(D, SPLITB ? 8 : 4);
-    // merge scratch: one row of slot weights per warp of the merging CTA
-    s += sizeof(float) * ((size_t)((nslot > 128 ? nslot : 128) + 8) * NW + 2 * GP);
-    return s;
+    return s + sizeof(float) * (size_t)GP * (nslot + 1);   // weights and sums of the merge
 }
 
 template <int D, int MSE_BITS, int VAL_BITS, bool SPLITB, int NW, int R = 1>
@@ -745,7 +861,6 @@ int launch_mma_nw(const DecodeParams& p_in, int batch, cudaStream_t st) {
     const TqLayout L = tq_make_layout(D, MSE_BITS + 1, VAL_BITS);
     const int nslot = p.num_splits + p.ring_splits;
     const size_t smem = mma_smem_bytes<D, SPLITB, NW>(L.block_bytes, nslot);
-    p.land_bytes = (uint32_t)mma_land_bytes<D, SPLITB, NW>(L.block_bytes, nslot);
     auto kern = tq_decode_mma_kernel<D, MSE_BITS, VAL_BITS, SPLITB, NW, R>;
     static TqSmemOptIn opt_in;
     if (tq_opt_in_smem(kern, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;
@@ -789,7 +904,7 @@ int launch_mma(const DecodeParams& p, int batch, cudaStream_t st, int* handled) 
         return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_MULTI>(p, batch, st);
     }
     if constexpr (D == 128)
-        if (batch == 1 && (p.host_io || (p.max_ring_len >= SINGLE_RING && records <= SINGLE_RECORDS)) && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
+        if (batch == 1 && p.host_io && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
             return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_SINGLE>(p, batch, st);
     if (fits_wave) return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_WAVE>(p, batch, st);
     *handled = 0;

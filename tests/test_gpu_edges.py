@@ -77,3 +77,27 @@ def test_merge_of_any_number_of_partial_results(d, h, qh, kb, vb, dev):
             ks, vs = ((torch.cat((a, b.double().transpose(0, 1)), 1) if ring else a) for a, b in ((k64, rk), (v64, rv)))
             assert _rel(out, _attend64(q, ks, vs, qh // h)) <= 1e-3, (splits, ring)
     assert store.workspace.status() == 0
+
+
+@pytest.mark.parametrize("d,kb,vb", [(128, 3, 2), (128, 4, 4), (256, 3, 4), (256, 4, 2)])
+@pytest.mark.parametrize("n,buf", [(1, 1), (63, 0), (65, 5), (129, 64), (1000, 129)])
+def test_cache_object_for_every_group_of_queries(d, kb, vb, n, buf, dev):
+    """Sums of up to 1129 fp32 products: (log2(1129) + 8) 2^-24 = 1.1e-6 of the sum of magnitudes, which for random signs is
+    some sqrt(1129) times the sum."""
+    from turboquant_b200 import TurboQuantKVCache, _engine as E
+    g = torch.Generator(device=dev).manual_seed(n + d)
+    cache = TurboQuantKVCache(d, kb, vb, buffer_size=max(buf, 1), device=dev, dtype=torch.float16)
+    k, v = (torch.randn(1, 2, n + buf, d, generator=g, device=dev, dtype=torch.float16) for _ in range(2))
+    if buf:
+        cache.prefill(k, v)
+    else:
+        cache._append_compressed(k, v)
+    k64, v64 = _history64(cache.consts, E.pool_to_planes(cache.consts, cache._pool, cache._bt, n), n, vb)
+    k64, v64 = (torch.cat((a, b[0, :, n:].double()), 1) for a, b in ((k64, k), (v64, v)))
+    for n_q in (1, 2, 3, 4, 5, 8, 9):
+        q = torch.randn(1, 2, n_q, d, generator=g, device=dev, dtype=torch.float16)
+        logits = cache.attention_scores(q)
+        want = torch.einsum("hqd,hnd->hqn", q[0].double(), k64) / math.sqrt(d)
+        assert logits.dtype == torch.float32 and _rel(logits[0], want) <= 2e-6, n_q
+        w = torch.softmax(logits, -1)
+        assert _rel(cache.attend(w)[0], torch.einsum("hqn,hnd->hqd", w[0].double(), v64)) <= 4e-6, n_q

@@ -123,6 +123,51 @@ __device__ __forceinline__ void half_row_scores(const uint32_t* cw, const uint32
 #pragma unroll
     for (int g = 0; g < GP; ++g) out[g] = norm * am[g] + rn * aq[g];
 }
+// Half a key row, its code and sign words in registers (which are used up), against GP prepared queries in shared memory:
+// qs[g][0] rotated, qs[g][1] sketched.  am: sums over centroids, aq: over signs.
+template <int D, int MSE_BITS>
+struct HalfRow {
+    static constexpr int WIDTH = MSE_BITS == 2 ? 2 : 4, DIMS_PER_CW = 32 / WIDTH, CW_PER_SW = 32 / DIMS_PER_CW;
+    static constexpr int NSW = D / 64, NCW = NSW * CW_PER_SW;   // sign and code words
+};
+template <int D, int MSE_BITS, int GP>
+__device__ __forceinline__ void half_row_dots(uint32_t (&cw)[HalfRow<D, MSE_BITS>::NCW], uint32_t (&sw)[HalfRow<D, MSE_BITS>::NSW],
+                                              const float (&qs)[GP][2][D], const float* cent, int half, float (&am)[GP], float (&aq)[GP]) {
+    using R = HalfRow<D, MSE_BITS>;
+#pragma unroll
+    for (int g = 0; g < GP; ++g) am[g] = aq[g] = 0.f;
+    int j = half * (D / 2);
+#pragma unroll 1
+    for (int s = 0; s < R::NSW; ++s) {
+        uint32_t sg = sw[0];
+#pragma unroll
+        for (int c = 0; c < R::CW_PER_SW; ++c) {
+            uint32_t w = cw[c];
+#pragma unroll
+            for (int i = 0; i < R::DIMS_PER_CW; i += 4, j += 4) {
+                float cv[4], sv[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    cv[k] = cent[w & ((1u << R::WIDTH) - 1u)];
+                    w >>= R::WIDTH;
+                    sv[k] = (sg & 1u) ? 1.f : -1.f;
+                    sg >>= 1;
+                }
+#pragma unroll
+                for (int g = 0; g < GP; ++g) {
+                    const float4 a = *reinterpret_cast<const float4*>(&qs[g][0][j]), b = *reinterpret_cast<const float4*>(&qs[g][1][j]);
+                    am[g] = fmaf(a.x, cv[0], am[g]); am[g] = fmaf(a.y, cv[1], am[g]); am[g] = fmaf(a.z, cv[2], am[g]); am[g] = fmaf(a.w, cv[3], am[g]);
+                    aq[g] = fmaf(b.x, sv[0], aq[g]); aq[g] = fmaf(b.y, sv[1], aq[g]); aq[g] = fmaf(b.z, sv[2], aq[g]); aq[g] = fmaf(b.w, sv[3], aq[g]);
+                }
+            }
+        }
+        // the next words move down: the loop stays rolled and the words in registers
+#pragma unroll
+        for (int k = 0; k + R::CW_PER_SW < R::NCW; ++k) cw[k] = cw[k + R::CW_PER_SW];
+#pragma unroll
+        for (int k = 0; k + 1 < R::NSW; ++k) sw[k] = sw[k + 1];
+    }
+}
 // The same for token tl of a block record.
 template <int D, int MSE_BITS, int GP>
 __device__ __forceinline__ void token_half_scores(const uint8_t* rec, const TqLayout& L, int tl, int half,

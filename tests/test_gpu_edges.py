@@ -101,3 +101,43 @@ def test_cache_object_for_every_group_of_queries(d, kb, vb, n, buf, dev):
         assert logits.dtype == torch.float32 and _rel(logits[0], want) <= 2e-6, n_q
         w = torch.softmax(logits, -1)
         assert _rel(cache.attend(w)[0], torch.einsum("hqn,hnd->hqd", w[0].double(), v64)) <= 4e-6, n_q
+
+
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_key_rows_do_not_depend_on_their_place(bits, dtype, dev):
+    """The rows of one call are the rows of another: ends of row groups, tiles and waves."""
+    from turboquant_b200 import TurboQuantProd
+    z = TurboQuantProd(128, bits, device=dev)
+    n_all = 148 * 128 + 300
+    x = torch.randn(n_all, 128, generator=torch.Generator(device=dev).manual_seed(bits), device=dev).to(dtype)
+    x[5] = 0
+    full = z.quantize(x)
+    back = z.dequantize(full)
+    for lo, n in ((0, 1), (3, 7), (0, 8), (1, 9), (2, 15), (0, 16), (0, 17), (100, 127), (0, 128), (7, 129), (0, 255), (11, 148 * 128), (0, 148 * 128 + 1)):
+        part = z.quantize(x[lo:lo + n])
+        for a, b in zip(part[:4], full[:4]):
+            assert torch.equal(a, b[lo:lo + n]), (lo, n)
+        assert torch.equal(z.dequantize(part), back[lo:lo + n]), (lo, n)
+
+
+@pytest.mark.parametrize("d,bits", [(128, 2), (128, 4), (256, 2), (256, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_value_rows_for_any_number_of_groups(d, bits, dtype, dev):
+    """Codes, scales and zero points of n rows against the same arithmetic in torch, exactly; values back to the rounding of
+    one multiply-add."""
+    from turboquant_b200.kv_cache import dequantize_values, quantize_values
+    g = torch.Generator(device=dev).manual_seed(d + bits)
+    for n in (1, 2, 15, 16, 17, 63, 65, 1000):
+        v = torch.randn(1, n, d, generator=g, device=dev).to(dtype)
+        v[0, 0, :32] = 1.5                       # a group without a range
+        out = quantize_values(v, bits=bits)
+        x = v.view(n, d // 32, 32)
+        lo, hi = x.amin(-1, keepdim=True), x.amax(-1, keepdim=True)
+        scale = ((hi - lo) / torch.full_like(hi, 2 ** bits - 1)).clamp(min=1e-10)   # by a tensor: a number is multiplied by its inverse
+        code = ((x - lo) / scale).round().clamp(0, 2 ** bits - 1).nan_to_num(0).long().view(n, d)   # 0 / 0 where fp16 has no 1e-10
+        assert torch.equal(_unpack(out.data.view(n, -1), bits), code)
+        assert torch.equal(out.scales.view(n, -1), scale[..., 0].half().to(dtype)) and torch.equal(out.zeros.view(n, -1), lo[..., 0].half().to(dtype))
+        s64, z64 = (t.view(n, -1).half().double().repeat_interleave(32, -1) for t in (out.scales, out.zeros))
+        want = code.double() * s64 + z64
+        assert float((dequantize_values(out).view(n, d).double() - want).abs().max()) <= 2.0 ** -22 * float(want.abs().max() + s64.max() * (2 ** bits))

@@ -8,13 +8,15 @@
 //
 // The products run on mma.sync with fp16 limbs: a number scaled away from fp16's subnormals is the sum of two fp16 numbers
 // to 2^-22, and three products of limbs, accumulated in fp32, give the fp32 product to about the rounding of its own sum
-// (three bf16 limbs would need six).  A warp owns 16 rows from load to packed output with its A operand in registers; the
-// constant operands (two limbs of 128 x 128 each) stay in shared memory, so the kernel is bound by the MMA pipe (8 cycles
-// per m16n8k16 and scheduler) and not by fp32 FMAs, which needed 3 x 16384 per row at a fifth of their peak.
+// (three bf16 limbs would need six).  A pair of warps owns 16 rows from load to packed output with its A operand in registers;
+// the constant operands (two limbs of 128 x 128 each) stay in shared memory.  At these sizes - a tile per CTA - a kernel is
+// its chain of phases, so four warps a scheduler cover one another, the loops stay small enough to be fetched, and every
+// kernel starts under the launch ahead of it: its constants arrive while it waits.
 //
-// Measured (B200, 16000 rows of 128, 3-bit keys): quantise 51 us as half of a store into records plus 10 for the
-// conversion to planes -> 22 back to back; dequantise 80 -> 12.6; a whole quantise, score, dequantise pass of keys and
-// values 807 -> 67 to 73.
+// Measured (B200, 16000 rows of 128, fp32, 3-bit keys, 2-bit values, 4 queries, calls back to back; in brackets with a warp per
+// 16 rows, eight query slots whatever was asked for, a thread per group of values and plain launches): quantise 29.6 us
+// (31.7), dequantise 13.2 (14.6), scores 8.2 (12.0), values 6.9 (10.4) and 4.5 (6.2), everything in turn 59.7 (76.0); 480 rows
+// 41.5 (62.9).
 #include "tq_decode_common.cuh"
 
 using namespace tqdec;
@@ -23,98 +25,108 @@ namespace {
 
 // ------------------------------------------------------------------ values
 
-// One thread per group of 32 channels.  Arithmetic of kv_cache.py:64-90 with the rounding of the tensor's dtype after
-// every operation; scale and zero point pass through fp16, the form they are stored in.
+// What every kernel of this file does first: whatever it reads or writes of the caller's belongs to the launch ahead until the
+// wait; only then may the launch behind it begin, so that what it does before its own wait comes after everything ahead of here.
+__device__ __forceinline__ void wait_for_launch_ahead() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Four lanes per group of 32 channels, eight consecutive channels each.  Arithmetic of kv_cache.py:64-90 with the rounding of
+// the tensor's dtype after every operation; scale and zero point pass through fp16, the form they are stored in.
 template <int DT, int VAL_BITS>
 __global__ void __launch_bounds__(256) tq_rows_quantize_values_kernel(const void* __restrict__ v, int64_t n_groups, int groups_per_row, int64_t stride_row,
                                                                       uint8_t* __restrict__ data, void* __restrict__ scales, void* __restrict__ zeros) {
     using E = TqElem<DT>;
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= n_groups) return;
+    wait_for_launch_ahead();
+    const int64_t unit = (int64_t)blockIdx.x * 256 + threadIdx.x, i = unit >> 2;
+    const int part = (int)(unit & 3);
+    const bool live = i < n_groups;   // the four lanes of a group alike
     const int64_t row = i / groups_per_row;
-    const int grp = (int)(i % groups_per_row);
-    const int64_t at = row * stride_row + grp * 32;
-    float x[32];
-    if (DT == TQ_F32) {
-        const float4* src = reinterpret_cast<const float4*>((const float*)v + at);
+    const int64_t at = row * stride_row + (i - row * groups_per_row) * 32 + part * 8;
+    float x[8] = {};
+    if (live) {
+        if (DT == TQ_F32) {
+            const float4* src = reinterpret_cast<const float4*>((const float*)v + at);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float4 q = src[j];
-            x[4 * j] = q.x;
-            x[4 * j + 1] = q.y;
-            x[4 * j + 2] = q.z;
-            x[4 * j + 3] = q.w;
-        }
-    } else {
-        const uint4* src = reinterpret_cast<const uint4*>((const uint16_t*)v + at);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const uint4 q = src[j];
+            for (int j = 0; j < 2; ++j) {
+                const float4 q = src[j];
+                x[4 * j] = q.x;
+                x[4 * j + 1] = q.y;
+                x[4 * j + 2] = q.z;
+                x[4 * j + 3] = q.w;
+            }
+        } else {
+            const uint4 q = *reinterpret_cast<const uint4*>((const uint16_t*)v + at);
             const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if (DT == TQ_BF16) {
-                    x[8 * j + 2 * k] = __uint_as_float(w[k] << 16);
-                    x[8 * j + 2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
+                    x[2 * k] = __uint_as_float(w[k] << 16);
+                    x[2 * k + 1] = __uint_as_float(w[k] & 0xffff0000u);
                 } else {
                     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
-                    x[8 * j + 2 * k] = f.x;
-                    x[8 * j + 2 * k + 1] = f.y;
+                    x[2 * k] = f.x;
+                    x[2 * k + 1] = f.y;
                 }
             }
         }
     }
     float vmin = x[0], vmax = x[0];
 #pragma unroll
-    for (int j = 1; j < 32; ++j) {
+    for (int j = 1; j < 8; ++j) {
         vmin = fminf(vmin, x[j]);
         vmax = fmaxf(vmax, x[j]);
     }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+        vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
+        vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    }
+    if (!live) return;
     constexpr float LEVELS = (float)((1 << VAL_BITS) - 1);
     float scale = E::round(__fdiv_rn(E::round(vmax - vmin), LEVELS));
     scale = fmaxf(scale, E::round(1e-10f));
-    constexpr int PER_WORD = 32 / VAL_BITS, WORDS = VAL_BITS;
-    uint32_t out[WORDS];
+    uint32_t out = 0;
 #pragma unroll
-    for (int w = 0; w < WORDS; ++w) {
-        out[w] = 0;
-#pragma unroll
-        for (int j = 0; j < PER_WORD; ++j) {
-            const float r = rintf(E::round(__fdiv_rn(E::round(x[w * PER_WORD + j] - vmin), scale)));
-            out[w] |= (uint32_t)fminf(fmaxf(r, 0.f), LEVELS) << (VAL_BITS * j);
-        }
+    for (int j = 0; j < 8; ++j) {
+        const float r = rintf(E::round(__fdiv_rn(E::round(x[j] - vmin), scale)));
+        out |= (uint32_t)fminf(fmaxf(r, 0.f), LEVELS) << (VAL_BITS * j);
     }
-    if (WORDS == 2) *reinterpret_cast<uint2*>(data + i * 8) = make_uint2(out[0], out[1]);
-    else *reinterpret_cast<uint4*>(data + i * 16) = make_uint4(out[0], out[1], out[WORDS - 2], out[WORDS - 1]);
-    E::store(scales, i, __half2float(__float2half_rn(scale)));
-    E::store(zeros, i, __half2float(__float2half_rn(vmin)));
+    if (VAL_BITS == 2) reinterpret_cast<uint16_t*>(data)[unit] = (uint16_t)out;
+    else reinterpret_cast<uint32_t*>(data)[unit] = out;
+    if (part == 0) {
+        E::store(scales, i, __half2float(__float2half_rn(scale)));
+        E::store(zeros, i, __half2float(__float2half_rn(vmin)));
+    }
 }
 
-// code * scale + zero in fp32 (kv_cache.py:101-116); one thread per 32-bit word of codes
+// code * scale + zero in fp32 (kv_cache.py:101-116); one thread per four channels
 template <int VAL_BITS>
 __global__ void __launch_bounds__(256) tq_rows_dequantize_values_kernel(const uint8_t* __restrict__ data, const void* __restrict__ scales,
-                                                                        const void* __restrict__ zeros, int sdt, int64_t n_words, float* __restrict__ out) {
-    constexpr int PER_WORD = 32 / VAL_BITS, WORDS_PER_GROUP = 32 / PER_WORD;
+                                                                        const void* __restrict__ zeros, int sdt, int64_t n_quads, float* __restrict__ out) {
+    wait_for_launch_ahead();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= n_words) return;
-    const uint32_t w = reinterpret_cast<const uint32_t*>(data)[i];
-    const float sc = __half2float(__float2half_rn(tq_load_any(scales, i / WORDS_PER_GROUP, sdt)));
-    const float zr = __half2float(__float2half_rn(tq_load_any(zeros, i / WORDS_PER_GROUP, sdt)));
-    float4* dst = reinterpret_cast<float4*>(out + i * PER_WORD);
+    if (i >= n_quads) return;
+    const uint32_t w = VAL_BITS == 2 ? data[i] : reinterpret_cast<const uint16_t*>(data)[i];
+    const float sc = __half2float(__float2half_rn(tq_load_any(scales, i >> 3, sdt)));
+    const float zr = __half2float(__float2half_rn(tq_load_any(zeros, i >> 3, sdt)));
+    float v[4];
 #pragma unroll
-    for (int j = 0; j < PER_WORD / 4; ++j) {
-        float v[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = (float)((w >> (VAL_BITS * (4 * j + k))) & ((1u << VAL_BITS) - 1u)) * sc + zr;
-        dst[j] = make_float4(v[0], v[1], v[2], v[3]);
-    }
+    for (int k = 0; k < 4; ++k) v[k] = (float)((w >> (VAL_BITS * k)) & ((1u << VAL_BITS) - 1u)) * sc + zr;
+    reinterpret_cast<float4*>(out)[i] = make_float4(v[0], v[1], v[2], v[3]);
 }
 
 // ------------------------------------------------------------------ keys, head_dim 128
 
-constexpr int RD = 128, R_WARPS = 8, R_ROWS = 16 * R_WARPS;
+constexpr int RD = 128, R_GROUPS = 8, R_ROWS = 16 * R_GROUPS;   // row groups of a tile, 16 rows each
+constexpr int R_THREADS = 2 * R_GROUPS * 32;       // a pair of warps per row group, half of the columns each
 constexpr int R_MAT = RD * RD * 2;                 // one limb of a constant operand in shared memory
 constexpr int KSTEPS = RD / 16;
+constexpr int R_XCHG = R_GROUPS * KSTEPS * 2 * 32 * 16;   // A fragments that the warps of a pair hand each other
+
+// the two warps of a row group
+__device__ __forceinline__ void pair_sync(int group) { asm volatile("bar.sync %0, 64;" ::"r"(1 + group) : "memory"); }
 
 __device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -176,9 +188,9 @@ __device__ __forceinline__ void mma_f16_z(float (&c)[4], const uint32_t (&a)[4],
 // it together with the small ones, which have accumulators of their own.  STEPS: not with each other either - every k-step's
 // sum is added up in fp32.  Error of a product against 64 bits, unit vectors: one chain for all 4.6e-7 of the result (5.6e-7
 // with 3-bit codes), two chains 1.9e-7 (2.5e-7), STEPS 0.9e-7 (1.1e-7); the fp32 fused multiply-adds of the kernels on records
-// 2.0e-7.  Of 384 million fp32 coordinates 319, 129 and 58 sign bits came out wrong, 259 in the fp32 store.  A pass over 16000
-// rows (quantise, score, dequantise) takes 73 us with one chain, 67 with two for quantising and STEPS for dequantising, 75 with
-// STEPS everywhere.
+// 2.0e-7.  Of 384 million fp32 coordinates 319, 129 and 58 sign bits came out wrong, 259 in the fp32 store.  With a warp per
+// 16 rows a pass over 16000 (quantise, score, dequantise) took 73 us with one chain, 67 with two for quantising and STEPS for
+// dequantising, 75 with STEPS everywhere.
 template <int LA, bool TRANS, bool STEPS>
 __device__ __forceinline__ void product(float (&acc)[2][4], const uint32_t (*a)[KSTEPS][4], uint32_t mats, int n0, int lane) {
     float low[2][4] = {};
@@ -340,39 +352,54 @@ __device__ __noinline__ void redo_row(const RowsParams& p, int64_t row, float nd
     }
 }
 
-// quantizer.py:129-149,231-257 for 16 rows per warp: norm, x / |x| (rounded to the dtype like torch), Y = u Pi^T, bucket
-// search, residual in rotated space r' = (Y - c) + E, E = (x / |x| - u) Pi^T, sign bits of r' M^T with M = S Pi^T.
+// quantizer.py:129-149,231-257 for 16 rows per pair of warps: norm, x / |x| (rounded to the dtype like torch), Y = u Pi^T,
+// bucket search, residual in rotated space r' = (Y - c) + E, E = (x / |x| - u) Pi^T, sign bits of r' M^T with M = S Pi^T.
+// A warp works out half of the k-steps of its rows' A operands and half of the columns of both products; what the other needs
+// goes through shared memory as whole fragments.  Four warps a scheduler instead of two cover one another's chains, and the
+// loops over columns stay rolled: unrolled they were 100 KB of instructions that a call of one tile per CTA reads once.
 template <int DT, int MSE_BITS>
-__global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(const __grid_constant__ RowsParams p) {
+__global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(const __grid_constant__ RowsParams p) {
     using E = TqElem<DT>;
-    constexpr int LU = DT == TQ_F32 ? 2 : 1;   // limbs that hold u
+    constexpr int LU = DT == TQ_F32 ? 2 : 1;   // limbs that hold u; else the second place holds e = x / |x| - u
     constexpr int NB = (1 << MSE_BITS) - 1;
+    constexpr int HALF = KSTEPS / 2;           // k-steps, and blocks of 16 columns, of one warp of the pair
     extern __shared__ __align__(16) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+    __shared__ float s_ss[R_ROWS], s_n2[2][R_ROWS];
+    __shared__ uint32_t s_redo[R_GROUPS][2];
+    const int tid = threadIdx.x, group = (tid >> 5) & (R_GROUPS - 1), mine = tid >> 8, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
 #pragma unroll 1
-    for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_WARPS * 32);
+    for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_THREADS);
     asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll 1
-    for (int i = 0; i < 2; ++i) load_operand(smem + (2 + i) * R_MAT, p.other[i], tid, R_WARPS * 32);
+    for (int i = 0; i < 2; ++i) load_operand(smem + (2 + i) * R_MAT, p.other[i], tid, R_THREADS);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const uint32_t sp = tq_smem_u32(smem), sm = sp + 2 * R_MAT;
+    uint4* xchg = reinterpret_cast<uint4*>(smem + 4 * R_MAT) + group * (KSTEPS * 2 * 32) + lane;   // [k-step][limb][lane]
+    wait_for_launch_ahead();
     bool first = true;
 #pragma unroll 1
     for (int64_t tile = blockIdx.x; tile * R_ROWS < p.n; tile += gridDim.x) {
-        const int64_t r0 = tile * R_ROWS + warp * 16 + gid, r1 = r0 + 8;
-        uint32_t a[LU][KSTEPS][4], e[DT == TQ_F32 ? 1 : KSTEPS][4];
-        float nd[2], den[2];
-        {   // norms of the warp's 16 rows, in the fp32 store kernel's order: eight sums of 16 squares, added up in order.
-            // Lane = (row % 4, sum), four rows a lane.
-            const int ch = lane & 7;
-            float own[4];
+        const int64_t base_row = tile * R_ROWS + group * 16, r0 = base_row + gid, r1 = r0 + 8;
+        float x[HALF][2][2][2];   // this warp's k-steps: [row][half][element]
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int64_t row = tile * R_ROWS + warp * 16 + 4 * i + (lane >> 3);
+        for (int ks = 0; ks < HALF; ++ks)
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    const int64_t row = r ? r1 : r0;
+                    x[ks][r][hf][0] = x[ks][r][hf][1] = 0.f;
+                    if (row < p.n) load2<DT>(p.x, row * p.stride_row + (mine * HALF + ks) * 16 + hf * 8 + 2 * tig, x[ks][r][hf][0], x[ks][r][hf][1]);
+                }
+        {   // norms, in the fp32 store kernel's order: eight sums of 16 squares, added up in order.  Lane = (row % 4, sum), two rows a lane.
+            const int ch = lane & 7;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int row_l = 8 * mine + 4 * i + (lane >> 3);
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; j += 4)
-                    if (row < p.n) load4<DT>(p.x, row * p.stride_row + ch * 16 + j, v + j);
+                    if (base_row + row_l < p.n) load4<DT>(p.x, (base_row + row_l) * p.stride_row + ch * 16 + j, v + j);
                     else v[j] = v[j + 1] = v[j + 2] = v[j + 3] = 0.f;
                 float s = 0.f;
 #pragma unroll
@@ -380,40 +407,55 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
                 float tot = 0.f;
 #pragma unroll
                 for (int c = 0; c < 8; ++c) tot += __shfl_sync(0xffffffffu, s, (lane & 24) + c);
-                own[i] = tot;
-            }
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {   // rows gid, gid + 8: slot (row / 4), lanes 8 * (row % 4)
-                const float lo = __shfl_sync(0xffffffffu, own[2 * r], 8 * (gid & 3)), hi = __shfl_sync(0xffffffffu, own[2 * r + 1], 8 * (gid & 3));
-                nd[r] = E::round(__fsqrt_rn(gid < 4 ? lo : hi));
-                den[r] = E::round(nd[r] + 1e-10f);
+                if (ch == 0) s_ss[group * 16 + row_l] = tot;
             }
         }
+        pair_sync(group);
+        float nd[2], den[2];
 #pragma unroll
-        for (int ks = 0; ks < KSTEPS; ++ks)
+        for (int r = 0; r < 2; ++r) {
+            nd[r] = E::round(__fsqrt_rn(s_ss[group * 16 + gid + 8 * r]));
+            den[r] = E::round(nd[r] + 1e-10f);
+        }
+#pragma unroll
+        for (int ks = 0; ks < HALF; ++ks) {
+            uint32_t f[2][4];
 #pragma unroll
             for (int r = 0; r < 2; ++r)
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
-                    const int64_t row = r ? r1 : r0, at = row * p.stride_row + ks * 16 + hf * 8 + 2 * tig;
-                    float v0 = 0.f, v1 = 0.f;
-                    if (row < p.n) load2<DT>(p.x, at, v0, v1);
-                    const float q0 = __fdiv_rn(v0, den[r]), q1 = __fdiv_rn(v1, den[r]);
+                    const float q0 = __fdiv_rn(x[ks][r][hf][0], den[r]), q1 = __fdiv_rn(x[ks][r][hf][1], den[r]);
                     const float u0 = E::round(q0), u1 = E::round(q1);
-                    split<LU>(u0 * R_SCALE, u1 * R_SCALE, &a[0][ks][hf * 2 + r], KSTEPS * 4);
-                    if (DT != TQ_F32) e[DT == TQ_F32 ? 0 : ks][hf * 2 + r] = pack_h((q0 - u0) * R_SCALE, (q1 - u1) * R_SCALE);
+                    split<LU>(u0 * R_SCALE, u1 * R_SCALE, &f[0][hf * 2 + r], 4);
+                    if (DT != TQ_F32) f[1][hf * 2 + r] = pack_h((q0 - u0) * R_SCALE, (q1 - u1) * R_SCALE);
                 }
+#pragma unroll
+            for (int l = 0; l < 2; ++l) xchg[((mine * HALF + ks) * 2 + l) * 32] = make_uint4(f[l][0], f[l][1], f[l][2], f[l][3]);
+        }
+        uint32_t a[2][KSTEPS][4];
+        auto take = [&]() {   // all fragments of the pair's rows
+            pair_sync(group);
+#pragma unroll
+            for (int ks = 0; ks < KSTEPS; ++ks)
+#pragma unroll
+                for (int l = 0; l < 2; ++l) {
+                    const uint4 v = xchg[(ks * 2 + l) * 32];
+                    a[l][ks][0] = v.x; a[l][ks][1] = v.y; a[l][ks][2] = v.z; a[l][ks][3] = v.w;
+                }
+            pair_sync(group);
+        };
+        take();
         if (first) {
             asm volatile("cp.async.wait_group 1;" ::: "memory");
             __syncthreads();
         }
         // ---- codes, r' as limbs in the A layout of the second product ----
-        uint32_t rl[2][KSTEPS][4];
-        uint32_t cw[2][MSE_BITS == 2 ? 2 : 4];    // code words of the two rows, word j in lane j % 4
+        uint32_t cw[2][MSE_BITS == 2 ? 1 : 2] = {};   // this warp's code words of the two rows, word j in lane j % 4
         float rn2[2] = {0.f, 0.f};
-        uint32_t near_lo = 0, near_hi = 0;        // coordinates next to a boundary, bit 8 * nb + 4 * n8 + c
-#pragma unroll
-        for (int nb = 0; nb < RD / 16; ++nb) {
+        uint32_t near = 0;                            // coordinates next to a boundary, bit 8 * j + 4 * n8 + c
+#pragma unroll 1
+        for (int j = 0; j < HALF; ++j) {
+            const int nb = mine * HALF + j;
             float acc[2][4] = {};
             product<LU, false, false>(acc, a, sp, nb * 16, lane);
             float er[2][4] = {};
@@ -422,11 +464,11 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
                 for (int ks = 0; ks < KSTEPS; ++ks) {   // |q - u| <= 2^-12: Pi's first limb is enough
                     uint32_t b[4];
                     b_frag<false>(sp, nb * 16, ks, lane, b);
-                    mma_f16(er[0], e[DT == TQ_F32 ? 0 : ks], b[0], b[1]);
-                    mma_f16(er[1], e[DT == TQ_F32 ? 0 : ks], b[2], b[3]);
+                    mma_f16(er[0], a[1][ks], b[0], b[1]);
+                    mma_f16(er[1], a[1][ks], b[2], b[3]);
                 }
             }
-            uint32_t half[2];   // 2-bit codes: the word's first 16 bits
+            uint32_t word[2] = {0u, 0u}, rl[2][4];
 #pragma unroll
             for (int n8 = 0; n8 < 2; ++n8) {
                 uint32_t code[4];
@@ -434,7 +476,6 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float y = acc[n8][c] * (1.f / (R_SCALE * R_SCALE));
-                    const uint32_t bit = 1u << ((nb & 3) * 8 + n8 * 4 + c);
                     uint32_t k = 0;
                     float cv = p.cb.centroids[0], gap = 1.f;
 #pragma unroll
@@ -446,7 +487,7 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
                             cv = p.cb.centroids[i + 1];
                         }
                     }
-                    if (gap < NEAR) (nb < 4 ? near_lo : near_hi) |= bit;
+                    if (gap < NEAR) near |= (1u << (n8 * 4 + c)) << (8 * j);
                     if (y != y) {   // searchsorted orders NaN after every number
                         k = NB;
                         cv = p.cb.centroids[NB];
@@ -455,21 +496,24 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
                     r[c] = fmaf(er[n8][c], 1.f / (R_SCALE * R_SCALE), y - cv);
                     rn2[c >> 1] = fmaf(r[c], r[c], rn2[c >> 1]);
                 }
-                split<2>(r[0] * R_SCALE, r[1] * R_SCALE, &rl[0][nb][n8 * 2], KSTEPS * 4);       // row r0
-                split<2>(r[2] * R_SCALE, r[3] * R_SCALE, &rl[0][nb][n8 * 2 + 1], KSTEPS * 4);   // row r1
+                split<2>(r[0] * R_SCALE, r[1] * R_SCALE, &rl[0][n8 * 2], 4);       // row r0
+                split<2>(r[2] * R_SCALE, r[3] * R_SCALE, &rl[0][n8 * 2 + 1], 4);   // row r1
 #pragma unroll
                 for (int r2 = 0; r2 < 2; ++r2) {
                     uint32_t w = MSE_BITS == 2 ? (code[2 * r2] | (code[2 * r2 + 1] << 2)) << (4 * tig) : (code[2 * r2] | (code[2 * r2 + 1] << 4)) << (8 * tig);
                     w |= __shfl_xor_sync(0xffffffffu, w, 1);
                     w |= __shfl_xor_sync(0xffffffffu, w, 2);
-                    if (MSE_BITS == 2) {
-                        if (n8) w = half[r2] | (w << 16);
-                        else half[r2] = w;
+                    if (MSE_BITS == 2) {   // 16 bits of one word for each n8
+                        word[r2] |= w << (16 * n8);
+                        if (n8 && tig == j) cw[r2][0] = word[r2];
+                    } else if (tig == ((2 * j + n8) & 3)) {
+                        if (j < 2) cw[r2][0] = w;
+                        else cw[r2][MSE_BITS == 2 ? 0 : 1] = w;
                     }
-                    const int j = MSE_BITS == 2 ? nb : nb * 2 + n8;
-                    if (tig == (j & 3)) cw[r2][j >> 2] = w;
                 }
             }
+#pragma unroll
+            for (int l = 0; l < 2; ++l) xchg[(nb * 2 + l) * 32] = make_uint4(rl[l][0], rl[l][1], rl[l][2], rl[l][3]);
         }
         if (first) {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -477,18 +521,22 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
             first = false;
         }
         // ---- sign bits of r' M^T ----
-        uint32_t sw[2][4] = {};
-#pragma unroll
-        for (int nb = 0; nb < RD / 16; ++nb) {
+        take();
+        uint32_t sw[2][2] = {};
+#pragma unroll 1
+        for (int j = 0; j < HALF; ++j) {
             float acc[2][4] = {};
-            product<2, false, false>(acc, rl, sm, nb * 16, lane);
+            product<2, false, false>(acc, a, sm, (mine * HALF + j) * 16, lane);
 #pragma unroll
-            for (int n8 = 0; n8 < 2; ++n8)
+            for (int r2 = 0; r2 < 2; ++r2) {
+                uint32_t w = 0;
 #pragma unroll
-                for (int r2 = 0; r2 < 2; ++r2) {
-                    uint32_t w = ((acc[n8][2 * r2] > 0.f ? 1u : 0u) | (acc[n8][2 * r2 + 1] > 0.f ? 2u : 0u)) << (2 * tig);
-                    sw[r2][nb >> 1] |= w << (8 * (2 * (nb & 1) + n8));
-                }
+                for (int n8 = 0; n8 < 2; ++n8)
+                    w |= ((acc[n8][2 * r2] > 0.f ? 1u : 0u) | (acc[n8][2 * r2 + 1] > 0.f ? 2u : 0u)) << (2 * tig + 8 * n8);
+                w <<= 16 * (j & 1);
+                if (j < 2) sw[r2][0] |= w;
+                else sw[r2][1] |= w;
+            }
         }
         // ---- out ----
 #pragma unroll
@@ -497,9 +545,10 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
             float n2 = rn2[r2];
             n2 += __shfl_xor_sync(0xffffffffu, n2, 1);
             n2 += __shfl_xor_sync(0xffffffffu, n2, 2);
-            uint32_t s[4];
+            if (tig == 0) s_n2[mine][group * 16 + gid + 8 * r2] = n2;
+            uint32_t s[2];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 2; ++i) {
                 uint32_t w = sw[r2][i];
                 w |= __shfl_xor_sync(0xffffffffu, w, 1);
                 w |= __shfl_xor_sync(0xffffffffu, w, 2);
@@ -507,29 +556,23 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
             }
             if (row >= p.n) continue;
             constexpr int CB = MSE_BITS == 2 ? RD / 4 : RD / 2;
-            if (tig == 0) *reinterpret_cast<uint4*>(p.signs + row * (RD / 8)) = make_uint4(s[0], s[1], s[2], s[3]);
+            if (tig == 0) *reinterpret_cast<uint2*>(p.signs + row * (RD / 8) + 8 * mine) = make_uint2(s[0], s[1]);
 #pragma unroll
-            for (int q = 0; q < CB / 16; ++q) *reinterpret_cast<uint32_t*>(p.codes + row * CB + 16 * q + 4 * tig) = cw[r2][q];
-            if (tig == 3) {
-                tq_store_any(p.norms, row, __half2float(__float2half_rn(nd[r2])), p.norm_dt);
-                tq_store_any(p.rnorms, row, nd[r2] == 0.f ? 0.f : __half2float(__float2half_rn(nd[r2] * __fsqrt_rn(n2))), p.rnorm_dt);
-            }
+            for (int q = 0; q < CB / 32; ++q) *reinterpret_cast<uint32_t*>(p.codes + row * CB + mine * (CB / 2) + 16 * q + 4 * tig) = cw[r2][q];
         }
         // ---- coordinates next to a boundary, by the fp32 store kernel's chain; a row where it decides differently is redone ----
-        if (r0 >= p.n || nd[0] == 0.f) { near_lo &= 0xccccccccu; near_hi &= 0xccccccccu; }
-        if (r1 >= p.n || nd[1] == 0.f) { near_lo &= 0x33333333u; near_hi &= 0x33333333u; }
-        if (__any_sync(0xffffffffu, (near_lo | near_hi) != 0)) {
+        if (r0 >= p.n || nd[0] == 0.f) near &= 0xccccccccu;
+        if (r1 >= p.n || nd[1] == 0.f) near &= 0x33333333u;
+        uint32_t redo = 0;   // rows of the pair's sixteen
+        if (__any_sync(0xffffffffu, near != 0)) {
             __syncwarp();   // the warp's codes, read back below
-            uint32_t redo = 0;   // rows of the warp's sixteen
 #pragma unroll 1
-            for (uint32_t who; (who = __ballot_sync(0xffffffffu, (near_lo | near_hi) != 0)) != 0;) {
+            for (uint32_t who; (who = __ballot_sync(0xffffffffu, near != 0)) != 0;) {
                 const int from = __ffs(who) - 1;   // this lane's next coordinate, for the whole warp
-                const bool upper = near_lo == 0;
-                const uint32_t m = upper ? near_hi : near_lo, one = m & (0u - m);
-                const int bit = __shfl_sync(0xffffffffu, __ffs(m) - 1 + (upper ? 32 : 0), from);
-                if (lane == from) (upper ? near_hi : near_lo) ^= one;
-                const int col = (bit >> 2) * 8 + 2 * (from & 3) + (bit & 1), rw = (from >> 2) + (bit & 2 ? 8 : 0);
-                const int64_t row = tile * R_ROWS + warp * 16 + rw;
+                const int bit = __shfl_sync(0xffffffffu, __ffs(near) - 1, from);
+                if (lane == from) near &= near - 1;
+                const int col = mine * (RD / 2) + (bit >> 2) * 8 + 2 * (from & 3) + (bit & 1), rw = (from >> 2) + (bit & 2 ? 8 : 0);
+                const int64_t row = base_row + rw;
                 const float y = serial_product<DT>(p.x, row * p.stride_row, __shfl_sync(0xffffffffu, bit & 2 ? den[1] : den[0], from), p.pi_t + col, lane);
                 int k = 0;
 #pragma unroll
@@ -538,37 +581,95 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_quantize_keys_kernel(
                 const int had = (*(volatile const uint8_t*)(p.codes + row * (RD / PER) + col / PER) >> (W * (col % PER))) & ((1 << W) - 1);
                 if (k != had) redo |= 1u << rw;
             }
+        }
+        if (lane == 0) s_redo[group][mine] = redo;
+        pair_sync(group);   // both halves of every row are written
+        if (mine == 0) {
+            if (tig == 3)
+#pragma unroll
+                for (int r2 = 0; r2 < 2; ++r2) {
+                    const int64_t row = r2 ? r1 : r0;
+                    const float n2 = s_n2[0][group * 16 + gid + 8 * r2] + s_n2[1][group * 16 + gid + 8 * r2];
+                    if (row >= p.n) continue;
+                    tq_store_any(p.norms, row, __half2float(__float2half_rn(nd[r2])), p.norm_dt);
+                    tq_store_any(p.rnorms, row, nd[r2] == 0.f ? 0.f : __half2float(__float2half_rn(nd[r2] * __fsqrt_rn(n2))), p.rnorm_dt);
+                }
+            __syncwarp();   // redo_row writes a residual norm again
+            redo = s_redo[group][0] | s_redo[group][1];
 #pragma unroll 1
             for (; redo != 0; redo &= redo - 1) {
                 const int rw = __ffs(redo) - 1, from = 4 * (rw & 7);
-                redo_row<DT, MSE_BITS>(p, tile * R_ROWS + warp * 16 + rw, __shfl_sync(0xffffffffu, rw & 8 ? nd[1] : nd[0], from),
+                redo_row<DT, MSE_BITS>(p, base_row + rw, __shfl_sync(0xffffffffu, rw & 8 ? nd[1] : nd[0], from),
                                        __shfl_sync(0xffffffffu, rw & 8 ? den[1] : den[0], from), sm, lane);
             }
         }
     }
 }
 
-// quantizer.py:151-165,259-272 for 16 rows per warp: (c[idx] Pi) * norm + qjl_scale * rnorm * (signs S)
+// quantizer.py:151-165,259-272 for 16 rows per pair of warps, half of the columns each: (c[idx] Pi) * norm + qjl_scale * rnorm *
+// (signs S).  The codes' product first; a thread leaves its sums in shared memory while the signs take over the operand's registers.
 template <int MSE_BITS>
-__global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_dequantize_keys_kernel(const RowsParams p) {
+__global__ void __launch_bounds__(R_THREADS, 1) tq_rows_dequantize_keys_kernel(const RowsParams p) {
+    constexpr int HALF = KSTEPS / 2;   // blocks of 16 columns of one warp
     extern __shared__ __align__(16) uint8_t smem[];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
+    const int tid = threadIdx.x, group = (tid >> 5) & (R_GROUPS - 1), mine = tid >> 8, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
 #pragma unroll 1
-    for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_WARPS * 32);
+    for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_THREADS);
     if (p.with_qjl)
 #pragma unroll 1
-        for (int i = 0; i < 2; ++i) load_operand(smem + (2 + i) * R_MAT, p.other[i], tid, R_WARPS * 32);
+        for (int i = 0; i < 2; ++i) load_operand(smem + (2 + i) * R_MAT, p.other[i], tid, R_THREADS);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const uint32_t sp = tq_smem_u32(smem), ssg = sp + 2 * R_MAT;
-    float* cen = reinterpret_cast<float*>(smem + 4 * R_MAT);
+    float4* held = reinterpret_cast<float4*>(smem + 4 * R_MAT) + tid;   // [block of columns][n8][thread]
+    float* cen = reinterpret_cast<float*>(smem + 4 * R_MAT + HALF * 2 * R_THREADS * sizeof(float4));
     if (tid < (1 << MSE_BITS)) cen[tid] = p.cb.centroids[tid];
+    wait_for_launch_ahead();
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     constexpr int CB = MSE_BITS == 2 ? RD / 4 : RD / 2;
 #pragma unroll 1
     for (int64_t tile = blockIdx.x; tile * R_ROWS < p.n; tile += gridDim.x) {
-        const int64_t rows[2] = {tile * R_ROWS + warp * 16 + gid, tile * R_ROWS + warp * 16 + gid + 8};
-        uint32_t a[2][KSTEPS][4], sg[1][KSTEPS][4];
+        const int64_t rows[2] = {tile * R_ROWS + group * 16 + gid, tile * R_ROWS + group * 16 + gid + 8};
+        {
+            uint32_t a[2][KSTEPS][4];
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int ks = 0; ks < KSTEPS; ++ks) {
+                    uint32_t cbits = 0, cbits2 = 0;   // 16 coordinates of the k-step: 2-bit codes in one word, nibbles in two
+                    if (rows[r] < p.n) {
+                        if (MSE_BITS == 2) {
+                            cbits = reinterpret_cast<const uint32_t*>(p.codes + rows[r] * CB)[ks];
+                        } else {
+                            const uint2 v = reinterpret_cast<const uint2*>(p.codes + rows[r] * CB)[ks];
+                            cbits = v.x;
+                            cbits2 = v.y;
+                        }
+                    }
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        const int k = hf * 8 + 2 * tig;
+                        float c0, c1;
+                        if (MSE_BITS == 2) {
+                            c0 = cen[(cbits >> (2 * k)) & 3u];
+                            c1 = cen[(cbits >> (2 * k + 2)) & 3u];
+                        } else {
+                            const uint32_t w = hf ? cbits2 : cbits;
+                            c0 = cen[(w >> (8 * tig)) & 7u];
+                            c1 = cen[(w >> (8 * tig + 4)) & 7u];
+                        }
+                        split<2>(c0 * R_SCALE, c1 * R_SCALE, &a[0][ks][hf * 2 + r], KSTEPS * 4);
+                    }
+                }
+#pragma unroll 1
+            for (int j = 0; j < HALF; ++j) {
+                float ak[2][4] = {};
+                product<2, true, true>(ak, a, sp, (mine * HALF + j) * 16, lane);
+#pragma unroll
+                for (int n8 = 0; n8 < 2; ++n8) held[(j * 2 + n8) * R_THREADS] = make_float4(ak[n8][0], ak[n8][1], ak[n8][2], ak[n8][3]);
+            }
+        }
+        uint32_t sg[1][KSTEPS][4];   // +1 / -1
         float norm[2], rn[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -577,48 +678,26 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_dequantize_keys_kerne
             rn[r] = live && p.with_qjl ? p.qjl_scale * __half2float(__float2half_rn(tq_load_any(p.rnorms, rows[r], p.rnorm_dt))) : 0.f;
 #pragma unroll
             for (int ks = 0; ks < KSTEPS; ++ks) {
-                uint32_t cbits = 0, sbits = 0;   // 16 coordinates of the k-step: 2-bit codes in one word, nibbles in two
-                uint32_t cbits2 = 0;
-                if (live) {
-                    if (MSE_BITS == 2) {
-                        cbits = reinterpret_cast<const uint32_t*>(p.codes + rows[r] * CB)[ks];
-                    } else {
-                        const uint2 v = reinterpret_cast<const uint2*>(p.codes + rows[r] * CB)[ks];
-                        cbits = v.x;
-                        cbits2 = v.y;
-                    }
-                    if (p.with_qjl) sbits = reinterpret_cast<const uint16_t*>(p.signs + rows[r] * (RD / 8))[ks];
-                }
+                const uint32_t bits = live && p.with_qjl ? reinterpret_cast<const uint16_t*>(p.signs + rows[r] * (RD / 8))[ks] : 0u;
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
-                    const int k = hf * 8 + 2 * tig;
-                    float c0, c1;
-                    if (MSE_BITS == 2) {
-                        c0 = cen[(cbits >> (2 * k)) & 3u];
-                        c1 = cen[(cbits >> (2 * k + 2)) & 3u];
-                    } else {
-                        const uint32_t w = hf ? cbits2 : cbits;
-                        c0 = cen[(w >> (8 * tig)) & 7u];
-                        c1 = cen[(w >> (8 * tig + 4)) & 7u];
-                    }
-                    split<2>(c0 * R_SCALE, c1 * R_SCALE, &a[0][ks][hf * 2 + r], KSTEPS * 4);
-                    const uint32_t b = (sbits >> k) & 3u;   // +1 / -1
+                    const uint32_t b = bits >> (hf * 8 + 2 * tig);
                     sg[0][ks][hf * 2 + r] = ((b & 1u) ? 0x3c00u : 0xbc00u) | ((b & 2u) ? 0x3c000000u : 0xbc000000u);
                 }
             }
         }
 #pragma unroll 1
-        for (int nb = 0; nb < RD / 16; ++nb) {
-            float ak[2][4] = {}, as[2][4] = {};
-            product<2, true, true>(ak, a, sp, nb * 16, lane);
-            if (p.with_qjl) product<1, true, true>(as, sg, ssg, nb * 16, lane);
+        for (int j = 0; j < HALF; ++j) {
+            const int n0 = (mine * HALF + j) * 16;
+            float as[2][4] = {};
+            if (p.with_qjl) product<1, true, true>(as, sg, ssg, n0, lane);
 #pragma unroll
-            for (int n8 = 0; n8 < 2; ++n8)
-#pragma unroll
-                for (int r = 0; r < 2; ++r)
-                    if (rows[r] < p.n)
-                        *reinterpret_cast<float2*>(p.out + rows[r] * RD + nb * 16 + n8 * 8 + 2 * tig) =
-                            make_float2(ak[n8][2 * r] * norm[r] + as[n8][2 * r] * rn[r], ak[n8][2 * r + 1] * norm[r] + as[n8][2 * r + 1] * rn[r]);
+            for (int n8 = 0; n8 < 2; ++n8) {
+                const float4 ak = held[(j * 2 + n8) * R_THREADS];
+                float* out = p.out + n0 + n8 * 8 + 2 * tig;
+                if (rows[0] < p.n) *reinterpret_cast<float2*>(out + rows[0] * RD) = make_float2(ak.x * norm[0] + as[n8][0] * rn[0], ak.y * norm[0] + as[n8][1] * rn[0]);
+                if (rows[1] < p.n) *reinterpret_cast<float2*>(out + rows[1] * RD) = make_float2(ak.z * norm[1] + as[n8][2] * rn[1], ak.w * norm[1] + as[n8][3] * rn[1]);
+            }
         }
     }
 }
@@ -627,6 +706,7 @@ __global__ void __launch_bounds__(R_WARPS * 32, 1) tq_rows_dequantize_keys_kerne
 __global__ void __launch_bounds__(256) tq_rows_dequantize_keys256_kernel(const RowsParams p, const float* __restrict__ pi, const float* __restrict__ s, int mse_bits) {
     constexpr int D = 256;
     __shared__ __align__(16) float yh[D][20], sg[D][20];   // [coordinate][16 rows], padded
+    wait_for_launch_ahead();
     const int j = threadIdx.x;
     const int64_t row0 = (int64_t)blockIdx.x * 16;
     const int width = mse_bits == 2 ? 2 : 4, vpb = 8 / width, cb = D / vpb;
@@ -672,41 +752,80 @@ __global__ void __launch_bounds__(256) tq_rows_dequantize_keys256_kernel(const R
 
 // ------------------------------------------------------------------ scores of key planes
 
-// Unscaled logits of 64 tokens of one head (two threads per token) for up to eight queries; the queries are prepared (qprep).
-template <int D, int MSE_BITS>
-__global__ void __launch_bounds__(128) tq_rows_scores_kernel(const RowsParams p, const float* __restrict__ qprep, int64_t n_k, int n_q, float* __restrict__ logits) {
-    constexpr int GP = 8;
-    __shared__ __align__(16) float qr[D * GP], qs[D * GP], sp[2 * GP * 64], cent[TQ_MAX_CENTROIDS];
+// Unscaled logits of 64 tokens of one head (two threads per token) for GP queries; the queries are prepared (qprep).  A thread
+// asks for its whole half row at once (16 bytes at a time where the planes are aligned: `vec`), and a CTA holds no more queries
+// than it was asked for.
+template <int D, int MSE_BITS, int GP>
+__global__ void __launch_bounds__(128) tq_rows_scores_kernel(const RowsParams p, const float* __restrict__ qprep, int64_t n_k, int n_q, int vec, float* __restrict__ logits) {
+    constexpr int NSW = HalfRow<D, MSE_BITS>::NSW, NCW = HalfRow<D, MSE_BITS>::NCW;
+    __shared__ __align__(16) float qs[GP][2][D];
+    __shared__ float sp[GP * 64], cent[TQ_MAX_CENTROIDS];
     const int tid = threadIdx.x, h = blockIdx.y, q0 = blockIdx.z * GP, nq = min(GP, n_q - q0);
     if (tid < TQ_MAX_CENTROIDS) cent[tid] = p.cb.centroids[tid];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int i = tid; i < D * GP; i += 128) {
-        const int j = i / GP, g = i % GP;
-        const float* src = qprep + (((int64_t)h * n_q + q0 + g) * 2) * D;
-        qr[i] = g < nq ? src[j] : 0.f;
-        qs[i] = g < nq ? src[D + j] : 0.f;
-    }
-    __syncthreads();
     const int tk = tid & 63, half = tid >> 6;
     const int64_t t = (int64_t)blockIdx.x * 64 + tk, row = (int64_t)h * n_k + t;
-    float part[GP];
-#pragma unroll
-    for (int g = 0; g < GP; ++g) part[g] = 0.f;
+    wait_for_launch_ahead();
+    uint32_t cw[NCW], sw[NSW];
+    float norm = 0.f, rn = 0.f;
     if (t < n_k) {
-        constexpr int CB = MSE_BITS == 2 ? D / 4 : D / 2;
-        const float norm = __half2float(__float2half_rn(tq_load_any(p.norms, row, p.norm_dt)));
-        const float rn = __half2float(__float2half_rn(tq_load_any(p.rnorms, row, p.rnorm_dt))) * p.qjl_scale;
-        half_row_scores<D, MSE_BITS, GP>(reinterpret_cast<const uint32_t*>(p.codes + row * CB), reinterpret_cast<const uint32_t*>(p.signs + row * (D / 8)),
-                                         norm, rn, half, qr, qs, cent, part);
-    }
+        const uint32_t* c = reinterpret_cast<const uint32_t*>(p.codes + row * (8 * NCW)) + half * NCW;
+        const uint32_t* g = reinterpret_cast<const uint32_t*>(p.signs + row * (D / 8)) + half * NSW;
+        if (vec) {
 #pragma unroll
-    for (int g = 0; g < GP; ++g) sp[(half * GP + g) * 64 + tk] = part[g];
-    __syncthreads();
-    for (int i = tid; i < nq * 64; i += 128) {
-        const int g = i / 64, tt = i % 64;
-        const int64_t at = (int64_t)blockIdx.x * 64 + tt;
-        if (at < n_k) logits[((int64_t)h * n_q + q0 + g) * n_k + at] = sp[g * 64 + tt] + sp[(GP + g) * 64 + tt];
+            for (int k = 0; k < NCW; k += 4) {
+                const uint4 v = *reinterpret_cast<const uint4*>(c + k);
+                cw[k] = v.x; cw[k + 1] = v.y; cw[k + 2] = v.z; cw[k + 3] = v.w;
+            }
+#pragma unroll
+            for (int k = 0; k < NSW; k += 2) {
+                const uint2 v = *reinterpret_cast<const uint2*>(g + k);
+                sw[k] = v.x; sw[k + 1] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NCW; ++k) cw[k] = c[k];
+#pragma unroll
+            for (int k = 0; k < NSW; ++k) sw[k] = g[k];
+        }
+        norm = __half2float(__float2half_rn(tq_load_any(p.norms, row, p.norm_dt)));
+        rn = __half2float(__float2half_rn(tq_load_any(p.rnorms, row, p.rnorm_dt))) * p.qjl_scale;
     }
+    const float4* src = reinterpret_cast<const float4*>(qprep + ((int64_t)h * n_q + q0) * 2 * D);
+    for (int i = tid; i < GP * 2 * D / 4; i += 128)
+        reinterpret_cast<float4*>(qs)[i] = i < nq * 2 * D / 4 ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncthreads();
+    float part[GP];
+    if (t < n_k) {
+        float am[GP], aq[GP];
+        half_row_dots<D, MSE_BITS, GP>(cw, sw, qs, cent, half, am, aq);
+#pragma unroll
+        for (int g = 0; g < GP; ++g) part[g] = norm * am[g] + rn * aq[g];
+        if (half)
+#pragma unroll
+            for (int g = 0; g < GP; ++g) sp[g * 64 + tk] = part[g];
+    }
+    __syncthreads();
+    if (!half && t < n_k)
+#pragma unroll
+        for (int g = 0; g < GP; ++g)
+            if (g < nq) logits[((int64_t)h * n_q + q0 + g) * n_k + t] = part[g] + sp[g * 64 + tk];
+}
+
+// A kernel of this file behind whatever was launched last: its constants are loaded under that launch.
+template <class Kern, class... Args>
+int launch_rows(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+    return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
 }
 
 bool aligned(const void* p, size_t n) { return ((uintptr_t)p & (n - 1)) == 0; }
@@ -742,20 +861,16 @@ extern "C" int tq_rows_quantize_values(const void* v, tq_dtype dtype, int64_t n_
     if (n_rows == 0) return TQ_OK;
     const int gpr = head_dim / 32;
     const int64_t n = n_rows * gpr;
-    const unsigned grid = (unsigned)((n + 255) / 256);
+    const dim3 grid((unsigned)((4 * n + 255) / 256));
     cudaStream_t st = (cudaStream_t)stream;
-    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
 #define TQ_QV(DT)                                                                                                     \
-    do {                                                                                                              \
-        if (bits == 2) tq_rows_quantize_values_kernel<DT, 2><<<grid, 256, 0, st>>>(v, n, gpr, stride_row, data, scales, zeros); \
-        else tq_rows_quantize_values_kernel<DT, 4><<<grid, 256, 0, st>>>(v, n, gpr, stride_row, data, scales, zeros);  \
-    } while (0)
+    return bits == 2 ? launch_rows(tq_rows_quantize_values_kernel<DT, 2>, grid, 256, 0, st, v, n, gpr, stride_row, data, scales, zeros) \
+                     : launch_rows(tq_rows_quantize_values_kernel<DT, 4>, grid, 256, 0, st, v, n, gpr, stride_row, data, scales, zeros)
     if (dtype == TQ_F32) TQ_QV(TQ_F32);
-    else if (dtype == TQ_BF16) TQ_QV(TQ_BF16);
-    else if (dtype == TQ_F16) TQ_QV(TQ_F16);
-    else return TQ_ERR_UNSUPPORTED;
+    if (dtype == TQ_BF16) TQ_QV(TQ_BF16);
+    if (dtype == TQ_F16) TQ_QV(TQ_F16);
 #undef TQ_QV
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+    return TQ_ERR_UNSUPPORTED;
 }
 
 extern "C" int tq_rows_dequantize_values(const uint8_t* data, const void* scales, const void* zeros, tq_dtype scale_dtype, int64_t n_rows,
@@ -765,13 +880,11 @@ extern "C" int tq_rows_dequantize_values(const uint8_t* data, const void* scales
     if (bits != 2 && bits != 4) return TQ_ERR_UNSUPPORTED;
     if (!aligned(data, 4) || !aligned(out, 16)) return TQ_ERR_ALIGN;
     if (n_rows == 0) return TQ_OK;
-    const int64_t words = n_rows * head_dim * bits / 32;
-    const unsigned grid = (unsigned)((words + 255) / 256);
+    const int64_t quads = n_rows * head_dim / 4;
+    const dim3 grid((unsigned)((quads + 255) / 256));
     cudaStream_t st = (cudaStream_t)stream;
-    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
-    if (bits == 2) tq_rows_dequantize_values_kernel<2><<<grid, 256, 0, st>>>(data, scales, zeros, scale_dtype, words, out);
-    else tq_rows_dequantize_values_kernel<4><<<grid, 256, 0, st>>>(data, scales, zeros, scale_dtype, words, out);
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+    return bits == 2 ? launch_rows(tq_rows_dequantize_values_kernel<2>, grid, 256, 0, st, data, scales, zeros, (int)scale_dtype, quads, out)
+                     : launch_rows(tq_rows_dequantize_values_kernel<4>, grid, 256, 0, st, data, scales, zeros, (int)scale_dtype, quads, out);
 }
 
 extern "C" int tq_rows_quantize_keys(const tq_consts* consts, const void* x, tq_dtype dtype, int64_t n_rows, int64_t stride_row, uint8_t* codes,
@@ -795,20 +908,18 @@ extern "C" int tq_rows_quantize_keys(const tq_consts* consts, const void* x, tq_
     p.norm_dt = norm_dtype;
     p.rnorm_dt = residual_dtype;
     cudaStream_t st = (cudaStream_t)stream;
-    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
-    constexpr size_t smem = 4 * R_MAT;
+    constexpr size_t smem = 4 * R_MAT + R_XCHG;
 #define TQ_QK(DT, MB)                                                                            \
     do {                                                                                         \
         static TqSmemOptIn opt_in;                                                               \
         if (tq_opt_in_smem(tq_rows_quantize_keys_kernel<DT, MB>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA; \
-        tq_rows_quantize_keys_kernel<DT, MB><<<rows_grid(n_rows), R_WARPS * 32, smem, st>>>(p);   \
+        return launch_rows(tq_rows_quantize_keys_kernel<DT, MB>, dim3(rows_grid(n_rows)), R_THREADS, smem, st, p); \
     } while (0)
     const int mb = consts->cfg.key_bits - 1;
     if (dtype == TQ_F32) { if (mb == 2) TQ_QK(TQ_F32, 2); else TQ_QK(TQ_F32, 3); }
-    else if (dtype == TQ_F16) { if (mb == 2) TQ_QK(TQ_F16, 2); else TQ_QK(TQ_F16, 3); }
-    else return TQ_ERR_UNSUPPORTED;
+    if (dtype == TQ_F16) { if (mb == 2) TQ_QK(TQ_F16, 2); else TQ_QK(TQ_F16, 3); }
 #undef TQ_QK
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+    return TQ_ERR_UNSUPPORTED;
 }
 
 extern "C" int tq_rows_dequantize_keys(const tq_consts* consts, const uint8_t* codes, const uint8_t* signs, const void* norms, tq_dtype norm_dtype,
@@ -833,22 +944,17 @@ extern "C" int tq_rows_dequantize_keys(const tq_consts* consts, const uint8_t* c
     p.with_qjl = with_qjl;
     p.out = out;
     cudaStream_t st = (cudaStream_t)stream;
-    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
     const int mb = consts->cfg.key_bits - 1;
-    if (consts->cfg.head_dim != RD) {
-        tq_rows_dequantize_keys256_kernel<<<(unsigned)((n_rows + 15) / 16), 256, 0, st>>>(p, consts->pi, consts->s, mb);
-        return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
-    }
-    constexpr size_t smem = 4 * R_MAT + 16 * sizeof(float);
+    if (consts->cfg.head_dim != RD)
+        return launch_rows(tq_rows_dequantize_keys256_kernel, dim3((unsigned)((n_rows + 15) / 16)), 256, 0, st, p, (const float*)consts->pi, (const float*)consts->s, mb);
+    constexpr size_t smem = 4 * R_MAT + KSTEPS * R_THREADS * sizeof(float4) + 16 * sizeof(float);
     static TqSmemOptIn opt2, opt3;
     if (mb == 2) {
         if (tq_opt_in_smem(tq_rows_dequantize_keys_kernel<2>, smem, opt2) != TQ_OK) return TQ_ERR_CUDA;
-        tq_rows_dequantize_keys_kernel<2><<<rows_grid(n_rows), R_WARPS * 32, smem, st>>>(p);
-    } else {
-        if (tq_opt_in_smem(tq_rows_dequantize_keys_kernel<3>, smem, opt3) != TQ_OK) return TQ_ERR_CUDA;
-        tq_rows_dequantize_keys_kernel<3><<<rows_grid(n_rows), R_WARPS * 32, smem, st>>>(p);
+        return launch_rows(tq_rows_dequantize_keys_kernel<2>, dim3(rows_grid(n_rows)), R_THREADS, smem, st, p);
     }
-    return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+    if (tq_opt_in_smem(tq_rows_dequantize_keys_kernel<3>, smem, opt3) != TQ_OK) return TQ_ERR_CUDA;
+    return launch_rows(tq_rows_dequantize_keys_kernel<3>, dim3(rows_grid(n_rows)), R_THREADS, smem, st, p);
 }
 
 extern "C" int tq_rows_scores(const tq_consts* consts, const uint8_t* codes, const uint8_t* signs, const void* norms, tq_dtype norm_dtype,
@@ -877,22 +983,21 @@ extern "C" int tq_rows_scores(const tq_consts* consts, const uint8_t* codes, con
     float* qprep = reinterpret_cast<float*>((uint8_t*)workspace + TQ_WS_HEADER_BYTES);
     cudaStream_t st = (cudaStream_t)stream;
     if ((rc = tq_prepare_queries(consts, query, q_dtype, (int64_t)n_heads * n_q, qprep, st)) != TQ_OK) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3((unsigned)((n_keys + 63) / 64), (unsigned)n_heads, (unsigned)((n_q + 7) / 8));
-    cfg.blockDim = dim3(128);
-    cfg.stream = st;
+    const int gp = n_q > 4 ? 8 : n_q > 2 ? 4 : n_q, vec = aligned(codes, 16) && aligned(signs, 8);
+    const dim3 grid((unsigned)((n_keys + 63) / 64), (unsigned)n_heads, (unsigned)((n_q + gp - 1) / gp));
+#define TQ_RS_(DD, MB, GP) return launch_rows(tq_rows_scores_kernel<DD, MB, GP>, grid, 128, 0, st, p, (const float*)qprep, n_keys, (int)n_q, vec, logits)
+#define TQ_RS(DD, MB)                      \
+    do {                                   \
+        if (gp == 1) TQ_RS_(DD, MB, 1);    \
+        if (gp == 2) TQ_RS_(DD, MB, 2);    \
+        if (gp == 4) TQ_RS_(DD, MB, 4);    \
+        TQ_RS_(DD, MB, 8);                 \
+    } while (0)
     const int mb = consts->cfg.key_bits - 1;
-    cudaError_t e;
-    if (consts->cfg.head_dim == 128)
-        e = mb == 2 ? cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<128, 2>, p, (const float*)qprep, n_keys, (int)n_q, logits)
-                    : cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<128, 3>, p, (const float*)qprep, n_keys, (int)n_q, logits);
-    else
-        e = mb == 2 ? cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<256, 2>, p, (const float*)qprep, n_keys, (int)n_q, logits)
-                    : cudaLaunchKernelEx(&cfg, tq_rows_scores_kernel<256, 3>, p, (const float*)qprep, n_keys, (int)n_q, logits);
-    return e == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+    if (consts->cfg.head_dim == 128 && mb == 2) TQ_RS(128, 2);
+    if (consts->cfg.head_dim == 128) TQ_RS(128, 3);
+    if (mb == 2) TQ_RS(256, 2);
+    TQ_RS(256, 3);
+#undef TQ_RS
+#undef TQ_RS_
 }

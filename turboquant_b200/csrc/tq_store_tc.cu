@@ -837,8 +837,13 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 // channels), each box used for every product that needs it while it is resident: Pi_hi for Y and E, Pi_lo
 // for Y, M_hi for r'_hi and r'_lo, M_lo for r'_hi - 512 KB from L2 per tile.  One tile in flight.
 // 3-bit keys with 2-bit values have 25 KB of record images and leave room for the two slots of 256 rows;
-// the wider records (33 or 41 KB) take a ring of three 16 KB boxes of 128 rows, every product in two
-// halves of 128 columns: the same number of tensor-core cycles and of bytes, 48 KB of them in flight.
+// the wider records (33 or 41 KB) take a ring of four or three 16 KB boxes of 128 rows, every product in two
+// halves of 128 columns: the same number of tensor-core cycles and of bytes, 64 or 48 KB of them in flight.
+// What bounds it is the chain of one tile: products, of which a box is a round trip of load, products and
+// commit, then the element-wise phases.  A warp that only loads keeps the boxes coming; with one warp for loads
+// and products each box was its own round trip (0.7 us a 16 KB box, on 32 CTAs as on 148).  8192 tokens of 4
+// heads back to back: 45.8 -> 38.5 us (3-bit keys, 2-bit values), 67.1 -> 52.2 (4-bit both); 4875 tokens with
+// 4-bit keys 42.4 -> 33.5.
 // They also keep the precision of the fp32 kernel, on which these widths ran before (with the products of the narrow records
 // codes next to a boundary came out wrong eleven times as often, sign bits next to zero eight times):
 //   * fp16 limbs in the place of bf16 ones, scaled clear of the subnormals by powers of two: 22 bits of Pi, r' and M;
@@ -846,35 +851,35 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
 //     accumulators of 128 channels each, P one of the high limbs and one of the rest, small products first, sums in fp32.
 //     Two accumulators of Y leave room for half of its columns beside E: the first half's r' limbs wait in registers
 //     until the products of the second have read u and e'.  A box holds 32 columns of each compute thread's 64.
-// Measured (5003 tokens, 4 heads, 4-bit keys, 2-bit values, with the gather in front): 376 us with the fp32 kernel, 120.5 with
-// the narrow records' products, 122.8 so; codes and sign bits that 64-bit arithmetic decides otherwise, of 384 million each with
+// Measured (5003 tokens, 4 heads, 4-bit keys, 2-bit values, with the gather in front, one warp for loads and products): 376 us
+// with the fp32 kernel, 120.5 with the narrow records' products, 122.8 so; codes and sign bits that 64-bit arithmetic decides otherwise, of 384 million each with
 // 4-bit keys: 127 and 394, 1390 and 3070, 106 and 331.
 // A compute thread (row, q) owns channels [64q, 64q+64): two value groups, one 128-byte row of a box.
 constexpr int D2 = 256;
 constexpr int D2_TILE_BYTES = 4 * BOX_BYTES;      // 128 rows x 256 bf16: four boxes
-template <int ROWS>
-struct D2Ring {                                   // boxes of ROWS rows x 64 bf16 of a constant operand
-    static constexpr int BYTES = ROWS * 128, SLOTS = ROWS == 256 ? 2 : 3;
-    static constexpr int HALVES = D2 / ROWS, PER_MAT = 4 * HALVES, CHUNKS = 4 * PER_MAT;
-    static constexpr int BOX_ROWS = ROWS == 256 ? 256 : 32;   // a slot of 128 rows: 32 of each 64
-};
+constexpr int D2_LAUNCH = TC_THREADS + 64;        // compute threads, the issuing warp, the loading warp
 template <int MSE_BITS, int VAL_BITS>
-constexpr int d2_ring_rows() { return MSE_BITS == 2 && VAL_BITS == 2 ? 256 : 128; }
+struct D2Ring {                                   // boxes of ROWS rows x 64 channels of a constant operand
+    static constexpr bool WIDE = MSE_BITS != 2 || VAL_BITS != 2;
+    static constexpr int ROWS = WIDE ? 128 : 256, BYTES = ROWS * 128;
+    static constexpr int SLOTS = !WIDE ? 2 : MSE_BITS == 3 && VAL_BITS == 4 ? 3 : 4;   // what the record image leaves room for
+    static constexpr int HALVES = D2 / ROWS, PER_MAT = 4 * HALVES, CHUNKS = 4 * PER_MAT;
+    static constexpr int BOX_ROWS = WIDE ? 32 : 256;   // a slot of 128 rows: 32 of each 64
+};
 // What the operands of the wide records carry: u, e' and Pi are 64 times theirs, so Y, E and r' are 4096 times.
 constexpr float D2_OP = 64.f, D2_ACC = D2_OP * D2_OP;
 __device__ __forceinline__ uint32_t pack_f16(float lo, float hi) {
     const __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
-constexpr int D2_BARS = 15;
-template <int ROWS>
+constexpr int D2_BARS = 17;
+template <class Ring>
 constexpr size_t d2_smem(size_t img) {
-    return 2 * (size_t)D2_TILE_BYTES + (size_t)D2Ring<ROWS>::SLOTS * D2Ring<ROWS>::BYTES + img + 4 * TC_TOK * sizeof(float) +
-           D2_BARS * sizeof(uint64_t) + 16 + 1024;
+    return 2 * (size_t)D2_TILE_BYTES + (size_t)Ring::SLOTS * Ring::BYTES + img + 4 * TC_TOK * sizeof(float) + D2_BARS * sizeof(uint64_t) + 16;
 }
 
-template <int MSE_BITS, int VAL_BITS, bool SCATTER, int ROWS = d2_ring_rows<MSE_BITS, VAL_BITS>()>
-__global__ void __launch_bounds__(TC_LAUNCH, 1)
+template <int MSE_BITS, int VAL_BITS, bool SCATTER>
+__global__ void __launch_bounds__(D2_LAUNCH, 1)
 tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                       const __grid_constant__ CUtensorMap tm_kt, const __grid_constant__ CUtensorMap tm_vt,
                       const __grid_constant__ CUtensorMap tm_b0, const __grid_constant__ CUtensorMap tm_b1,
@@ -882,12 +887,13 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                       const TcParams p) {
     const TqLayout L = tq_make_layout(D2, MSE_BITS + 1, VAL_BITS);
     const int BB = L.block_bytes;
-    using Ring = D2Ring<ROWS>;
-    constexpr bool F16 = MSE_BITS != 2 || VAL_BITS != 2;
+    using Ring = D2Ring<MSE_BITS, VAL_BITS>;
+    constexpr bool F16 = Ring::WIDE;
+    constexpr int ROWS = Ring::ROWS;
     constexpr float OP = F16 ? D2_OP : 1.f, ACC = F16 ? D2_ACC : 1.f;
 
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = smem_raw + ((1024u - (tq_smem_u32(smem_raw) & 1023u)) & 1023u);
+    extern __shared__ __align__(1024) uint8_t smem_aligned[];   // swizzled boxes
+    uint8_t* smem = smem_aligned;
     uint8_t* sA0 = smem;                              // key rows -> u -> r'_hi
     uint8_t* sA1 = sA0 + D2_TILE_BYTES;               // value rows -> e' -> r'_lo
     uint8_t* sBr = sA1 + D2_TILE_BYTES;               // the constant-operand ring
@@ -895,10 +901,10 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     float* s_ss = reinterpret_cast<float*>(sRec + 8 * BB);   // [4][128] partial sums of squares (x, then r')
     uint64_t* bars = reinterpret_cast<uint64_t*>(s_ss + 4 * TC_TOK);
     uint64_t *bar_k = bars, *bar_v = bars + 1, *bar_m1 = bars + 2, *bar_m2 = bars + 3, *bar_r = bars + 4;
-    uint64_t *bar_full = bars + 5, *bar_empty = bars + 8;     // [2 or 3] each: ring slot filled / its products done
-    uint64_t* bar_m1b = bars + 11;                            // F16: the second half of Y and E (bar_m1: the first)
-    uint64_t *bar_n = bars + 12, *bar_c = bars + 13;          // 512 arrivals: u, e' written / r' written
-    uint64_t* bar_y = bars + 14;                              // F16, 512 arrivals: the first half of Y has been read
+    uint64_t *bar_full = bars + 5, *bar_empty = bars + 9;     // [2 to 4] each: ring slot filled / its products done
+    uint64_t* bar_m1b = bars + 13;                            // F16: the second half of Y and E (bar_m1: the first)
+    uint64_t *bar_n = bars + 14, *bar_c = bars + 15;          // 512 arrivals: u, e' written / r' written
+    uint64_t* bar_y = bars + 16;                              // F16, 512 arrivals: the first half of Y has been read
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + D2_BARS);
     volatile int* s_fail = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -916,7 +922,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     }
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 12; ++i) tq_mbar_init(bars + i, 1);
+        for (int i = 0; i < 14; ++i) tq_mbar_init(bars + i, 1);
         tq_mbar_init(bar_n, TC_THREADS);
         tq_mbar_init(bar_c, TC_THREADS);
         tq_mbar_init(bar_y, TC_THREADS);
@@ -934,8 +940,10 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
     const int tile0 = blockIdx.x;
     const bool rmw = !slot_mode && p.lead != 0 && tile0 < p.H;
 
-    if (warp == TC_THREADS / 32) {
-        // =============================== issuing warp (uniform, one elected lane issues) ===============================
+    if (warp >= TC_THREADS / 32) {
+        // =============================== issuing and loading warp (uniform, one elected lane issues) ===============================
+        // Two warps, so that a slot is asked for again the moment its products are done while the next slot's products are
+        // already queued: with one warp for both every box was a round trip of products, commit and load by itself.
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
         auto wait1 = [&](uint64_t* bar, uint32_t parity) -> bool {
             uint32_t ok = 0;
@@ -944,7 +952,6 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                     ok = 1;
                     break;
                 }
-                __nanosleep(40);
                 if ((i & 255) == 255 && *s_fail) break;
             }
             ok = __all_sync(0xffffffffu, ok != 0);
@@ -983,8 +990,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
             const int cm = c % Ring::PER_MAT;
             return {c / Ring::PER_MAT, cm / Ring::HALVES, cm % Ring::HALVES};
         };
-        int g_loaded = 0;       // chunks requested so far, over all tiles of this CTA
-        auto load_chunk = [&](int c) -> bool {
+        auto load_chunk = [&](int c, int g_loaded) -> bool {   // g_loaded: chunks requested before, over all tiles of this CTA
             const int slot = g_loaded % Ring::SLOTS;
             const Chunk ch = chunk(c);
             if (g_loaded >= Ring::SLOTS && !wait1(bar_empty + slot, (g_loaded / Ring::SLOTS - 1) & 1)) return false;
@@ -1000,11 +1006,9 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 }
             }
             __syncwarp();
-            ++g_loaded;
             return true;
         };
-        int g_used = 0;
-        auto use_chunk = [&](int c) -> bool {   // issue every product that reads chunk c, then release its slot
+        auto use_chunk = [&](int c, int g_used) -> bool {   // issue every product that reads chunk c, then release its slot
             const int slot = g_used % Ring::SLOTS;
             const Chunk ch = chunk(c);
             const int mat = ch.mat, kc = ch.kc;
@@ -1044,46 +1048,52 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 if (c == Ring::CHUNKS - 1) umma_commit(bar_m2);
             }
             __syncwarp();
-            ++g_used;
             return true;
         };
 
-        issue_rows(sA0, &tm_k, &tm_kt, bar_k, tile0);
-        issue_rows(sA1, &tm_v, &tm_vt, bar_v, tile0);
-        if (rmw) {
-            pool_writes_may_begin();
-            if (elected()) {
-                const int64_t phys = p.block_table[p.start_pos >> 4];
-                if (phys >= 0 && phys < p.num_blocks) {
-                    tq_mbar_expect_tx(bar_r, (uint32_t)BB);
-                    tq_bulk_g2s(sRec, p.pool + (phys * p.H + tile_head(tile0)) * (int64_t)BB, (uint32_t)BB, bar_r);
-                } else {
-                    atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_RANGE);
-                    tq_mbar_expect_tx(bar_r, 0);
+        if (warp == TC_THREADS / 32) {
+            bool ok = true;
+            int i = 0, used = 0;
+#pragma unroll 1
+            for (int tile = tile0; tile < p.n_tiles && ok; tile += (int)gridDim.x, ++i) {
+                if (!(ok = wait1(bar_n, i & 1))) break;              // u, e' in shared memory
+#pragma unroll 1
+                for (int c = 0; c < Ring::CHUNKS && ok; ++c) {
+                    if (F16 && c == Ring::CHUNKS / 4 && !(ok = wait1(bar_y, i & 1))) break;   // Y's columns are free for its second half
+                    if (c == Ring::CHUNKS / 2 && !(ok = wait1(bar_c, i & 1))) break;   // r' limbs in shared memory
+                    ok = use_chunk(c, used++);
                 }
             }
-            __syncwarp();
-        }
-        bool ok = load_chunk(0) && load_chunk(1) && (Ring::SLOTS < 3 || load_chunk(2));
-        int i = 0;
-#pragma unroll 1
-        for (int tile = tile0; tile < p.n_tiles && ok; tile += (int)gridDim.x, ++i) {
-            const int next = tile + (int)gridDim.x;
-            if (!(ok = wait1(bar_n, i & 1))) break;              // u, e' in shared memory
-#pragma unroll 1
-            for (int c = 0; c < Ring::CHUNKS && ok; ++c) {
-                if (F16 && c == Ring::CHUNKS / 4 && !(ok = wait1(bar_y, i & 1))) break;   // Y's columns are free for its second half
-                if (c == Ring::CHUNKS / 2 && !(ok = wait1(bar_c, i & 1))) break;   // r' limbs in shared memory
-                ok = use_chunk(c);
-                // keep the ring full: the chunk SLOTS ahead (of this tile, or the first ones of the next tile)
-                const int ahead = c + Ring::SLOTS;
-                if (ok && (ahead < Ring::CHUNKS || next < p.n_tiles)) ok = load_chunk(ahead % Ring::CHUNKS);
+        } else {
+            issue_rows(sA0, &tm_k, &tm_kt, bar_k, tile0);
+            issue_rows(sA1, &tm_v, &tm_vt, bar_v, tile0);
+            if (rmw) {
+                pool_writes_may_begin();
+                if (elected()) {
+                    const int64_t phys = p.block_table[p.start_pos >> 4];
+                    if (phys >= 0 && phys < p.num_blocks) {
+                        tq_mbar_expect_tx(bar_r, (uint32_t)BB);
+                        tq_bulk_g2s(sRec, p.pool + (phys * p.H + tile_head(tile0)) * (int64_t)BB, (uint32_t)BB, bar_r);
+                    } else {
+                        atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_RANGE);
+                        tq_mbar_expect_tx(bar_r, 0);
+                    }
+                }
+                __syncwarp();
             }
-            if (!ok) break;
-            if (next < p.n_tiles) {
-                if (!(ok = wait1(bar_m2, i & 1))) break;         // the A tiles are free again
-                issue_rows(sA0, &tm_k, &tm_kt, bar_k, next);
-                issue_rows(sA1, &tm_v, &tm_vt, bar_v, next);
+            bool ok = true;
+            int i = 0, loaded = 0;
+#pragma unroll 1
+            for (int tile = tile0; tile < p.n_tiles && ok; tile += (int)gridDim.x, ++i) {
+#pragma unroll 1
+                for (int c = 0; c < Ring::CHUNKS && ok; ++c) {
+                    if (i > 0 && c == Ring::SLOTS - 1) {             // the last slot's products were the tile's last: the A tiles are free too
+                        if (!(ok = wait1(bar_m2, (i - 1) & 1))) break;
+                        issue_rows(sA0, &tm_k, &tm_kt, bar_k, tile);
+                        issue_rows(sA1, &tm_v, &tm_vt, bar_v, tile);
+                    }
+                    ok = load_chunk(c, loaded++);
+                }
             }
         }
     } else {
@@ -1500,7 +1510,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
         tm_kt = tm_k;
         tm_vt = tm_v;
     }
-    if (!maps_ok || !operand_maps(tm_b, limbs, D, d2_wide ? D2Ring<128>::BOX_ROWS : D))
+    if (!maps_ok || !operand_maps(tm_b, limbs, D, d2_wide ? D2Ring<3, 4>::BOX_ROWS : D))
         return TQ_OK;   // a stride pattern the tensor map cannot express: the fp32 kernel takes the call
     *handled = 1;
 
@@ -1522,11 +1532,11 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     cudaError_t launched = cudaSuccess;
     if (D == D2) {
         p.n_rec_buf = 1;
+        lc.blockDim = dim3(D2_LAUNCH);
 #define TQ_TC256_(MB, VB, SL)                                                                                         \
     do {                                                                                                         \
         static TqSmemOptIn opt_in;                                                                               \
-        const size_t smem = d2_smem<d2_ring_rows<MB, VB>()>(img);                                                \
-        static_assert(d2_ring_rows<2, 2>() == 256 && d2_ring_rows<2, 4>() == 128, "boxes of the operand maps");  \
+        const size_t smem = d2_smem<D2Ring<MB, VB>>(img);                                                        \
         if (tq_opt_in_smem(tq_store_tc256_kernel<MB, VB, SL>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA;            \
         lc.dynamicSmemBytes = smem;                                                                              \
         launched = cudaLaunchKernelEx(&lc, tq_store_tc256_kernel<MB, VB, SL>, tm_k, tm_v, tm_kt, tm_vt, tm_b[0], tm_b[1], \

@@ -225,6 +225,23 @@ int tq_store_paged(const tq_consts* consts, const void* key_cache, const void* v
                    int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t n_tokens,
                    const int32_t* block_table, int64_t start_pos, const tq_pool* pool, void* stream);
 
+/* The same for every bit width at head_dim 256 too (4-bit keys or values need
+ * the rows_pi / rows_m operands in `consts`). */
+int tq_store_paged_any(const tq_consts* consts, const void* key_cache, const void* value_cache, tq_dtype dtype,
+                       int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int64_t stride_block,
+                       int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t n_tokens,
+                       const int32_t* block_table, int64_t start_pos, const tq_pool* pool, void* stream);
+
+/* `n_tokens` tokens from position `first_token` of a sequence in such a cache
+ * (any block size, any dtype) into the ring at `position`, key and value in one
+ * launch; a token whose block index is out of range is left out and reported by
+ * tq_store_read_status.  Planes, strides and rows 16-byte aligned. */
+int tq_ring_write_paged(const void* key_cache, const void* value_cache, tq_dtype dtype, int64_t src_num_blocks,
+                        int32_t src_block_size, int32_t n_heads, int32_t head_dim, int64_t stride_block,
+                        int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t first_token,
+                        int64_t n_tokens, void* ring_k, void* ring_v, int64_t ring_stride_token, int64_t position,
+                        void* stream);
+
 /* Status left by the tensor-core store kernels since the last call: 0, or
  * TQ_ERR_TIMEOUT / TQ_ERR_RANGE if one of their bounded waits ran out or a
  * block index (destination or paged source) was out of range - such a

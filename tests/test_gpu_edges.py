@@ -141,3 +141,56 @@ def test_value_rows_for_any_number_of_groups(d, bits, dtype, dev):
         s64, z64 = (t.view(n, -1).half().double().repeat_interleave(32, -1) for t in (out.scales, out.zeros))
         want = code.double() * s64 + z64
         assert float((dequantize_values(out).view(n, d).double() - want).abs().max()) <= 2.0 ** -22 * float(want.abs().max() + s64.max() * (2 ** bits))
+
+
+@pytest.mark.parametrize("kb,vb", [(4, 2), (3, 4), (4, 4)])
+@pytest.mark.parametrize("n", [1, 127, 129, 700])
+def test_d256_wide_records_from_a_paged_cache(kb, vb, n, dev):
+    """The table-walking launch writes what the launch on gathered rows writes; without `any_width` it is refused as before."""
+    from turboquant_b200 import CompressedKVStore, _engine as E
+    h, bs, d = 3, 16, 256
+    g = torch.Generator(device=dev).manual_seed(n)
+    used = (n + bs - 1) // bs
+    table = torch.randperm(used + 5, generator=g, device=dev)[:used].int()
+    cache = torch.randn(2, used + 5, bs, h, d, generator=g, device=dev, dtype=torch.bfloat16)
+    k, v = (cache[i][table.long()].flatten(0, 1)[:n] for i in range(2))
+    a = CompressedKVStore(d, h, kb, vb, device=dev, capacity_tokens=n)
+    a.append_chunk(k, v)
+    pool = E.BlockPool(a.consts, h, E.blocks_for(n))
+    args = dict(src_block_table=table, n_tokens=n, block_table=E.identity_block_table(E.blocks_for(n), dev))
+    assert not E.store_paged(a.consts, pool, cache[0], cache[1], **args)
+    assert E.store_paged(a.consts, pool, cache[0], cache[1], any_width=True, **args)
+    size = E.blocks_for(n) * h * a.consts.block_bytes
+    assert torch.equal(pool.data[:size], a.pool.data[:size]) and E.store_status() == 0
+
+
+@pytest.mark.parametrize("bs", [1, 5, 16, 48])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_ring_is_filled_from_a_paged_cache(bs, dtype, dev):
+    """The last tokens of a prompt, into an empty ring and behind tokens that it holds; a full ring or a table of another type
+    takes the general way with the same result."""
+    from turboquant_b200 import CompressedKVStore, KVCaptureEngine
+    h, d, cap = 2, 128, 32
+    g = torch.Generator(device=dev).manual_seed(bs)
+    for n, held, wide in ((1, 0, False), (31, 0, False), (32, 0, True), (20, 12, False), (20, 13, False), (75, 0, False), (75, 3, False)):
+        used = (n + bs - 1) // bs
+        table = torch.randperm(used + 3, generator=g, device=dev)[:used].to(torch.int64 if wide else torch.int32)
+        cache = torch.randn(2, used + 3, bs, h, d, generator=g, device=dev).to(dtype)
+        k, v = (cache[i][table.long()].flatten(0, 1)[:n] for i in range(2))
+        k0, v0 = (torch.randn(max(held, 1), h, d, generator=g, device=dev).to(dtype) for _ in range(2))
+        both = []
+        for paged in (True, False):
+            e = KVCaptureEngine(CompressedKVStore(d, h, 3, 2, device=dev), ring_capacity=cap, device=dev, dtype=dtype)
+            if held:
+                e.ring.write(k0[:held], v0[:held], held)
+            if paged:
+                e.ingest_prefill_from_paged_cache(cache, n, table, bs)
+            else:
+                m = max(n - cap, 0)
+                if m:
+                    e.store.append_chunk(k[:m], v[:m])
+                e.ring.write(k[m:], v[m:], n - m)
+            both.append(e)
+        a, b = both
+        assert (a.ring.size, a.ring.total_written, a.store.num_tokens) == (b.ring.size, b.ring.total_written, b.store.num_tokens)
+        assert all(torch.equal(x, y) for x, y in zip(a.ring.peek(), b.ring.peek())), (n, held)

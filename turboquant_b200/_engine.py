@@ -291,13 +291,15 @@ def store(consts: LayerConstants, pool: BlockPool, key: torch.Tensor, value: tor
 
 
 def store_paged(consts: LayerConstants, pool: BlockPool, key_cache: torch.Tensor, value_cache: torch.Tensor, *,
-                src_block_table: torch.Tensor, n_tokens: int, block_table: torch.Tensor, start_pos: int = 0) -> bool:
+                src_block_table: torch.Tensor, n_tokens: int, block_table: torch.Tensor, start_pos: int = 0,
+                any_width: bool = False) -> bool:
     """Compress the first n_tokens tokens of a sequence held in a paged cache.
 
     key_cache / value_cache: (num_blocks, block_size, H, D) views (any block / token / head strides, D
     contiguous, same strides for both); src_block_table: int32 device tensor, logical -> physical block.
     Returns False, with nothing launched, when the call does not fit the table-walking tensor-core
-    kernel (the caller then gathers the rows and uses `store`).
+    kernel (the caller then gathers the rows and uses `store`).  any_width: take head_dim 256 with 4-bit
+    keys or values too.
     """
     require_cuda(key_cache, "key_cache")
     require_cuda(value_cache, "value_cache")
@@ -309,13 +311,34 @@ def store_paged(consts: LayerConstants, pool: BlockPool, key_cache: torch.Tensor
     nb, bs, h, _ = key_cache.shape
     if n_tokens > src_block_table.numel() * bs:
         raise ValueError("src_block_table is shorter than n_tokens")
-    rc = lib().tq_store_paged(C.byref(consts.c), key_cache.data_ptr(), value_cache.data_ptr(), dtype_code(key_cache.dtype),
-                              nb, bs, h, key_cache.stride(0), key_cache.stride(1), key_cache.stride(2),
-                              src_block_table.data_ptr(), n_tokens, block_table.data_ptr(), start_pos,
-                              C.byref(pool.c), stream_ptr(consts.device))
+    fn = lib().tq_store_paged_any if any_width else lib().tq_store_paged
+    rc = fn(C.byref(consts.c), key_cache.data_ptr(), value_cache.data_ptr(), dtype_code(key_cache.dtype), nb, bs, h,
+            key_cache.stride(0), key_cache.stride(1), key_cache.stride(2), src_block_table.data_ptr(), n_tokens,
+            block_table.data_ptr(), start_pos, C.byref(pool.c), stream_ptr(consts.device))
     if rc == _lib.TQ_ERR_UNSUPPORTED:
         return False
     check(rc, "tq_store_paged")
+    return True
+
+
+def ring_write_paged(ring_k: torch.Tensor, ring_v: torch.Tensor, position: int, key_cache: torch.Tensor, value_cache: torch.Tensor,
+                     src_block_table: torch.Tensor, first: int, n: int) -> bool:
+    """Tokens [first, first + n) of a sequence in a paged cache ((num_blocks, block_size, H, D) planes of one layout,
+    `src_block_table` int32, contiguous) into the ring's buffers from `position` on, in one launch.  False, with nothing
+    launched, for tensors that the kernel does not take."""
+    nb, bs, h, d = key_cache.shape
+    if not (key_cache.is_cuda and ring_k.device == key_cache.device == value_cache.device == src_block_table.device
+            and ring_k.dtype == key_cache.dtype == value_cache.dtype and key_cache.dtype in _DTYPES
+            and key_cache.stride() == value_cache.stride() and key_cache.shape == value_cache.shape and key_cache.stride(3) == 1
+            and min(key_cache.stride()) >= 0 and tuple(ring_k.shape[1:]) == (h, d) and src_block_table.dtype == torch.int32
+            and src_block_table.is_contiguous() and first + n <= src_block_table.numel() * bs and position + n <= ring_k.shape[0]):
+        return False
+    rc = lib().tq_ring_write_paged(key_cache.data_ptr(), value_cache.data_ptr(), _DTYPES[key_cache.dtype], nb, bs, h, d, key_cache.stride(0),
+                                   key_cache.stride(1), key_cache.stride(2), src_block_table.data_ptr(), first, n, ring_k.data_ptr(),
+                                   ring_v.data_ptr(), ring_k.stride(0), position, stream_ptr(ring_k.device))
+    if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
+        return False
+    check(rc, "tq_ring_write_paged")
     return True
 
 

@@ -81,6 +81,12 @@ SIGNATURES = {
     "tq_store_paged": (C.c_int, [C.POINTER(tq_consts), C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int32,
                                  C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64,
                                  C.POINTER(tq_pool), C.c_void_p]),
+    "tq_store_paged_any": (C.c_int, [C.POINTER(tq_consts), C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int32,
+                                     C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_int64, C.c_void_p, C.c_int64,
+                                     C.POINTER(tq_pool), C.c_void_p]),
+    "tq_ring_write_paged": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int64,
+                                      C.c_int64, C.c_int64, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p,
+                                      C.c_int64, C.c_int64, C.c_void_p]),
     "tq_store_read_status": (C.c_int, [C.POINTER(C.c_int32)]),
     "tq_prefill_attention": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int64, C.c_int32,
                                        C.c_int32, C.c_int32, C.c_int64, C.c_int64, C.c_int64, C.c_int64, C.c_int64,

@@ -96,6 +96,19 @@ class RingBuffer:
         self._fill = stay
         return out_k, out_v
 
+    def write_from_paged(self, key_cache: torch.Tensor, value_cache: torch.Tensor, block_table: torch.Tensor, first: int,
+                         num_tokens: int) -> bool:
+        """`write` of tokens [first, first + num_tokens) of a sequence in a paged cache, where nothing is evicted and the
+        tensors are the kernel's; False, with nothing changed, otherwise."""
+        held = self._fill
+        if num_tokens <= 0 or held + num_tokens > self.capacity or not self._keys.is_cuda:
+            return False
+        if not E.ring_write_paged(self._keys, self._values, held, key_cache, value_cache, block_table, first, num_tokens):
+            return False
+        self._fill = held + num_tokens
+        self._seen += num_tokens
+        return True
+
     def drain(self):
         """Everything held, as copies; the ring is empty afterwards."""
         if self._fill == 0:
@@ -162,7 +175,11 @@ class KVCaptureEngine:
             raise ValueError(f"block_size {block_size} does not match the cache's {kv_cache_tensor.shape[2]}")
         cap = self.ring.capacity
         n = max(num_tokens - cap, 0)
-        self.store.append_from_paged(kv_cache_tensor[0], kv_cache_tensor[1], block_table, n)
+        keys, values = kv_cache_tensor[0], kv_cache_tensor[1]
+        self.store.append_from_paged(keys, values, block_table, n)
+        if self.ring.write_from_paged(keys, values, block_table, n, num_tokens - n):
+            self._prefill_done = True
+            return
         b0, b1 = n // block_size, (num_tokens + block_size - 1) // block_size
         phys = block_table[b0:b1].long()
         lo = n - b0 * block_size

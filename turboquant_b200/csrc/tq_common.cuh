@@ -257,6 +257,7 @@ struct TqPagedSource {
     int64_t num_blocks;      // physical blocks in the cache
     int32_t block_size;      // tokens per block
     int64_t stride_block;    // elements between blocks
+    bool any_width;          // head_dim 256 with 4-bit keys or values too
 };
 
 struct TqSmemOptIn {

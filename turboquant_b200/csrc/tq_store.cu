@@ -346,11 +346,11 @@ extern "C" int tq_store(const tq_consts* consts, const void* key, const void* va
 #undef TQ_LAUNCH
 }
 
-extern "C" int tq_store_paged(const tq_consts* consts, const void* key_cache, const void* value_cache, tq_dtype dtype,
-                              int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int64_t stride_block,
-                              int64_t stride_token, int64_t stride_head, const int32_t* src_block_table,
-                              int64_t n_tokens, const int32_t* block_table, int64_t start_pos, const tq_pool* pool,
-                              void* stream) {
+static int store_paged(const tq_consts* consts, const void* key_cache, const void* value_cache, tq_dtype dtype,
+                       int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int64_t stride_block,
+                       int64_t stride_token, int64_t stride_head, const int32_t* src_block_table,
+                       int64_t n_tokens, const int32_t* block_table, int64_t start_pos, const tq_pool* pool,
+                       void* stream, bool any_width) {
     if (!consts || !key_cache || !value_cache || !src_block_table || !block_table || !pool || !pool->base)
         return TQ_ERR_NULL;
     int rc = tq_check_config(&consts->cfg);
@@ -365,9 +365,28 @@ extern "C" int tq_store_paged(const tq_consts* consts, const void* key_cache, co
     src.num_blocks = src_num_blocks;
     src.block_size = src_block_size;
     src.stride_block = stride_block;
+    src.any_width = any_width;
     int handled = 0;
     rc = tq_store_tc_launch(consts, key_cache, value_cache, dtype, n_tokens, n_heads, stride_token, stride_head, nullptr,
                             block_table, start_pos, pool, (cudaStream_t)stream, &handled, &src);
     if (rc != TQ_OK) return rc;
     return handled ? TQ_OK : TQ_ERR_UNSUPPORTED;
+}
+
+extern "C" int tq_store_paged(const tq_consts* consts, const void* key_cache, const void* value_cache, tq_dtype dtype,
+                              int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int64_t stride_block,
+                              int64_t stride_token, int64_t stride_head, const int32_t* src_block_table,
+                              int64_t n_tokens, const int32_t* block_table, int64_t start_pos, const tq_pool* pool,
+                              void* stream) {
+    return store_paged(consts, key_cache, value_cache, dtype, src_num_blocks, src_block_size, n_heads, stride_block, stride_token, stride_head,
+                       src_block_table, n_tokens, block_table, start_pos, pool, stream, false);
+}
+
+extern "C" int tq_store_paged_any(const tq_consts* consts, const void* key_cache, const void* value_cache, tq_dtype dtype,
+                                  int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int64_t stride_block,
+                                  int64_t stride_token, int64_t stride_head, const int32_t* src_block_table,
+                                  int64_t n_tokens, const int32_t* block_table, int64_t start_pos, const tq_pool* pool,
+                                  void* stream) {
+    return store_paged(consts, key_cache, value_cache, dtype, src_num_blocks, src_block_size, n_heads, stride_block, stride_token, stride_head,
+                       src_block_table, n_tokens, block_table, start_pos, pool, stream, true);
 }

@@ -1445,7 +1445,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     const TqLayout L = tq_make_layout(D, cfg.key_bits, cfg.value_bits);
     const size_t img = (size_t)8 * L.block_bytes;
     const bool d2_wide = D == D2 && (cfg.key_bits != 3 || cfg.value_bits != 2);   // records of 33 or 41 KB a tile
-    if (paged && d2_wide) return TQ_OK;   // tq_store_paged answers "not supported" for these; its callers gather first
+    if (paged && d2_wide && !paged->any_width) return TQ_OK;   // tq_store_paged answers "not supported" for these
     // wide records: fp16 limbs of 64 Pi and M; elsewhere bf16 limbs
     const void* const* pi = d2_wide ? consts->rows_pi : consts->pi_limbs;
     const void* const* m = d2_wide ? consts->rows_m : consts->m_limbs;
@@ -1570,6 +1570,65 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
 #undef TQ_TC
 #undef TQ_TC_
     return launched == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}
+
+namespace {
+// The last tokens of a prompt from its paged cache into the ring, key and value in one launch.  Bound by its launch (128 tokens
+// of 4 heads x 256 are 512 KB): two gathers, a conversion of the table and a ring write took 15 us of the device and 40 of the host.
+__global__ void __launch_bounds__(256) tq_ring_gather_kernel(const char* __restrict__ k, const char* __restrict__ v, const int32_t* __restrict__ table,
+                                                             int64_t num_blocks, int block_size, int row16, int n_heads, int64_t first, int64_t total,
+                                                             int64_t src_block, int64_t src_token, int64_t src_head, char* __restrict__ rk,
+                                                             char* __restrict__ rv, int64_t dst_token) {
+    // the ring may still be read by the launch ahead; only then may the next one begin (it reads pool and tables early)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;   // (token, head, 16-byte chunk)
+    if (i >= total) return;
+    const int c = (int)(i % row16);
+    const int h = (int)((i / row16) % n_heads);
+    const int64_t t = i / ((int64_t)row16 * n_heads), tok = first + t;
+    const int64_t phys = table[tok / block_size];
+    if (phys < 0 || phys >= num_blocks) {
+        atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_RANGE);
+        return;
+    }
+    const int64_t src = phys * src_block + tok % block_size * src_token + h * src_head + 16 * c;
+    const int64_t dst = t * dst_token + ((int64_t)h * row16 + c) * 16;
+    const uint4 a = *reinterpret_cast<const uint4*>(k + src), b = *reinterpret_cast<const uint4*>(v + src);
+    *reinterpret_cast<uint4*>(rk + dst) = a;
+    *reinterpret_cast<uint4*>(rv + dst) = b;
+}
+}  // namespace
+
+extern "C" int tq_ring_write_paged(const void* key_cache, const void* value_cache, tq_dtype dtype, int64_t src_num_blocks,
+                                   int32_t src_block_size, int32_t n_heads, int32_t head_dim, int64_t stride_block,
+                                   int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t first_token,
+                                   int64_t n_tokens, void* ring_k, void* ring_v, int64_t ring_stride_token, int64_t position,
+                                   void* stream) {
+    if (!key_cache || !value_cache || !src_block_table || !ring_k || !ring_v) return TQ_ERR_NULL;
+    if (src_num_blocks <= 0 || src_block_size <= 0 || n_heads <= 0 || head_dim <= 0 || first_token < 0 || n_tokens <= 0 || position < 0)
+        return TQ_ERR_SHAPE;
+    if (n_tokens > (1 << 20) || n_heads > (1 << 12)) return TQ_ERR_UNSUPPORTED;
+    const int64_t eb = (int64_t)tq_dtype_size(dtype);
+    if (((uintptr_t)key_cache | (uintptr_t)value_cache | (uintptr_t)ring_k | (uintptr_t)ring_v | (uintptr_t)(stride_block * eb) |
+         (uintptr_t)(stride_token * eb) | (uintptr_t)(stride_head * eb) | (uintptr_t)(ring_stride_token * eb) | (uintptr_t)(head_dim * eb)) & 15)
+        return TQ_ERR_ALIGN;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int row16 = (int)(head_dim * eb / 16);
+    const int64_t total = n_tokens * n_heads * row16, off = position * ring_stride_token * eb;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((total + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    tq_note_launch(st, TQ_LAUNCH_DECODE);   // a store behind it may be about to read the ring
+    return cudaLaunchKernelEx(&cfg, tq_ring_gather_kernel, (const char*)key_cache, (const char*)value_cache, src_block_table, src_num_blocks,
+                              (int)src_block_size, row16, (int)n_heads, first_token, total, stride_block * eb, stride_token * eb, stride_head * eb,
+                              (char*)ring_k + off, (char*)ring_v + off, ring_stride_token * eb) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
 }
 
 // Status left by the tensor-core store kernels since the last call (0, or a tq_status if a bounded wait ran

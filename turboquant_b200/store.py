@@ -113,7 +113,7 @@ class CompressedKVStore:
         self.reserve(self._num_tokens + num_tokens)
         table = src_block_table.to(device=self.device, dtype=torch.int32).contiguous()
         if not E.store_paged(self.consts, self.pool, key_cache, value_cache, src_block_table=table,
-                             n_tokens=num_tokens, block_table=self.block_table, start_pos=self._num_tokens):
+                             n_tokens=num_tokens, block_table=self.block_table, start_pos=self._num_tokens, any_width=True):
             bs = key_cache.shape[1]
             phys = table[:(num_tokens + bs - 1) // bs].long()
             k = key_cache.index_select(0, phys).flatten(0, 1)[:num_tokens]

@@ -129,6 +129,35 @@ __device__ __forceinline__ RecUnit rec_unit(const TqLayout& L, int u) {
 }
 constexpr int REC_UNITS_MAX = (128 + 32 + 4 + 128 + 32) / 2;   // head_dim 256, four bits each
 
+// Two fp32 numbers in a register pair: one instruction for both, each rounded as by itself.  These kernels are bound by the
+// instructions they issue, not by the fp32 pipes: with everything that is not a saturating step in pairs, and one saturating
+// product for a sign bit in the place of two, 8192 tokens of 8 heads x 128 back to back 19.9 -> 18.7 us (3-bit keys, 2-bit
+// values), 26.7 -> 24.6 (4-bit both), of 4 heads x 256 38.5 -> 37.2 and 52.2 -> 48.7.  The records are the same bytes.
+struct F2 {
+    uint64_t v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+
 // ---------------------------------------------------------------------------
 // Values: asymmetric min/max quantisation of ONE 32-channel group of one row in
 // bf16 arithmetic (kv_cache.py:64-90), on packed pairs.
@@ -165,7 +194,9 @@ __device__ __forceinline__ void quantize_value_group(const uint4 (&raw)[4], uint
     for (int i = 0; i < 16; ++i) {
         const uint32_t d = as_u32(__hsub2(as_bf162(w[i]), zero2));
         // z <= levels * (1 + 2^-7) < levels + 1/2: the rounding below cannot leave the field
-        const __nv_bfloat162 z = as_bf162(pack_bf16(bf_lo(d) * rscale, bf_hi(d) * rscale));
+        float za, zb;
+        unpack(mul2(f2(bf_lo(d), bf_hi(d)), f2(rscale, rscale)), za, zb);
+        const __nv_bfloat162 z = as_bf162(pack_bf16(za, zb));
         code[i] = as_u32(__hadd2(z, magic)) & FIELD;
     }
     if (!wr) return;
@@ -191,7 +222,7 @@ __device__ __forceinline__ void quantize_value_group(const uint4 (&raw)[4], uint
 // bit logic run at half rate and would bound this kernel.  For finite a:
 //     step_gt(a, BIG, -b * BIG) = saturate((a - b) * 2^126)  is exactly 1 when a > b and exactly 0 when
 // a <= b, as long as |a - b| is either 0 or at least 2^-126 - true for every boundary that is not itself
-// tiny; the second saturating multiply of step_gt2 extends that to every float (2^-149 * 2^252 >= 1).
+// tiny.
 // NaN saturates to 0.
 constexpr float BIG = 8.507059173023462e37f;   // 2^126
 __device__ __forceinline__ float fma_sat(float a, float b, float c) {
@@ -199,35 +230,42 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
-__device__ __forceinline__ float mul_sat(float a, float b) {
+// The same with subnormal numbers taken for 0, so that 0 and 1 are the only results where a sum of products may come
+// next to zero without reaching it (the middle boundary, sign bits): the sums have steps far above 2^-126.
+__device__ __forceinline__ float fma_sat_ftz(float a, float b, float c) {
     float d;
-    asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    asm("fma.rn.ftz.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float mul_sat_ftz(float a, float b) {
+    float d;
+    asm("mul.rn.ftz.sat.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
     return d;
 }
 
-// The code book prepared for that arithmetic (registers): nb[i] = -boundary[i] * 2^126, c0 = centroid[0],
-// step[i] = centroid[i+1] - centroid[i].
+// The code book prepared for that arithmetic (registers): nb[i] = -boundary[i] * 2^126, c0 = -centroid[0],
+// step[i] = centroid[i] - centroid[i+1].
 template <int MSE_BITS>
 struct BookRegs {
     float nb[(1 << MSE_BITS) - 1], step[(1 << MSE_BITS) - 1], c0;
 };
 
-// Bucket search of one rotated coordinate y (torch.searchsorted on the interior boundaries, left: the
-// code is the number of boundaries below y) and y minus its centroid.  `code` comes back as a float.
+// Bucket search of two rotated coordinates (torch.searchsorted on the interior boundaries, left: the
+// code is the number of boundaries below y) and what is left of them without their centroids.  Codes come back as floats.
 // SCALE: y, c0 and the steps are this power of two times theirs, the boundaries in nb are not.
 template <int MSE_BITS, int SCALE = 1>
-__device__ __forceinline__ void bucket(const BookRegs<MSE_BITS>& bk, float y, float& code, float& y_minus_c) {
+__device__ __forceinline__ void bucket2(const BookRegs<MSE_BITS>& bk, float& ya, float& yb, float& code_a, float& code_b) {
     constexpr int NB = (1 << MSE_BITS) - 1, MID = NB / 2;   // the middle boundary is (next to) zero
-    float k = 0.f, r = y - bk.c0;
+    F2 k, r = add2(f2(ya, yb), f2(bk.c0, bk.c0));
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
-        float t = fma_sat(y, BIG / SCALE, bk.nb[i]);
-        if (i == MID) t = mul_sat(t, BIG);
-        k += t;
-        r = fmaf(-t, bk.step[i], r);
+        const F2 t = i == MID ? f2(fma_sat_ftz(ya, BIG / SCALE, bk.nb[i]), fma_sat_ftz(yb, BIG / SCALE, bk.nb[i]))
+                              : f2(fma_sat(ya, BIG / SCALE, bk.nb[i]), fma_sat(yb, BIG / SCALE, bk.nb[i]));
+        k = i == 0 ? t : add2(k, t);
+        r = fma2(t, f2(bk.step[i], bk.step[i]), r);
     }
-    code = k;
-    y_minus_c = r;
+    unpack(k, code_a, code_b);
+    unpack(r, ya, yb);
 }
 
 // Destination of one image block (16 rows) of a tile: asked for early, looked at when the records leave
@@ -616,11 +654,11 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
         const int blk_l = row >> 4, tl = row & 15;
         const uint32_t lane_base = (uint32_t)(row & ~31) << 16;   // this warp's quarter of the 128 TMEM lanes
         BookRegs<MSE_BITS> bk;   // the code book, in registers
-        bk.c0 = p.cb.centroids[0];
+        bk.c0 = -p.cb.centroids[0];
 #pragma unroll
         for (int i = 0; i < (1 << MSE_BITS) - 1; ++i) {
             bk.nb[i] = -p.cb.boundaries[i] * BIG;
-            bk.step[i] = p.cb.centroids[i + 1] - p.cb.centroids[i];
+            bk.step[i] = p.cb.centroids[i] - p.cb.centroids[i + 1];
         }
         bool bad = false;      // one of this warp's waits ran out; reported at the next compute barrier
         float nd = 0.f;        // |x| of this thread's row in the input dtype, from N to S of the same tile
@@ -653,10 +691,13 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
             for (int i = 0; i < 16; ++i) {
                 // numerator and denominator are bf16 numbers: the product with the reciprocal rounds to
                 // the same bf16 as the division (see quantize_value_group)
-                const float q0 = bf_lo(xw[i]) * rden, q1 = bf_hi(xw[i]) * rden;
+                const F2 q2 = mul2(f2(bf_lo(xw[i]), bf_hi(xw[i])), f2(rden, rden));
+                float q0, q1;
+                unpack(q2, q0, q1);
                 const uint32_t u = pack_bf16(q0, q1);
                 up[i] = u;
-                ep[i] = pack_bf16(q0 - bf_lo(u), q1 - bf_hi(u));   // what the bf16 normalisation lost
+                unpack(fma2(f2(bf_lo(u), bf_hi(u)), f2(-1.f, -1.f), q2), q0, q1);
+                ep[i] = pack_bf16(q0, q1);   // what the bf16 normalisation lost
             }
             tmem_st16(tmem + lane_base + COL_U + q * 16, up);
             tmem_st16(tmem + lane_base + COL_EP + q * 16, ep);
@@ -721,10 +762,11 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 for (int w = 0; w < 32 / PER_HALF; ++w) {
                     float wf = 0.f;
 #pragma unroll
-                    for (int jj = 0; jj < PER_HALF; ++jj) {
-                        float code;
-                        bucket<MSE_BITS>(bk, y[w * PER_HALF + jj], code, y[w * PER_HALF + jj]);   // quantizer.py:144
-                        wf = fmaf(code, (float)(1u << (WIDTH * jj)), wf);
+                    for (int jj = 0; jj < PER_HALF; jj += 2) {
+                        float ca, cb;
+                        bucket2<MSE_BITS>(bk, y[w * PER_HALF + jj], y[w * PER_HALF + jj + 1], ca, cb);   // quantizer.py:144
+                        wf = fmaf(ca, (float)(1u << (WIDTH * jj)), wf);
+                        wf = fmaf(cb, (float)(1u << (WIDTH * (jj + 1))), wf);
                     }
                     halves[w] = __float_as_uint(wf + 8388608.f) & 0xffffu;   // 2^23 + integer: the integer sits in the mantissa
                 }
@@ -741,12 +783,15 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 uint32_t hi[16], lo[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const float a = y[2 * i] + er[2 * i], b = y[2 * i + 1] + er[2 * i + 1];   // r' = (Y - c) + E
+                    const F2 s2 = add2(f2(y[2 * i], y[2 * i + 1]), f2(er[2 * i], er[2 * i + 1]));   // r' = (Y - c) + E
+                    float a, b;
+                    unpack(s2, a, b);
                     rn2 = fmaf(a, a, rn2);
                     rn2 = fmaf(b, b, rn2);
                     const uint32_t hh = pack_bf16(a, b);
                     hi[i] = hh;
-                    lo[i] = pack_bf16(a - bf_lo(hh), b - bf_hi(hh));
+                    unpack(fma2(f2(bf_lo(hh), bf_hi(hh)), f2(-1.f, -1.f), s2), a, b);
+                    lo[i] = pack_bf16(a, b);
                 }
                 tmem_st16(tmem + lane_base + COL_RH + q * 16, hi);
                 tmem_st16(tmem + lane_base + COL_RL + q * 16, lo);
@@ -784,8 +829,8 @@ tq_store_tc_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_consta
                 float w_lo = 0.f, w_hi = 0.f;   // bit j = (P_j > 0), sixteen bits per float
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    w_lo = fmaf(mul_sat(mul_sat(pr[j], BIG), BIG), (float)(1u << j), w_lo);
-                    w_hi = fmaf(mul_sat(mul_sat(pr[16 + j], BIG), BIG), (float)(1u << j), w_hi);
+                    w_lo = fmaf(mul_sat_ftz(pr[j], BIG), (float)(1u << j), w_lo);
+                    w_hi = fmaf(mul_sat_ftz(pr[16 + j], BIG), (float)(1u << j), w_hi);
                 }
                 uint32_t w = (__float_as_uint(w_lo + 8388608.f) & 0xffffu) | (__float_as_uint(w_hi + 8388608.f) << 16);
                 if (nd == 0.f) w = 0;   // x = 0: the reference's residual is exactly 0, r' is not
@@ -1102,11 +1147,11 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         const int blk_l = row >> 4, tl = row & 15;
         const uint32_t lane_base = (uint32_t)(row & ~31) << 16;
         BookRegs<MSE_BITS> bk;
-        bk.c0 = p.cb.centroids[0] * ACC;
+        bk.c0 = -p.cb.centroids[0] * ACC;
 #pragma unroll
         for (int i = 0; i < (1 << MSE_BITS) - 1; ++i) {
             bk.nb[i] = -p.cb.boundaries[i] * BIG;
-            bk.step[i] = (p.cb.centroids[i + 1] - p.cb.centroids[i]) * ACC;
+            bk.step[i] = (p.cb.centroids[i] - p.cb.centroids[i + 1]) * ACC;
         }
         auto wait_warp = [&](uint64_t* bar, uint32_t parity) -> bool {
             uint32_t ok = 1;
@@ -1224,10 +1269,11 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 for (int w = 0; w < 32 / PER_HALF; ++w) {
                     float wf = 0.f;
 #pragma unroll
-                    for (int jj = 0; jj < PER_HALF; ++jj) {
-                        float code;
-                        bucket<MSE_BITS, (int)ACC>(bk, y[w * PER_HALF + jj], code, y[w * PER_HALF + jj]);
-                        wf = fmaf(code, (float)(1u << (WIDTH * jj)), wf);
+                    for (int jj = 0; jj < PER_HALF; jj += 2) {
+                        float ca, cb;
+                        bucket2<MSE_BITS, (int)ACC>(bk, y[w * PER_HALF + jj], y[w * PER_HALF + jj + 1], ca, cb);
+                        wf = fmaf(ca, (float)(1u << (WIDTH * jj)), wf);
+                        wf = fmaf(cb, (float)(1u << (WIDTH * (jj + 1))), wf);
                     }
                     halves[w] = __float_as_uint(wf + 8388608.f) & 0xffffu;
                 }
@@ -1293,8 +1339,8 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
                 float w_lo = 0.f, w_hi = 0.f;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    w_lo = fmaf(mul_sat(mul_sat(pr[j], BIG), BIG), (float)(1u << j), w_lo);
-                    w_hi = fmaf(mul_sat(mul_sat(pr[16 + j], BIG), BIG), (float)(1u << j), w_hi);
+                    w_lo = fmaf(mul_sat_ftz(pr[j], BIG), (float)(1u << j), w_lo);
+                    w_hi = fmaf(mul_sat_ftz(pr[16 + j], BIG), (float)(1u << j), w_hi);
                 }
                 uint32_t w = (__float_as_uint(w_lo + 8388608.f) & 0xffffu) | (__float_as_uint(w_hi + 8388608.f) << 16);
                 if (nd == 0.f) w = 0;
@@ -1469,7 +1515,8 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
         const int nb = (1 << (cfg.key_bits - 1)) - 1;
         for (int i = 0; i < nb; ++i)
             if (i != nb / 2 && !(fabsf(consts->boundaries[i]) >= 1e-30f && fabsf(consts->boundaries[i]) < 2.f)) return TQ_OK;
-        if (!(fabsf(consts->boundaries[nb / 2]) < 2.f)) return TQ_OK;
+        const float mid = fabsf(consts->boundaries[nb / 2]);
+        if (!(mid < 2.f) || (mid > 0.f && mid < 1e-25f)) return TQ_OK;
     }
 
     TcParams p;

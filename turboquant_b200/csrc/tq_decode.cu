@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
         uint32_t* base = frag + (int64_t)(seq * (uint32_t)(Qh / G) + kvh) * qf_words(D, split ? 8 : 4);   // (sequence, kv head)
         const int gid = split ? g : g + 4 * which, set = split ? which : 0;
         return {reinterpret_cast<float*>(base) + which * 8 + g,
-                reinterpret_cast<__half*>(base + QF_HDR + ((set * (D / 8) + r) * 32 + gid * 4 + tig)) + half};
+                reinterpret_cast<__half*>(base + qf_at(set * (D / 8) + r, gid * 4 + tig)) + half};
     };
     Place at = {nullptr, nullptr};
     if (frag != nullptr && threadIdx.x < VPC * 32) at = place(v0 + (threadIdx.x >> 5));
@@ -305,8 +305,8 @@ __global__ void __launch_bounds__(256) tq_qprep_batched_kernel(const void* __res
         if (v0 + v < nvec) out[((v0 + v) * 2 + which) * D + column(lc)] = res[v * RP + lc];
     }
     if (frag == nullptr) return;
-    // fragment words: thread = (quarter, vector); lanes (quarter, vector % 8) write one 128-byte fragment row
-    // when eight query heads share a kv head.  Element layout as in tq_qprep_kernel.
+    // fragment words: thread = (quarter, vector); lanes (quarter, vector % 8) write 512 bytes of four fragment
+    // registers when eight query heads share a kv head.  Element layout as in tq_qprep_kernel.
     const int tig = tid & 3, v = tid >> 2;
     if (v0 + v >= nvec) return;
     const int64_t vec = v0 + v;
@@ -323,12 +323,17 @@ __global__ void __launch_bounds__(256) tq_qprep_batched_kernel(const void* __res
     const int gid = split ? g : g + 4 * which;
     const int set = split ? which : 0;
 #pragma unroll
-    for (int rl = 0; rl < 8; ++rl) {
-        const int lc0 = tig * 16 + (nibble ? 2 * rl : rl), lc1 = tig * 16 + (nibble ? 2 * rl + 1 : rl + 8);
-        const int sh = nibble ? 0 : (which ? sign_pos(sign_bit(strip, rl)) : 2 * code_pos(rl));
-        const float scale = __int_as_float((127 + e - sh) << 23);
-        const __half2 h2 = __floats2half2_rn(res[v * RP + lc0] * scale, res[v * RP + lc1] * scale);
-        base[QF_HDR + (set * (D / 8) + 8 * strip + rl) * 32 + gid * 4 + tig] = *reinterpret_cast<const uint32_t*>(&h2);
+    for (int rl = 0; rl < 8; rl += 4) {
+        uint32_t w[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int lc0 = tig * 16 + (nibble ? 2 * (rl + k) : rl + k), lc1 = tig * 16 + (nibble ? 2 * (rl + k) + 1 : rl + k + 8);
+            const int sh = nibble ? 0 : (which ? sign_pos(sign_bit(strip, rl + k)) : 2 * code_pos(rl + k));
+            const float scale = __int_as_float((127 + e - sh) << 23);
+            const __half2 h2 = __floats2half2_rn(res[v * RP + lc0] * scale, res[v * RP + lc1] * scale);
+            w[k] = *reinterpret_cast<const uint32_t*>(&h2);
+        }
+        *reinterpret_cast<uint4*>(base + qf_at(set * (D / 8) + 8 * strip + rl, gid * 4 + tig)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 

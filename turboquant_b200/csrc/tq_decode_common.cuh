@@ -54,11 +54,14 @@ __host__ __device__ constexpr int sign_pos(int b) { return b <= 9 ? b : b - 6; }
 
 // Query fragments of one (sequence, kv head): QF_HDR floats (exponent of the
 // rotated query per head [8], of the sketched query per head [8]) followed by
-// `sets` x (D/8) registers x 32 lanes of packed fp16 pairs.  With G <= 4 there
+// `sets` x (D/8) registers x 32 lanes of packed fp16 pairs (qf_at).  With G <= 4 there
 // is one set: B-fragment columns 0-3 hold the rotated query of heads 0-3
 // scaled by 2^(e - 2*code_pos), columns 4-7 the sketched query scaled by
 // 2^(e - sign_pos); with G > 4 set 0 is the rotated, set 1 the sketched query.
 constexpr int QF_HDR = 16;
+// Word of register r (of all sets, in order) of a lane: four registers of a lane lie together, so that two k-steps are one
+// 16-byte load (32-bit loads were a tenth of the instructions of the kernels that read the fragments from shared memory).
+__host__ __device__ constexpr int qf_at(int r, int lane) { return QF_HDR + (r >> 2) * 128 + lane * 4 + (r & 3); }
 __host__ __device__ constexpr int qf_words(int D, int G) { return QF_HDR + (G > 4 ? 2 : 1) * (D / 8) * 32; }
 
 struct ScoreParams {

@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         bt_s[i] = phys;
     }
     if (tid < NW * NSTW + 1) {   // one barrier per thread
-        tq_mbar_init(bars + tid, 1);
+        tq_mbar_init(bars + tid, tid < NW * NSTW ? R : 1);
         tq_mbar_fence_init();
     }
     __syncthreads();
@@ -317,11 +317,20 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         tq_bulk_g2s(qf_s, p.qfrag + (int64_t)(b * p.H + h) * qf_words(D, SPLITB ? 8 : 4), QF_BYTES, bars + NW * NSTW);
     }
     __syncwarp();
-    if (lane < NSTW && lane < cnt) {   // one stage per lane
-        tq_mbar_expect_tx(my_bar + lane, (uint32_t)BB);
-        tq_bulk_g2s(my_stage + lane * BB, p.pool + ((int64_t)bt_s[warp + NW * lane] * p.H + h) * BB, (uint32_t)BB,
-                    my_bar + lane);
-    }
+    // Record `rec_no` of this warp into its stage; the R stages of an iteration share the first one's barrier, where a record
+    // that the warp does not have arrives without bytes.
+    auto ask = [&](int rec_no) {
+        const int st = rec_no % NSTW;
+        uint64_t* bar = my_bar + st / R * R;
+        if (rec_no < cnt) {
+            tq_mbar_expect_tx(bar, (uint32_t)BB);
+            // 2^32 records do not fit any memory
+            tq_bulk_g2s(my_stage + st * BB, p.pool + (uint64_t)((uint32_t)bt_s[warp + NW * rec_no] * (uint32_t)p.H + (uint32_t)h) * BB, (uint32_t)BB, bar);
+        } else if (R > 1 && rec_no / R * R < cnt) {
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tq_smem_u32(bar)) : "memory");
+        }
+    };
+    if (lane < NSTW) ask(lane);   // one stage per lane
 
     // ---- query fragments, prepared once per (sequence, kv head) by the query-prep kernel ----
     // (launched with programmatic stream serialisation: everything above overlapped that kernel)
@@ -329,11 +338,19 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     bool failed = !__all_sync(0xffffffffu, tq_mbar_wait_bounded(bars + NW * NSTW, 0u));   // then no record is processed
     // Head_dim 256, and separate rotated / sketched sets in a CTA of 128 registers a thread: the fragments do not fit
     // beside the value accumulators and two records' score accumulators; they stay in shared memory, read once per pair.
-    constexpr bool BSM = R == 2 ? D == 256 || SPLITB : SPLITB && (D == 256 || NW == NW_SINGLE);
-    uint32_t bq[BSM ? 1 : 2 * KS];
-    uint32_t bsk[(SPLITB && !BSM) ? 2 * KS : 1];
-#define BQ(r) (BSM ? qf_s[QF_HDR + (r) * 32 + lane] : bq[BSM ? 0 : (r)])
-#define BSK(r) (BSM ? qf_s[QF_HDR + (2 * KS + (r)) * 32 + lane] : bsk[(SPLITB && !BSM) ? (r) : 0])
+    constexpr bool BSM = D == 256 ? R == 2 || SPLITB || NW == NW_MULTI : SPLITB && (R == 2 || NW == NW_SINGLE);
+    uint32_t bq[BSM ? 1 : 2 * KS] = {};
+    uint32_t bsk[(SPLITB && !BSM) ? 2 * KS : 1] = {};
+    // registers r .. r + 3 of the rotated (SPLITB: else of the only) set, of the sketched set; r a multiple of four
+    auto bq4 = [&](int r) -> uint4 {
+        if constexpr (BSM) return *reinterpret_cast<const uint4*>(qf_s + qf_at(r, lane));
+        else return make_uint4(bq[r], bq[r + 1], bq[r + 2], bq[r + 3]);
+    };
+    auto bsk4 = [&](int r) -> uint4 {
+        if constexpr (!SPLITB) return bq4(r);
+        else if constexpr (BSM) return *reinterpret_cast<const uint4*>(qf_s + qf_at(2 * KS + r, lane));
+        else return make_uint4(bsk[r], bsk[r + 1], bsk[r + 2], bsk[r + 3]);
+    };
     float k0[2], k1[2], kb0[2], ksg[2], kq[2];
     {
         const uint32_t* qf = qf_s;
@@ -342,13 +359,19 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         const bool col_live = g_col < p.G;
         if (BSM) {
             if (!col_live)   // columns without a head: nobody wrote their fragments - clear this lane's words
-                for (int r = 0; r < (SPLITB ? 4 : 2) * KS; ++r) qf_s[QF_HDR + r * 32 + lane] = 0u;
+                for (int r = 0; r < (SPLITB ? 4 : 2) * KS; r += 4) *reinterpret_cast<uint4*>(qf_s + qf_at(r, lane)) = make_uint4(0u, 0u, 0u, 0u);
             __syncwarp();
         } else {
 #pragma unroll
-            for (int r = 0; r < 2 * KS; ++r) {
-                bq[BSM ? 0 : r] = col_live ? qf[QF_HDR + r * 32 + lane] : 0u;
-                if (SPLITB) bsk[(SPLITB && !BSM) ? r : 0] = col_live ? qf[QF_HDR + (2 * KS + r) * 32 + lane] : 0u;
+            for (int r = 0; r < 2 * KS; r += 4) {
+                const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+                const uint4 a = col_live ? *reinterpret_cast<const uint4*>(qf + qf_at(r, lane)) : zero;
+                bq[BSM ? 0 : r] = a.x; bq[BSM ? 0 : r + 1] = a.y; bq[BSM ? 0 : r + 2] = a.z; bq[BSM ? 0 : r + 3] = a.w;
+                if (SPLITB && !BSM) {
+                    constexpr bool REG = SPLITB && !BSM;
+                    const uint4 c = col_live ? *reinterpret_cast<const uint4*>(qf + qf_at(2 * KS + r, lane)) : zero;
+                    bsk[REG ? r : 0] = c.x; bsk[REG ? r + 1 : 0] = c.y; bsk[REG ? r + 2 : 0] = c.z; bsk[REG ? r + 3 : 0] = c.w;
+                }
             }
         }
         // Sums of the fp16-rounded query over all dims (the constant terms of the bit-plane form), taken
@@ -358,16 +381,19 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         float one_c[4] = {0.f, 0.f, 0.f, 0.f}, one_s[4] = {0.f, 0.f, 0.f, 0.f};
         float one_c2[4] = {0.f, 0.f, 0.f, 0.f}, one_s2[4] = {0.f, 0.f, 0.f, 0.f};   // odd k-steps: shorter chains
 #pragma unroll
-        for (int s = 0; s < KS; ++s) {
-            const int wi = s >> 2, jj = s & 3;
-            if (MSE_BITS == 2) {
-                const uint32_t m0 = 0x00010001u << (2 * code_pos(2 * jj)), m1 = 0x00010001u << (2 * code_pos(2 * jj + 1));
-                mma16816((s & 1) ? one_c2 : one_c, m0, m0, m1, m1, BQ(2 * s), BQ(2 * s + 1));
+        for (int s2 = 0; s2 < KS; s2 += 2) {
+            const uint4 q = bq4(2 * s2), z = bsk4(2 * s2);
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                const int wi = (s2 + o) >> 2, jj = (s2 + o) & 3;
+                if (MSE_BITS == 2) {
+                    const uint32_t m0 = 0x00010001u << (2 * code_pos(2 * jj)), m1 = 0x00010001u << (2 * code_pos(2 * jj + 1));
+                    mma16816(o ? one_c2 : one_c, m0, m0, m1, m1, o ? q.z : q.x, o ? q.w : q.y);
+                }
+                const uint32_t n0 = 0x00010001u << sign_pos(sign_bit(wi, 2 * jj));
+                const uint32_t n1 = 0x00010001u << sign_pos(sign_bit(wi, 2 * jj + 1));
+                mma16816(o ? one_s2 : one_s, n0, n0, n1, n1, o ? z.z : z.x, o ? z.w : z.y);
             }
-            const uint32_t n0 = 0x00010001u << sign_pos(sign_bit(wi, 2 * jj));
-            const uint32_t n1 = 0x00010001u << sign_pos(sign_bit(wi, 2 * jj + 1));
-            mma16816((s & 1) ? one_s2 : one_s, n0, n0, n1, n1, SPLITB ? BSK(2 * s) : BQ(2 * s),
-                     SPLITB ? BSK(2 * s + 1) : BQ(2 * s + 1));
         }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -410,6 +436,9 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         for (int c = 0; c < 4; ++c) o[mb][c] = 0.f;
     float zacc[4] = {0.f, 0.f, 0.f, 0.f};
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    // m_run, or 0 while there is no score but -Inf (or NaN); kept where a warp meets many records
+    constexpr bool USE = D == 128 && R == 2;
+    float m_use[2] = {0.f, 0.f};
 
     const int tokA = 4 * (gid >> 1) + (gid & 1), tokB = tokA + 2;   // tokens of score rows gid, gid+8
     // 3-bit codes: low / high bytes of the eight fp16 centroids, selectable by PRMT
@@ -430,36 +459,39 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
     // independent, which keeps the pipes of a quarter SM busy with the four warps that the registers allow.
     for (int it = 0; it < cnt && !failed; it += R) {
         const int st = it % NSTW;
-        const uint32_t phase = (uint32_t)((it / NSTW) & 1);
-        const bool both = R == 2 && it + 1 < cnt;
-        bool ok = tq_mbar_wait_bounded(my_bar + st, phase) && (!both || tq_mbar_wait_bounded(my_bar + st + 1, phase));
-        ok = __all_sync(0xffffffffu, ok);
+        const bool ok = __all_sync(0xffffffffu, tq_mbar_wait_bounded(my_bar + st, (uint32_t)((it / NSTW) & 1)));
         if (!ok) {
             failed = true;
             break;
         }
         uint8_t* rec[R];
-        int valid[R];   // an odd record's partner is itself, with no valid token
+        rec[0] = my_stage + st * BB;
+        int valid[R];
         bool ragged = false;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const bool there = r == 0 || both;
-            rec[r] = my_stage + (there ? st + r : st) * BB;
-            valid[r] = there ? min(TQ_BLOCK_TOKENS, n - (blk0 + warp + NW * (it + r)) * TQ_BLOCK_TOKENS) : 0;
-            ragged |= valid[r] < TQ_BLOCK_TOKENS;
-        }
-        if (ragged) {
-            // the sequence's last, partly filled record: unused slots may hold anything.  Their scores are
-            // masked below; their value scales and zero points ([grp][16 tok] fp16, contiguous) are cleared
-            // here, so that probability 0 times a stale Inf/NaN cannot reach the value MMAs.
-            for (int r = 0; r < 1 + (both ? 1 : 0); ++r) {
-                __half* sz = reinterpret_cast<__half*>(my_stage + (st + r) * BB + L.off_vscale);
-                const int live = r == 0 ? valid[0] : valid[R - 1];
-                for (int i = lane; i < 2 * NG * TQ_BLOCK_TOKENS; i += 32)
-                    if ((i & (TQ_BLOCK_TOKENS - 1)) >= live) sz[i] = __float2half(0.f);
+        for (int r = 0; r < R; ++r) valid[r] = TQ_BLOCK_TOKENS;
+        if (R == 2) rec[R - 1] = rec[0] + BB;
+        if (it + R >= cnt) {   // only here: the sequence's last record, or one without a partner (it then stands in for it, with no valid token)
+            const bool both = R == 1 || it + 1 < cnt;
+            if (!both) rec[R - 1] = rec[0];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                valid[r] = r == 0 || both ? min(TQ_BLOCK_TOKENS, n - (blk0 + warp + NW * (it + r)) * TQ_BLOCK_TOKENS) : 0;
+                ragged |= valid[r] < TQ_BLOCK_TOKENS;
             }
-            tq_fence_proxy_async();   // generic writes to a stage that a later bulk copy may refill
-            __syncwarp();
+            if (ragged) {
+                // the sequence's last, partly filled record: unused slots may hold anything.  Their scores are
+                // masked below; their value scales and zero points ([grp][16 tok] fp16, contiguous) are cleared
+                // here, so that probability 0 times a stale Inf/NaN cannot reach the value MMAs.
+                for (int r = 0; r < (both ? R : 1); ++r) {
+                    __half* sz = reinterpret_cast<__half*>(my_stage + (st + r) * BB + L.off_vscale);
+                    const int live = r == 0 ? valid[0] : valid[R - 1];
+                    for (int i = lane; i < 2 * NG * TQ_BLOCK_TOKENS; i += 32)
+                        if ((i & (TQ_BLOCK_TOKENS - 1)) >= live) sz[i] = __float2half(0.f);
+                }
+                tq_fence_proxy_async();   // generic writes to a stage that a later bulk copy may refill
+                __syncwarp();
+            }
         }
 
         // ------------------------------ scores ------------------------------
@@ -503,15 +535,20 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                     sa_hi[r] = sa_lo[r] >> 6;
                     sb_hi[r] = sb_lo[r] >> 6;
                 }
+                uint4 q4, z4;
 #pragma unroll
                 for (int jj = 0; jj < 4; ++jj) {
                     const int s = wi * 4 + jj;
+                    if (jj % 2 == 0) {
+                        q4 = bq4(2 * s);
+                        z4 = bsk4(2 * s);
+                    }
                     const int j0 = 2 * jj, j1 = j0 + 1;
                     const uint32_t m0 = 0x00010001u << (2 * code_pos(j0)), m1 = 0x00010001u << (2 * code_pos(j1));
                     const int sb0 = sign_bit(wi, j0), sb1 = sign_bit(wi, j1);
                     const uint32_t n0 = 0x00010001u << sign_pos(sb0), n1 = 0x00010001u << sign_pos(sb1);
-                    const uint32_t q0 = BQ(2 * s), q1 = BQ(2 * s + 1);
-                    const uint32_t z0 = SPLITB ? BSK(2 * s) : q0, z1 = SPLITB ? BSK(2 * s + 1) : q1;
+                    const uint32_t q0 = jj % 2 ? q4.z : q4.x, q1 = jj % 2 ? q4.w : q4.y;
+                    const uint32_t z0 = jj % 2 ? z4.z : z4.x, z1 = jj % 2 ? z4.w : z4.y;
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         const uint32_t xa0 = j0 <= 4 ? wA[r][wi] : a_hi[r], xb0 = j0 <= 4 ? wB[r][wi] : b_hi[r];
@@ -546,11 +583,12 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                 }
 #pragma unroll
                 for (int wi = 0; wi < 4; ++wi) {
+                    const uint4 q4r = bq4(2 * ((q4 * 4 + wi) * 2));   // two k-steps
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf) {
                         // k-step s covers dims 8*(4*q4+wi) + 4*hf + {0,1 | 2,3} of this thread's slice
                         const int s = (q4 * 4 + wi) * 2 + hf;
-                        const uint32_t q0 = BQ(2 * s), q1 = BQ(2 * s + 1);
+                        const uint32_t q0 = hf ? q4r.z : q4r.x, q1 = hf ? q4r.w : q4r.y;
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
                             const uint32_t sa = hf ? wa[r][wi] >> 16 : wa[r][wi], sb = hf ? wb[r][wi] >> 16 : wb[r][wi];
@@ -578,12 +616,14 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                 }
 #pragma unroll
                 for (int wi = 2 * sw; wi < 2 * sw + 2; ++wi) {
+                    uint4 z4;
 #pragma unroll
                     for (int jj = 0; jj < 4; ++jj) {
                         const int s = wi * 4 + jj;
+                        if (jj % 2 == 0) z4 = bsk4(2 * s);
                         const int sb0 = sign_bit(wi, 2 * jj), sb1 = sign_bit(wi, 2 * jj + 1);
                         const uint32_t n0 = 0x00010001u << sign_pos(sb0), n1 = 0x00010001u << sign_pos(sb1);
-                        const uint32_t z0 = BSK(2 * s), z1 = BSK(2 * s + 1);
+                        const uint32_t z0 = jj % 2 ? z4.z : z4.x, z1 = jj % 2 ? z4.w : z4.y;
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
                             const uint32_t ya0 = sb0 <= 9 ? sa_lo[r] : sa_hi[r], yb0 = sb0 <= 9 ? sb_lo[r] : sb_hi[r];
@@ -648,6 +688,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
                 alpha[i] = m_new == -INFINITY ? 1.f : ex2_fast(m_run[i] - m_new);
                 l_run[i] *= alpha[i];
                 m_run[i] = m_new;
+                if (USE) m_use[i] = m_new == -INFINITY ? 0.f : m_new;
             }
 #pragma unroll
             for (int mb = 0; mb < NMB; ++mb) {
@@ -668,9 +709,9 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
             float pA[2], pB[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const float m_use = m_run[i] == -INFINITY ? 0.f : m_run[i];   // no score yet but -Inf (or NaN)
-                pA[i] = ex2_fast(sc_[r][0][i] - m_use);
-                pB[i] = ex2_fast(sc_[r][1][i] - m_use);
+                const float m = USE ? m_use[i] : m_run[i] == -INFINITY ? 0.f : m_run[i];
+                pA[i] = ex2_fast(sc_[r][0][i] - m);
+                pB[i] = ex2_fast(sc_[r][1][i] - m);
                 l_run[i] += pA[i] + pB[i];
             }
             t0[r] = movmatrix_trans(col_ok ? pack_half2(pA[0] * 16.f, pA[1] * 16.f) : 0u);
@@ -746,11 +787,7 @@ __global__ void __launch_bounds__(NW * 32, NW == NW_MULTI ? 2 : 1) tq_decode_mma
         }
 
         __syncwarp();
-        if (lane < R && it + lane + NSTW < cnt) {   // refill the stages just consumed
-            tq_mbar_expect_tx(my_bar + st + lane, (uint32_t)BB);
-            tq_bulk_g2s(my_stage + (st + lane) * BB, p.pool + ((int64_t)bt_s[warp + NW * (it + lane + NSTW)] * p.H + h) * BB,
-                        (uint32_t)BB, my_bar + st + lane);
-        }
+        if (lane < R) ask(it + lane + NSTW);   // refill the stages just consumed
     }
     if (failed && lane == 0) atomicCAS(p.status, 0, (int)TQ_ERR_TIMEOUT);
 

@@ -166,22 +166,26 @@ tq_qprep_tc_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_consta
                 const bool nibble = p.mse_bits == 3 && which == 0;
                 const int gid = split ? g : g + 4 * which;
                 const int set = split ? which : 0;
-                // one 16-byte store per fragment row: the four quarters' words of this (vector, position) are
-                // adjacent, and the eight query heads of a kv head fill the 128-byte row
+                // a quarter's words of four registers lie together, two quarters' are one 32-byte store (a whole sector), and
+                // the eight query heads of a kv head fill 512 bytes
 #pragma unroll
-                for (int r = 0; r < 16; ++r) {   // element layout as in tq_qprep_kernel
-                    const int wi = r >> 3, jf = r & 7;
-                    const int c0 = nibble ? 2 * r : wi * 16 + jf, c1 = nibble ? 2 * r + 1 : wi * 16 + 8 + jf;
-                    const int sh = nibble ? 0 : (which ? sign_pos(sign_bit(wi, jf)) : 2 * code_pos(jf));
-                    const float scale = __int_as_float((127 + e - sh) << 23);
-                    uint32_t w[4];
+                for (int r = 0; r < 16; r += 4) {   // element layout as in tq_qprep_kernel
 #pragma unroll
-                    for (int tig = 0; tig < 4; ++tig) {
-                        const __half2 h2 = __floats2half2_rn(v[tig][c0] * scale, v[tig][c1] * scale);
-                        w[tig] = *reinterpret_cast<const uint32_t*>(&h2);
+                    for (int tig = 0; tig < 4; tig += 2) {
+                        uint32_t w[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const int rr = r + (k & 3), wi = rr >> 3, jf = rr & 7;
+                            const int c0 = nibble ? 2 * rr : wi * 16 + jf, c1 = nibble ? 2 * rr + 1 : wi * 16 + 8 + jf;
+                            const int sh = nibble ? 0 : (which ? sign_pos(sign_bit(wi, jf)) : 2 * code_pos(jf));
+                            const float scale = __int_as_float((127 + e - sh) << 23);
+                            const __half2 h2 = __floats2half2_rn(v[tig + (k >> 2)][c0] * scale, v[tig + (k >> 2)][c1] * scale);
+                            w[k] = *reinterpret_cast<const uint32_t*>(&h2);
+                        }
+                        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(base + qf_at(set * (QT_D / 8) + r, gid * 4 + tig)),
+                                     "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                                     : "memory");
                     }
-                    *reinterpret_cast<uint4*>(base + QF_HDR + (set * (QT_D / 8) + r) * 32 + gid * 4) =
-                        make_uint4(w[0], w[1], w[2], w[3]);
                 }
             }
             // fp32 results: transposed through shared memory, a warp's 32 rows one after the other, so that

@@ -225,8 +225,8 @@ int tq_sm_count();         // multiprocessors of the current device (148 when th
 // begin before they have finished (programmatic dependent launch) and do part of their work before they wait
 // for the launch ahead; that is only safe when the launch still in flight cannot be writing what is read early:
 //   * the tensor-core store kernels fetch their key / value rows before the wait.  The decode family appends
-//     the new token to the ring - rows a flush then reads - so a store behind a decode launch is launched in
-//     plain stream order;
+//     the new token to the ring - rows a flush then reads - so a store behind a decode launch only asks for its
+//     constant operands early, waits in front of its first row and lets its own dependents begin after that;
 //   * the decode family reads sequence lengths, block tables and the first pool records before the wait.
 //     The tensor-core store kernels write the pool and let their dependents begin at once.  The query
 //     preparation reads nothing that they write and may start under them; the decode kernel behind it is
@@ -243,7 +243,7 @@ inline void tq_note_prep_launch(cudaStream_t st) {
     const int k = tq_last_launch(st);
     tq_note_launch(st, k == TQ_LAUNCH_STORE_EARLY || k == TQ_LAUNCH_PREP_BEHIND_STORE ? TQ_LAUNCH_PREP_BEHIND_STORE : TQ_LAUNCH_DECODE);
 }
-// programmatic-launch attribute count (0 or 1) for a kernel of the decode family / of the early-starting stores
+// programmatic-launch attribute count (0 or 1) for a kernel of the decode family / whether a store may read its rows early
 inline int tq_pdl_for_decode(cudaStream_t st) { return tq_last_launch(st) == TQ_LAUNCH_STORE_EARLY ? 0 : 1; }
 inline int tq_pdl_for_store(cudaStream_t st) {
     const int k = tq_last_launch(st);

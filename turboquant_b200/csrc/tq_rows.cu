@@ -14,8 +14,8 @@
 // kernel starts under the launch ahead of it: its constants arrive while it waits.
 //
 // Measured (B200, 16000 rows of 128, fp32, 3-bit keys, 2-bit values, 4 queries, calls back to back; in brackets with a warp per
-// 16 rows, eight query slots whatever was asked for, a thread per group of values and plain launches): quantise 29.6 us
-// (31.7), dequantise 13.2 (14.6), scores 8.2 (12.0), values 6.9 (10.4) and 4.5 (6.2), everything in turn 59.7 (76.0); 480 rows
+// 16 rows, eight query slots whatever was asked for, a thread per group of values and plain launches): quantise 28.9 us
+// (31.7), dequantise 13.2 (14.6), scores 8.2 (12.0), values 6.9 (10.4) and 4.5 (6.2), everything in turn 58.9 (76.0); 480 rows
 // 41.5 (62.9).
 #include "tq_decode_common.cuh"
 
@@ -358,7 +358,7 @@ __device__ __noinline__ void redo_row(const RowsParams& p, int64_t row, float nd
 // goes through shared memory as whole fragments.  Four warps a scheduler instead of two cover one another's chains, and the
 // loops over columns stay rolled: unrolled they were 100 KB of instructions that a call of one tile per CTA reads once.
 template <int DT, int MSE_BITS>
-__global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(const __grid_constant__ RowsParams p) {
+__global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(const __grid_constant__ RowsParams p, int vec /* rows of x are 16-byte aligned */) {
     using E = TqElem<DT>;
     constexpr int LU = DT == TQ_F32 ? 2 : 1;   // limbs that hold u; else the second place holds e = x / |x| - u
     constexpr int NB = (1 << MSE_BITS) - 1;
@@ -375,11 +375,43 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
     asm volatile("cp.async.commit_group;" ::: "memory");
     const uint32_t sp = tq_smem_u32(smem), sm = sp + 2 * R_MAT;
     uint4* xchg = reinterpret_cast<uint4*>(smem + 4 * R_MAT) + group * (KSTEPS * 2 * 32) + lane;   // [k-step][limb][lane]
+    constexpr int ES = DT == TQ_F32 ? 4 : 2, RB = RD * ES;
+    static_assert(16 * RB <= KSTEPS * 2 * 32 * 16, "the rows of a pair fit the place of its fragments");
+    // chunk c of row r there: eight rows' same chunk (or four rows' same two, of fp32) in different banks
+    auto at_row = [&](int r, int c) -> uint8_t* {
+        return smem + 4 * R_MAT + group * (KSTEPS * 2 * 32 * 16) + r * RB + ((c ^ (DT == TQ_F32 ? (r & 3) << 1 : r & 7)) << 4);
+    };
     wait_for_launch_ahead();
     bool first = true;
 #pragma unroll 1
     for (int64_t tile = blockIdx.x; tile * R_ROWS < p.n; tile += gridDim.x) {
         const int64_t base_row = tile * R_ROWS + group * 16, r0 = base_row + gid, r1 = r0 + 8;
+        {   // the pair's rows, whole lines at a time, into the place of the fragments: chunks of 16 bytes, swizzled by row (each lane
+            // fetching its own pairs of numbers from global memory, twice over with the norms: 29.5 us, now 28.9; fp16 33.2, now 31.8)
+            constexpr int CHUNKS = 16 * RB / 16 / 64;   // of one thread
+            uint4 v[CHUNKS];
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) {
+                const int c = i * 64 + mine * 32 + lane;
+                const int64_t row = base_row + c / (RB / 16);
+                v[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (row < p.n) {
+                    const char* src = static_cast<const char*>(p.x) + row * p.stride_row * ES + c % (RB / 16) * 16;
+                    if (vec) {
+                        v[i] = *reinterpret_cast<const uint4*>(src);
+                    } else {
+                        const uint2 lo = reinterpret_cast<const uint2*>(src)[0], hi = reinterpret_cast<const uint2*>(src)[1];
+                        v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) {
+                const int c = i * 64 + mine * 32 + lane;
+                *reinterpret_cast<uint4*>(at_row(c / (RB / 16), c % (RB / 16))) = v[i];
+            }
+        }
+        pair_sync(group);
         float x[HALF][2][2][2];   // this warp's k-steps: [row][half][element]
 #pragma unroll
         for (int ks = 0; ks < HALF; ++ks)
@@ -387,9 +419,8 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
             for (int r = 0; r < 2; ++r)
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
-                    const int64_t row = r ? r1 : r0;
-                    x[ks][r][hf][0] = x[ks][r][hf][1] = 0.f;
-                    if (row < p.n) load2<DT>(p.x, row * p.stride_row + (mine * HALF + ks) * 16 + hf * 8 + 2 * tig, x[ks][r][hf][0], x[ks][r][hf][1]);
+                    const int byte = ((mine * HALF + ks) * 16 + hf * 8 + 2 * tig) * ES;
+                    load2<DT>(at_row(gid + 8 * r, byte >> 4) + (byte & 15), 0, x[ks][r][hf][0], x[ks][r][hf][1]);
                 }
         {   // norms, in the fp32 store kernel's order: eight sums of 16 squares, added up in order.  Lane = (row % 4, sum), two rows a lane.
             const int ch = lane & 7;
@@ -398,9 +429,9 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
                 const int row_l = 8 * mine + 4 * i + (lane >> 3);
                 float v[16];
 #pragma unroll
-                for (int j = 0; j < 16; j += 4)
-                    if (base_row + row_l < p.n) load4<DT>(p.x, (base_row + row_l) * p.stride_row + ch * 16 + j, v + j);
-                    else v[j] = v[j + 1] = v[j + 2] = v[j + 3] = 0.f;
+                for (int j = 0; j < 16; j += 16 / ES)
+#pragma unroll
+                    for (int k = 0; k < 16 / ES; k += 4) load4<DT>(at_row(row_l, (ch * 16 + j) * ES >> 4), k, v + j + k);
                 float s = 0.f;
 #pragma unroll
                 for (int j = 0; j < 16; ++j) s = fmaf(v[j], v[j], s);
@@ -908,12 +939,13 @@ extern "C" int tq_rows_quantize_keys(const tq_consts* consts, const void* x, tq_
     p.norm_dt = norm_dtype;
     p.rnorm_dt = residual_dtype;
     cudaStream_t st = (cudaStream_t)stream;
+    const int vec = aligned(x, 16) && (stride_row * (int64_t)tq_dtype_size(dtype)) % 16 == 0;
     constexpr size_t smem = 4 * R_MAT + R_XCHG;
 #define TQ_QK(DT, MB)                                                                            \
     do {                                                                                         \
         static TqSmemOptIn opt_in;                                                               \
         if (tq_opt_in_smem(tq_rows_quantize_keys_kernel<DT, MB>, smem, opt_in) != TQ_OK) return TQ_ERR_CUDA; \
-        return launch_rows(tq_rows_quantize_keys_kernel<DT, MB>, dim3(rows_grid(n_rows)), R_THREADS, smem, st, p); \
+        return launch_rows(tq_rows_quantize_keys_kernel<DT, MB>, dim3(rows_grid(n_rows)), R_THREADS, smem, st, p, vec); \
     } while (0)
     const int mb = consts->cfg.key_bits - 1;
     if (dtype == TQ_F32) { if (mb == 2) TQ_QK(TQ_F32, 2); else TQ_QK(TQ_F32, 3); }

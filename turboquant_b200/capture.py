@@ -30,6 +30,7 @@ class RingBuffer:
         self.device, self.dtype = device, dtype
         self._keys = torch.zeros(capacity, num_kv_heads, head_dim, device=device, dtype=dtype)
         self._values = torch.zeros_like(self._keys)
+        self._on_device = self._keys.is_cuda
         self._fill = 0                                     # tokens held
         self._seen = 0                                     # tokens ever written
         self._fill_dev: Optional[torch.Tensor] = None      # device mirror of _fill, kept by device_len()
@@ -95,6 +96,16 @@ class RingBuffer:
         self._values[:stay] = value[cut:num_tokens]
         self._fill = stay
         return out_k, out_v
+
+    def write_one(self, key: torch.Tensor, value: torch.Tensor) -> bool:
+        """`write` of one token where there is room and the kernel takes it, in as few steps as that can be; False, with
+        nothing changed, otherwise."""
+        held = self._fill
+        if held >= self.capacity or not self._on_device or E.host().ring_write(self._keys, self._values, key, value, held, 1) != 0:
+            return False
+        self._fill = held + 1
+        self._seen += 1
+        return True
 
     def write_from_paged(self, key_cache: torch.Tensor, value_cache: torch.Tensor, block_table: torch.Tensor, first: int,
                          num_tokens: int) -> bool:

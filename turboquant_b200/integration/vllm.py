@@ -170,7 +170,11 @@ def _make_patched_kv_update(orig_fn, state: LayerState, no_alloc: bool = False):
         if not no_alloc:
             orig_fn(self_impl, layer, key, value, kv_cache, slot_mapping)
         if _GLOBAL_MODE != MODE_OFF:
-            _capture(state, key, value, slot_mapping.shape[0])
+            n = slot_mapping.shape[0]
+            if n == 1 and state._engine is not None:    # a decode token into a ring with room: nothing between here and the launch
+                if state._engine.ring.write_one(key, value):
+                    return
+            _capture(state, key, value, n)
     return patched
 
 
@@ -178,9 +182,24 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
     def original(self_impl, layer, query, key, value, kv_cache, md, output, output_scale, output_block_scale):
         return orig_fn(self_impl, layer, query, key, value, kv_cache, md, output, output_scale, output_block_scale)
 
+    c, flash = state.config, state.supports_hybrid
+    head_dim, num_query_heads = c.head_dim, c.num_query_heads
+
+    def attend(st, ring, query, n, self_impl, output):
+        """The native call that writes into the engine's buffer: `output`, a status, or None where it does not apply."""
+        return E.host().hybrid(st.consts.addr, st.pool.addr, st.workspace, st.block_table, head_dim, st._num_tokens, query, n,
+                               num_query_heads, ring._keys, ring._values, ring._fill, getattr(self_impl, "scale", None),
+                               MIN_HISTORY, output)
+
     def patched(self_impl, layer, query, key, value, kv_cache, attn_metadata, output=None, output_scale=None,
                 output_block_scale=None):
         mode = _GLOBAL_MODE
+        if mode == MODE_HYBRID and output is not None and flash and not capture_in_forward and attn_metadata is not None and \
+                attn_metadata.max_query_len <= 1:       # a decode step in the engine's own layout: what such a step spends here, it waits for
+            st, engine = state._store, state._engine
+            if st is not None and engine is not None and st._num_tokens >= MIN_HISTORY and \
+                    attend(st, engine.ring, query, attn_metadata.num_actual_tokens, self_impl, output) is output:
+                return output
         args = (self_impl, layer, query, key, value, kv_cache, attn_metadata, output, output_scale,
                 output_block_scale)
         if capture_in_forward and mode != MODE_OFF and attn_metadata is not None:
@@ -199,7 +218,6 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
             _capture(state, key[:n], value[:n], n)
         if mode in (MODE_OFF, MODE_CAPTURE_ONLY) or attn_metadata is None:
             return original(*args)
-        c = state.config
         n = attn_metadata.num_actual_tokens
         if attn_metadata.max_query_len > 1:            # prefill
             if not no_alloc:
@@ -211,9 +229,7 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
         if mode == MODE_HYBRID and state.supports_hybrid and state.store.num_tokens >= MIN_HISTORY:
             if output is not None:                      # straight into the engine's buffer where its layout allows
                 st, ring = state.store, state.engine.ring
-                res = E.host().hybrid(st.consts.addr, st.pool.addr, st.workspace, st.block_table, c.head_dim, st._num_tokens,
-                                      query, n, c.num_query_heads, *ring.storage, ring.size, getattr(self_impl, "scale", None),
-                                      MIN_HISTORY, output)
+                res = attend(st, ring, query, n, self_impl, output)
                 if res is output:
                     return output
                 if res is not None:

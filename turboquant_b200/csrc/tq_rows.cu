@@ -14,8 +14,8 @@
 // kernel starts under the launch ahead of it: its constants arrive while it waits.
 //
 // Measured (B200, 16000 rows of 128, fp32, 3-bit keys, 2-bit values, 4 queries, calls back to back; in brackets with a warp per
-// 16 rows, eight query slots whatever was asked for, a thread per group of values and plain launches): quantise 28.9 us
-// (31.7), dequantise 13.2 (14.6), scores 8.2 (12.0), values 6.9 (10.4) and 4.5 (6.2), everything in turn 58.9 (76.0); 480 rows
+// 16 rows, eight query slots whatever was asked for, a thread per group of values and plain launches): quantise 20.2 us
+// (31.7), dequantise 13.2 (14.6), scores 8.2 (12.0), values 6.9 (10.4) and 4.5 (6.2), everything in turn 50.1 (76.0); 480 rows
 // 41.5 (62.9).
 #include "tq_decode_common.cuh"
 
@@ -257,10 +257,12 @@ __device__ __forceinline__ void load4(const void* p, int64_t i, float* x) {
 
 // The limb products and the fp32 store kernel's chain of fused multiply-adds agree to a few 1e-7 (|u| = 1, rows of Pi have
 // norm 1).  A coordinate that lies closer than this to a decision boundary - some 20 in a million - is computed again as
-// that chain, so that the codes are the fp32 kernel's on both sides of a tie.
+// that chain, so that the codes are the fp32 kernel's on both sides of a tie.  Where the chain decides differently, in one row of some
+// 30 000, its number takes the product's place before anything follows from it (as a whole row by that chain, behind the rest of
+// its tile, such a row made a call of 16000 rows take 28.9 us; now 20.2 with or without one).
 constexpr float NEAR = 1e-6f;
-// Both functions below are off the usual path and run from a cold instruction cache, where a line of eight instructions
-// costs more than the arithmetic in it: loops stay rolled (an unrolled row took 41 us, this form a few).
+// Off the usual path, from a cold instruction cache, where a line of eight instructions costs more than the arithmetic in
+// it: loops stay rolled.
 // One coordinate by the whole warp: lane l holds the terms l, 32 + l, ...; every lane returns the sum.
 template <int DT>
 __device__ __noinline__ float serial_product(const void* x, int64_t at, float den, const float* pi_t_col, int lane) {
@@ -276,81 +278,6 @@ __device__ __noinline__ float serial_product(const void* x, int64_t at, float de
         for (int l = 0; l < 32; ++l) y = fmaf(__shfl_sync(0xffffffffu, u[i], l), __shfl_sync(0xffffffffu, w[i], l), y);
     return y;
 }
-// A whole row by that chain, one warp, four coordinates a lane: for the row (one in some 30 000) where it decides
-// differently.  Overwrites the row's codes, sign bits and residual norm.
-template <int DT, int MSE_BITS>
-__device__ __noinline__ void redo_row(const RowsParams& p, int64_t row, float nd, float den, uint32_t sm, int lane) {
-    using E = TqElem<DT>;
-    float u[4], d[4], y[4] = {}, e[4] = {}, r[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const float q = __fdiv_rn(E::load(p.x, row * p.stride_row + 4 * lane + c), den);
-        u[c] = E::round(q);
-        d[c] = q - u[c];
-    }
-#pragma unroll 1
-    for (int l = 0; l < 32; l += 2) {
-        float4 w[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) w[k] = __ldg(reinterpret_cast<const float4*>(p.pi_t + (4 * l + k) * RD) + lane);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float uk = __shfl_sync(0xffffffffu, u[k & 3], l + (k >> 2));
-            y[0] = fmaf(uk, w[k].x, y[0]); y[1] = fmaf(uk, w[k].y, y[1]); y[2] = fmaf(uk, w[k].z, y[2]); y[3] = fmaf(uk, w[k].w, y[3]);
-            if (DT != TQ_F32) {
-                const float dk = __shfl_sync(0xffffffffu, d[k & 3], l + (k >> 2));
-                e[0] = fmaf(dk, w[k].x, e[0]); e[1] = fmaf(dk, w[k].y, e[1]); e[2] = fmaf(dk, w[k].z, e[2]); e[3] = fmaf(dk, w[k].w, e[3]);
-            }
-        }
-    }
-    uint32_t packed = 0;
-    float n2 = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        uint32_t k = 0;
-        float cv = p.cb.centroids[0];
-#pragma unroll
-        for (int i = 0; i < (1 << MSE_BITS) - 1; ++i)
-            if (p.cb.boundaries[i] < y[c]) {
-                k = i + 1;
-                cv = p.cb.centroids[i + 1];
-            }
-        packed |= k << ((MSE_BITS == 2 ? 2 : 4) * c);
-        r[c] = (y[c] - cv) + e[c];
-        n2 = fmaf(r[c], r[c], n2);
-    }
-    if (MSE_BITS == 2) p.codes[row * (RD / 4) + lane] = (uint8_t)packed;
-    else reinterpret_cast<uint16_t*>(p.codes + row * (RD / 2))[lane] = (uint16_t)packed;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
-    float pr[4] = {};
-#pragma unroll 1
-    for (int l = 0; l < 32; ++l) {   // columns 4 l .. 4 l + 3 of rows lane + 32 i of M
-        const float rk[4] = {__shfl_sync(0xffffffffu, r[0], l), __shfl_sync(0xffffffffu, r[1], l), __shfl_sync(0xffffffffu, r[2], l),
-                             __shfl_sync(0xffffffffu, r[3], l)};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row_m = lane + 32 * i;
-            const uint32_t a = sm + row_m * 256 + (((l >> 1) ^ (row_m & 7)) << 4) + (l & 1) * 8;
-            uint32_t h[2], t[2];
-            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(h[0]), "=r"(h[1]) : "r"(a));
-            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(t[0]), "=r"(t[1]) : "r"(a + R_MAT));
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h[k])), g = __half22float2(*reinterpret_cast<const __half2*>(&t[k]));
-                pr[i] = fmaf(rk[2 * k], f.x + g.x, pr[i]);
-                pr[i] = fmaf(rk[2 * k + 1], f.y + g.y, pr[i]);
-            }
-        }
-    }
-    uint32_t s[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) s[i] = __ballot_sync(0xffffffffu, pr[i] > 0.f);
-    if (lane == 0) {
-        *reinterpret_cast<uint4*>(p.signs + row * (RD / 8)) = make_uint4(s[0], s[1], s[2], s[3]);
-        tq_store_any(p.rnorms, row, __half2float(__float2half_rn(nd * __fsqrt_rn(n2))), p.rnorm_dt);
-    }
-}
 
 // quantizer.py:129-149,231-257 for 16 rows per pair of warps: norm, x / |x| (rounded to the dtype like torch), Y = u Pi^T,
 // bucket search, residual in rotated space r' = (Y - c) + E, E = (x / |x| - u) Pi^T, sign bits of r' M^T with M = S Pi^T.
@@ -365,7 +292,6 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
     constexpr int HALF = KSTEPS / 2;           // k-steps, and blocks of 16 columns, of one warp of the pair
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ float s_ss[R_ROWS], s_n2[2][R_ROWS];
-    __shared__ uint32_t s_redo[R_GROUPS][2];
     const int tid = threadIdx.x, group = (tid >> 5) & (R_GROUPS - 1), mine = tid >> 8, lane = tid & 31, gid = lane >> 2, tig = lane & 3;
 #pragma unroll 1
     for (int i = 0; i < 2; ++i) load_operand(smem + i * R_MAT, p.pi[i], tid, R_THREADS);
@@ -387,7 +313,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
     for (int64_t tile = blockIdx.x; tile * R_ROWS < p.n; tile += gridDim.x) {
         const int64_t base_row = tile * R_ROWS + group * 16, r0 = base_row + gid, r1 = r0 + 8;
         {   // the pair's rows, whole lines at a time, into the place of the fragments: chunks of 16 bytes, swizzled by row (each lane
-            // fetching its own pairs of numbers from global memory, twice over with the norms: 29.5 us, now 28.9; fp16 33.2, now 31.8)
+            // fetching its own pairs of numbers from global memory, twice over with the norms, added 0.6 us to 28.9, of fp16 1.4 to 31.8)
             constexpr int CHUNKS = 16 * RB / 16 / 64;   // of one thread
             uint4 v[CHUNKS];
 #pragma unroll
@@ -483,7 +409,6 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
         // ---- codes, r' as limbs in the A layout of the second product ----
         uint32_t cw[2][MSE_BITS == 2 ? 1 : 2] = {};   // this warp's code words of the two rows, word j in lane j % 4
         float rn2[2] = {0.f, 0.f};
-        uint32_t near = 0;                            // coordinates next to a boundary, bit 8 * j + 4 * n8 + c
 #pragma unroll 1
         for (int j = 0; j < HALF; ++j) {
             const int nb = mine * HALF + j;
@@ -499,6 +424,39 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
                     mma_f16(er[1], a[1][ks], b[2], b[3]);
                 }
             }
+            uint32_t near = 0;   // of the lane's eight: those next to a boundary, whose side the fp32 store kernel's chain decides
+#pragma unroll
+            for (int n8 = 0; n8 < 2; ++n8)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float gap = 1.f;
+#pragma unroll
+                    for (int i = 0; i < NB; ++i) gap = fminf(gap, fabsf(acc[n8][c] * (1.f / (R_SCALE * R_SCALE)) - p.cb.boundaries[i]));
+                    if (gap < NEAR) near |= 1u << (n8 * 4 + c);
+                }
+            if (r0 >= p.n || nd[0] == 0.f) near &= 0xccu;
+            if (r1 >= p.n || nd[1] == 0.f) near &= 0x33u;
+            if (__any_sync(0xffffffffu, near != 0)) {
+#pragma unroll 1
+                for (uint32_t who; (who = __ballot_sync(0xffffffffu, near != 0)) != 0;) {
+                    const int from = __ffs(who) - 1;   // this lane's next coordinate, for the whole warp
+                    const int bit = __shfl_sync(0xffffffffu, __ffs(near) - 1, from);
+                    const int64_t row = base_row + (from >> 2) + (bit & 2 ? 8 : 0);
+                    const float y = serial_product<DT>(p.x, row * p.stride_row, __shfl_sync(0xffffffffu, bit & 2 ? den[1] : den[0], from),
+                                                       p.pi_t + nb * 16 + (bit >> 2) * 8 + 2 * (from & 3) + (bit & 1), lane);
+                    if (lane == from) {
+                        near &= near - 1;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {   // where it decides differently, it is what is coded
+                            float& had = acc[i >> 2][i & 3];
+                            int k = 0;
+#pragma unroll
+                            for (int b = 0; b < NB; ++b) k += (p.cb.boundaries[b] < y) - (p.cb.boundaries[b] < had * (1.f / (R_SCALE * R_SCALE)));
+                            if (i == bit && k != 0) had = y * (R_SCALE * R_SCALE);
+                        }
+                    }
+                }
+            }
             uint32_t word[2] = {0u, 0u}, rl[2][4];
 #pragma unroll
             for (int n8 = 0; n8 < 2; ++n8) {
@@ -508,17 +466,13 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
                 for (int c = 0; c < 4; ++c) {
                     const float y = acc[n8][c] * (1.f / (R_SCALE * R_SCALE));
                     uint32_t k = 0;
-                    float cv = p.cb.centroids[0], gap = 1.f;
+                    float cv = p.cb.centroids[0];
 #pragma unroll
-                    for (int i = 0; i < NB; ++i) {
-                        const float d = y - p.cb.boundaries[i];
-                        gap = fminf(gap, fabsf(d));
-                        if (d > 0.f) {
+                    for (int i = 0; i < NB; ++i)
+                        if (p.cb.boundaries[i] < y) {
                             k = i + 1;
                             cv = p.cb.centroids[i + 1];
                         }
-                    }
-                    if (gap < NEAR) near |= (1u << (n8 * 4 + c)) << (8 * j);
                     if (y != y) {   // searchsorted orders NaN after every number
                         k = NB;
                         cv = p.cb.centroids[NB];
@@ -591,47 +545,15 @@ __global__ void __launch_bounds__(R_THREADS, 1) tq_rows_quantize_keys_kernel(con
 #pragma unroll
             for (int q = 0; q < CB / 32; ++q) *reinterpret_cast<uint32_t*>(p.codes + row * CB + mine * (CB / 2) + 16 * q + 4 * tig) = cw[r2][q];
         }
-        // ---- coordinates next to a boundary, by the fp32 store kernel's chain; a row where it decides differently is redone ----
-        if (r0 >= p.n || nd[0] == 0.f) near &= 0xccccccccu;
-        if (r1 >= p.n || nd[1] == 0.f) near &= 0x33333333u;
-        uint32_t redo = 0;   // rows of the pair's sixteen
-        if (__any_sync(0xffffffffu, near != 0)) {
-            __syncwarp();   // the warp's codes, read back below
-#pragma unroll 1
-            for (uint32_t who; (who = __ballot_sync(0xffffffffu, near != 0)) != 0;) {
-                const int from = __ffs(who) - 1;   // this lane's next coordinate, for the whole warp
-                const int bit = __shfl_sync(0xffffffffu, __ffs(near) - 1, from);
-                if (lane == from) near &= near - 1;
-                const int col = mine * (RD / 2) + (bit >> 2) * 8 + 2 * (from & 3) + (bit & 1), rw = (from >> 2) + (bit & 2 ? 8 : 0);
-                const int64_t row = base_row + rw;
-                const float y = serial_product<DT>(p.x, row * p.stride_row, __shfl_sync(0xffffffffu, bit & 2 ? den[1] : den[0], from), p.pi_t + col, lane);
-                int k = 0;
+        pair_sync(group);   // both halves of the residual norms are written
+        if (mine == 0 && tig == 3) {
 #pragma unroll
-                for (int i = 0; i < NB; ++i) k += p.cb.boundaries[i] < y ? 1 : 0;
-                constexpr int PER = MSE_BITS == 2 ? 4 : 2, W = 8 / PER;
-                const int had = (*(volatile const uint8_t*)(p.codes + row * (RD / PER) + col / PER) >> (W * (col % PER))) & ((1 << W) - 1);
-                if (k != had) redo |= 1u << rw;
-            }
-        }
-        if (lane == 0) s_redo[group][mine] = redo;
-        pair_sync(group);   // both halves of every row are written
-        if (mine == 0) {
-            if (tig == 3)
-#pragma unroll
-                for (int r2 = 0; r2 < 2; ++r2) {
-                    const int64_t row = r2 ? r1 : r0;
-                    const float n2 = s_n2[0][group * 16 + gid + 8 * r2] + s_n2[1][group * 16 + gid + 8 * r2];
-                    if (row >= p.n) continue;
-                    tq_store_any(p.norms, row, __half2float(__float2half_rn(nd[r2])), p.norm_dt);
-                    tq_store_any(p.rnorms, row, nd[r2] == 0.f ? 0.f : __half2float(__float2half_rn(nd[r2] * __fsqrt_rn(n2))), p.rnorm_dt);
-                }
-            __syncwarp();   // redo_row writes a residual norm again
-            redo = s_redo[group][0] | s_redo[group][1];
-#pragma unroll 1
-            for (; redo != 0; redo &= redo - 1) {
-                const int rw = __ffs(redo) - 1, from = 4 * (rw & 7);
-                redo_row<DT, MSE_BITS>(p, base_row + rw, __shfl_sync(0xffffffffu, rw & 8 ? nd[1] : nd[0], from),
-                                       __shfl_sync(0xffffffffu, rw & 8 ? den[1] : den[0], from), sm, lane);
+            for (int r2 = 0; r2 < 2; ++r2) {
+                const int64_t row = r2 ? r1 : r0;
+                const float n2 = s_n2[0][group * 16 + gid + 8 * r2] + s_n2[1][group * 16 + gid + 8 * r2];
+                if (row >= p.n) continue;
+                tq_store_any(p.norms, row, __half2float(__float2half_rn(nd[r2])), p.norm_dt);
+                tq_store_any(p.rnorms, row, nd[r2] == 0.f ? 0.f : __half2float(__float2half_rn(nd[r2] * __fsqrt_rn(n2))), p.rnorm_dt);
             }
         }
     }

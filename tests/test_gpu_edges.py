@@ -194,3 +194,52 @@ def test_ring_is_filled_from_a_paged_cache(bs, dtype, dev):
         a, b = both
         assert (a.ring.size, a.ring.total_written, a.store.num_tokens) == (b.ring.size, b.ring.total_written, b.store.num_tokens)
         assert all(torch.equal(x, y) for x, y in zip(a.ring.peek(), b.ring.peek())), (n, held)
+
+
+@pytest.mark.parametrize("d,bits", [(128, 3), (128, 4), (256, 3), (256, 4)])
+@pytest.mark.parametrize("mid", [0.0, 1e-25, -2e-25, 9e-26, -1e-30, 1e-39])
+def test_store_with_a_middle_boundary_next_to_zero(d, bits, mid, dev):
+    """The tensor-core kernels scale differences up and flush what is below the normal numbers, so a code book whose middle
+    boundary lies between 0 and 1e-25 is the fp32 kernel's, byte for byte.  With others at most 1e-4 of the codes and of the
+    sign bits differ, as with any code book: a byte holds up to four codes, or eight bits."""
+    from turboquant_b200 import _engine as E
+    n, h = 300, 2
+    base = E.LayerConstants(d, bits, 2, dev)
+    edges = base.boundaries_cpu.clone()
+    edges[len(edges) // 2] = mid
+    g = torch.Generator(device=dev).manual_seed(d + bits)
+    k, v = (torch.randn(n, h, d, generator=g, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    pools = []
+    for fast in (True, False):
+        c = E.LayerConstants(d, bits, 2, dev, centroids=base.centroids_cpu, boundaries=edges, tensor_core_store=fast)
+        pool = E.BlockPool(c, h, E.blocks_for(n))
+        E.store(c, pool, k, v, stride_token=h * d, stride_head=d, n_tokens=n, n_heads=h,
+                block_table=E.identity_block_table(E.blocks_for(n), dev))
+        pools.append((pool.data[:E.blocks_for(n) * h * c.block_bytes].clone(),
+                      E.pool_to_planes(c, pool, E.identity_block_table(E.blocks_for(n), dev), n)))
+    (a, pa), (b, pb) = pools
+    if 0 < abs(mid) < 1e-25:
+        assert torch.equal(a, b)
+    assert float((pa.mse_indices[:, :n] != pb.mse_indices[:, :n]).float().mean()) <= 4e-4
+    assert float((pa.qjl_signs[:, :n] != pb.qjl_signs[:, :n]).float().mean()) <= 8e-4
+
+
+@pytest.mark.parametrize("d,kb,vb", [(128, 3, 2), (128, 4, 4), (256, 3, 2), (256, 4, 2)])
+def test_store_right_behind_the_call_that_writes_its_last_row(d, kb, vb, dev):
+    """The decode call writes a token into the ring and the store behind it, which begins under it, reads that row."""
+    from turboquant_b200 import CompressedKVStore, KVCaptureEngine
+    h, cap, n = 2, 48, 4000
+    g = torch.Generator(device=dev).manual_seed(d + kb)
+    k, v = (torch.randn(n + cap, h, d, generator=g, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    q = torch.randn(1, 4 * h, d, generator=g, device=dev, dtype=torch.bfloat16)
+    want = CompressedKVStore(d, h, kb, vb, device=dev, capacity_tokens=n + cap)
+    for lo, hi in ((0, n), (n, n + cap)):
+        want.append_chunk(k[lo:hi], v[lo:hi])
+    size = (n + cap) // 16 * h * want.consts.block_bytes
+    for _ in range(10):
+        engine = KVCaptureEngine(CompressedKVStore(d, h, kb, vb, device=dev, capacity_tokens=n + cap), ring_capacity=cap, device=dev)
+        engine.store.append_chunk(k[:n], v[:n])
+        engine.ingest_decode(k[n:-1], v[n:-1], cap - 1)
+        engine.decode_step(q, k[-1:], v[-1:], 4 * h)
+        engine.flush()
+        assert torch.equal(engine.store.pool.data[:size], want.pool.data[:size])

@@ -35,14 +35,19 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 // Warps per CTA.  A launch that fits one wave runs 12-warp CTAs, one per SM (all of an SM's warps
 // share one set of query fragments and one merge).  A launch of several waves runs 8-warp CTAs, two
 // per SM, so that the set-up and the merge of one CTA overlap the main loop of the other.
-// At head_dim 128 a single sequence whose query lies in host memory runs 16 warps an SM: 128 registers are enough there, and
-// the ring's CTAs fetch the query from the host, the more at a time the more threads.  Steps of decode_step_host, sixteen warps /
-// twelve: 0.94 to 0.99 (13.0 us for 13.7 at 4000 tokens of 8 heads, 17.3 for 17.6 at 16000; two sets of fragments 16.6 for 17.3).
-// With everything on the device they are no faster: 1.00 to 1.01 with the ring's tokens a warp each, 1.06 with 3-bit codes.  At
-// head_dim 256 sixteen warps cost registers.
+// At head_dim 128 a single sequence runs 16 warps an SM where its ring fills a second pass of 32 tokens and a CTA has few records,
+// and wherever its query lies in host memory: 128 registers are enough there.  With the data on the device that is for exactness:
+// the largest probability of each warp is 1 and exact in fp16, so sixteen warps leave less to round than twelve (fp32 queries, 24
+// sequences of 4096 tokens and 77 in the ring: 3.68e-4 of the output against 64 bits, twelve 3.77e-4; 12000 tokens 4.44e-4 and
+// 4.52e-4).  It costs 1.00 to 1.01 of twelve's time with one set of fragments (4096 tokens 9.33 us for 9.30), 1.00 to 1.06 with two
+// (10.6 for 10.1).
+// With the query in host memory the ring's CTAs fetch it from there, the more at a time the more threads: steps of
+// decode_step_host, sixteen / twelve, 0.94 to 0.99 (13.0 us for 13.7 at 4000 tokens of 8 heads, 17.3 for 17.6 at 16000; two
+// sets of fragments 16.6 for 17.3).  At head_dim 256 sixteen warps cost registers.
 constexpr int NW_WAVE = 12;
 constexpr int NW_SINGLE = 16;
 constexpr int NW_MULTI = 8;
+constexpr int SINGLE_RING = 33, SINGLE_RECORDS = 48;   // at least so many ring tokens, at most so many records a CTA
 constexpr int BT_MAX = 1024;   // block-table entries a CTA keeps in shared memory
 
 
@@ -953,7 +958,7 @@ int launch_mma(const DecodeParams& p, int batch, cudaStream_t st, int* handled) 
         return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_MULTI>(p, batch, st);
     }
     if constexpr (D == 128)
-        if (batch == 1 && p.host_io && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
+        if (batch == 1 && (p.host_io || (p.max_ring_len >= SINGLE_RING && records <= SINGLE_RECORDS)) && mma_smem_bytes<D, SPLITB, NW_SINGLE>(L.block_bytes, nslot) <= SMEM_PER_CTA_MAX)
             return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_SINGLE>(p, batch, st);
     if (fits_wave) return launch_mma_nw<D, MSE_BITS, VAL_BITS, SPLITB, NW_WAVE>(p, batch, st);
     *handled = 0;

@@ -243,3 +243,46 @@ def test_store_right_behind_the_call_that_writes_its_last_row(d, kb, vb, dev):
         engine.decode_step(q, k[-1:], v[-1:], 4 * h)
         engine.flush()
         assert torch.equal(engine.store.pool.data[:size], want.pool.data[:size])
+
+
+def _others_launch(dev, streams):
+    """Something of the library on each of the streams."""
+    from turboquant_b200.kv_cache import quantize_values
+    v = torch.randn(1, 4, 128, device=dev, dtype=torch.bfloat16)
+    for s in streams:
+        with torch.cuda.stream(s):
+            quantize_values(v, bits=2)
+
+
+@pytest.mark.parametrize("d,kb,vb", [(128, 3, 2), (256, 4, 4)])
+def test_scores_right_behind_a_store_with_nine_streams_between(d, kb, vb, dev):
+    """A store lets what follows on its stream begin at once.  With queued work in front of it and launches on more streams than
+    are kept in mind behind it, neither the cache object nor the decode may read records that are not written."""
+    from turboquant_b200 import CompressedKVStore, TurboQuantKVCache, compute_hybrid_attention
+    n, h = 3000, 4
+    g = torch.Generator(device=dev).manual_seed(d + kb)
+    k, v = (torch.randn(1, h, n, d, generator=g, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    q = torch.randn(1, h, 1, d, generator=g, device=dev, dtype=torch.bfloat16)
+    qd = torch.randn(1, 4 * h, d, generator=g, device=dev, dtype=torch.bfloat16)
+    rows_k, rows_v = (t[0].transpose(0, 1) for t in (k, v))
+    mine, *others = (torch.cuda.Stream(dev) for _ in range(10))
+    _others_launch(dev, others)
+    torch.cuda.synchronize()
+    for _ in range(8):
+        cache = TurboQuantKVCache(d, kb, vb, buffer_size=8, device=dev, dtype=torch.bfloat16)
+        store = CompressedKVStore(d, h, kb, vb, device=dev, capacity_tokens=n)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(mine):
+            torch.cuda._sleep(4_000_000)          # about 2 ms, so that everything below is queued behind it
+            cache.prefill(k, v)
+        _others_launch(dev, others)
+        with torch.cuda.stream(mine):
+            logits = cache.attention_scores(q)
+            torch.cuda._sleep(4_000_000)
+            store.append_chunk(rows_k, rows_v)
+        _others_launch(dev, others)
+        with torch.cuda.stream(mine):
+            out = compute_hybrid_attention(qd, store, None, None, 4 * h)
+        torch.cuda.synchronize()
+        assert torch.equal(logits, cache.attention_scores(q))
+        assert torch.equal(out, compute_hybrid_attention(qd, store, None, None, 4 * h))

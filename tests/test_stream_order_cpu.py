@@ -1,0 +1,121 @@
+"""What may begin before the launch ahead has finished (csrc/tq_stream_order.h), stepped through on the CPU for every
+sequence of the library's launches on a stream, with other streams' notes taking the place of this one's anywhere between.
+
+The model of a launch follows the places that launch it: whether it is a programmatic dependent, whether it lets its own
+dependents begin at entry, after its wait or only by finishing, what it writes, and whether it reads the pool or rows in front of
+its wait.  What a launch wrote is there for an early reader only if some launch in between has waited for it.
+"""
+
+import ctypes as C
+import itertools
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "turboquant_b200", "csrc")
+UNKNOWN, DECODE, STORE_EARLY, NEUTRAL, PREP_BEHIND_STORE, WAITED = range(6)
+GLUE = """
+#include "tq_stream_order.h"
+extern "C" {
+int kind_of_prep(int k) { return tq_kind_of_prep(k); }
+int may_overlap(int k) { return tq_reader_may_overlap(k); }
+int pool_is_late(int k) { return tq_pool_is_late(k); }
+int rows_at_rest(int k) { return tq_rows_are_at_rest(k); }
+void* notes_new() { return new TqStreamNotes; }
+void notes_free(void* n) { delete static_cast<TqStreamNotes*>(n); }
+void note(void* n, unsigned long st, int k) { static_cast<TqStreamNotes*>(n)->note(reinterpret_cast<const void*>(st), k); }
+int last(void* n, unsigned long st) { return static_cast<TqStreamNotes*>(n)->last(reinterpret_cast<const void*>(st)); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("stream_order")
+    (d / "glue.cpp").write_text(GLUE)
+    subprocess.run([os.environ.get("CXX", "g++"), "-std=c++17", "-O1", "-shared", "-fPIC", "-I", CSRC, "-o", str(d / "glue.so"), str(d / "glue.cpp")],
+                   check=True)
+    lib = C.CDLL(str(d / "glue.so"))
+    lib.notes_new.restype = C.c_void_p
+    lib.notes_free.argtypes = [C.c_void_p]
+    lib.note.argtypes = [C.c_void_p, C.c_ulong, C.c_int]
+    lib.last.argtypes = [C.c_void_p, C.c_ulong]
+    return lib
+
+
+def _launch(r, name, ahead):
+    """(programmatic, lets others begin, writes, reads early, note or None) of a launch behind one noted as `ahead`."""
+    if name == "store":
+        late = not r.rows_at_rest(ahead)
+        return True, "waited" if late else "entry", "pool", None if late else "rows", STORE_EARLY
+    if name == "ring write":
+        return True, "waited", "rows", None, DECODE
+    if name == "prepare":                     # may append a row to the ring
+        return True, "entry", "rows", None, r.kind_of_prep(ahead)
+    if name == "decode":
+        prog, late = bool(r.may_overlap(ahead)), bool(r.pool_is_late(ahead))
+        return prog, "waited" if late else "entry", None, "pool" if prog and not late else None, DECODE
+    if name == "cache scores":
+        return True, "done", None, None if r.pool_is_late(ahead) else "pool", None
+    if name == "cache attend":
+        return True, "done", None, None, WAITED
+    if name == "plain rows":
+        return True, "waited", "rows", None, WAITED
+    assert name == "prefill"
+    return False, "entry", None, None, NEUTRAL
+
+
+LAUNCHES = ("store", "ring write", "prepare", "decode", "cache scores", "cache attend", "plain rows", "prefill")
+
+
+def _run(r, steps):
+    """None, or what went wrong."""
+    notes, loose = r.notes_new(), set()
+    try:
+        for name in steps:
+            if name == "others":              # eight other streams launch something
+                for st in range(100, 108):
+                    r.note(notes, st, DECODE)
+                continue
+            prog, begin, writes, early, kind = _launch(r, name, r.last(notes, 7))
+            if prog and early in loose:
+                return "%s reads %s that may not be written" % (name, early)
+            loose = (loose if prog and begin == "entry" else set()) | ({writes} if writes else set())
+            if kind is not None:
+                r.note(notes, 7, kind)
+    finally:
+        r.notes_free(notes)
+    return None
+
+
+def test_nobody_reads_early_what_may_not_be_written(rules):
+    wrong = []
+    for n in range(1, 6):
+        for steps in itertools.product(LAUNCHES + ("others",), repeat=n):
+            bad = _run(rules, steps)
+            if bad:
+                wrong.append((steps, bad))
+                if len(wrong) > 3:
+                    break
+    assert not wrong, wrong
+
+
+@pytest.mark.parametrize("reader", ["decode", "cache scores"])
+def test_readers_overlap_where_the_pool_is_known_to_be_at_rest(rules, reader):
+    """The usual steps keep their early reads: behind another step, a ring write, attention of the cache object or a prefill."""
+    for ahead in (DECODE, NEUTRAL, WAITED):
+        kind = rules.kind_of_prep(ahead)
+        assert kind == DECODE and _launch(rules, reader, kind)[3] == "pool"
+    assert rules.rows_at_rest(STORE_EARLY) and rules.rows_at_rest(NEUTRAL)
+
+
+def test_notes_keep_the_last_eight_streams(rules):
+    notes = rules.notes_new()
+    for st in range(1, 9):
+        rules.note(notes, st, STORE_EARLY)
+    rules.note(notes, 3, DECODE)
+    assert [rules.last(notes, st) for st in (1, 3, 8)] == [STORE_EARLY, DECODE, STORE_EARLY]
+    rules.note(notes, 9, NEUTRAL)
+    assert rules.last(notes, 1) == UNKNOWN and rules.last(notes, 9) == NEUTRAL and rules.last(notes, 2) == STORE_EARLY
+    rules.notes_free(notes)

@@ -26,7 +26,7 @@ def sources() -> list[str]:
 
 def needs_build() -> bool:
     headers = glob.glob(os.path.join(INCLUDE, "*.h"))
-    return (_stale(LIB_PATH, sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + headers)
+    return (_stale(LIB_PATH, sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + headers)
             or _stale(HOST_PATH, [HOST_SRC] + headers))
 
 

@@ -1,6 +1,4 @@
 // Host-only entry points: configuration checks, layout queries, messages.
-#include <mutex>
-
 #include "tq_common.cuh"
 
 int tq_check_config(const tq_config* cfg) {
@@ -30,38 +28,17 @@ int tq_sm_count() {
 }
 
 namespace {
-struct StreamNote {
-    cudaStream_t st;
-    int kind;
-};
-std::mutex g_note_mu;
-StreamNote g_notes[TQ_MAX_DEVICES][8];
-int g_note_count[TQ_MAX_DEVICES], g_note_next[TQ_MAX_DEVICES];
+TqStreamNotes g_notes[TQ_MAX_DEVICES];
 }  // namespace
 
 void tq_note_launch(cudaStream_t st, int kind) {
     const int dev = tq_current_device();
-    if (dev < 0 || dev >= TQ_MAX_DEVICES) return;
-    std::lock_guard<std::mutex> lock(g_note_mu);
-    for (int i = 0; i < g_note_count[dev]; ++i)
-        if (g_notes[dev][i].st == st) {
-            g_notes[dev][i].kind = kind;
-            return;
-        }
-    const int slot = g_note_next[dev];
-    g_notes[dev][slot] = StreamNote{st, kind};
-    g_note_next[dev] = (slot + 1) % 8;
-    if (g_note_count[dev] < 8) ++g_note_count[dev];
+    if (dev >= 0 && dev < TQ_MAX_DEVICES) g_notes[dev].note(st, kind);
 }
 
-// Kind of the library's latest launch on the stream (a stream never noted, or whose note was displaced: unknown).
 int tq_last_launch(cudaStream_t st) {
     const int dev = tq_current_device();
-    if (dev < 0 || dev >= TQ_MAX_DEVICES) return TQ_LAUNCH_UNKNOWN;
-    std::lock_guard<std::mutex> lock(g_note_mu);
-    for (int i = 0; i < g_note_count[dev]; ++i)
-        if (g_notes[dev][i].st == st) return g_notes[dev][i].kind;
-    return TQ_LAUNCH_UNKNOWN;
+    return dev >= 0 && dev < TQ_MAX_DEVICES ? g_notes[dev].last(st) : TQ_LAUNCH_UNKNOWN;
 }
 
 extern "C" int tq_get_layout(const tq_config* cfg, tq_layout* out) {

@@ -382,7 +382,7 @@ extern "C" int tq_cache_scores(const tq_consts* consts, const tq_pool* pool, con
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    p.pool_late = tq_last_launch(st) == TQ_LAUNCH_PREP_BEHIND_STORE ? 1 : 0;
+    p.pool_late = tq_pool_is_late(tq_last_launch(st));
     const int gp = n_q > 4 ? 8 : n_q > 2 ? 4 : n_q;
     cfg.gridDim = dim3((unsigned)(tiles(n_tokens, CA_TOK) + tiles(n_buf, CA_TOK)), (unsigned)p.H, (unsigned)tiles(n_q, gp));
     cfg.blockDim = dim3(128);
@@ -432,7 +432,7 @@ extern "C" int tq_cache_attend(const tq_consts* consts, const tq_pool* pool, con
     cfg.gridDim = dim3((unsigned)p.splits, (unsigned)p.H, (unsigned)zs);
     cfg.blockDim = dim3(AT_THREADS);
     cfg.stream = st;
-    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+    tq_note_launch(st, TQ_LAUNCH_WAITED);
     const int kb = consts->cfg.key_bits, vb = consts->cfg.value_bits;
     cudaError_t e = cudaSuccess;
 #define TQ_CA(DD, VB)                                                                             \

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "turboquant_b200.h"
+#include "tq_stream_order.h"
 
 #define TQ_HD __host__ __device__ __forceinline__
 
@@ -221,34 +222,10 @@ constexpr int TQ_MAX_DEVICES = 64;
 int tq_current_device();   // ordinal of the calling thread's current device, -1 on error
 int tq_sm_count();         // multiprocessors of the current device (148 when the query fails)
 
-// Which of the library's kernels was launched last on a stream.  Several kernels let the launch behind them
-// begin before they have finished (programmatic dependent launch) and do part of their work before they wait
-// for the launch ahead; that is only safe when the launch still in flight cannot be writing what is read early:
-//   * the tensor-core store kernels fetch their key / value rows before the wait.  The decode family appends
-//     the new token to the ring - rows a flush then reads - so a store behind a decode launch only asks for its
-//     constant operands early, waits in front of its first row and lets its own dependents begin after that;
-//   * the decode family reads sequence lengths, block tables and the first pool records before the wait.
-//     The tensor-core store kernels write the pool and let their dependents begin at once.  The query
-//     preparation reads nothing that they write and may start under them; the decode kernel behind it is
-//     then told to wait before its first record (and to let its own dependents begin only after that, so
-//     that no later kernel's early reads reach back to the store).  A decode kernel directly behind a
-//     store is launched in plain stream order.
-// Kernels of other libraries between two of ours never start early and only make the order stricter; a
-// stream the library has not seen counts as unknown.
-enum TqLaunchKind { TQ_LAUNCH_UNKNOWN = 0, TQ_LAUNCH_DECODE = 1, TQ_LAUNCH_STORE_EARLY = 2, TQ_LAUNCH_NEUTRAL = 3, TQ_LAUNCH_PREP_BEHIND_STORE = 4 };
+// the library's latest launch on a stream of the current device (tq_stream_order.h has the rules)
 void tq_note_launch(cudaStream_t st, int kind);
 int tq_last_launch(cudaStream_t st);
-// notes a launch that prepares a decode call (and neither reads nor writes the pool)
-inline void tq_note_prep_launch(cudaStream_t st) {
-    const int k = tq_last_launch(st);
-    tq_note_launch(st, k == TQ_LAUNCH_STORE_EARLY || k == TQ_LAUNCH_PREP_BEHIND_STORE ? TQ_LAUNCH_PREP_BEHIND_STORE : TQ_LAUNCH_DECODE);
-}
-// programmatic-launch attribute count (0 or 1) for a kernel of the decode family / whether a store may read its rows early
-inline int tq_pdl_for_decode(cudaStream_t st) { return tq_last_launch(st) == TQ_LAUNCH_STORE_EARLY ? 0 : 1; }
-inline int tq_pdl_for_store(cudaStream_t st) {
-    const int k = tq_last_launch(st);
-    return (k == TQ_LAUNCH_STORE_EARLY || k == TQ_LAUNCH_NEUTRAL) ? 1 : 0;
-}
+inline void tq_note_prep_launch(cudaStream_t st) { tq_note_launch(st, tq_kind_of_prep(tq_last_launch(st))); }
 
 // Largest dynamic shared-memory size a kernel has been opted in for, per device.
 // A paged bf16 cache as the source of a store call (see tq_store_paged).

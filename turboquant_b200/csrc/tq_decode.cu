@@ -851,7 +851,7 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     p.ring_splits = rsplits;
     p.ring_tok = ring_tok;
     p.host_io = early_inputs;
-    p.pool_late = tq_last_launch(st) == TQ_LAUNCH_PREP_BEHIND_STORE ? 1 : 0;
+    p.pool_late = tq_pool_is_late(tq_last_launch(st));
 
     const int mse_bits = consts->cfg.key_bits - 1, vb = consts->cfg.value_bits;
     if (a->kernel != 1) {   // tensor-core kernel where it applies

@@ -777,7 +777,7 @@ int launch_rows(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t st,
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    tq_note_launch(st, TQ_LAUNCH_UNKNOWN);
+    tq_note_launch(st, TQ_LAUNCH_WAITED);
     return cudaLaunchKernelEx(&cfg, kern, args...) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
 }
 

@@ -1605,7 +1605,7 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     lc.attrs = attr;
     lc.numAttrs = 1;
-    p.rows_late = tq_pdl_for_store(st) ? 0 : 1;   // behind a decode launch (ring append) and others
+    p.rows_late = !tq_rows_are_at_rest(tq_last_launch(st));   // behind a decode launch (ring append) and others
     tq_note_launch(st, TQ_LAUNCH_STORE_EARLY);
     lc.stream = st;
     lc.gridDim = dim3(grid);

@@ -286,3 +286,30 @@ def test_scores_right_behind_a_store_with_nine_streams_between(d, kb, vb, dev):
         torch.cuda.synchronize()
         assert torch.equal(logits, cache.attention_scores(q))
         assert torch.equal(out, compute_hybrid_attention(qd, store, None, None, 4 * h))
+
+
+@pytest.mark.parametrize("d,kb,vb", [(128, 3, 2), (256, 4, 4)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32, torch.bfloat16])
+def test_scores_right_behind_a_flush(d, kb, vb, dtype, dev):
+    """History, scores and output with nothing launched in between, over a pool that grows on the way, and the same again once
+    everything is at rest."""
+    from turboquant_b200 import TurboQuantKVCache
+    h, n = 2, 2600
+    g = torch.Generator(device=dev).manual_seed(d + kb)
+    k, v = (torch.randn(1, h, n, d, generator=g, device=dev, dtype=dtype) for _ in range(2))
+    q = torch.randn(1, h, 2, d, generator=g, device=dev, dtype=dtype)
+    for _ in range(5):
+        cache = TurboQuantKVCache(d, kb, vb, buffer_size=4, device=dev, dtype=dtype)
+        got = []
+        cache.prefill(k[..., :600, :], v[..., :600, :])
+        for at in (600, 1100, 1101, 2400):       # 1024 tokens of room, then twice that, then more
+            got.append((cache._n_quant, cache.attention_scores(q)))
+            m = {600: 500, 1100: 1, 1101: 1299, 2400: 200}[at]
+            cache.append(k[..., at:at + m, :], v[..., at:at + m, :])
+        last = cache.attention_scores(q)
+        torch.cuda.synchronize()
+        assert cache._n_quant == n - 4
+        full = cache.attention_scores(q)
+        assert torch.equal(last, full)
+        for m, logits in got:
+            assert torch.equal(logits[..., :m], full[..., :m]), m

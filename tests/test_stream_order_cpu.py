@@ -14,7 +14,7 @@ import subprocess
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "turboquant_b200", "csrc")
-UNKNOWN, DECODE, STORE_EARLY, NEUTRAL, PREP_BEHIND_STORE, WAITED = range(6)
+UNKNOWN, DECODE, STORE_EARLY, NEUTRAL, PREP_BEHIND_STORE, WAITED, STORE_PLAIN = range(7)
 GLUE = """
 #include "tq_stream_order.h"
 extern "C" {
@@ -49,6 +49,8 @@ def _launch(r, name, ahead):
     if name == "store":
         late = not r.rows_at_rest(ahead)
         return True, "waited" if late else "entry", "pool", None if late else "rows", STORE_EARLY
+    if name == "fp32 store":                  # and planes into the pool
+        return False, "done", "pool", None, STORE_PLAIN
     if name == "ring write":
         return True, "waited", "rows", None, DECODE
     if name == "prepare":                     # may append a row to the ring
@@ -66,7 +68,7 @@ def _launch(r, name, ahead):
     return False, "entry", None, None, NEUTRAL
 
 
-LAUNCHES = ("store", "ring write", "prepare", "decode", "cache scores", "cache attend", "plain rows", "prefill")
+LAUNCHES = ("store", "fp32 store", "ring write", "prepare", "decode", "cache scores", "cache attend", "plain rows", "prefill")
 
 
 def _run(r, steps):
@@ -107,7 +109,7 @@ def test_readers_overlap_where_the_pool_is_known_to_be_at_rest(rules, reader):
     for ahead in (DECODE, NEUTRAL, WAITED):
         kind = rules.kind_of_prep(ahead)
         assert kind == DECODE and _launch(rules, reader, kind)[3] == "pool"
-    assert rules.rows_at_rest(STORE_EARLY) and rules.rows_at_rest(NEUTRAL)
+    assert all(rules.rows_at_rest(k) for k in (STORE_EARLY, NEUTRAL, STORE_PLAIN))
 
 
 def test_notes_keep_the_last_eight_streams(rules):

@@ -207,6 +207,7 @@ int convert(const tq_config* cfg, const tq_pool* pool, const int32_t* block_tabl
     const int64_t first = start_pos >> 4, last = (start_pos + n_tokens - 1) >> 4;
     dim3 grid((unsigned)(last - first + 1), (unsigned)pool->num_kv_heads);
     const bool words = (((uintptr_t)planes->mse_indices | (uintptr_t)planes->qjl_signs | (uintptr_t)planes->v_data) & 3) == 0;
+    if (TO_POOL) tq_note_launch((cudaStream_t)stream, TQ_LAUNCH_STORE_PLAIN);
     if (words) tq_convert_kernel<TO_POOL, uint32_t><<<grid, 128, 0, (cudaStream_t)stream>>>(p);
     else tq_convert_kernel<TO_POOL, uint8_t><<<grid, 128, 0, (cudaStream_t)stream>>>(p);
     return cudaGetLastError() == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;

@@ -10,7 +10,9 @@
 //     the wait.  The tensor-core store kernels write the pool and let their dependents begin at once.  The query preparation
 //     reads nothing that they write and may start under them; the kernel behind it is then told to wait before its first record
 //     (and to let its own dependents begin only after that, so that no later kernel's early reads reach back to the store).
-//     A decode kernel directly behind a store is launched in plain stream order.
+//     A decode kernel directly behind a store is launched in plain stream order.  The fp32 store and the planes' converter let
+//     nobody begin, but a launch that begins when they have finished has not waited for them either, and only the wait makes
+//     what they wrote visible: the same holds behind them.
 // Kernels of other libraries between two of ours never start early and only make the order stricter.  Of a stream that has no
 // note - the library has not seen it, or other streams' notes took its place - anything may be in flight.
 #pragma once
@@ -24,6 +26,7 @@ enum TqLaunchKind {
     TQ_LAUNCH_NEUTRAL = 3,             // in plain stream order, writes neither rows nor pool
     TQ_LAUNCH_PREP_BEHIND_STORE = 4,   // prepares a call, a store may still be in flight
     TQ_LAUNCH_WAITED = 5,              // writes no pool (rows perhaps), and waits before it lets anyone begin
+    TQ_LAUNCH_STORE_PLAIN = 6,         // writes the pool, in plain stream order, and lets nobody begin before it has finished
 };
 
 // what a launch is noted as that prepares a call (and neither reads nor writes the pool) and lets its dependents begin at once
@@ -31,11 +34,15 @@ inline int tq_kind_of_prep(int ahead) {
     return ahead == TQ_LAUNCH_DECODE || ahead == TQ_LAUNCH_NEUTRAL || ahead == TQ_LAUNCH_WAITED ? TQ_LAUNCH_DECODE : TQ_LAUNCH_PREP_BEHIND_STORE;
 }
 // whether a kernel that reads the pool early may be launched as a programmatic dependent (else: plain stream order) ...
-inline bool tq_reader_may_overlap(int ahead) { return ahead != TQ_LAUNCH_STORE_EARLY && ahead != TQ_LAUNCH_UNKNOWN; }
+inline bool tq_reader_may_overlap(int ahead) {
+    return ahead != TQ_LAUNCH_STORE_EARLY && ahead != TQ_LAUNCH_STORE_PLAIN && ahead != TQ_LAUNCH_UNKNOWN;
+}
 // ... and whether it then has to wait before its first record
 inline bool tq_pool_is_late(int ahead) { return ahead == TQ_LAUNCH_PREP_BEHIND_STORE || !tq_reader_may_overlap(ahead); }
 // whether a store may read its rows early
-inline bool tq_rows_are_at_rest(int ahead) { return ahead == TQ_LAUNCH_STORE_EARLY || ahead == TQ_LAUNCH_NEUTRAL; }
+inline bool tq_rows_are_at_rest(int ahead) {
+    return ahead == TQ_LAUNCH_STORE_EARLY || ahead == TQ_LAUNCH_STORE_PLAIN || ahead == TQ_LAUNCH_NEUTRAL;
+}
 
 // The notes of one device: the streams noted last, up to eight.
 class TqStreamNotes {

@@ -9,6 +9,7 @@ its wait.  What a launch wrote is there for an early reader only if some launch 
 import ctypes as C
 import itertools
 import os
+import re
 import subprocess
 
 import pytest
@@ -121,3 +122,21 @@ def test_notes_keep_the_last_eight_streams(rules):
     rules.note(notes, 9, NEUTRAL)
     assert rules.last(notes, 1) == UNKNOWN and rules.last(notes, 9) == NEUTRAL and rules.last(notes, 2) == STORE_EARLY
     rules.notes_free(notes)
+
+
+@pytest.mark.parametrize("kernel,begin,first_use", [
+    ("tq_store_tc_kernel", "in the order they are needed", "if (rmw)"),                  # loads and products
+    ("tq_store_tc_kernel", "compute warps ====", "bool ok = phase_n_and_arrive(0"),
+    ("tq_store_tc256_kernel", "if (warp == TC_THREADS / 32) {\n", "wait1(bar_n"),         # products
+    ("tq_store_tc256_kernel", "int loaded = 0;", "issue_rows(sA0"),                       # loads; the operands' first boxes wait for nobody
+    ("tq_store_tc256_kernel", "compute warps ====", "const int64_t tok0 = tile_tok0(tile);"),
+])
+def test_every_warp_of_a_late_store_waits_for_the_launch_ahead_first(kernel, begin, first_use):
+    """The waits on barriers are bounded, and their bound is meant for the kernel's own phases: behind a launch that may be
+    writing rows no warp of a store polls a barrier before it has waited for that launch.  Read from the source, role by role."""
+    text = open(os.path.join(CSRC, "tq_store_tc.cu")).read()
+    body = text[text.index(kernel + "("):]
+    body = body[body.index("issuing"):]
+    body = body[body.index(begin):]
+    body = body[:body.index(first_use)]
+    assert re.search(r"if \(p\.rows_late\)[\s{].*(pool_writes_may_begin|rows_may_be_read)\(\)", body, re.S), body

@@ -1014,7 +1014,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem, 0);
         auto wait1 = [&](uint64_t* bar, uint32_t parity) -> bool {
             uint32_t ok = 0;
-            for (int i = 0; i < (1 << 20); ++i) {
+            for (int i = 0; i < (1 << 22); ++i) {
                 if (tq_mbar_try_wait(bar, parity)) {
                     ok = 1;
                     break;
@@ -1121,6 +1121,7 @@ tq_store_tc256_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_con
         if (warp == TC_THREADS / 32) {
             bool ok = true;
             int i = 0, used = 0;
+            if (p.rows_late) pool_writes_may_begin();   // the bound of its waits is for this kernel's own phases
 #pragma unroll 1
             for (int tile = tile0; tile < p.n_tiles && ok; tile += (int)gridDim.x, ++i) {
                 if (!(ok = wait1(bar_n, i & 1))) break;              // u, e' in shared memory

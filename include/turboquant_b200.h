@@ -234,13 +234,23 @@ int tq_store_paged_any(const tq_consts* consts, const void* key_cache, const voi
 
 /* `n_tokens` tokens from position `first_token` of a sequence in such a cache
  * (any block size, any dtype) into the ring at `position`, key and value in one
- * launch; a token whose block index is out of range is left out and reported by
- * tq_store_read_status.  Planes, strides and rows 16-byte aligned. */
+ * launch; a token whose block index is out of range becomes zeros and is reported
+ * by tq_store_read_status.  Planes, strides and rows 16-byte aligned. */
 int tq_ring_write_paged(const void* key_cache, const void* value_cache, tq_dtype dtype, int64_t src_num_blocks,
                         int32_t src_block_size, int32_t n_heads, int32_t head_dim, int64_t stride_block,
                         int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t first_token,
                         int64_t n_tokens, void* ring_k, void* ring_v, int64_t ring_stride_token, int64_t position,
                         void* stream);
+
+/* The same; such a token also sets *report to `report_value`.  `report` is memory
+ * the device can write (mapped host memory, to be looked at without a
+ * synchronisation) that outlives the launch, or NULL. */
+int tq_ring_write_paged_reported(const void* key_cache, const void* value_cache, tq_dtype dtype,
+                                 int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int32_t head_dim,
+                                 int64_t stride_block, int64_t stride_token, int64_t stride_head,
+                                 const int32_t* src_block_table, int64_t first_token, int64_t n_tokens, void* ring_k,
+                                 void* ring_v, int64_t ring_stride_token, int64_t position, int32_t* report,
+                                 int32_t report_value, void* stream);
 
 /* Status left by the tensor-core store kernels since the last call: 0, or
  * TQ_ERR_TIMEOUT / TQ_ERR_RANGE if one of their bounded waits ran out or a

@@ -313,3 +313,38 @@ def test_scores_right_behind_a_flush(d, kb, vb, dtype, dev):
         assert torch.equal(last, full)
         for m, logits in got:
             assert torch.equal(logits[..., :m], full[..., :m]), m
+
+
+@pytest.mark.parametrize("bad", [-1, 9, 2 ** 30])
+@pytest.mark.parametrize("n", [20, 75])
+def test_ring_filled_through_a_table_with_a_bad_index(bad, n, dev):
+    """The tokens of that block become zeros - nothing of what the ring held for another sequence - the others arrive, and the
+    engine's next calls raise until it is reset."""
+    from turboquant_b200 import CompressedKVStore, KVCaptureEngine, _engine as E
+    h, d, cap, bs = 2, 128, 32, 16
+    g = torch.Generator(device=dev).manual_seed(n)
+    cache = torch.randn(2, 9, bs, h, d, generator=g, device=dev, dtype=torch.bfloat16)
+    used = (n + bs - 1) // bs
+    table = torch.randperm(9, generator=g, device=dev)[:used].int()
+    wrong = table.clone()
+    wrong[-1] = bad
+    e = KVCaptureEngine(CompressedKVStore(d, h, 3, 2, device=dev), ring_capacity=cap, device=dev)
+    e.ring.write(*(torch.full((cap, h, d), 7.0, device=dev, dtype=torch.bfloat16) for _ in range(2)), cap)
+    for tab in (table, wrong, table):
+        e.reset()
+        e.ingest_prefill_from_paged_cache(cache, n, tab, bs)
+        torch.cuda.synchronize()
+        m = min(n, cap)
+        want = cache[:, table.long()].flatten(1, 2)[:, n - m:n].clone()
+        if tab is wrong:
+            want[:, bs * (used - 1) - n:] = 0
+            row = torch.zeros(1, h, d, device=dev, dtype=torch.bfloat16)
+            q = torch.zeros(1, 4 * h, d, device=dev, dtype=torch.bfloat16)
+            for call in (e.ring.peek, e.flush, e.ring.drain, lambda: e.ingest_decode(row, row, 1), lambda: e.ring.write_one(row, row),
+                         lambda: e.decode_step(q, row, row, 4 * h)):
+                with pytest.raises(IndexError):
+                    call()
+            assert E.store_status() == -7
+        else:
+            assert e.ring.peek()[0].shape[0] == m and E.store_status() == 0
+        assert torch.equal(e.ring._keys[:m], want[0]) and torch.equal(e.ring._values[:m], want[1])

@@ -8,6 +8,7 @@ store and read paths runs in the CUDA library.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import math
 import threading
 from typing import Optional
@@ -321,8 +322,41 @@ def store_paged(consts: LayerConstants, pool: BlockPool, key_cache: torch.Tensor
     return True
 
 
+_REPORT_WORDS = 1024
+_report_page: Optional[torch.Tensor] = None     # page-locked: a launch may write a word as long as the process lives
+_report_ticket = itertools.count(1)
+_report_lock = threading.Lock()
+
+
+class RangeReport:
+    """A word of host memory that a launch sets to a number of its own when it meets an index out of range: looked at
+    without a synchronisation, so an error shows once the launch has run.  Two launches 1024 apart share a word, and the
+    later error then hides the earlier one; neither is taken for the other's."""
+
+    def __init__(self, page: torch.Tensor):
+        self.ticket = next(_report_ticket) & 0x7fffffff
+        self.address = page.data_ptr() + 4 * (self.ticket % _REPORT_WORDS)
+        self._word = C.c_int32.from_address(self.address)
+
+    @property
+    def failed(self) -> bool:
+        return self._word.value == self.ticket
+
+
+def range_report() -> Optional[RangeReport]:
+    """None while the page would have to be made under stream capture."""
+    global _report_page
+    if _report_page is None:
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        with _report_lock:
+            if _report_page is None:
+                _report_page = torch.zeros(_REPORT_WORDS, dtype=torch.int32).pin_memory()
+    return RangeReport(_report_page)
+
+
 def ring_write_paged(ring_k: torch.Tensor, ring_v: torch.Tensor, position: int, key_cache: torch.Tensor, value_cache: torch.Tensor,
-                     src_block_table: torch.Tensor, first: int, n: int) -> bool:
+                     src_block_table: torch.Tensor, first: int, n: int, report: Optional[RangeReport] = None) -> bool:
     """Tokens [first, first + n) of a sequence in a paged cache ((num_blocks, block_size, H, D) planes of one layout,
     `src_block_table` int32, contiguous) into the ring's buffers from `position` on, in one launch.  False, with nothing
     launched, for tensors that the kernel does not take."""
@@ -333,9 +367,10 @@ def ring_write_paged(ring_k: torch.Tensor, ring_v: torch.Tensor, position: int, 
             and min(key_cache.stride()) >= 0 and tuple(ring_k.shape[1:]) == (h, d) and src_block_table.dtype == torch.int32
             and src_block_table.is_contiguous() and first + n <= src_block_table.numel() * bs and position + n <= ring_k.shape[0]):
         return False
-    rc = lib().tq_ring_write_paged(key_cache.data_ptr(), value_cache.data_ptr(), _DTYPES[key_cache.dtype], nb, bs, h, d, key_cache.stride(0),
-                                   key_cache.stride(1), key_cache.stride(2), src_block_table.data_ptr(), first, n, ring_k.data_ptr(),
-                                   ring_v.data_ptr(), ring_k.stride(0), position, stream_ptr(ring_k.device))
+    rc = lib().tq_ring_write_paged_reported(
+        key_cache.data_ptr(), value_cache.data_ptr(), _DTYPES[key_cache.dtype], nb, bs, h, d, key_cache.stride(0), key_cache.stride(1),
+        key_cache.stride(2), src_block_table.data_ptr(), first, n, ring_k.data_ptr(), ring_v.data_ptr(), ring_k.stride(0), position,
+        report.address if report else None, report.ticket if report else 0, stream_ptr(ring_k.device))
     if rc in (_lib.TQ_ERR_UNSUPPORTED, _lib.TQ_ERR_ALIGN):
         return False
     check(rc, "tq_ring_write_paged")

@@ -35,6 +35,13 @@ class RingBuffer:
         self._seen = 0                                     # tokens ever written
         self._fill_dev: Optional[torch.Tensor] = None      # device mirror of _fill, kept by device_len()
         self._fill_dev_val = -1
+        self._report: Optional[E.RangeReport] = None       # of the launch that filled the ring from a paged cache
+
+    def check(self) -> None:
+        """Raises once a launch that filled the ring from a paged cache has met a block index out of range."""
+        if self._report is not None and self._report.failed:
+            raise IndexError("the block table given to ingest_prefill_from_paged_cache has an index out of range; "
+                             "the tokens of that block are missing (reset() starts anew)")
 
     def device_len(self) -> torch.Tensor:
         """(1,) int32 device tensor equal to `size`.  The fused decode step lets the kernel write the new
@@ -73,6 +80,7 @@ class RingBuffer:
         """Append `num_tokens` tokens.  Seen as one stream - the tokens held, then the new ones - every
         full buffer's worth that is followed by at least one more token leaves; what stays is the tail of
         1..capacity tokens.  No loop over buffers: the split point is arithmetic."""
+        self.check()
         held, cap = self._fill, self.capacity
         total = held + num_tokens
         self._seen += num_tokens
@@ -100,6 +108,8 @@ class RingBuffer:
     def write_one(self, key: torch.Tensor, value: torch.Tensor) -> bool:
         """`write` of one token where there is room and the kernel takes it, in as few steps as that can be; False, with
         nothing changed, otherwise."""
+        if self._report is not None:
+            self.check()
         held = self._fill
         if held >= self.capacity or not self._on_device or E.host().ring_write(self._keys, self._values, key, value, held, 1) != 0:
             return False
@@ -110,18 +120,23 @@ class RingBuffer:
     def write_from_paged(self, key_cache: torch.Tensor, value_cache: torch.Tensor, block_table: torch.Tensor, first: int,
                          num_tokens: int) -> bool:
         """`write` of tokens [first, first + num_tokens) of a sequence in a paged cache, where nothing is evicted and the
-        tensors are the kernel's; False, with nothing changed, otherwise."""
+        tensors are the kernel's; False, with nothing changed, otherwise.  A block index out of range is met on the device:
+        such tokens are zeros, and a later call on the ring raises."""
+        self.check()
         held = self._fill
         if num_tokens <= 0 or held + num_tokens > self.capacity or not self._keys.is_cuda:
             return False
-        if not E.ring_write_paged(self._keys, self._values, held, key_cache, value_cache, block_table, first, num_tokens):
+        report = E.range_report()
+        if not E.ring_write_paged(self._keys, self._values, held, key_cache, value_cache, block_table, first, num_tokens, report):
             return False
+        self._report = report
         self._fill = held + num_tokens
         self._seen += num_tokens
         return True
 
     def drain(self):
         """Everything held, as copies; the ring is empty afterwards."""
+        self.check()
         if self._fill == 0:
             return None
         taken = self._keys[: self._fill].clone(), self._values[: self._fill].clone()
@@ -134,6 +149,7 @@ class RingBuffer:
 
     def peek(self):
         """Views of what is held (None when empty)."""
+        self.check()
         if self._fill == 0:
             return None
         return self._keys[: self._fill], self._values[: self._fill]
@@ -141,6 +157,7 @@ class RingBuffer:
     def reset(self) -> None:
         self._fill = 0
         self._seen = 0
+        self._report = None
 
 
 class KVCaptureEngine:
@@ -181,7 +198,9 @@ class KVCaptureEngine:
                                         block_table: torch.Tensor, block_size: int) -> None:
         """kv_cache_tensor (2, num_blocks, block_size, H, D); block_table maps logical to physical blocks
         (reference capture.py:187-217).  All but the last `capacity` tokens go from the paged cache into
-        the compressed store in one launch that walks the table; only the ring's tokens are gathered."""
+        the compressed store in one launch that walks the table, the ring's tokens in another; where tensors or a full ring do
+        not allow that, the ring's tokens are gathered.  A block index out of range among the ring's tokens raises IndexError
+        from a later call on this engine, one among the others leaves its records out (`_engine.store_status`)."""
         if kv_cache_tensor.shape[2] != block_size:
             raise ValueError(f"block_size {block_size} does not match the cache's {kv_cache_tensor.shape[2]}")
         cap = self.ring.capacity
@@ -219,6 +238,8 @@ class KVCaptureEngine:
         single call.
         """
         ring, store = self.ring, self.store
+        if ring._report is not None:
+            ring.check()
         if ring.is_full:                      # the rare step: compress the full ring first
             self._compress_ring()
         if num_query_heads == query.shape[-2]:
@@ -257,6 +278,8 @@ class KVCaptureEngine:
         before reading host_out).  Same results as `decode_step`.
         """
         ring, store = self.ring, self.store
+        if ring._report is not None:
+            ring.check()
         if ring.is_full:
             self._compress_ring()
         h, d, qh = store.num_kv_heads, store.head_dim, num_query_heads

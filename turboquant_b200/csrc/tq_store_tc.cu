@@ -1657,10 +1657,11 @@ int tq_store_tc_launch(const tq_consts* consts, const void* key, const void* val
 namespace {
 // The last tokens of a prompt from its paged cache into the ring, key and value in one launch.  Bound by its launch (128 tokens
 // of 4 heads x 256 are 512 KB): two gathers, a conversion of the table and a ring write took 15 us of the device and 40 of the host.
+// A token whose block is out of range becomes zeros - what the ring held there belongs to another sequence - and is reported.
 __global__ void __launch_bounds__(256) tq_ring_gather_kernel(const char* __restrict__ k, const char* __restrict__ v, const int32_t* __restrict__ table,
                                                              int64_t num_blocks, int block_size, int row16, int n_heads, int64_t first, int64_t total,
                                                              int64_t src_block, int64_t src_token, int64_t src_head, char* __restrict__ rk,
-                                                             char* __restrict__ rv, int64_t dst_token) {
+                                                             char* __restrict__ rv, int64_t dst_token, int32_t* report, int32_t report_value) {
     // the ring may still be read by the launch ahead; only then may the next one begin (it reads pool and tables early)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -1670,23 +1671,29 @@ __global__ void __launch_bounds__(256) tq_ring_gather_kernel(const char* __restr
     const int h = (int)((i / row16) % n_heads);
     const int64_t t = i / ((int64_t)row16 * n_heads), tok = first + t;
     const int64_t phys = table[tok / block_size];
+    const int64_t dst = t * dst_token + ((int64_t)h * row16 + c) * 16;
+    uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
     if (phys < 0 || phys >= num_blocks) {
         atomicCAS(&g_tq_store_status, 0, (int)TQ_ERR_RANGE);
-        return;
+        if (report) {
+            *reinterpret_cast<volatile int32_t*>(report) = report_value;
+            __threadfence_system();
+        }
+    } else {
+        const int64_t src = phys * src_block + tok % block_size * src_token + h * src_head + 16 * c;
+        a = *reinterpret_cast<const uint4*>(k + src);
+        b = *reinterpret_cast<const uint4*>(v + src);
     }
-    const int64_t src = phys * src_block + tok % block_size * src_token + h * src_head + 16 * c;
-    const int64_t dst = t * dst_token + ((int64_t)h * row16 + c) * 16;
-    const uint4 a = *reinterpret_cast<const uint4*>(k + src), b = *reinterpret_cast<const uint4*>(v + src);
     *reinterpret_cast<uint4*>(rk + dst) = a;
     *reinterpret_cast<uint4*>(rv + dst) = b;
 }
 }  // namespace
 
-extern "C" int tq_ring_write_paged(const void* key_cache, const void* value_cache, tq_dtype dtype, int64_t src_num_blocks,
+extern "C" int tq_ring_write_paged_reported(const void* key_cache, const void* value_cache, tq_dtype dtype, int64_t src_num_blocks,
                                    int32_t src_block_size, int32_t n_heads, int32_t head_dim, int64_t stride_block,
                                    int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t first_token,
                                    int64_t n_tokens, void* ring_k, void* ring_v, int64_t ring_stride_token, int64_t position,
-                                   void* stream) {
+                                   int32_t* report, int32_t report_value, void* stream) {
     if (!key_cache || !value_cache || !src_block_table || !ring_k || !ring_v) return TQ_ERR_NULL;
     if (src_num_blocks <= 0 || src_block_size <= 0 || n_heads <= 0 || head_dim <= 0 || first_token < 0 || n_tokens <= 0 || position < 0)
         return TQ_ERR_SHAPE;
@@ -1710,7 +1717,17 @@ extern "C" int tq_ring_write_paged(const void* key_cache, const void* value_cach
     tq_note_launch(st, TQ_LAUNCH_DECODE);   // a store behind it may be about to read the ring
     return cudaLaunchKernelEx(&cfg, tq_ring_gather_kernel, (const char*)key_cache, (const char*)value_cache, src_block_table, src_num_blocks,
                               (int)src_block_size, row16, (int)n_heads, first_token, total, stride_block * eb, stride_token * eb, stride_head * eb,
-                              (char*)ring_k + off, (char*)ring_v + off, ring_stride_token * eb) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+                              (char*)ring_k + off, (char*)ring_v + off, ring_stride_token * eb, report, report_value) == cudaSuccess ? TQ_OK : TQ_ERR_CUDA;
+}
+
+extern "C" int tq_ring_write_paged(const void* key_cache, const void* value_cache, tq_dtype dtype, int64_t src_num_blocks,
+                                   int32_t src_block_size, int32_t n_heads, int32_t head_dim, int64_t stride_block,
+                                   int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t first_token,
+                                   int64_t n_tokens, void* ring_k, void* ring_v, int64_t ring_stride_token, int64_t position,
+                                   void* stream) {
+    return tq_ring_write_paged_reported(key_cache, value_cache, dtype, src_num_blocks, src_block_size, n_heads, head_dim, stride_block,
+                                        stride_token, stride_head, src_block_table, first_token, n_tokens, ring_k, ring_v,
+                                        ring_stride_token, position, nullptr, 0, stream);
 }
 
 // Status left by the tensor-core store kernels since the last call (0, or a tq_status if a bounded wait ran

@@ -140,3 +140,25 @@ def test_every_warp_of_a_late_store_waits_for_the_launch_ahead_first(kernel, beg
     body = body[body.index(begin):]
     body = body[:body.index(first_use)]
     assert re.search(r"if \(p\.rows_late\)[\s{].*(pool_writes_may_begin|rows_may_be_read)\(\)", body, re.S), body
+
+
+def test_no_read_only_loads_of_what_the_launch_ahead_may_write():
+    """A grid that is resident while the launch ahead still writes must not read that through pointers which promise the compiler
+    that nobody does (`const ... __restrict__`: such loads may move in front of the wait).  Constant operands are written once,
+    before any launch; the staging kernel's source is host memory."""
+    constants = {"pi", "s", "pi_t", "s_t"}
+    seen, wrong = 0, []
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith(".cu"):
+            continue
+        text = open(os.path.join(CSRC, name)).read()
+        starts = [m.start() for m in re.finditer(r"__global__ void", text)] + [len(text)]
+        for a, b in zip(starts, starts[1:]):
+            kernel, args = re.match(r"__global__ void (?:__launch_bounds__\([^)]*\)\s*)?(\w+)\((.*?)\) \{", text[a:b], re.S).groups()
+            if not re.search(r"griddepcontrol\.wait|wait_for_launch_ahead\(\)|pool_writes_may_begin\(\)", text[a:b]):
+                continue
+            seen += 1
+            for ptr in re.findall(r"const \w+\* __restrict__ (\w+)", args):
+                if ptr not in constants and kernel != "tq_stage_in_kernel":
+                    wrong.append((kernel, ptr))
+    assert seen >= 12 and not wrong, (seen, wrong)

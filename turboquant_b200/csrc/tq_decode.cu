@@ -62,7 +62,7 @@ __device__ __forceinline__ void load_query(const void* q, int64_t at, int n, int
 // VPC = query vectors per CTA; OCC = CTAs per SM the registers are budgeted for (2 for a grid that is resident
 // all at once - fewer CTAs share an SM for the latency-critical part after the wait - 3 for throughput).
 template <int D, int VPC, int OCC>
-__global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restrict__ q, int dt, int64_t nvec,
+__global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* q, int dt, int64_t nvec,
                                                        const float* __restrict__ pi_t,
                                                        const float* __restrict__ s_t, float* __restrict__ out,
                                                        uint32_t* __restrict__ frag, int G, int Qh, int mse_bits,
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(256, OCC) tq_qprep_kernel(const void* __restri
 // one position): the results are staged in shared memory and leave as full 128-byte rows.
 constexpr int QB_V = 64, QB_C = 64, QB_K = 32;
 template <int D>
-__global__ void __launch_bounds__(256) tq_qprep_batched_kernel(const void* __restrict__ q, int dt, int64_t nvec,
+__global__ void __launch_bounds__(256) tq_qprep_batched_kernel(const void* q, int dt, int64_t nvec,
                                                                const float* __restrict__ pi_t,
                                                                const float* __restrict__ s_t, float* __restrict__ out,
                                                                uint32_t* __restrict__ frag, int G, int Qh, int mse_bits) {
@@ -877,9 +877,9 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
 namespace {
 // One or a few exact tokens into the ring, key and value in one launch.  Bound by its launch (a token of 8 heads x 128
 // is 4 KB): two torch slice assignments cost two launches and ~10 us of host time instead of one and ~3 us.
-__global__ void __launch_bounds__(256) tq_ring_write_kernel(const char* __restrict__ k, const char* __restrict__ v, int row16, int n_heads,
-                                                            int64_t total, int64_t src_token, int64_t src_head, char* __restrict__ rk,
-                                                            char* __restrict__ rv, int64_t dst_token) {
+__global__ void __launch_bounds__(256) tq_ring_write_kernel(const char* k, const char* v, int row16, int n_heads,
+                                                            int64_t total, int64_t src_token, int64_t src_head, char* rk,
+                                                            char* rv, int64_t dst_token) {
     // the ring may still be read by the launch ahead; only then may the next one begin (it reads pool and tables early)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -35,8 +35,8 @@ __device__ __forceinline__ void wait_for_launch_ahead() {
 // Four lanes per group of 32 channels, eight consecutive channels each.  Arithmetic of kv_cache.py:64-90 with the rounding of
 // the tensor's dtype after every operation; scale and zero point pass through fp16, the form they are stored in.
 template <int DT, int VAL_BITS>
-__global__ void __launch_bounds__(256) tq_rows_quantize_values_kernel(const void* __restrict__ v, int64_t n_groups, int groups_per_row, int64_t stride_row,
-                                                                      uint8_t* __restrict__ data, void* __restrict__ scales, void* __restrict__ zeros) {
+__global__ void __launch_bounds__(256) tq_rows_quantize_values_kernel(const void* v, int64_t n_groups, int groups_per_row, int64_t stride_row,
+                                                                      uint8_t* data, void* scales, void* zeros) {
     using E = TqElem<DT>;
     wait_for_launch_ahead();
     const int64_t unit = (int64_t)blockIdx.x * 256 + threadIdx.x, i = unit >> 2;
@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(256) tq_rows_quantize_values_kernel(const void
 
 // code * scale + zero in fp32 (kv_cache.py:101-116); one thread per four channels
 template <int VAL_BITS>
-__global__ void __launch_bounds__(256) tq_rows_dequantize_values_kernel(const uint8_t* __restrict__ data, const void* __restrict__ scales,
-                                                                        const void* __restrict__ zeros, int sdt, int64_t n_quads, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) tq_rows_dequantize_values_kernel(const uint8_t* data, const void* scales,
+                                                                        const void* zeros, int sdt, int64_t n_quads, float* out) {
     wait_for_launch_ahead();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     if (i >= n_quads) return;
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(256) tq_rows_dequantize_keys256_kernel(const R
 // asks for its whole half row at once (16 bytes at a time where the planes are aligned: `vec`), and a CTA holds no more queries
 // than it was asked for.
 template <int D, int MSE_BITS, int GP>
-__global__ void __launch_bounds__(128) tq_rows_scores_kernel(const RowsParams p, const float* __restrict__ qprep, int64_t n_k, int n_q, int vec, float* __restrict__ logits) {
+__global__ void __launch_bounds__(128) tq_rows_scores_kernel(const RowsParams p, const float* qprep, int64_t n_k, int n_q, int vec, float* logits) {
     constexpr int NSW = HalfRow<D, MSE_BITS>::NSW, NCW = HalfRow<D, MSE_BITS>::NCW;
     __shared__ __align__(16) float qs[GP][2][D];
     __shared__ float sp[GP * 64], cent[TQ_MAX_CENTROIDS];

@@ -1658,10 +1658,10 @@ namespace {
 // The last tokens of a prompt from its paged cache into the ring, key and value in one launch.  Bound by its launch (128 tokens
 // of 4 heads x 256 are 512 KB): two gathers, a conversion of the table and a ring write took 15 us of the device and 40 of the host.
 // A token whose block is out of range becomes zeros - what the ring held there belongs to another sequence - and is reported.
-__global__ void __launch_bounds__(256) tq_ring_gather_kernel(const char* __restrict__ k, const char* __restrict__ v, const int32_t* __restrict__ table,
+__global__ void __launch_bounds__(256) tq_ring_gather_kernel(const char* k, const char* v, const int32_t* table,
                                                              int64_t num_blocks, int block_size, int row16, int n_heads, int64_t first, int64_t total,
-                                                             int64_t src_block, int64_t src_token, int64_t src_head, char* __restrict__ rk,
-                                                             char* __restrict__ rv, int64_t dst_token, int32_t* report, int32_t report_value) {
+                                                             int64_t src_block, int64_t src_token, int64_t src_head, char* rk,
+                                                             char* rv, int64_t dst_token, int32_t* report, int32_t report_value) {
     // the ring may still be read by the launch ahead; only then may the next one begin (it reads pool and tables early)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -348,3 +348,22 @@ def test_ring_filled_through_a_table_with_a_bad_index(bad, n, dev):
         else:
             assert e.ring.peek()[0].shape[0] == m and E.store_status() == 0
         assert torch.equal(e.ring._keys[:m], want[0]) and torch.equal(e.ring._values[:m], want[1])
+
+
+@pytest.mark.parametrize("d,h,qh", [(128, 8, 32), (128, 2, 16), (256, 4, 16)])
+def test_large_scores_of_ring_tokens_keep_their_differences(d, h, qh, dev):
+    """Scores of 1024, 1025 and 1026, exact in fp32: only differences reach an exponential, whose argument below 2 and its
+    product with log2(e) are rounded to 2^-23 each, its result to 2^-22.  (Scaled to base 2 first, a score of 1477 is rounded by up
+    to 6e-5, and so is every probability.)"""
+    from turboquant_b200 import CompressedKVStore, compute_hybrid_attention
+    store = CompressedKVStore(d, h, 3, 2, device=dev)
+    g = torch.Generator(device=dev).manual_seed(d)
+    k, q = torch.zeros(256, h, d, device=dev), torch.zeros(1, qh, d, device=dev)
+    k[..., 0], k[..., 1] = 32, torch.randint(0, 3, (256, h), generator=g, device=dev).float()
+    q[..., 0], q[..., 1] = 32, 1
+    v = torch.randn(256, h, d, generator=g, device=dev)
+    for r in (5, 33, 64, 128, 256):
+        out = compute_hybrid_attention(q, store, k[:r], v[:r], qh, scale=1.0)
+        kk, vv = (t[:r].double().transpose(0, 1).repeat_interleave(qh // h, 0) for t in (k, v))
+        want = torch.einsum("thn,hnd->thd", torch.softmax(torch.einsum("thd,hnd->thn", q.double(), kk), -1), vv)
+        assert _rel(out, want) <= 2e-6, r

@@ -110,3 +110,34 @@ def test_compressed_cache_specs_follow_the_layer_configuration():
     assert (s.head_dim, s.num_kv_heads, s.page_size_bytes) == (128, 2, 16 * 2 * 100)
     assert specs["layers.0.attn"].page_size_bytes == 16 * 2 * 132      # 4-bit keys: 3-bit codes in nibbles, 32 bytes more per token
     assert adapter.compressed_cache_specs(types.SimpleNamespace()) == {}
+
+
+def test_decode_step_reads_the_layer_configuration_of_the_call(monkeypatch):
+    """A layer whose configuration is replaced behind the hooks - another number of query heads, another kind of backend - is
+    attended with what it says at the call."""
+    import dataclasses
+    r = _runner(1)
+    state = adapter.install_hooks(r, mode=adapter.MODE_HYBRID)["layers.0.attn"]
+    impl = r.compilation_config.static_forward_context["layers.0.attn"].impl
+    ring = types.SimpleNamespace(_keys=None, _values=None, _fill=3, storage=(None, None), size=3)
+    state._store = types.SimpleNamespace(consts=types.SimpleNamespace(addr=1), pool=types.SimpleNamespace(addr=2), workspace=None,
+                                         block_table=None, _num_tokens=64, num_tokens=64)
+    state._engine = types.SimpleNamespace(ring=ring)
+    seen = []
+
+    def hybrid(*args):
+        seen.append((args[4], args[8]))                 # head_dim, query heads
+        return args[-1]
+
+    monkeypatch.setattr(adapter.E, "host", lambda: types.SimpleNamespace(hybrid=hybrid))
+    md = types.SimpleNamespace(num_actual_tokens=1, max_query_len=1)
+    try:
+        for heads in (8, 4):
+            state.config = dataclasses.replace(state.config, num_query_heads=heads)
+            q, out = torch.zeros(1, heads, 128), torch.zeros(1, heads, 128)
+            assert impl.forward(None, q, None, None, None, md, output=out) is out
+        assert seen == [(128, 8), (128, 4)]
+        state.config = dataclasses.replace(state.config, backend_kind="mla")
+        assert impl.forward(None, q, None, None, None, md, output=out) == "flash-output" and len(seen) == 2
+    finally:
+        adapter.set_mode(adapter.MODE_OFF)

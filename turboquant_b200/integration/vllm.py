@@ -182,29 +182,25 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
     def original(self_impl, layer, query, key, value, kv_cache, md, output, output_scale, output_block_scale):
         return orig_fn(self_impl, layer, query, key, value, kv_cache, md, output, output_scale, output_block_scale)
 
-    c, flash = state.config, state.supports_hybrid
-    head_dim, num_query_heads = c.head_dim, c.num_query_heads
-
-    def attend(st, ring, query, n, self_impl, output):
+    def attend(c, st, ring, query, n, self_impl, output):
         """The native call that writes into the engine's buffer: `output`, a status, or None where it does not apply."""
-        return E.host().hybrid(st.consts.addr, st.pool.addr, st.workspace, st.block_table, head_dim, st._num_tokens, query, n,
-                               num_query_heads, ring._keys, ring._values, ring._fill, getattr(self_impl, "scale", None),
+        return E.host().hybrid(st.consts.addr, st.pool.addr, st.workspace, st.block_table, c.head_dim, st._num_tokens, query, n,
+                               c.num_query_heads, ring._keys, ring._values, ring._fill, getattr(self_impl, "scale", None),
                                MIN_HISTORY, output)
 
     def patched(self_impl, layer, query, key, value, kv_cache, attn_metadata, output=None, output_scale=None,
                 output_block_scale=None):
-        mode = _GLOBAL_MODE
-        if mode == MODE_HYBRID and output is not None and flash and not capture_in_forward and attn_metadata is not None and \
+        mode, c = _GLOBAL_MODE, state.config
+        if mode == MODE_HYBRID and output is not None and c.backend_kind == "flash" and not capture_in_forward and attn_metadata is not None and \
                 attn_metadata.max_query_len <= 1:       # a decode step in the engine's own layout: what such a step spends here, it waits for
             st, engine = state._store, state._engine
             if st is not None and engine is not None and st._num_tokens >= MIN_HISTORY and \
-                    attend(st, engine.ring, query, attn_metadata.num_actual_tokens, self_impl, output) is output:
+                    attend(c, st, engine.ring, query, attn_metadata.num_actual_tokens, self_impl, output) is output:
                 return output
         args = (self_impl, layer, query, key, value, kv_cache, attn_metadata, output, output_scale,
                 output_block_scale)
         if capture_in_forward and mode != MODE_OFF and attn_metadata is not None:
             n = getattr(attn_metadata, "num_actual_tokens", key.shape[0])
-            c = state.config
             if (mode == MODE_HYBRID and n == 1 and getattr(attn_metadata, "max_query_len", 1) == 1
                     and state.supports_hybrid and state.store.num_tokens >= MIN_HISTORY
                     and key.dtype == state.engine.ring.dtype and query.dtype == key.dtype):
@@ -229,7 +225,7 @@ def _make_patched_forward(orig_fn, state: LayerState, no_alloc: bool = False, ca
         if mode == MODE_HYBRID and state.supports_hybrid and state.store.num_tokens >= MIN_HISTORY:
             if output is not None:                      # straight into the engine's buffer where its layout allows
                 st, ring = state.store, state.engine.ring
-                res = attend(st, ring, query, n, self_impl, output)
+                res = attend(c, st, ring, query, n, self_impl, output)
                 if res is output:
                     return output
                 if res is not None:

@@ -188,15 +188,16 @@ int tq_prefill_attention_read_status(int32_t* out);
  * skip) when slot_mapping is given, else position start_pos+t of the
  * sequence whose blocks are block_table[0..].
  * bf16 input with 16-byte aligned rows runs on the tensor cores (head_dim 128;
- * head_dim 256 with 3-bit keys and 2-bit values); those kernels are launched
- * as programmatic dependents: one that follows another store or
- * tq_prefill_attention on the stream may fetch its key / value rows while
- * that launch is still running, and touches the pool only after it has
- * completed.  A store that follows one of the tq_decode* calls on the stream
- * (whose ring append may still be writing rows the store is about to read)
- * is launched in plain stream order; likewise the first kernel of a tq_decode*
- * call that follows one of these stores (the decode kernels fetch lengths,
- * block tables and their first records before they wait for the launch ahead).
+ * head_dim 256, with 4-bit keys or values where `consts` has the rows_pi /
+ * rows_m operands); those kernels are launched as programmatic dependents: one
+ * that follows another store or tq_prefill_attention on the stream may fetch
+ * its key / value rows while that launch is still running, and touches the pool
+ * only after it has completed.  A store that follows anything else of the
+ * library (a ring append may still be writing rows the store is about to read)
+ * begins early too, but waits for that launch in front of its first row.  The
+ * tq_decode* and tq_cache_scores kernels fetch lengths, block tables and their
+ * first records before they wait for the launch ahead; behind a store, or on a
+ * stream that the library has no note of, they wait first.
  * With a block table the kernels may fill the slots of the last block behind the last token (a later
  * append overwrites them): tokens are appended, not rewritten in the middle of a sequence.
  * Device-side status: tq_store_read_status. */
@@ -226,7 +227,8 @@ int tq_store_paged(const tq_consts* consts, const void* key_cache, const void* v
                    const int32_t* block_table, int64_t start_pos, const tq_pool* pool, void* stream);
 
 /* The same for every bit width at head_dim 256 too (4-bit keys or values need
- * the rows_pi / rows_m operands in `consts`). */
+ * the rows_pi / rows_m operands in `consts`).  Take this one; tq_store_paged is
+ * for callers that rely on its refusal of those widths. */
 int tq_store_paged_any(const tq_consts* consts, const void* key_cache, const void* value_cache, tq_dtype dtype,
                        int64_t src_num_blocks, int32_t src_block_size, int32_t n_heads, int64_t stride_block,
                        int64_t stride_token, int64_t stride_head, const int32_t* src_block_table, int64_t n_tokens,

@@ -95,3 +95,27 @@ def test_null_and_shape_errors_come_before_any_launch(lib):
     assert lib.tq_decode_static(C.byref(consts), C.byref(pool), None, None) == -1
     assert lib.tq_scores(C.byref(consts), C.byref(pool), None, 16, None, 0, 1, None, None, 0, None) == -1
     assert lib.tq_workspace_init(None, 1024, None) == -1
+
+
+@pytest.mark.parametrize("what", ["ring_k", "ring_v", "ring_stride_token", "ring_stride_seq"])
+def test_misaligned_ring_is_refused_before_any_launch(lib, what):
+    """The decode kernels read ring rows 16 bytes at a time.  (The addresses are never touched: an aligned ring is only compared,
+    and a ring stride of a single sequence is not used.)"""
+    page = (C.c_uint8 * 65536)()
+    base = (C.addressof(page) + 255) // 256 * 256
+    consts = _lib.tq_consts()
+    consts.cfg = _lib.tq_config(128, 3, 2, 32)
+    consts.pi_t = consts.s_t = base
+    pool = _lib.tq_pool(base, 4, 2)
+    a = _lib.tq_decode_args()
+    a.query = a.out = a.workspace = a.block_table = a.seq_lens = a.ring_k = a.ring_v = a.ring_lens = base
+    a.batch, a.num_q_heads, a.block_table_stride, a.max_seq_len, a.max_ring_len = 2, 8, 4, 64, 16
+    a.q_dtype = a.ring_dtype = 1
+    a.ring_stride_seq, a.ring_stride_token = 16 * 256, 256
+    a.workspace_bytes = 0
+    assert lib.tq_decode(C.byref(consts), C.byref(pool), C.byref(a), None) == -6       # aligned: the workspace is what is missing
+    setattr(a, what, getattr(a, what) + 4)
+    assert lib.tq_decode(C.byref(consts), C.byref(pool), C.byref(a), None) == -3
+    if what == "ring_stride_seq":
+        a.batch = 1
+        assert lib.tq_decode(C.byref(consts), C.byref(pool), C.byref(a), None) == -6

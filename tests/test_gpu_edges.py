@@ -367,3 +367,30 @@ def test_large_scores_of_ring_tokens_keep_their_differences(d, h, qh, dev):
         kk, vv = (t[:r].double().transpose(0, 1).repeat_interleave(qh // h, 0) for t in (k, v))
         want = torch.einsum("thn,hnd->thd", torch.softmax(torch.einsum("thd,hnd->thn", q.double(), kk), -1), vv)
         assert _rel(out, want) <= 2e-6, r
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("d", [128, 256])
+def test_recent_tokens_from_any_address(d, dtype, dev):
+    """Views that begin, or whose rows begin, beside a 16-byte boundary: the same result as from tensors of their own."""
+    from turboquant_b200 import CompressedKVStore, compute_hybrid_attention
+    h, qh, r, n = 2, 8, 40, 200
+    g = torch.Generator(device=dev).manual_seed(d)
+    k, v = (torch.randn(n, h, d, generator=g, device=dev, dtype=torch.bfloat16) for _ in range(2))
+    store = CompressedKVStore(d, h, 3, 2, device=dev)
+    store.append_chunk(k, v)
+    rk, rv = (torch.randn(r, h, d, generator=g, device=dev).to(dtype) for _ in range(2))
+    q = torch.randn(1, qh, d, generator=g, device=dev, dtype=torch.bfloat16)
+
+    def moved(t, first, stride):
+        flat = torch.zeros(first + r * stride, device=dev, dtype=dtype)
+        view = flat.as_strided(t.shape, (stride, d, 1), first)
+        view.copy_(t)
+        return view
+
+    want = compute_hybrid_attention(q, store, rk, rv, qh)
+    one = compute_hybrid_attention(q, store, rk[:1], rv[:1], qh)
+    for kf, vf, stride in ((1, 0, h * d), (0, 1, h * d), (3, 3, h * d), (0, 0, h * d + 1), (5, 2, h * d + 2)):
+        a, b = moved(rk, kf, stride), moved(rv, vf, stride)
+        assert torch.equal(compute_hybrid_attention(q, store, a, b, qh), want), (kf, vf, stride)
+        assert torch.equal(compute_hybrid_attention(q, store, a[:1], b[:1], qh), one), (kf, vf, stride)

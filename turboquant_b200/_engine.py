@@ -300,7 +300,7 @@ def store_paged(consts: LayerConstants, pool: BlockPool, key_cache: torch.Tensor
     contiguous, same strides for both); src_block_table: int32 device tensor, logical -> physical block.
     Returns False, with nothing launched, when the call does not fit the table-walking tensor-core
     kernel (the caller then gathers the rows and uses `store`).  any_width: take head_dim 256 with 4-bit
-    keys or values too.
+    keys or values too, which callers without it may rely on being refused.
     """
     require_cuda(key_cache, "key_cache")
     require_cuda(value_cache, "value_cache")

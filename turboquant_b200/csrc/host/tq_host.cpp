@@ -174,7 +174,8 @@ PyObject* hybrid(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
             rk->stride(0) != rv->stride(0) || rk->size(0) < r || rv->size(0) != rk->size(0) || rk->scalar_type() != rv->scalar_type() || r > 256)
             Py_RETURN_NONE;
         const int rdt = dtype_code(rk->scalar_type());
-        if (rdt < 0) Py_RETURN_NONE;
+        if (rdt < 0 || !aligned16(rk->data_ptr()) || !aligned16(rv->data_ptr()) || (r > 1 && rk->stride(0) * rk->element_size() % 16 != 0))
+            Py_RETURN_NONE;
         a.ring_k = rk->data_ptr();
         a.ring_v = rv->data_ptr();
         a.ring_dtype = (tq_dtype)rdt;

@@ -227,7 +227,6 @@ void tq_note_launch(cudaStream_t st, int kind);
 int tq_last_launch(cudaStream_t st);
 inline void tq_note_prep_launch(cudaStream_t st) { tq_note_launch(st, tq_kind_of_prep(tq_last_launch(st))); }
 
-// Largest dynamic shared-memory size a kernel has been opted in for, per device.
 // A paged bf16 cache as the source of a store call (see tq_store_paged).
 struct TqPagedSource {
     const int32_t* table;    // device: logical block of the sequence -> physical block
@@ -237,6 +236,7 @@ struct TqPagedSource {
     bool any_width;          // head_dim 256 with 4-bit keys or values too
 };
 
+// Largest dynamic shared-memory size a kernel has been opted in for, per device.
 struct TqSmemOptIn {
     size_t bytes[TQ_MAX_DEVICES] = {};
 };

@@ -751,6 +751,11 @@ static int decode_impl(const tq_consts* consts, const tq_pool* pool, const tq_de
     const bool has_ring = a->ring_k != nullptr && a->max_ring_len > 0;
     if (has_ring && (!a->ring_v || (!host_lens && !a->ring_lens))) return TQ_ERR_NULL;
     if (has_ring && a->max_ring_len > 256) return TQ_ERR_UNSUPPORTED;
+    if (has_ring) {   // its rows are read 16 bytes at a time
+        const int64_t eb = (int64_t)tq_dtype_size(a->ring_dtype);
+        if (((uintptr_t)a->ring_k | (uintptr_t)a->ring_v) & 15) return TQ_ERR_ALIGN;
+        if ((a->max_ring_len > 1 && (a->ring_stride_token * eb) % 16) || (a->batch > 1 && (a->ring_stride_seq * eb) % 16)) return TQ_ERR_ALIGN;
+    }
     if (((uintptr_t)pool->base & 15) || ((uintptr_t)a->workspace & 255) || ((uintptr_t)a->out & 15)) return TQ_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
 

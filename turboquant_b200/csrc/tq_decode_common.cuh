@@ -171,7 +171,7 @@ __device__ __forceinline__ void half_row_dots(uint32_t (&cw)[HalfRow<D, MSE_BITS
         for (int k = 0; k + 1 < R::NSW; ++k) sw[k] = sw[k + 1];
     }
 }
-// The same for token tl of a block record.
+// half_row_scores for token tl of a block record.
 template <int D, int MSE_BITS, int GP>
 __device__ __forceinline__ void token_half_scores(const uint8_t* rec, const TqLayout& L, int tl, int half,
                                                   const float* __restrict__ qr, const float* __restrict__ qs,

@@ -221,10 +221,9 @@ __device__ __forceinline__ void quantize_value_group(const uint4 (&raw)[4], uint
 
 // Comparisons as arithmetic.  The fp32 pipes are the only full-rate ones of an SM; compares, selects and
 // bit logic run at half rate and would bound this kernel.  For finite a:
-//     step_gt(a, BIG, -b * BIG) = saturate((a - b) * 2^126)  is exactly 1 when a > b and exactly 0 when
+//     fma_sat(a, BIG, -b * BIG) = saturate((a - b) * 2^126)  is exactly 1 when a > b and exactly 0 when
 // a <= b, as long as |a - b| is either 0 or at least 2^-126 - true for every boundary that is not itself
-// tiny.
-// NaN saturates to 0.
+// tiny.  NaN saturates to 0.
 constexpr float BIG = 8.507059173023462e37f;   // 2^126
 __device__ __forceinline__ float fma_sat(float a, float b, float c) {
     float d;
@@ -395,7 +394,7 @@ __device__ __forceinline__ void issue_paged_rows(uint8_t* dst, const CUtensorMap
 
 // This launch may have started while the launch ahead of it in the stream still runs (programmatic
 // dependent launch; only when that launch is one of the library's that cannot be writing key / value
-// rows, see TqLaunchKind): the rows may be fetched at once, but the pool - which that launch
+// rows, see tq_stream_order.h): the rows may be fetched at once, but the pool - which that launch
 // may write, and whose stream order of writes the caller relies on - is touched only after this wait.
 __device__ __forceinline__ void pool_writes_may_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // The same in front of the first row, for a launch behind one that may be writing rows: what does not depend on it - tensor

@@ -66,6 +66,8 @@ def compute_hybrid_attention(query: torch.Tensor, store: CompressedKVStore, rece
     if r > 0:
         if recent_k.stride(2) != 1 or recent_k.stride(1) != d or recent_v.stride() != recent_k.stride():
             recent_k, recent_v = recent_k.contiguous(), recent_v.contiguous()
+        if (recent_k.data_ptr() | recent_v.data_ptr() | recent_k.stride(0) * recent_k.element_size()) % 16:
+            recent_k, recent_v = (x.clone(memory_format=torch.contiguous_format) for x in (recent_k, recent_v))
         kwargs = dict(ring_k=recent_k, ring_v=recent_v,
                       ring_lens=E.const_i32(dev, r, t), max_ring_len=r,
                       ring_stride_seq=0, ring_stride_token=recent_k.stride(0))

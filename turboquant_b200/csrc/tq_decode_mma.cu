@@ -39,8 +39,8 @@ constexpr int NSTW = 4;    // bulk-copy stages per warp, one block record each
 // and wherever its query lies in host memory: 128 registers are enough there.  With the data on the device that is for exactness:
 // the largest probability of each warp is 1 and exact in fp16, so sixteen warps leave less to round than twelve (fp32 queries, 24
 // sequences of 4096 tokens and 77 in the ring: 3.68e-4 of the output against 64 bits, twelve 3.77e-4; 12000 tokens 4.44e-4 and
-// 4.52e-4).  It costs 1.00 to 1.01 of twelve's time with one set of fragments (4096 tokens 9.33 us for 9.30), 1.00 to 1.06 with two
-// (10.6 for 10.1).
+// 4.52e-4).  It takes 1.00 to 1.01 of twelve's time with one set of fragments (4096 tokens 9.35 us for 9.28, but 9.7 for 9.0 at 300),
+// 1.00 to 1.06 with two (10.6 for 10.1).
 // With the query in host memory the ring's CTAs fetch it from there, the more at a time the more threads: steps of
 // decode_step_host, sixteen / twelve, 0.94 to 0.99 (13.0 us for 13.7 at 4000 tokens of 8 heads, 17.3 for 17.6 at 16000; two
 // sets of fragments 16.6 for 17.3).  At head_dim 256 sixteen warps cost registers.
